@@ -140,6 +140,14 @@ int tdt_test_barrier_timeout(void *workspace, long long limit_ns, cudaStream_t s
 int tdt_segment_add(const int32_t *col_indices, int64_t num_values, const int32_t *col_ptr,
                     int32_t *output, int64_t num_rows, tdt_stream_t stream);
 
+/* Per-segment maximum (no counterpart in the reference; the batched call's
+ * per-graph kmax): output[g] = max(output[g], values[offsets[g]:offsets[g+1]])
+ * for num_segments segments.  offsets: int64[num_segments+1], non-decreasing
+ * (segments are clamped to the num_values values); empty segments are left
+ * untouched. */
+int tdt_segment_max(const int32_t *values, int64_t num_values, const int64_t *offsets,
+                    int64_t num_segments, int64_t *output, tdt_stream_t stream);
+
 /* segment_isin2 (myhpu_extension.cpp:24-34; kernel.cu:28-79) and
  * segment_isin2tile (myhpu_extension.cpp:43-56; kernel.cu:81-141):
  * output[i] += number of triangles containing edge i (its support).

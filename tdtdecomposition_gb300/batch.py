@@ -16,7 +16,7 @@ from typing import List, NamedTuple
 import numpy as np
 import torch
 
-from . import truss as T
+from . import _lib, truss as T
 from .graph import CSRCOO
 
 
@@ -70,15 +70,30 @@ def batch_from_union(graph, edge_offsets, vertex_offsets):
                       torch.as_tensor(edge_offsets, dtype=torch.int64).cpu())
 
 
+def _device_offsets(batch, dev, num_edges):
+    """The batch's edge offsets on the device, checked: graph g owns
+    eo[g] - eo[0] .. eo[g + 1] - eo[0] of the union's edges."""
+    eo = batch.edge_offsets.to(torch.int64)
+    if bool((eo[1:] < eo[:-1]).any()) or int(eo[-1] - eo[0]) > num_edges:
+        raise RuntimeError("edge_offsets must be non-decreasing and within the union's %d edges" % num_edges)
+    return (eo - eo[0]).to(dev)
+
+
+def _graph_kmax(truss, offsets, kmax):
+    """kmax[g] = max(kmax[g], truss numbers of graph g), on the current stream."""
+    with torch.cuda.device(truss.device):
+        _lib.check(_lib.load().tdt_segment_max(truss.data_ptr(), truss.shape[0], offsets.data_ptr(),
+                                               kmax.shape[0], kmax.data_ptr(),
+                                               torch.cuda.current_stream(truss.device).cuda_stream),
+                   "tdt_segment_max")
+
+
 def decompose(batch, workspace=None, lists="auto", sync=True, list_budget=None):
     """Decompose every graph of the batch in one device-resident run."""
     res = T.truss_decompose(batch.graph, workspace=workspace, lists=lists, sync=sync, list_budget=list_budget)
     tr = res.truss if sync else res[0]
-    eo = batch.edge_offsets.to(tr.device)
-    G = batch.num_graphs
-    seg = torch.repeat_interleave(torch.arange(G, device=tr.device), eo[1:] - eo[:-1])
-    kmax = torch.full((G,), 2, dtype=torch.int64, device=tr.device)
-    kmax.scatter_reduce_(0, seg, tr.to(torch.int64), reduce="amax", include_self=True)
+    kmax = torch.full((batch.num_graphs,), 2, dtype=torch.int64, device=tr.device)
+    _graph_kmax(tr, _device_offsets(batch, tr.device, tr.shape[0]), kmax)
     return BatchResult(tr, kmax, res)
 
 
@@ -93,13 +108,12 @@ class CapturedBatch:
 
     Everything a replay touches is allocated at capture: the outputs, the
     workspace (base part plus a fixed triangle-list tail; the device decides
-    per replay whether the lists fit) and the per-graph segment ids.  A replay
+    per replay whether the lists fit) and the per-graph edge offsets.  A replay
     re-reads the batch's CSR tensors in place, so new graphs of the same
     shape can be copied into them between replays.  replay() returns the
     per-graph results after checking the run's device status."""
 
     def __init__(self, batch: GraphBatch, workspace=None, lists="auto", list_budget=None, stream=None):
-        from . import _lib
         L = _lib.load()
         g = batch.graph
         rows, cols, rp = T._graph_arrays(g)
@@ -116,10 +130,8 @@ class CapturedBatch:
         tail = int(list_budget) if list_budget is not None else T._list_bytes(wso, cols, rp, lists, base, rows)
         self.ws = wso.get(base + tail)
         self.ws_bytes = base + tail
-        eo = batch.edge_offsets.to(dev)
-        G = batch.num_graphs
-        self.seg = torch.repeat_interleave(torch.arange(G, device=dev), eo[1:] - eo[:-1])
-        self.kmax = torch.full((G,), 2, dtype=torch.int64, device=dev)
+        self.offsets = _device_offsets(batch, dev, E)
+        self.kmax = torch.full((batch.num_graphs,), 2, dtype=torch.int64, device=dev)
         self.stream = stream or torch.cuda.Stream(dev)
         args = (rows.data_ptr() if rows is not None else None, cols.data_ptr(), rp.data_ptr(), V, E,
                 self.truss.data_ptr(), self.e_truss.data_ptr(), self.ptr.data_ptr(), self.cap,
@@ -129,7 +141,7 @@ class CapturedBatch:
             s = torch.cuda.current_stream(dev).cuda_stream
             _lib.check(L.tdt_truss_decompose(*args, s), "tdt_truss_decompose")
             self.kmax.fill_(2)
-            self.kmax.scatter_reduce_(0, self.seg, self.truss.to(torch.int64), reduce="amax", include_self=True)
+            _graph_kmax(self.truss, self.offsets, self.kmax)
 
         # one eager run on the capture stream (kernel attributes, caches), then capture
         self.stream.wait_stream(torch.cuda.current_stream(dev))

@@ -109,6 +109,51 @@ __global__ void segment_add_kernel(const int32_t* __restrict__ vals, const int32
     }
 }
 
+// ------------------------------------------------------------------ segment_max
+// out[g] = max(out[g], values of segment g): the per-graph kmax of a batch.
+// One pass over the values.  Each warp owns one contiguous slab, finds the
+// segment of its first value by binary search and walks on from there, so a
+// long segment spreads over many warps and a slab of short ones stays in one;
+// one atomic per (slab, segment).  Bound by reading the values; one 64-bit
+// atomic per value on the segments' addresses (14 M values, 512 segments) took
+// 5.6 ms of an 11.7 ms batch, which takes 5.9 ms with this kernel.
+constexpr int kSegMaxUnroll = 4;
+
+__global__ void __launch_bounds__(kOpsBlock) segment_max_kernel(const int32_t* __restrict__ vals,
+                                                                const int64_t* __restrict__ off, int64_t nseg,
+                                                                int64_t nvals, int64_t slab,
+                                                                long long* __restrict__ out) {
+    const unsigned lane = lane_id();
+    const int64_t w = (blockIdx.x * (int64_t)kOpsBlock + threadIdx.x) / kWarp;
+    int64_t p = w * slab;
+    const int64_t pe = p + slab < nvals ? p + slab : nvals;
+    if (p >= pe) return;
+    int64_t g = 0, hi = nseg;  // first segment that ends past p
+    while (g < hi) {
+        const int64_t mid = (g + hi) >> 1;
+        if (__ldg(off + mid + 1) <= p) g = mid + 1; else hi = mid;
+    }
+    for (; g < nseg; g++) {
+        const int64_t b = __ldg(off + g), e = __ldg(off + g + 1);
+        if (b >= pe) break;
+        p = p < b ? b : p;
+        const int64_t end = e < pe ? e : pe;
+        int32_t m = INT32_MIN;
+        for (int64_t i = p + lane; i < end; i += kSegMaxUnroll * kWarp) {
+            int32_t x[kSegMaxUnroll];
+#pragma unroll
+            for (int k = 0; k < kSegMaxUnroll; k++) x[k] = i + k * kWarp < end ? __ldg(vals + i + k * kWarp) : INT32_MIN;
+#pragma unroll
+            for (int k = 0; k < kSegMaxUnroll; k++) m = x[k] > m ? x[k] : m;
+        }
+        if (p < end) {
+            m = __reduce_max_sync(kFull, m);
+            if (lane == 0) atomicMax(out + g, (long long)m);
+            p = end;
+        }
+    }
+}
+
 // ------------------------------------------------------------------ peel-update operators
 enum AffectMode { kAffectDeleted = 0, kAffectNot = 1, kAffectNotWin = 2 };
 
@@ -277,6 +322,26 @@ int launch_segment_add(const int32_t* vals, const int32_t* ptr, int32_t* out, in
     if (rc) return rc;
     segment_add_kernel<<<grid_for(nrows, 256, di.sms, 16), 256, 0, st>>>(vals, ptr, out, nrows, nvals);
     TDT_LAUNCH_CHECK("segment_add");
+    return TDT_OK;
+}
+
+int launch_segment_max(const int32_t* vals, const int64_t* off, int64_t nseg, int64_t nvals, int64_t* out,
+                       cudaStream_t st) {
+    TDT_CHECK_ARG(nseg >= 0 && nvals >= 0, "negative size");
+    if (nseg == 0 || nvals == 0) return TDT_OK;
+    TDT_CHECK_ARG(vals && off && out, "null pointer");
+    DeviceInfo di;
+    int rc = device_info(&di);
+    if (rc) return rc;
+    // whole steps of a warp, at most one wave of 8 blocks per SM
+    constexpr int64_t step = kSegMaxUnroll * kWarp;
+    const int64_t warps = (int64_t)di.sms * 8 * (kOpsBlock / kWarp);
+    int64_t slab = ((nvals + warps - 1) / warps + step - 1) / step * step;
+    const int64_t used = (nvals + slab - 1) / slab;
+    const unsigned blocks = (unsigned)((used + kOpsBlock / kWarp - 1) / (kOpsBlock / kWarp));
+    segment_max_kernel<<<blocks, kOpsBlock, 0, st>>>(vals, off, nseg, nvals, slab,
+                                                     reinterpret_cast<long long*>(out));
+    TDT_LAUNCH_CHECK("segment_max");
     return TDT_OK;
 }
 
