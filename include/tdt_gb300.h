@@ -71,26 +71,24 @@ int tdt_profile_stop(float *ms_phase, int *ncalls);
  * around synchronize calls (demo_truss/singlegpu_truss.py:69-77, :153-157). */
 int tdt_peel_clock(const void *workspace, long long *ns, cudaStream_t stream);
 
-/* Testing knob of the support/listing kernels: rows with out-degree <=
- * warp_cap are processed by one warp, heavier rows by a block with the row
- * staged in shared memory up to heavy_cap entries, and beyond that in place.
- * Lower values let small graphs exercise every path; 0 restores the
- * defaults.  Affects calls launched afterwards from any thread. */
+/* Testing knob of the triangle walks: rows with out-degree <= warp_cap (and,
+ * in the whole-path calls, few in-edges) are processed by one warp, others by a
+ * block with the row staged in shared memory up to heavy_cap entries, and
+ * beyond that in place (the drop-in support operator) or in column chunks of
+ * heavy_cap entries (the whole-path calls).  Lower values let small graphs
+ * exercise every path; 0 restores the defaults.  Affects calls launched
+ * afterwards from any thread. */
 void tdt_set_support_caps(int warp_cap, int heavy_cap);
 
-/* Testing knob of the support/listing kernels: 0 makes their wedge walk load
+/* Testing knob of the drop-in support operator: 0 makes its wedge walk load
  * one column index per lane and step, 1 (the default) four at a time from
  * 16-byte chunks (used when the columns array is 16-byte aligned and the
  * graph has fewer than 2^30 edges).  Results do not depend on it.  Affects
  * calls launched afterwards from any thread. */
 void tdt_set_vector_walk(int on);
 
-/* Knob of the support/listing kernels: 1 stages the rows that a whole block
- * walks (out-degree above 256) into shared memory by one bulk copy
- * (cp.async.bulk, tracked by an mbarrier with a bounded wait) plus plain
- * loads of the ragged ends; 0 (the default) loads them with plain loads.
- * Needs the vectorised walk.  Results do not depend on it.  Affects calls
- * launched afterwards from any thread. */
+/* Accepted for callers that set it; rows are staged by plain loads either
+ * way.  Results do not depend on it. */
 void tdt_set_bulk_staging(int on);
 
 /* Knob of the persistent peel (no counterpart in the reference): its grid in

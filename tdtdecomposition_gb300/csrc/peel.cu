@@ -61,12 +61,10 @@ struct PeelCtl {
     int dmin[2];                   // minimum decrement result above the level during level L_t, at t & 1
     long long passes;              // level-change passes run (diagnostic)
     int listed;                   // 1: per-edge triangle lists were built (they fit the workspace)
-    int list_skip;                // gate of the role-C transpose (no lists)
-    int rewalk_skip;              // gate of the second walk (lists written by kSupList)
-    int compact_skip;             // gate of the staging compaction (lists from the one-walk pass)
-    int stage_skip;               // gate of the one-walk pass (kSupStage)
-    int roles_skip;               // gate of the count-only walk (kSupRoles)
-    int pad0[2];
+    int list_skip;                // gate of the listing kernels (no lists)
+    int stage_skip;               // the walk only counts
+    int compact_skip;             // the role-A entries are not taken from the staging slots
+    int rewalk_skip;              // gate of the list walk
     long long rounds;
     long long triangles;
     unsigned long long alive;
@@ -1139,151 +1137,26 @@ __global__ void init_state_kernel(const int32_t* __restrict__ cA, const int32_t*
     }
 }
 
-// Staging bounds of the one-walk pass, per edge e = (u, v) at position i of
-// row u: role A (triangles (u, v, w)) at most min(d+(u) - i - 1, d+(v)) --
-// w lies in N+(u) after v and in N+(v); role B (triangles (u, x, v), x in
-// N+(u) before v and in N-(v) \ {u}) at most min(i, d-(v) - 1).  bnd[e] =
-// the role-A bound, sz[e] = both (the staging region of e).
-__global__ void stage_bounds_kernel(const int32_t* __restrict__ rows, const int32_t* __restrict__ cols,
-                                    const int64_t* __restrict__ rp, const int64_t* __restrict__ cp, int64_t E,
-                                    int32_t* __restrict__ bnd, int32_t* __restrict__ sz, const PeelCtl* ctl) {
-    if (*(volatile const int*)&ctl->g.status != 0) return;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t u = rows[e], v = cols[e];
-        const int64_t bu = rp[u];
-        const int64_t i = e - bu, du = rp[u + 1] - bu;
-        const int64_t dv = rp[v + 1] - rp[v], inv = cp[v + 1] - cp[v];
-        const int64_t a = du - i - 1 < dv ? du - i - 1 : dv;
-        const int64_t b = i < inv - 1 ? i : inv - 1;
-        const int64_t aa = a < 0 ? 0 : a, bb = b < 0 ? 0 : b;
-        bnd[e] = (int32_t)aa;
-        sz[e] = (int32_t)(aa + bb);  // < 2^31: the one-walk pass is only chosen for V < 2^30
-    }
+// One walk that counts and lists when the staging slots fit the list tail,
+// else a walk that only counts.
+__global__ void stage_decide_kernel(const int64_t* __restrict__ sbase, int64_t V, unsigned long long tail_bytes,
+                                    PeelCtl* ctl) {
+    ctl->stage_skip = !(ctl->g.status == 0 && (unsigned long long)sbase[V] <= tail_bytes / 8);
 }
 
-// Count-only walk or one walk with staging: the one walk when the staging
-// regions (8 bytes x soff[E]) fit the list tail.
-__global__ void stage_decide_kernel(const int64_t* __restrict__ soff, int64_t E, int64_t V,
-                                    unsigned long long tail_bytes, int want_lists, PeelCtl* ctl) {
-    const int ok0 = ctl->g.status == 0;
-    const int st = ok0 && want_lists && V < (1ll << 30) && 8ull * (unsigned long long)soff[E] <= tail_bytes;
-    ctl->stage_skip = !st;
-    ctl->roles_skip = !ok0 || st;
-}
-
-// Global cursors of the one walk's staging slots (used by rows searched in
-// place): role A at soff[e], role B at soff[e] + bnd[e].
-__global__ void stage_cursor_kernel(const int64_t* __restrict__ soff, const int32_t* __restrict__ bnd, int64_t E,
-                                    unsigned long long* __restrict__ curA, unsigned long long* __restrict__ curB,
-                                    const PeelCtl* ctl) {
-    if (*(volatile const int*)&ctl->stage_skip) return;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const unsigned long long o = (unsigned long long)soff[e];
-        curA[e] = o;
-        curB[e] = o + (unsigned long long)bnd[e];
-    }
-}
-
-// Lists fit when 8 bytes x (3T = off[E]) fit the workspace tail.  After the
-// one walk they are packed from the staging area (which sits at the end of
-// the tail) when both fit side by side; otherwise, when the lists alone fit,
-// the second walk writes them; otherwise the peel searches.
-__global__ void list_decide_kernel(const int64_t* __restrict__ off, const int64_t* __restrict__ soff, int64_t E,
-                                   unsigned long long tail_bytes, int want_lists, PeelCtl* ctl) {
-    const unsigned long long need = 8ull * (unsigned long long)off[E];
-    const int ok0 = want_lists && ctl->g.status == 0;
-    const int staged = !ctl->stage_skip;
-    const unsigned long long stage = staged ? 8ull * (unsigned long long)soff[E] : 0ull;
-    const int compact = ok0 && staged && need <= tail_bytes - stage;
-    const int rewalk = ok0 && !compact && need <= tail_bytes;
-    ctl->listed = compact || rewalk;
-    ctl->list_skip = !(compact || rewalk);
+// Lists fit when 8 bytes x (3T = off[E]) fit the list tail.  After the one
+// walk the role-A entries are moved from the staging slots (at the end of the
+// tail) when both fit side by side; otherwise, when the lists alone fit, a
+// second walk writes them; otherwise the peel searches.
+__global__ void list_decide_kernel(const int64_t* __restrict__ off, const int64_t* __restrict__ sbase, int64_t E,
+                                   int64_t V, unsigned long long tail_bytes, PeelCtl* ctl) {
+    const unsigned long long need = (unsigned long long)off[E], slots = tail_bytes / 8;
+    const int ok = ctl->g.status == 0 && need <= slots;
+    const int compact = ok && !ctl->stage_skip && need <= slots - (unsigned long long)sbase[V];
+    ctl->listed = ok;
+    ctl->list_skip = !ok;
     ctl->compact_skip = !compact;
-    ctl->rewalk_skip = !rewalk;
-}
-
-// Pack the role-A / role-B entries of every edge from its staging region
-// (slot s at stage_end[-1-s]) into its final list: role A at off[e], role B
-// at off[e] + cA[e].  A warp takes 32 edges at a time: their entries form one
-// flat index space (lane-held exclusive starts S), each lane finds the edge
-// of its entry by a 5-step search over S (shuffles), and four 32-entry
-// windows are copied per step so four loads per lane are in flight.
-#ifndef TDT_CMP_WIN
-#define TDT_CMP_WIN 4
-#endif
-#ifndef TDT_CMP_MINB
-#define TDT_CMP_MINB 6
-#endif
-constexpr int kCmpBlock = 256;
-__global__ void __launch_bounds__(kCmpBlock, TDT_CMP_MINB)
-stage_compact_kernel(const int64_t* __restrict__ soff, const int32_t* __restrict__ bnd,
-                                     const int32_t* __restrict__ cA, const int32_t* __restrict__ cB,
-                                     const int64_t* __restrict__ off, const int2* __restrict__ stage_end,
-                                     int2* __restrict__ lists, int64_t E, const PeelCtl* ctl) {
-    if (*(volatile const int*)&ctl->compact_skip) return;
-    const unsigned lane = lane_id();
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    constexpr int kWin = TDT_CMP_WIN;
-    for (int64_t base = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kWarp; base < E;
-         base += nw * kWarp) {
-        const int64_t e = base + lane;
-        int64_t so = 0, o = 0;
-        int32_t b = 0, na = 0, n = 0;
-        if (e < E) {
-            so = soff[e];
-            b = bnd[e];
-            na = cA[e];
-            n = na + cB[e];
-            o = off[e];
-        }
-        const int32_t incl = warp_incl_scan(n);
-        const int32_t total = __shfl_sync(kFull, incl, 31);
-        const int32_t S = incl - n;  // first flat entry of this lane's edge
-        for (int32_t tb = 0; tb < total; tb += kWin * kWarp) {
-            int2 v[kWin];
-            int64_t dst[kWin];
-#pragma unroll
-            for (int w = 0; w < kWin; w++) {
-                const int32_t t = tb + w * kWarp + (int)lane;
-                // last lane k with S_k <= t (S is non-decreasing, S_0 = 0)
-                int k = 0;
-#pragma unroll
-                for (int step = 16; step > 0; step >>= 1) {
-                    const int32_t Sc = __shfl_sync(kFull, S, k + step);
-                    if (Sc <= t) k += step;
-                }
-                const int32_t Sk = __shfl_sync(kFull, S, k), ak = __shfl_sync(kFull, na, k),
-                              bk = __shfl_sync(kFull, b, k);
-                const int64_t sk = __shfl_sync(kFull, so, k), ok = __shfl_sync(kFull, o, k);
-                const int32_t loc = t - Sk;
-                dst[w] = -1;
-                if (t < total) {
-                    const int64_t src = sk + (loc < ak ? loc : bk + (loc - ak));
-                    v[w] = __ldcs(stage_end - 1 - src);
-                    dst[w] = ok + loc;
-                }
-            }
-#pragma unroll
-            for (int w = 0; w < kWin; w++)
-                if (dst[w] >= 0) lists[dst[w]] = v[w];
-        }
-    }
-}
-
-// Global slot cursors of the second walk (used by rows listed in place):
-// role A at off[e], role B at off[e] + cA[e].
-__global__ void list_cursor_kernel(const int64_t* __restrict__ off, const int32_t* __restrict__ cA, int64_t E,
-                                   unsigned long long* __restrict__ curA, unsigned long long* __restrict__ curB,
-                                   const PeelCtl* ctl) {
-    if (*(volatile const int*)&ctl->rewalk_skip) return;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const unsigned long long o = (unsigned long long)off[e];
-        curA[e] = o;
-        curB[e] = o + cA[e];
-    }
+    ctl->rewalk_skip = !ok || compact;
 }
 
 __global__ void truss_out_kernel(const int32_t* __restrict__ rnd, const int32_t* __restrict__ round_level,
@@ -1428,20 +1301,19 @@ int test_barrier_timeout(void* ws, long long limit_ns, cudaStream_t st) {
     return status;
 }
 
-int launch_support_roles(const int64_t* rp, const int32_t* cols, int64_t nv, int64_t ne, int32_t* cA, int32_t* cB,
-                         int32_t* cC, void* ctl, const int* gate, int* status, cudaStream_t st);
-int launch_support_list(const int64_t* rp, const int32_t* cols, int64_t nv, int64_t ne, const int64_t* off,
-                        const int32_t* cA, const int32_t* cB, unsigned long long* curA_g,
-                        unsigned long long* curB_g, int2* lists, void* ctl, const int* gate, int* status,
-                        cudaStream_t st);
-int launch_support_stage(const int64_t* rp, const int32_t* cols, int64_t nv, int64_t ne, const int64_t* soff,
-                         const int32_t* bnd, int32_t* cA, int32_t* cB, int32_t* cC, unsigned long long* curA_g,
-                         unsigned long long* curB_g, int2* stage_end, unsigned long long stage_slots, void* ctl,
-                         const int* gate, int* status, cudaStream_t st);
-int launch_list_transpose(const int64_t* cp, const int64_t* rp, const int32_t* cols, const int32_t* in_eid,
-                          int64_t nv, int64_t ne, const int64_t* off,
-                          const int32_t* cA, const int32_t* cB, int2* lists, unsigned long long* cur, void* next,
-                          const int* gate, int* status, cudaStream_t st);
+int launch_stage_rows(const int64_t* rp, int64_t nv, int64_t* slots, const int* status, cudaStream_t st);
+int launch_walk_count(const int64_t* rp, const int32_t* cols, const int64_t* cp, const int32_t* in_src,
+                      const int32_t* in_eid, int64_t nv, int64_t ne, int32_t* cA, int32_t* cB, int32_t* cC,
+                      const int64_t* sbase, int2* stage_end, const int* stage_skip, int32_t* runA, void* units,
+                      void* ctl, int* status, cudaStream_t st);
+int launch_walk_list(const int64_t* rp, const int32_t* cols, const int64_t* cp, const int32_t* in_src,
+                     const int32_t* in_eid, int64_t nv, int64_t ne, const int64_t* off, int32_t* cA, int2* lists,
+                     int32_t* runA, void* units, void* ctl, const int* gate, int* status, cudaStream_t st);
+int launch_distribute(const int64_t* rp, const int32_t* cols, const int32_t* rows, const int64_t* cp,
+                      const int32_t* in_eid, int64_t nv, int64_t ne, const int64_t* off, const int32_t* cA,
+                      const int32_t* cB, const int64_t* sbase, const int2* stage_end, const int* stage_skip,
+                      int2* lists, uint32_t* cnt, void* units, void* ctl, const int* gate, int* status,
+                      cudaStream_t st);
 
 namespace {
 struct Carver {
@@ -1471,8 +1343,7 @@ struct Layout {
     int4* qi[3];
     long long* qb[3];
     int64_t* off;
-    int64_t* soff;
-    int32_t* bnd;
+    int64_t* sbase;
     int32_t* alive[2];
     unsigned* dead;
     unsigned* code;
@@ -1501,8 +1372,7 @@ Layout carve(void* ws, int64_t V, int64_t E) {
         L.qb[b] = (long long*)c.take(8 * e);
     }
     L.off = (int64_t*)c.take(8 * (e + 1));
-    L.soff = (int64_t*)c.take(8 * (e + 1));
-    L.bnd = (int32_t*)c.take(4 * e);
+    L.sbase = (int64_t*)c.take(8 * (v + 1));
     L.alive[0] = (int32_t*)c.take(4 * e);
     L.alive[1] = (int32_t*)c.take(4 * e);
     L.dead = (unsigned*)c.take(4 * (e / 32 + 1));
@@ -1565,30 +1435,8 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     int32_t* cB = cA + E;
     int32_t* cC = cB + E;
     prof_mark(0, st);
-    TDT_CUDA(cudaMemsetAsync(cA, 0, 12 * (size_t)E, st));
-    if (mode == 2) {
-        // triangle count: the count-only walk (skipped on the device when
-        // validation failed)
-        rc = launch_support_roles(rp, cols, V, E, cA, cB, cC, L.sup_ctl, &L.ctl->g.status, &L.ctl->g.status, st);
-        if (rc) return rc;
-        init_state_kernel<<<g_e, tb, 0, st>>>(cA, cB, cC, L.sup, L.live, L.rnd, E, L.ctl);
-        TDT_LAUNCH_CHECK("init_state");
-        prof_mark(1, st);
-        if (support_out) TDT_CUDA(cudaMemcpyAsync(support_out, L.sup, 4 * (size_t)E, cudaMemcpyDeviceToDevice, st));
-        stats_final_kernel<<<1, 1, 0, st>>>(L.ctl, stats, 1);
-        TDT_LAUNCH_CHECK("stats_final");
-        for (int ph = 2; ph <= 4; ph++) prof_mark(ph, st);
-        return TDT_OK;
-    }
-    // The list tail: final lists grow from its start, the one walk's staging
-    // area (indexed backwards) ends at its end.
-    const size_t list_base = (need + 255) & ~(size_t)255;
-    const unsigned long long tail = ws_bytes > list_base ? (unsigned long long)(ws_bytes - list_base) : 0ull;
-    int2* lists = reinterpret_cast<int2*>(reinterpret_cast<char*>(ws) + list_base);
-    const unsigned long long stage_slots = tail / 8;
-    int2* stage_end = lists + stage_slots;
-    // in-adjacency (CSC) of the oriented graph: staging bounds, role-C
-    // transpose, and the peel without lists
+    // in-adjacency (CSC) of the oriented graph: the walk's middle vertices, and
+    // the peel without lists
     TDT_CUDA(cudaMemsetAsync(L.indeg, 0, 4 * (size_t)V, st));
     indeg_kernel<<<g_e, tb, 0, st>>>(rows_use, cols, E, V, L.indeg, L.ctl);
     TDT_LAUNCH_CHECK("indeg");
@@ -1597,53 +1445,52 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     TDT_CUDA(cudaMemsetAsync(L.indeg, 0, 4 * (size_t)V, st));
     csc_fill_kernel<<<g_e, tb, 0, st>>>(rows_use, cols, E, V, L.cp, L.indeg, L.in_src, L.in_eid, L.ctl);
     TDT_LAUNCH_CHECK("csc_fill");
-    // staging regions of the one walk (L.sup holds their sizes until
-    // init_state overwrites it), and the choice of walk
-    stage_bounds_kernel<<<g_e, tb, 0, st>>>(rows_use, cols, rp, L.cp, E, L.bnd, L.sup, L.ctl);
-    TDT_LAUNCH_CHECK("stage_bounds");
-    rc = exclusive_scan<int32_t, int64_t>(L.sup, L.soff, E, L.soff + E, L.scan_ws, st);
-    if (rc) return rc;
-    stage_decide_kernel<<<1, 1, 0, st>>>(L.soff, E, V, tail, tail > 0, L.ctl);
-    TDT_LAUNCH_CHECK("stage_decide");
-    unsigned long long* curA = reinterpret_cast<unsigned long long*>(L.qb[0]);
-    unsigned long long* curB = reinterpret_cast<unsigned long long*>(L.qb[1]);
-    stage_cursor_kernel<<<g_e, tb, 0, st>>>(L.soff, L.bnd, E, curA, curB, L.ctl);
-    TDT_LAUNCH_CHECK("stage_cursor");
-    // the walk: counts and staged role-A/B entries, or counts only (each
-    // launch returns at once when its gate is set)
-    rc = launch_support_stage(rp, cols, V, E, L.soff, L.bnd, cA, cB, cC, curA, curB, stage_end, stage_slots,
-                              L.sup_ctl, &L.ctl->stage_skip, &L.ctl->g.status, st);
-    if (rc) return rc;
-    rc = launch_support_roles(rp, cols, V, E, cA, cB, cC, L.sup_ctl, &L.ctl->roles_skip, &L.ctl->g.status, st);
+    // The list tail: final lists grow from its start, the staging slots of the
+    // one walk end at its end.
+    const size_t list_base = (need + 255) & ~(size_t)255;
+    const unsigned long long tail =
+        mode != 2 && ws_bytes > list_base ? (unsigned long long)(ws_bytes - list_base) : 0ull;
+    int2* lists = reinterpret_cast<int2*>(reinterpret_cast<char*>(ws) + list_base);
+    int2* stage_end = lists + tail / 8;
+    if (tail > 0) {
+        rc = launch_stage_rows(rp, V, L.sbase, &L.ctl->g.status, st);
+        if (rc) return rc;
+        rc = exclusive_scan<int64_t, int64_t>(L.sbase, L.sbase, V, L.sbase + V, L.scan_ws, st);
+        if (rc) return rc;
+        stage_decide_kernel<<<1, 1, 0, st>>>(L.sbase, V, tail, L.ctl);
+        TDT_LAUNCH_CHECK("stage_decide");
+    }
+    // the walk: counts, and the role-A entries when they can be staged (skipped
+    // on the device when validation failed); the plan of its units stays for
+    // the list walk
+    TDT_CUDA(cudaMemsetAsync(cA, 0, 16 * (size_t)E, st));  // cA, cB, cC and the distribution's counters
+    rc = launch_walk_count(rp, cols, L.cp, L.in_src, L.in_eid, V, E, cA, cB, cC, tail > 0 ? L.sbase : nullptr,
+                           stage_end, &L.ctl->stage_skip, L.alive[0], L.qi[2], L.sup_ctl, &L.ctl->g.status, st);
     if (rc) return rc;
     init_state_kernel<<<g_e, tb, 0, st>>>(cA, cB, cC, L.sup, L.live, L.rnd, E, L.ctl);
     TDT_LAUNCH_CHECK("init_state");
     prof_mark(1, st);
-    // per-edge triangle lists in the workspace tail when 24 T bytes fit
-    rc = exclusive_scan<int32_t, int64_t>(L.sup, L.off, E, L.off + E, L.scan_ws, st);
-    if (rc) return rc;
-    list_decide_kernel<<<1, 1, 0, st>>>(L.off, L.soff, E, tail, tail > 0, L.ctl);
-    TDT_LAUNCH_CHECK("list_decide");
-    {
-        // one wave of resident blocks (the loop is grid-strided)
-        int occ_c = 0;
-        TDT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_c, stage_compact_kernel, kCmpBlock, 0));
-        if (occ_c < 1) occ_c = 1;
-        const unsigned g_c = grid_for(E * 32, kCmpBlock, di.sms, occ_c);
-        stage_compact_kernel<<<g_c, kCmpBlock, 0, st>>>(L.soff, L.bnd, cA, cB, L.off, stage_end, lists, E, L.ctl);
+    if (mode == 2) {
+        if (support_out) TDT_CUDA(cudaMemcpyAsync(support_out, L.sup, 4 * (size_t)E, cudaMemcpyDeviceToDevice, st));
+        stats_final_kernel<<<1, 1, 0, st>>>(L.ctl, stats, 1);
+        TDT_LAUNCH_CHECK("stats_final");
+        for (int ph = 2; ph <= 4; ph++) prof_mark(ph, st);
+        return TDT_OK;
     }
-    TDT_LAUNCH_CHECK("stage_compact");
-    // second walk, when the lists fit but not beside the staging area
-    list_cursor_kernel<<<g_e, tb, 0, st>>>(L.off, cA, E, curA, curB, L.ctl);
-    TDT_LAUNCH_CHECK("list_cursor");
-    rc = launch_support_list(rp, cols, V, E, L.off, cA, cB, curA, curB, lists, L.sup_ctl, &L.ctl->rewalk_skip,
-                             &L.ctl->g.status, st);
-    if (rc) return rc;
-    // role C of every list, from the role-A lists of each vertex's in-edges
-    rc = launch_list_transpose(L.cp, rp, cols, L.in_eid, V, E, L.off, cA, cB, lists,
-                               reinterpret_cast<unsigned long long*>(L.qi[1]), L.sup_ctl, &L.ctl->list_skip,
-                               &L.ctl->g.status, st);
-    if (rc) return rc;
+    // per-edge triangle lists in the workspace tail when 24 T bytes fit
+    if (tail > 0) {
+        rc = exclusive_scan<int32_t, int64_t>(L.sup, L.off, E, L.off + E, L.scan_ws, st);
+        if (rc) return rc;
+        list_decide_kernel<<<1, 1, 0, st>>>(L.off, L.sbase, E, V, tail, L.ctl);
+        TDT_LAUNCH_CHECK("list_decide");
+        // second walk, when the lists fit but not beside the staging slots
+        rc = launch_walk_list(rp, cols, L.cp, L.in_src, L.in_eid, V, E, L.off, cA, lists, L.alive[0], L.qi[2],
+                              L.sup_ctl, &L.ctl->rewalk_skip, &L.ctl->g.status, st);
+        if (rc) return rc;
+        rc = launch_distribute(rp, cols, rows_use, L.cp, L.in_eid, V, E, L.off, cA, cB, L.sbase, stage_end,
+                               &L.ctl->compact_skip, lists, reinterpret_cast<uint32_t*>(cC + E), L.qi[2], L.sup_ctl, &L.ctl->list_skip, &L.ctl->g.status, st);
+        if (rc) return rc;
+    }
     prof_mark(2, st);
 
     // persistent peel

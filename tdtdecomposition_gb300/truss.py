@@ -58,24 +58,13 @@ STAGE_BUDGET_FRACTION = 0.75
 
 
 def stage_bytes(cols, rp, rows=None):
-    """Bytes of the one-walk pass's staging area: 8 per slot of the role-A /
-    role-B bounds of every edge e = (u, v) at position i of row u:
-    min(d+(u) - i - 1, d+(v)) + min(i, d-(v) - 1), the bounds the device
-    computes (stage_bounds_kernel)."""
-    rp = rp.to(torch.int64)
-    V, E = rp.shape[0] - 1, cols.shape[0]
-    if E == 0:
+    """Bytes of the one-walk pass's staging slots: 8 per role-A entry an edge
+    at position i of a row of d edges may have, d - i - 1, so d (d - 1) / 2 per
+    row (the slots the device lays out, walk.cu)."""
+    if cols.shape[0] == 0:
         return 0
-    dplus = rp[1:] - rp[:-1]
-    if rows is None:
-        rows = torch.repeat_interleave(torch.arange(V, device=cols.device), dplus)
-    u = rows.to(torch.int64)
-    v = cols.to(torch.int64)
-    i = torch.arange(E, device=cols.device) - rp[u]
-    indeg = torch.bincount(v, minlength=V)
-    a = torch.minimum(dplus[u] - i - 1, dplus[v]).clamp_min_(0)
-    b = torch.minimum(i, indeg[v] - 1).clamp_min_(0)
-    return 8 * int((a + b).sum())
+    d = rp[1:].to(torch.int64) - rp[:-1].to(torch.int64)
+    return 4 * int((d * (d - 1)).sum())
 
 
 def _list_bytes(ws, cols, rp, lists, base, rows=None):
