@@ -89,6 +89,8 @@ struct PeelArgs {
     int4* qi[3];
     long long* qb[3];
     int32_t* alive[2];    // compacted alive-edge lists (level transitions)
+    // listed mode, round r at r & 1: the item that holds slot 32 j, for j < kSlotIdx
+    int32_t* sidx[2];
     // bit e set: edge e was peeled in a sub-round before the current one (a
     // filter in L2 before the state checks, used only in builds without the
     // round codes; a bit not set yet only costs the check it would have saved)
@@ -110,6 +112,67 @@ struct PeelArgs {
 __device__ __forceinline__ void set_status(PeelCtl* c, int s) {
     atomicMax(&c->g.status, s);
     grid_abort(&c->g);
+}
+
+// Round-boundary barrier of the persistent loop: arrivals counted against an
+// epoch that every thread keeps (no returned value on the arrival), and the
+// next sub-round's counters fetched by the waiting thread and handed to the
+// block through shared memory, so no warp pays a load for them.
+struct RoundBar {
+    unsigned long long target;   // arrivals that complete the next barrier
+    unsigned long long q, fe;    // after wait(): counters of the round asked for
+};
+
+struct RoundShared {
+    unsigned long long q, fe;
+    int ok;
+    int dmin;                    // smallest decrement result of the block's sub-round
+};
+
+__device__ __forceinline__ void red_release_add(unsigned long long* p, unsigned long long v) {
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// Barrier over all blocks; next: the round whose counters are wanted.  dmin:
+// where the block's smallest decrement result goes (reset for the next
+// sub-round).  False when the run is being aborted.
+__device__ __forceinline__ bool round_barrier(PeelCtl* ctl, RoundBar& B, RoundShared* S, int next, int* dmin) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int ok = 1;
+        if (S->dmin != INT32_MAX) {
+            atomicMin(dmin, S->dmin);
+            S->dmin = INT32_MAX;
+        }
+        red_release_add(&ctl->g.arrive, 1ull);
+        const uint64_t t0 = globaltimer_ns();
+        unsigned spins = 0;
+        for (;;) {
+            const unsigned long long v = ld_acquire_u64(&ctl->g.arrive);
+            if (v & kGridAbortBit) {
+                ok = 0;
+                break;
+            }
+            if (v >= B.target) break;
+            if ((++spins & 31u) == 0) {
+                if (globaltimer_ns() - t0 > kBarrierTimeoutNs) {
+                    atomicMax(&ctl->g.status, (int)TDT_ERR_TIMEOUT);
+                    grid_abort(&ctl->g);
+                    ok = 0;
+                    break;
+                }
+                if (spins > 4096) __nanosleep(200);
+            }
+        }
+        S->q = __ldcg(&ctl->q[next & 3]);
+        S->fe = __ldcg(&ctl->fe[next & 3]);
+        S->ok = ok;
+    }
+    __syncthreads();
+    B.target += gridDim.x;
+    B.q = S->q;
+    B.fe = S->fe;
+    return S->ok != 0;
 }
 
 __device__ __forceinline__ unsigned long long ld_cg_u64(const unsigned long long* p) {
@@ -167,6 +230,18 @@ __device__ __forceinline__ bool make_item(const PeelArgs& A, bool want, int32_t 
     if (du <= dv) { it.y = u; it.z = v; dx = du; it.w = (int32_t)duo; }
     else { it.y = v; it.z = u; dx = dv; it.w = (int32_t)dvo; }
     return dx > 1;
+}
+
+// 32-slot windows covered by the slot index.
+constexpr int kSlotIdx = 32768;
+// A listed sub-round takes the short chain up to this many windows a warp
+// (peel at R-MAT scale 16 / 18 / 20: 7.52 / 14.04 / 34.55 ms with one, 7.38 /
+// 13.79 / 33.95 with four, the same with six).
+constexpr int kLeanWindows = 4;
+
+// Records item idx, slots [c, c + dx), in the slot index of its round.
+__device__ __forceinline__ void index_item(int32_t* sidx, long long idx, long long c, long long dx) {
+    for (long long j = (c + kWarp - 1) / kWarp; j < kSlotIdx && j * kWarp < c + dx; j++) sidx[j] = (int32_t)idx;
 }
 
 // Reserve n items and tot candidate slots of the round in `slot` (lane 0's
@@ -242,6 +317,7 @@ __device__ __forceinline__ void append_flush(const PeelArgs& A, int slot, int bu
                     if (idx < A.E) {
                         A.qi[buf][idx] = it[k];
                         A.qb[buf][idx] = cc;
+                        if (Listed) index_item(A.sidx[slot & 1], idx, cc, dx[k]);
                     }
                     idx++;
                     cc += dx[k];
@@ -421,7 +497,7 @@ __device__ __forceinline__ void pass_start(const PeelArgs& A, int np) {
 }
 
 __device__ __forceinline__ bool level_transition(const PeelArgs& A, bool listed, int r_next, int t, int& np,
-                                              int32_t* l_out, int32_t* app_e) {
+                                              int32_t* l_out, int32_t* app_e, RoundBar& RB, RoundShared* RS) {
     const unsigned lane = lane_id();
     const long long gw = (long long)blockIdx.x * kPeelWarps + threadIdx.x / kWarp;
     const long long nw = (long long)gridDim.x * kPeelWarps;
@@ -513,7 +589,7 @@ __device__ __forceinline__ bool level_transition(const PeelArgs& A, bool listed,
         pass_min(A, np, mloc);
     }
     np++;
-    if (!grid_barrier(&A.ctl->g, gridDim.x)) return false;
+    if (!round_barrier(A.ctl, RB, RS, r_next, &A.ctl->dmin[t & 1])) return false;
     if (ld_cg_u64(&A.ctl->pfe[(np + 2) % 3]) > 0) {
         *l_out = g;
         return true;
@@ -546,7 +622,7 @@ __device__ __forceinline__ bool level_transition(const PeelArgs& A, bool listed,
     else append_flush_call<false>(A, slot, buf, B, &A.ctl->pfe[np % 3]);
     pass_min(A, np, mloc);
     np++;
-    return grid_barrier(&A.ctl->g, gridDim.x);
+    return round_barrier(A.ctl, RB, RS, r_next, &A.ctl->dmin[t & 1]);
 }
 
 // k-truss search (fixed level l): the frontier is every alive edge with
@@ -604,12 +680,14 @@ __device__ __forceinline__ void warp_append_capped(const PeelArgs& A, bool liste
         if (idx < A.E) {
             A.qi[buf][idx] = it;
             A.qb[buf][idx] = (long long)(old & kCandMask) + incl - c;
+            if (listed) index_item(A.sidx[slot & 1], idx, (long long)(old & kCandMask) + incl - c, dx);
         }
     }
 }
 
 // One collection pass for sub-round r_next; true when it took an edge.
-__device__ bool fixed_collect(const PeelArgs& A, bool listed, int32_t l, int r_next, int& np) {
+__device__ bool fixed_collect(const PeelArgs& A, bool listed, int32_t l, int r_next, int& np, RoundBar& RB,
+                              RoundShared* RS) {
     const unsigned lane = lane_id();
     const int64_t nthreads = (int64_t)gridDim.x * blockDim.x;
     const int slot = r_next & 3, buf = r_next % 3;
@@ -627,7 +705,7 @@ __device__ bool fixed_collect(const PeelArgs& A, bool listed, int32_t l, int r_n
         warp_append_capped(A, listed, slot, buf, want, (int32_t)e, s, r_next, &A.ctl->pfe[np % 3]);
     }
     np++;
-    if (!grid_barrier(&A.ctl->g, gridDim.x)) return false;
+    if (!round_barrier(A.ctl, RB, RS, r_next, &A.ctl->dmin[0])) return false;
     return ld_cg_u64(&A.ctl->pfe[(np + 2) % 3]) > 0;
 }
 
@@ -786,6 +864,72 @@ __device__ __forceinline__ void settle(const PeelArgs& A, const Pending& P, int 
     }
 }
 
+// A listed sub-round of a few windows a warp: a chain of dependent loads with
+// nothing to hide it (300 cycles each in L2, 500 for an atomic's result), so
+// the chain is kept short.  The slot index gives the window's first item, the
+// records and first slots of the 32 items from it on come together, and a lane
+// takes its record by shuffles: slot index, items, list entry, round codes,
+// decrement, instead of counters, item search (a load per factor of 32), item,
+// window starts, records, list entry, codes, decrement.  With the counters
+// handed over by the barrier, peel of R-MAT scale 12 / 16 / 20 / 22: 2.58 /
+// 9.70 / 40.3 / 116.6 -> 1.72 / 7.32 / 33.6 / 104.2 ms.
+__device__ __forceinline__ void lean_round(const PeelArgs& A, int r, int32_t l, int N, int T, int gwarp, int nwarps,
+                                           int32_t* ebuf, int* s_dmin) {
+    if (gwarp * kWarp >= T) return;
+    const unsigned lane = lane_id();
+    const unsigned le = lanemask_lt() | (1u << lane);
+    const int buf = r % 3, nslot = (r + 1) & 3, nbuf = (r + 1) % 3;
+    const unsigned cm = l > 0 ? ((unsigned)(r + 1) & 3u) : kCodeDead;
+    int32_t dm = INT32_MAX;
+    AppendBuf B{ebuf, 0, 0ull};
+    for (int cb = gwarp * kWarp; cb < T; cb += nwarps * kWarp) {
+        const int i0 = __ldcg(A.sidx[r & 1] + (cb >> 5));
+        int4 it = make_int4(0, 0, 0, 0);
+        int S = INT32_MAX;  // first slot of item i0 + lane
+        if (i0 + (int)lane < N) {
+            it = __ldcg(A.qi[buf] + i0 + lane);
+            S = (int)__ldcg(A.qb[buf] + i0 + lane);
+        }
+        const unsigned d = (unsigned)(S - cb);
+        const unsigned mk = __reduce_or_sync(kFull, lane > 0 && d < (unsigned)kWarp ? 1u << d : 0u);
+        const int k = __popc(mk & le);
+        const int t = cb + (int)lane - __shfl_sync(kFull, S, k);
+        const int32_t e = __shfl_sync(kFull, it.x, k);
+        const long long o =
+            (long long)(unsigned)__shfl_sync(kFull, it.y, k) | ((long long)__shfl_sync(kFull, it.z, k) << 32);
+        const bool v = cb + (int)lane < T;
+        int2 fg = make_int2(0, 0);
+        if (v) fg = __ldg(A.lists + o + t);
+        unsigned xf = 0, xg = 0;
+        if (v) {
+            xf = __ldcg(A.code + (fg.x >> 3));
+            xg = __ldcg(A.code + (fg.y >> 3));
+        }
+        // the ownership rules of process_round
+        const int32_t rf = code_round(xf, fg.x, r), rg = code_round(xg, fg.y, r);
+        const bool on = v && rf != -2 && rg != -2;
+        const bool cf = rf == r, cg = rg == r;
+        int32_t of = INT32_MIN, og = INT32_MIN;
+        if (on && !cf && (!cg || e < fg.y) && (!kSkipMarked || rf != r + 1)) of = atomicSub(A.live + fg.x, 1);
+        if (on && !cg && (!cf || e < fg.x) && (!kSkipMarked || rg != r + 1)) og = atomicSub(A.live + fg.y, 1);
+        if (of > l + 1 && of - 1 < dm) dm = of - 1;
+        if (og > l + 1 && og - 1 < dm) dm = og - 1;
+        const bool wf = of == l + 1, wg = og == l + 1;
+        if (wf) {
+            A.rnd[fg.x] = r + 1;
+            code_mark(A.code, fg.x, cm);
+        }
+        if (wg) {
+            A.rnd[fg.y] = r + 1;
+            code_mark(A.code, fg.y, cm);
+        }
+        warp_append2_staged<true>(A, nslot, nbuf, wf, fg.x, wg, fg.y, l, B, &A.ctl->fe[nslot]);
+    }
+    dm = warp_min(dm);
+    if (lane == 0 && dm != INT32_MAX) atomicMin(s_dmin, dm);
+    append_flush<true>(A, nslot, nbuf, B, &A.ctl->fe[nslot]);
+}
+
 // One sub-round: warps gwarp = 0..nwarps-1 share the candidate slots of round r.
 // The smallest decrement result above l is folded into *dmin (the lower bound
 // of the next level).  Each step covers two 32-slot windows whose loads and
@@ -794,8 +938,9 @@ __device__ __forceinline__ void settle(const PeelArgs& A, const Pending& P, int 
 // so no call passes a local copy of them, and no call frame is saved around
 // every sub-round.
 template <bool Listed>
-__device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t l, long long gwarp, long long nwarps,
-                                           int* dmin, int32_t* app_e) {
+__device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t l, unsigned long long packed,
+                                              long long nprev, long long gwarp, long long nwarps, int* s_dmin,
+                                              int32_t* app_e) {
     const unsigned lane = lane_id();
     const unsigned le = lanemask_lt() | (1u << lane);
     int32_t dm = INT32_MAX;
@@ -803,7 +948,6 @@ __device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t 
     const int nslot = (r + 1) & 3, nbuf = (r + 1) % 3;
     const int wib = threadIdx.x / kWarp;
     AppendBuf B{app_e + wib * kAppBuf, 0, 0ull};
-    const unsigned long long packed = ld_cg_u64(&A.ctl->q[slot]);
     const long long N = (long long)(packed >> kCandBits);
     const long long T = (long long)(packed & kCandMask);
     const long long* __restrict__ qb = A.qb[buf];
@@ -813,14 +957,16 @@ __device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t 
     // the next round"), or, without the codes, their dead bits are set (a bit
     // read before it is set only sends that triangle to the state check)
     if ((kPeelCodes || kDeadFilter) && r > 0) {
-        long long nprev = (long long)(ld_cg_u64(&A.ctl->q[(r - 1) & 3]) >> kCandBits);
-        if (nprev > A.E) nprev = A.E;
         const int4* __restrict__ qp = A.qi[(r - 1) % 3];
         for (long long i = gwarp * kWarp + lane; i < nprev; i += nwarps * kWarp) {
             const int32_t e = __ldcg(&qp[i].x);
             if (kPeelCodes) atomicOr(A.code + (e >> 3), kCodeDead << ((unsigned)(e & 7) * 4u));
             else atomicOr(A.dead + (e >> 5), 1u << (e & 31));
         }
+    }
+    if (Listed && T <= nwarps * kWarp * kLeanWindows && T <= (long long)kSlotIdx * kWarp) {
+        lean_round(A, r, l, (int)N, (int)T, (int)gwarp, (int)nwarps, app_e + wib * kAppBuf, s_dmin);
+        return;
     }
     // listed mode: each warp owns a contiguous range of candidate slots (a
     // multiple of 64).  Search mode with many slots: warps take ranges of
@@ -969,7 +1115,8 @@ __device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t 
     }
     if (kPeelDefer) settle<Listed>(A, P, r, l, nslot, nbuf, B, dm);
     if (Listed) append_flush<Listed>(A, nslot, nbuf, B, &A.ctl->fe[nslot]);
-    fold_min(dmin, dm);
+    dm = warp_min(dm);
+    if (lane == 0 && dm != INT32_MAX) atomicMin(s_dmin, dm);
 }
 
 #ifndef TDT_PEEL_MINB
@@ -979,6 +1126,7 @@ __device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t 
 // read its fields from the parameter bank instead of a local copy.
 __global__ void __launch_bounds__(kPeelBlock, TDT_PEEL_MINB) peel_kernel(const __grid_constant__ PeelArgs A) {
     __shared__ int32_t s_app_e[kPeelWarps * kAppBuf];  // per-warp append staging
+    __shared__ RoundShared s_round;
     const bool listed = A.lists != nullptr && *(volatile int*)&A.ctl->listed != 0;
     const int wib = threadIdx.x / kWarp;
     const int64_t gwarp = (int64_t)blockIdx.x * kPeelWarps + wib;
@@ -991,11 +1139,14 @@ __global__ void __launch_bounds__(kPeelBlock, TDT_PEEL_MINB) peel_kernel(const _
     int32_t l = 0;
     int ntrans = 0, np = 0;
     bool ok;
+    if (threadIdx.x == 0) s_round.dmin = INT32_MAX;
+    RoundBar RB{gridDim.x, 0ull, 0ull};
+    long long nprev = 0;  // items of the sub-round before
     if (A.mode == 0) {
-        ok = level_transition(A, listed, 0, ntrans++, np, &l, s_app_e);
+        ok = level_transition(A, listed, 0, ntrans++, np, &l, s_app_e, RB, &s_round);
     } else {
         l = A.fixed_level;
-        ok = fixed_collect(A, listed, l, 0, np);
+        ok = fixed_collect(A, listed, l, 0, np, RB, &s_round);
     }
     if (!ok) {
         if (master) A.ctl->rounds = 0;
@@ -1010,12 +1161,14 @@ __global__ void __launch_bounds__(kPeelBlock, TDT_PEEL_MINB) peel_kernel(const _
             A.ctl->grab[(r + 2) & 3] = 0;
             if (globaltimer_ns() - t_start > A.deadline_ns) set_status(A.ctl, TDT_ERR_TIMEOUT);
         }
-        // level L_t (t = ntrans - 1) folds its decrement results into dmin[t & 1]
-        if (listed) process_round<true>(A, r, l, gwarp, nwarps, &A.ctl->dmin[(ntrans + 1) & 1], s_app_e);
-        else process_round<false>(A, r, l, gwarp, nwarps, &A.ctl->dmin[(ntrans + 1) & 1], s_app_e);
+        if (listed) process_round<true>(A, r, l, RB.q, nprev, gwarp, nwarps, &s_round.dmin, s_app_e);
+        else process_round<false>(A, r, l, RB.q, nprev, gwarp, nwarps, &s_round.dmin, s_app_e);
+        nprev = (long long)(RB.q >> kCandBits);
+        if (nprev > A.E) nprev = A.E;
         __syncthreads();
         const uint64_t t_p = globaltimer_ns();
-        if (!grid_barrier(&A.ctl->g, gridDim.x)) return;
+        // level L_t (t = ntrans - 1) folds its decrement results into dmin[t & 1]
+        if (!round_barrier(A.ctl, RB, &s_round, r + 1, &A.ctl->dmin[(ntrans + 1) & 1])) return;
         const uint64_t t_b = globaltimer_ns();
         if (master) {
             A.ctl->t_proc += t_p - t_mark;
@@ -1027,16 +1180,16 @@ __global__ void __launch_bounds__(kPeelBlock, TDT_PEEL_MINB) peel_kernel(const _
         }
         // fe[(r+1) & 3] is only written by sub-round r (level changes count
         // into pfe), and cleared again at the top of sub-round r+3
-        if (ld_cg_u64(&A.ctl->fe[(r + 1) & 3]) == 0) {
+        if (RB.fe == 0) {
             if (A.mode != 0) {
                 // k-truss search: the next batch of low-support edges, if any
-                if (!fixed_collect(A, listed, l, r + 1, np)) break;
+                if (!fixed_collect(A, listed, l, r + 1, np, RB, &s_round)) break;
                 t_mark = globaltimer_ns();
                 r++;
                 continue;
             }
             int32_t nl;
-            const bool more = level_transition(A, listed, r + 1, ntrans++, np, &nl, s_app_e);
+            const bool more = level_transition(A, listed, r + 1, ntrans++, np, &nl, s_app_e, RB, &s_round);
             if (master) A.ctl->t_trans += globaltimer_ns() - t_b;
             if (!more) break;
             l = nl;
@@ -1344,6 +1497,7 @@ struct Layout {
     long long* qb[3];
     int64_t* off;
     int64_t* sbase;
+    int32_t* sidx;
     int32_t* alive[2];
     unsigned* dead;
     unsigned* code;
@@ -1373,6 +1527,7 @@ Layout carve(void* ws, int64_t V, int64_t E) {
     }
     L.off = (int64_t*)c.take(8 * (e + 1));
     L.sbase = (int64_t*)c.take(8 * (v + 1));
+    L.sidx = (int32_t*)c.take(8 * (size_t)kSlotIdx);
     L.alive[0] = (int32_t*)c.take(4 * e);
     L.alive[1] = (int32_t*)c.take(4 * e);
     L.dead = (unsigned*)c.take(4 * (e / 32 + 1));
@@ -1513,6 +1668,7 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     TDT_CUDA(cudaMemsetAsync(L.code, 0xff, 4 * (size_t)(E / 8 + 1), st));
     A.off = L.off; A.lists = lists;
     A.alive[0] = L.alive[0]; A.alive[1] = L.alive[1];
+    A.sidx[0] = L.sidx; A.sidx[1] = L.sidx + kSlotIdx;
     A.V = V; A.E = E; A.round_cap = E + 2;
     A.mode = mode == 0 ? 0 : 1;
     A.fixed_level = fixed_level;
@@ -1524,15 +1680,15 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
                            ? (unsigned long long)g_fixed_cand_cap : kFixedCandCap;
     A.ctl = L.ctl;
     if (di.sms * occ > 4096) occ = 4096 / di.sms;
-    // Smaller graphs peel their lists faster on fewer blocks: the sub-rounds
-    // are short, so the grid barrier and the idle warps cost more than the
-    // parallelism gives (R-MAT scale 10-18 measured 4-15 % faster on one block
-    // per SM, scales 10-14 on one per two SMs; scale 20 and up fastest on
-    // all).  The search peel (no list tail) keeps every block: its slots are
-    // binary searches, and scale 18 ran 22 % slower on half the blocks.
+    // Small graphs peel their lists on one block per SM: their sub-rounds fit
+    // one window a warp there, and a grid barrier of fewer blocks is shorter.
+    // 76 / 152 / 304 blocks: R-MAT scale 12 1.77 / 1.80 / 1.92 ms, scale 14
+    // 4.42 / 4.36 / 4.64, scale 16 (0.9 M edges) 8.43 / 7.53 / 7.52, scale 18
+    // 18.2 / 14.0 / 13.3, scale 20 61.4 / 40.2 / 34.1; Chung-Lu (1.5 M edges)
+    // 10.6 / 9.6 / 9.8.  The search peel (no list tail) keeps every block: its
+    // slots are binary searches.
     int nblk = di.sms * occ;
-    if (tail > 0 && E < (1ll << 18)) nblk = (di.sms + 1) / 2;
-    else if (tail > 0 && E < (1ll << 22)) nblk = di.sms;
+    if (tail > 0 && E < (1ll << 20)) nblk = di.sms;
     if (g_peel_half_sms > 0) nblk = (g_peel_half_sms * di.sms + 1) / 2;
     if (nblk > di.sms * occ) nblk = di.sms * occ;
     dim3 grid(nblk), block(kPeelBlock);
