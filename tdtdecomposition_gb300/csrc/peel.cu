@@ -52,7 +52,7 @@ constexpr uint64_t kPeelDeadlineNs = 120ull * 1000ull * 1000ull * 1000ull;
 struct PeelCtl {
     GridCtl g;
     // round r's counters live at r & 3: round r reads slot r, appends to r+1,
-    // sets the dead bits of round r-1's edges, and the top of round r clears r+2
+    // turns round r-1's edges dead, and the top of round r clears r+2
     unsigned long long q[4];      // packed (items << kCandBits | candidates) per round slot
     unsigned long long fe[4];     // frontier edges per round slot (queued or not)
     unsigned long long cnt[3];     // survivors written by level change t, at t % 3
@@ -85,16 +85,12 @@ struct PeelArgs {
     int32_t* rnd;         // sub-round that peeled each edge (-1: alive)
     int32_t* round_level;
     // queue of round r in buffer r % 3: round r reads r, appends r+1, and the
-    // items of round r-1 stay intact for the dead bits set during round r
+    // items of round r-1 stay intact for the codes turned dead during round r
     int4* qi[3];
     long long* qb[3];
     int32_t* alive[2];    // compacted alive-edge lists (level transitions)
-    // listed mode, round r at r & 1: the item that holds slot 32 j, for j < kSlotIdx
+    // round r at r & 1: the item that holds slot 32 j, for j < kSlotIdx
     int32_t* sidx[2];
-    // bit e set: edge e was peeled in a sub-round before the current one (a
-    // filter in L2 before the state checks, used only in builds without the
-    // round codes; a bit not set yet only costs the check it would have saved)
-    unsigned* dead;
     // round code of edge e in the 4 bits at (e & 7) * 4 of word e >> 3 (the
     // listed peel's partner-state check; see code_round)
     unsigned* code;
@@ -182,8 +178,8 @@ __device__ __forceinline__ unsigned long long ld_cg_u64(const unsigned long long
 // Round codes: 4 bits per edge, 32 MB at 64 M edges, so they stay in L2.
 // 0xF: never marked (alive); 0-3: marked for sub-round y, stored as y & 3;
 // bit 3 set: peeled and done.  A code is set once, when its edge is marked
-// (0xF -> y & 3, one atomicAnd), and turned dead during sub-round y + 1 with
-// the dead bits of that round's items (atomicOr 0x8).  An edge marked without
+// (0xF -> y & 3, one atomicAnd), and turned dead during sub-round y + 1
+// (atomicOr 0x8 over the items of round y).  An edge marked without
 // an item (no triangle left to enumerate) is dead at once: each of its
 // triangles is already destroyed by a partner peeled before it.  Hence, in
 // sub-round r (a grid barrier after every sub-round), a code reads 0xF
@@ -238,6 +234,11 @@ constexpr int kSlotIdx = 32768;
 // (peel at R-MAT scale 16 / 18 / 20: 7.52 / 14.04 / 34.55 ms with one, 7.38 /
 // 13.79 / 33.95 with four, the same with six).
 constexpr int kLeanWindows = 4;
+// A search sub-round, whose slots cost from one load to twenty, takes its
+// windows strided over the warps up to this many a warp: neighbouring slots,
+// which cost alike, spread out (Chung-Lu, 1 M vertices: 120 ms of peel with one
+// range a warp, 104 ms).
+constexpr int kLeanSearch = 8;
 
 // Records item idx, slots [c, c + dx), in the slot index of its round.
 __device__ __forceinline__ void index_item(int32_t* sidx, long long idx, long long c, long long dx) {
@@ -317,7 +318,7 @@ __device__ __forceinline__ void append_flush(const PeelArgs& A, int slot, int bu
                     if (idx < A.E) {
                         A.qi[buf][idx] = it[k];
                         A.qb[buf][idx] = cc;
-                        if (Listed) index_item(A.sidx[slot & 1], idx, cc, dx[k]);
+                        index_item(A.sidx[slot & 1], idx, cc, dx[k]);
                     }
                     idx++;
                     cc += dx[k];
@@ -385,6 +386,7 @@ __device__ __forceinline__ void warp_append2_direct(const PeelArgs& A, int slot,
         if (idx < A.E) {
             A.qi[buf][idx] = itf;
             A.qb[buf][idx] = cc;
+            index_item(A.sidx[slot & 1], idx, cc, dxf);
         }
         idx++;
         cc += dxf;
@@ -392,6 +394,7 @@ __device__ __forceinline__ void warp_append2_direct(const PeelArgs& A, int slot,
     if (qg && idx < A.E) {
         A.qi[buf][idx] = itg;
         A.qb[buf][idx] = cc;
+        index_item(A.sidx[slot & 1], idx, cc, dxg);
     }
 }
 
@@ -463,26 +466,6 @@ static_assert(kDynChunk % 64 == 0, "dynamic ranges are whole 64-slot steps");
 #define TDT_SKIP_MARKED 1
 #endif
 constexpr bool kSkipMarked = TDT_SKIP_MARKED != 0;
-// The 1-bit dead-edge filter before the edge-state loads of a slot.
-#ifndef TDT_DEAD_FILTER
-#define TDT_DEAD_FILTER 1
-#endif
-constexpr bool kDeadFilter = TDT_DEAD_FILTER != 0;
-
-// The decrement results of a peel step are used one step later, after the
-// next step's loads are in flight (0: used at once).
-#ifndef TDT_PEEL_DEFER
-#define TDT_PEEL_DEFER 1
-#endif
-constexpr bool kPeelDefer = TDT_PEEL_DEFER != 0;
-
-// The listed peel reads its partners' round codes instead of the dead bits
-// and the edge states (0: dead bits, then edge states).
-#ifndef TDT_PEEL_CODES
-#define TDT_PEEL_CODES 1
-#endif
-constexpr bool kPeelCodes = TDT_PEEL_CODES != 0;
-
 #ifndef TDT_PEEL_STEP
 #define TDT_PEEL_STEP 8
 #endif
@@ -680,7 +663,7 @@ __device__ __forceinline__ void warp_append_capped(const PeelArgs& A, bool liste
         if (idx < A.E) {
             A.qi[buf][idx] = it;
             A.qb[buf][idx] = (long long)(old & kCandMask) + incl - c;
-            if (listed) index_item(A.sidx[slot & 1], idx, (long long)(old & kCandMask) + incl - c, dx);
+            index_item(A.sidx[slot & 1], idx, (long long)(old & kCandMask) + incl - c, dx);
         }
     }
 }
@@ -786,52 +769,92 @@ __device__ __forceinline__ void window_items(const long long* __restrict__ qb, c
     nst = w.nsn;
 }
 
-// The other two edges (f, g) of slot tl of item it; false when the slot is
-// not a triangle (search mode only).
-template <bool Listed>
-__device__ __forceinline__ bool slot_edges(const PeelArgs& A, const int4& it, long long tl, int r, int32_t& f,
-                                           int32_t& g) {
-    if (Listed) {
-        const long long lo = (long long)(unsigned)it.y | ((long long)it.z << 32);
-        const int2 fg = __ldg(A.lists + lo + tl);
-        f = fg.x;
-        g = fg.y;
-        return true;
+// Search mode: the other two edges (f, g) of slot tl[h] of item it[h] and their
+// sub-round stamps, for the kWin windows of a step; tr[h] (in: the slot exists)
+// turns false when the slot is no triangle or needs no decrement from here.
+// A slot is a chain of loads, most of them the binary search for the third
+// edge, so the windows go through each stage together: their searches run in
+// step, kWin loads in flight instead of one.
+#ifndef TDT_PEEL_WIN
+#define TDT_PEEL_WIN 2
+#endif
+constexpr int kWin = TDT_PEEL_WIN;  // 32-slot windows per peel step
+
+__device__ __forceinline__ void search_slots(const PeelArgs& A, const int4 (&it)[kWin], const int (&tl)[kWin], int r,
+                                             bool (&tr)[kWin], int32_t (&f)[kWin], int32_t (&g)[kWin],
+                                             int32_t (&rf)[kWin], int32_t (&rg)[kWin]) {
+    int32_t w[kWin];
+#pragma unroll
+    for (int h = 0; h < kWin; h++) {
+        w[h] = f[h] = g[h] = 0;
+        rf[h] = rg[h] = -2;
+        if (tr[h]) {
+            if (tl[h] < it[h].w) {
+                f[h] = (int32_t)(__ldg(A.rp + it[h].y) + tl[h]);
+                w[h] = __ldg(A.cols + f[h]);
+            } else {
+                const int64_t kk = __ldg(A.cp + it[h].y) + (tl[h] - it[h].w);
+                w[h] = __ldg(A.in_src + kk);
+                f[h] = __ldg(A.in_eid + kk);
+            }
+            tr[h] = w[h] != it[h].z;
+        }
     }
-    const int32_t x = it.y, y = it.z, dxo = it.w;
-    int32_t w;
-    if (tl < dxo) {
-        f = (int32_t)(__ldg(A.rp + x) + tl);
-        w = __ldg(A.cols + f);
-    } else {
-        const int64_t kk = __ldg(A.cp + x) + (tl - dxo);
-        w = __ldg(A.in_src + kk);
-        f = __ldg(A.in_eid + kk);
-    }
-    if (w == y) return false;
-    if (kPeelCodes) {
+    unsigned x[kWin];
+#pragma unroll
+    for (int h = 0; h < kWin; h++) x[h] = tr[h] ? __ldcg(A.code + (f[h] >> 3)) : 0u;
+    int64_t b[kWin];
+    int n[kWin];
+    int32_t key[kWin];
+    bool any = false;
+#pragma unroll
+    for (int h = 0; h < kWin; h++) {
+        b[h] = 0;
+        n[h] = 0;
+        key[h] = 0;
         // no search when (x,w) was peeled before this round, or peels in it
         // too with the smaller index: then the other edge of the triangle is
         // decremented from (x,w)'s own slot, not from this one
-        const int32_t cf = code_round(__ldcg(A.code + (f >> 3)), f, r);
-        if (cf == -2 || (cf == r && it.x > f)) return false;
-    } else if (kDeadFilter && ((A.dead[f >> 5] >> (f & 31)) & 1u)) {
-        return false;  // (x,w) peeled before this round
+        rf[h] = tr[h] ? code_round(x[h], f[h], r) : -2;
+        tr[h] = tr[h] && rf[h] != -2 && !(rf[h] == r && it[h].x > f[h]);
+        if (tr[h]) {
+            const int32_t y = it[h].z, src = w[h] < y ? w[h] : y;
+            key[h] = w[h] < y ? y : w[h];
+            b[h] = __ldg(A.rp + src);
+            n[h] = (int)(__ldg(A.rp + src + 1) - b[h]);
+        }
+        tr[h] = n[h] > 0;
+        any |= n[h] > 1;
     }
-    const int64_t gg = (w < y) ? find_sorted<int64_t>(A.cols, __ldg(A.rp + w), __ldg(A.rp + w + 1), y)
-                               : find_sorted<int64_t>(A.cols, __ldg(A.rp + y), __ldg(A.rp + y + 1), w);
-    g = (int32_t)gg;
-    return gg >= 0;
+    // the last entry <= key of each list, in step
+    while (any) {
+        any = false;
+        int32_t c[kWin];
+#pragma unroll
+        for (int h = 0; h < kWin; h++) c[h] = n[h] > 1 ? __ldg(A.cols + b[h] + (n[h] >> 1)) : INT32_MAX;
+#pragma unroll
+        for (int h = 0; h < kWin; h++) {
+            const int half = n[h] >> 1;
+            if (c[h] <= key[h]) b[h] += half;
+            n[h] -= half;
+            any |= n[h] > 1;
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < kWin; h++) tr[h] = tr[h] && __ldg(A.cols + b[h]) == key[h];
+#pragma unroll
+    for (int h = 0; h < kWin; h++) {
+        g[h] = (int32_t)b[h];
+        x[h] = tr[h] ? __ldcg(A.code + (g[h] >> 3)) : 0u;
+    }
+#pragma unroll
+    for (int h = 0; h < kWin; h++) rg[h] = tr[h] ? code_round(x[h], g[h], r) : -2;
 }
 
 // The decrements of one peel step: the four edges and the supports before
 // their decrements (INT32_MIN: no decrement).  An edge whose support fell to
 // l is marked for sub-round r+1 and queued; a larger result lowers the bound
 // dm of the next level.
-#ifndef TDT_PEEL_WIN
-#define TDT_PEEL_WIN 2
-#endif
-constexpr int kWin = TDT_PEEL_WIN;  // 32-slot windows per peel step
 struct Pending {
     int32_t e[2 * kWin];
     int32_t o[2 * kWin];
@@ -873,6 +896,7 @@ __device__ __forceinline__ void settle(const PeelArgs& A, const Pending& P, int 
 // window starts, records, list entry, codes, decrement.  With the counters
 // handed over by the barrier, peel of R-MAT scale 12 / 16 / 20 / 22: 2.58 /
 // 9.70 / 40.3 / 116.6 -> 1.72 / 7.32 / 33.6 / 104.2 ms.
+template <bool Listed>
 __device__ __forceinline__ void lean_round(const PeelArgs& A, int r, int32_t l, int N, int T, int gwarp, int nwarps,
                                            int32_t* ebuf, int* s_dmin) {
     if (gwarp * kWarp >= T) return;
@@ -882,52 +906,90 @@ __device__ __forceinline__ void lean_round(const PeelArgs& A, int r, int32_t l, 
     const unsigned cm = l > 0 ? ((unsigned)(r + 1) & 3u) : kCodeDead;
     int32_t dm = INT32_MAX;
     AppendBuf B{ebuf, 0, 0ull};
-    for (int cb = gwarp * kWarp; cb < T; cb += nwarps * kWarp) {
-        const int i0 = __ldcg(A.sidx[r & 1] + (cb >> 5));
-        int4 it = make_int4(0, 0, 0, 0);
-        int S = INT32_MAX;  // first slot of item i0 + lane
-        if (i0 + (int)lane < N) {
-            it = __ldcg(A.qi[buf] + i0 + lane);
-            S = (int)__ldcg(A.qb[buf] + i0 + lane);
+    constexpr int kL = Listed ? 1 : kWin;  // windows in flight
+    for (int cb0 = gwarp * kWarp; cb0 < T; cb0 += kL * nwarps * kWarp) {
+        int i0[kL];
+#pragma unroll
+        for (int h = 0; h < kL; h++) {
+            const int cb = cb0 + h * nwarps * kWarp;
+            i0[h] = cb < T ? __ldcg(A.sidx[r & 1] + (cb >> 5)) : N;
         }
-        const unsigned d = (unsigned)(S - cb);
-        const unsigned mk = __reduce_or_sync(kFull, lane > 0 && d < (unsigned)kWarp ? 1u << d : 0u);
-        const int k = __popc(mk & le);
-        const int t = cb + (int)lane - __shfl_sync(kFull, S, k);
-        const int32_t e = __shfl_sync(kFull, it.x, k);
-        const long long o =
-            (long long)(unsigned)__shfl_sync(kFull, it.y, k) | ((long long)__shfl_sync(kFull, it.z, k) << 32);
-        const bool v = cb + (int)lane < T;
-        int2 fg = make_int2(0, 0);
-        if (v) fg = __ldg(A.lists + o + t);
-        unsigned xf = 0, xg = 0;
-        if (v) {
-            xf = __ldcg(A.code + (fg.x >> 3));
-            xg = __ldcg(A.code + (fg.y >> 3));
+        int4 it[kL];
+        int S[kL];  // first slot of item i0 + lane
+#pragma unroll
+        for (int h = 0; h < kL; h++) {
+            it[h] = make_int4(0, 0, 0, 0);
+            S[h] = INT32_MAX;
+            if (i0[h] + (int)lane < N) {
+                it[h] = __ldcg(A.qi[buf] + i0[h] + lane);
+                S[h] = (int)__ldcg(A.qb[buf] + i0[h] + lane);
+            }
+        }
+        int tl[kL];
+        bool v[kL];
+#pragma unroll
+        for (int h = 0; h < kL; h++) {
+            const int cb = cb0 + h * nwarps * kWarp;
+            const unsigned d = (unsigned)(S[h] - cb);
+            const unsigned mk = __reduce_or_sync(kFull, lane > 0 && d < (unsigned)kWarp ? 1u << d : 0u);
+            const int k = __popc(mk & le);
+            v[h] = cb + (int)lane < T;
+            tl[h] = cb + (int)lane - __shfl_sync(kFull, S[h], k);
+            it[h].x = __shfl_sync(kFull, it[h].x, k);
+            it[h].y = __shfl_sync(kFull, it[h].y, k);
+            it[h].z = __shfl_sync(kFull, it[h].z, k);
+            if (!Listed) it[h].w = __shfl_sync(kFull, it[h].w, k);
+        }
+        int32_t f[kL], g[kL], rf[kL], rg[kL];
+        if constexpr (Listed) {
+            int2 fg = make_int2(0, 0);
+            if (v[0]) fg = __ldg(A.lists + ((long long)(unsigned)it[0].y | ((long long)it[0].z << 32)) + tl[0]);
+            f[0] = fg.x;
+            g[0] = fg.y;
+            unsigned xf = 0, xg = 0;
+            if (v[0]) {
+                xf = __ldcg(A.code + (fg.x >> 3));
+                xg = __ldcg(A.code + (fg.y >> 3));
+            }
+            rf[0] = v[0] ? code_round(xf, fg.x, r) : -2;
+            rg[0] = v[0] ? code_round(xg, fg.y, r) : -2;
+        } else {
+            search_slots(A, it, tl, r, v, f, g, rf, rg);
+#pragma unroll
+            for (int h = 0; h < kL; h++)
+                if (!v[h]) rf[h] = -2;
         }
         // the ownership rules of process_round
-        const int32_t rf = code_round(xf, fg.x, r), rg = code_round(xg, fg.y, r);
-        const bool on = v && rf != -2 && rg != -2;
-        const bool cf = rf == r, cg = rg == r;
-        int32_t of = INT32_MIN, og = INT32_MIN;
-        if (on && !cf && (!cg || e < fg.y) && (!kSkipMarked || rf != r + 1)) of = atomicSub(A.live + fg.x, 1);
-        if (on && !cg && (!cf || e < fg.x) && (!kSkipMarked || rg != r + 1)) og = atomicSub(A.live + fg.y, 1);
-        if (of > l + 1 && of - 1 < dm) dm = of - 1;
-        if (og > l + 1 && og - 1 < dm) dm = og - 1;
-        const bool wf = of == l + 1, wg = og == l + 1;
-        if (wf) {
-            A.rnd[fg.x] = r + 1;
-            code_mark(A.code, fg.x, cm);
+        int32_t of[kL], og[kL];
+#pragma unroll
+        for (int h = 0; h < kL; h++) {
+            const bool on = rf[h] != -2 && rg[h] != -2;
+            const bool cf = rf[h] == r, cg = rg[h] == r;
+            of[h] = og[h] = INT32_MIN;
+            if (on && !cf && (!cg || it[h].x < g[h]) && (!kSkipMarked || rf[h] != r + 1))
+                of[h] = atomicSub(A.live + f[h], 1);
+            if (on && !cg && (!cf || it[h].x < f[h]) && (!kSkipMarked || rg[h] != r + 1))
+                og[h] = atomicSub(A.live + g[h], 1);
         }
-        if (wg) {
-            A.rnd[fg.y] = r + 1;
-            code_mark(A.code, fg.y, cm);
+#pragma unroll
+        for (int h = 0; h < kL; h++) {
+            if (of[h] > l + 1 && of[h] - 1 < dm) dm = of[h] - 1;
+            if (og[h] > l + 1 && og[h] - 1 < dm) dm = og[h] - 1;
+            const bool wf = of[h] == l + 1, wg = og[h] == l + 1;
+            if (wf) {
+                A.rnd[f[h]] = r + 1;
+                code_mark(A.code, f[h], cm);
+            }
+            if (wg) {
+                A.rnd[g[h]] = r + 1;
+                code_mark(A.code, g[h], cm);
+            }
+            warp_append2_staged<Listed>(A, nslot, nbuf, wf, f[h], wg, g[h], l, B, &A.ctl->fe[nslot]);
         }
-        warp_append2_staged<true>(A, nslot, nbuf, wf, fg.x, wg, fg.y, l, B, &A.ctl->fe[nslot]);
     }
     dm = warp_min(dm);
     if (lane == 0 && dm != INT32_MAX) atomicMin(s_dmin, dm);
-    append_flush<true>(A, nslot, nbuf, B, &A.ctl->fe[nslot]);
+    append_flush<Listed>(A, nslot, nbuf, B, &A.ctl->fe[nslot]);
 }
 
 // One sub-round: warps gwarp = 0..nwarps-1 share the candidate slots of round r.
@@ -954,18 +1016,16 @@ __device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t 
     const int4* __restrict__ qi = A.qi[buf];
     // the edges of round r-1 are dead from this round on: their round codes
     // turn dead (needed by round r+2, where (r-1) & 3 would read "marked for
-    // the next round"), or, without the codes, their dead bits are set (a bit
-    // read before it is set only sends that triangle to the state check)
-    if ((kPeelCodes || kDeadFilter) && r > 0) {
+    // the next round")
+    if (r > 0) {
         const int4* __restrict__ qp = A.qi[(r - 1) % 3];
         for (long long i = gwarp * kWarp + lane; i < nprev; i += nwarps * kWarp) {
             const int32_t e = __ldcg(&qp[i].x);
-            if (kPeelCodes) atomicOr(A.code + (e >> 3), kCodeDead << ((unsigned)(e & 7) * 4u));
-            else atomicOr(A.dead + (e >> 5), 1u << (e & 31));
+            atomicOr(A.code + (e >> 3), kCodeDead << ((unsigned)(e & 7) * 4u));
         }
     }
-    if (Listed && T <= nwarps * kWarp * kLeanWindows && T <= (long long)kSlotIdx * kWarp) {
-        lean_round(A, r, l, (int)N, (int)T, (int)gwarp, (int)nwarps, app_e + wib * kAppBuf, s_dmin);
+    if (T <= nwarps * kWarp * (Listed ? kLeanWindows : kLeanSearch) && T <= (long long)kSlotIdx * kWarp) {
+        lean_round<Listed>(A, r, l, (int)N, (int)T, (int)gwarp, (int)nwarps, app_e + wib * kAppBuf, s_dmin);
         return;
     }
     // listed mode: each warp owns a contiguous range of candidate slots (a
@@ -1024,21 +1084,26 @@ __device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t 
             v[h] = cbh + lane < cb1;
             if (cbh < cb1) window_items(qb, qi, N, cbh, v[h], le, i0, base0, nst, rec, rv, it[h], bl[h]);
         }
-        int32_t f[kWin], g[kWin];
+        int32_t f[kWin], g[kWin], rf[kWin], rg[kWin];
         bool tr[kWin];
-#pragma unroll
-        for (int h = 0; h < kWin; h++) {
-            f[h] = 0;
-            g[h] = 0;
-            tr[h] = false;
-            if (v[h]) tr[h] = slot_edges<Listed>(A, it[h], cb + h * kWarp + lane - bl[h], r, f[h], g[h]);
-        }
-        int32_t rf[kWin], rg[kWin];
-#pragma unroll
-        for (int h = 0; h < kWin; h++) rf[h] = rg[h] = -2;
-        if (kPeelCodes) {
-            // the partners' round codes (L2): dead, alive, peeling now, marked
+        if (Listed) {
+            // list entry, then the partners' round codes (L2): dead, alive,
+            // peeling now, marked
             unsigned x[kWin], y[kWin];
+#pragma unroll
+            for (int h = 0; h < kWin; h++) {
+                f[h] = g[h] = 0;
+                tr[h] = false;
+                if (v[h]) {
+                    const long long lo = (long long)(unsigned)it[h].y | ((long long)it[h].z << 32);
+                    const int2 fg = __ldg(A.lists + lo + (cb + h * kWarp + lane - bl[h]));
+                    f[h] = fg.x;
+                    g[h] = fg.y;
+                    tr[h] = true;
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < kWin; h++) rf[h] = rg[h] = -2;
 #pragma unroll
             for (int h = 0; h < kWin; h++) {
                 x[h] = y[h] = 0;
@@ -1048,7 +1113,7 @@ __device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t 
                 }
             }
             // the previous step's decrement results, while these loads are in flight
-            if (kPeelDefer) settle<Listed>(A, P, r, l, nslot, nbuf, B, dm);
+            settle<Listed>(A, P, r, l, nslot, nbuf, B, dm);
 #pragma unroll
             for (int h = 0; h < kWin; h++) {
                 if (tr[h]) {
@@ -1057,30 +1122,14 @@ __device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t 
                 }
             }
         } else {
-            // dead-bit filter: a triangle with an edge peeled before round r is gone
-            if (kDeadFilter) {
-                unsigned x[kWin], y[kWin];
-#pragma unroll
-                for (int h = 0; h < kWin; h++) {
-                    x[h] = y[h] = 0;
-                    if (tr[h]) {
-                        x[h] = A.dead[f[h] >> 5];
-                        y[h] = A.dead[g[h] >> 5];
-                    }
-                }
-#pragma unroll
-                for (int h = 0; h < kWin; h++)
-                    if (tr[h] && (((x[h] >> (f[h] & 31)) | (y[h] >> (g[h] & 31))) & 1u)) tr[h] = false;
-            }
+            int tl[kWin];
 #pragma unroll
             for (int h = 0; h < kWin; h++) {
-                if (tr[h]) {
-                    rf[h] = __ldcg(A.rnd + f[h]);
-                    rg[h] = __ldcg(A.rnd + g[h]);
-                }
+                tl[h] = (int)(cb + h * kWarp + lane - bl[h]);
+                tr[h] = v[h];
             }
-            // the previous step's decrement results, while these loads are in flight
-            if (kPeelDefer) settle<Listed>(A, P, r, l, nslot, nbuf, B, dm);
+            search_slots(A, it, tl, r, tr, f, g, rf, rg);
+            settle<Listed>(A, P, r, l, nslot, nbuf, B, dm);
         }
         // a triangle is alive when both other edges are alive or peel in r or r+1;
         // which of f, g this lane decrements: the ownership rules above
@@ -1105,15 +1154,10 @@ __device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t 
             P.o[2 * h] = df[h] ? atomicSub(A.live + f[h], 1) : INT32_MIN;
             P.o[2 * h + 1] = dg[h] ? atomicSub(A.live + g[h], 1) : INT32_MIN;
         }
-        if (!kPeelDefer) {
-            settle<Listed>(A, P, r, l, nslot, nbuf, B, dm);
-#pragma unroll
-            for (int j = 0; j < 2 * kWin; j++) P.o[j] = INT32_MIN;
-        }
     }
     if (!dyn) break;
     }
-    if (kPeelDefer) settle<Listed>(A, P, r, l, nslot, nbuf, B, dm);
+    settle<Listed>(A, P, r, l, nslot, nbuf, B, dm);
     if (Listed) append_flush<Listed>(A, nslot, nbuf, B, &A.ctl->fe[nslot]);
     dm = warp_min(dm);
     if (lane == 0 && dm != INT32_MAX) atomicMin(s_dmin, dm);
@@ -1123,11 +1167,15 @@ __device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t 
 #define TDT_PEEL_MINB 2
 #endif
 // A is a __grid_constant__ parameter: the helpers take it by reference and
-// read its fields from the parameter bank instead of a local copy.
+// read its fields from the parameter bank instead of a local copy.  Lists:
+// the caller gave a list tail, and whether the lists fit is decided on the
+// device; without a tail the search peel has a kernel, and its registers, of
+// its own (Chung-Lu, 1 M vertices: 121 -> 104 ms).
+template <bool Lists>
 __global__ void __launch_bounds__(kPeelBlock, TDT_PEEL_MINB) peel_kernel(const __grid_constant__ PeelArgs A) {
     __shared__ int32_t s_app_e[kPeelWarps * kAppBuf];  // per-warp append staging
     __shared__ RoundShared s_round;
-    const bool listed = A.lists != nullptr && *(volatile int*)&A.ctl->listed != 0;
+    const bool listed = Lists && *(volatile int*)&A.ctl->listed != 0;
     const int wib = threadIdx.x / kWarp;
     const int64_t gwarp = (int64_t)blockIdx.x * kPeelWarps + wib;
     const int64_t nwarps = (int64_t)gridDim.x * kPeelWarps;
@@ -1499,7 +1547,6 @@ struct Layout {
     int64_t* sbase;
     int32_t* sidx;
     int32_t* alive[2];
-    unsigned* dead;
     unsigned* code;
     void* scan_ws;
     void* sort_ws;
@@ -1530,7 +1577,6 @@ Layout carve(void* ws, int64_t V, int64_t E) {
     L.sidx = (int32_t*)c.take(8 * (size_t)kSlotIdx);
     L.alive[0] = (int32_t*)c.take(4 * e);
     L.alive[1] = (int32_t*)c.take(4 * e);
-    L.dead = (unsigned*)c.take(4 * (e / 32 + 1));
     L.code = (unsigned*)c.take(4 * (e / 8 + 1));
     size_t scan_b = scan_scratch_bytes((int64_t)(e > v ? e : v) + 1);
     L.scan_ws = c.take(scan_b);
@@ -1649,12 +1695,6 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     prof_mark(2, st);
 
     // persistent peel
-    int occ = 0;
-    TDT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, peel_kernel, kPeelBlock, 0));
-    if (occ < 1) {
-        set_error("peel kernel cannot be resident");
-        return TDT_ERR_UNSUPPORTED;
-    }
     PeelArgs A;
     A.rp = rp; A.cols = cols; A.rows = rows_use; A.cp = L.cp; A.in_src = L.in_src; A.in_eid = L.in_eid;
     A.live = L.live; A.rnd = L.rnd; A.round_level = L.round_level;
@@ -1662,8 +1702,6 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
         A.qi[b] = L.qi[b];
         A.qb[b] = L.qb[b];
     }
-    A.dead = L.dead;
-    TDT_CUDA(cudaMemsetAsync(L.dead, 0, 4 * (size_t)(E / 32 + 1), st));
     A.code = L.code;
     TDT_CUDA(cudaMemsetAsync(L.code, 0xff, 4 * (size_t)(E / 8 + 1), st));
     A.off = L.off; A.lists = lists;
@@ -1679,21 +1717,27 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     A.fixed_cand_cap = g_fixed_cand_cap > 0 && (unsigned long long)g_fixed_cand_cap < kFixedCandCap
                            ? (unsigned long long)g_fixed_cand_cap : kFixedCandCap;
     A.ctl = L.ctl;
-    if (di.sms * occ > 4096) occ = 4096 / di.sms;
     // Small graphs peel their lists on one block per SM: their sub-rounds fit
     // one window a warp there, and a grid barrier of fewer blocks is shorter.
     // 76 / 152 / 304 blocks: R-MAT scale 12 1.77 / 1.80 / 1.92 ms, scale 14
     // 4.42 / 4.36 / 4.64, scale 16 (0.9 M edges) 8.43 / 7.53 / 7.52, scale 18
     // 18.2 / 14.0 / 13.3, scale 20 61.4 / 40.2 / 34.1; Chung-Lu (1.5 M edges)
-    // 10.6 / 9.6 / 9.8.  The search peel (no list tail) keeps every block: its
-    // slots are binary searches.
+    // 10.6 / 9.6 / 9.8.  The search peel keeps every block: its slots are
+    // binary searches.
+    void* kern = tail > 0 ? (void*)peel_kernel<true> : (void*)peel_kernel<false>;
+    int occ = 0;
+    TDT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kPeelBlock, 0));
+    if (occ < 1) {
+        set_error("peel kernel cannot be resident");
+        return TDT_ERR_UNSUPPORTED;
+    }
+    if (di.sms * occ > 4096) occ = 4096 / di.sms;
     int nblk = di.sms * occ;
     if (tail > 0 && E < (1ll << 20)) nblk = di.sms;
     if (g_peel_half_sms > 0) nblk = (g_peel_half_sms * di.sms + 1) / 2;
     if (nblk > di.sms * occ) nblk = di.sms * occ;
-    dim3 grid(nblk), block(kPeelBlock);
     void* args[] = {&A};
-    TDT_CUDA(cudaLaunchCooperativeKernel((void*)peel_kernel, grid, block, args, 0, st));
+    TDT_CUDA(cudaLaunchCooperativeKernel(kern, dim3(nblk), dim3(kPeelBlock), args, 0, st));
     note_launch();
     prof_mark(3, st);
 
