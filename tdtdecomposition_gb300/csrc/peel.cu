@@ -74,13 +74,20 @@ struct PeelCtl {
     unsigned long long grab[4];    // slot cursor of search-mode sub-round r, at r & 3
 };
 
+// How the peel finds an edge's triangles: in its list, by search in the graph's
+// adjacency, or by search in an adjacency that is compacted as edges die.
+enum PeelMode { kListed = 0, kSearch = 1, kCompact = 2 };
+// The compacted adjacency: still the graph's own; compacted, with items queued
+// before that; compacted.
+enum CompactState { kWhole = 0, kStale = 1, kFresh = 2 };
+
 struct PeelArgs {
     const int64_t* rp;
     const int32_t* cols;
     const int32_t* rows;
     const int64_t* cp;
-    const int32_t* in_src;
-    const int32_t* in_eid;
+    int32_t* in_src;
+    int32_t* in_eid;
     int32_t* live;        // support of each edge, decremented as its triangles are destroyed
     int32_t* rnd;         // sub-round that peeled each edge (-1: alive)
     int32_t* round_level;
@@ -91,6 +98,13 @@ struct PeelArgs {
     int32_t* alive[2];    // compacted alive-edge lists (level transitions)
     // round r at r & 1: the item that holds slot 32 j, for j < kSlotIdx
     int32_t* sidx[2];
+    // compacted adjacency (see compact_rows): row u's out-edges at rp[u] of
+    // out_col / out_eid, its in-edges at cp[u] of in_src / in_eid, as many as its
+    // lengths say
+    int32_t* out_col;
+    int32_t* out_eid;
+    int32_t* out_len;
+    int32_t* in_len;
     // round code of edge e in the 4 bits at (e & 7) * 4 of word e >> 3 (the
     // listed peel's partner-state check; see code_round)
     unsigned* code;
@@ -102,6 +116,7 @@ struct PeelArgs {
     unsigned long long deadline_ns;  // wall-clock budget of the launch
     unsigned long long fixed_item_cap, fixed_cand_cap;  // k-truss collection batch limits
     long long dyn_min_slots;      // search mode: sub-rounds of at least this many slots take dynamic ranges
+    int search_next;      // a search kernel follows the one that may find no lists
     PeelCtl* ctl;
 };
 
@@ -116,7 +131,7 @@ __device__ __forceinline__ void set_status(PeelCtl* c, int s) {
 // block through shared memory, so no warp pays a load for them.
 struct RoundBar {
     unsigned long long target;   // arrivals that complete the next barrier
-    unsigned long long q, fe;    // after wait(): counters of the round asked for
+    unsigned long long q, fe;    // counters of the round asked for (fe after a level change: edges it queued)
 };
 
 struct RoundShared {
@@ -204,13 +219,13 @@ __device__ __forceinline__ int32_t code_round(unsigned word, int32_t e, int r) {
 // Queue item of edge e (listed: e's list offset and length; search: the
 // lower-degree endpoint x, the other endpoint y, x's out-degree dxo and the
 // candidate count dx).  Returns false when e has nothing to enumerate.
-template <bool Listed>
+template <int Mode>
 __device__ __forceinline__ bool make_item(const PeelArgs& A, bool want, int32_t cur_sup, int32_t e, int4& it,
                                           long long& dx) {
     it = make_int4(e, 0, 0, 0);
     dx = 0;
     if (!want || cur_sup <= 0) return false;
-    if (Listed) {
+    if (Mode == kListed) {
         // the edge's original triangles; the item carries the list offset
         const long long o = __ldg(A.off + e);
         dx = __ldg(A.off + e + 1) - o;
@@ -219,6 +234,15 @@ __device__ __forceinline__ bool make_item(const PeelArgs& A, bool want, int32_t 
         return dx > 0;
     }
     const int32_t u = __ldg(A.rows + e), v = __ldg(A.cols + e);
+    if (Mode == kCompact) {
+        const int32_t uo = __ldcg(A.out_len + u), vo = __ldcg(A.out_len + v);
+        const int32_t du = uo + __ldcg(A.in_len + u), dv = vo + __ldcg(A.in_len + v);
+        it.y = du <= dv ? u : v;
+        it.z = du <= dv ? v : u;
+        it.w = du <= dv ? uo : vo;
+        dx = du <= dv ? du : dv;
+        return dx > 1;
+    }
     const long long duo = __ldg(A.rp + u + 1) - __ldg(A.rp + u);
     const long long du = duo + __ldg(A.cp + u + 1) - __ldg(A.cp + u);
     const long long dvo = __ldg(A.rp + v + 1) - __ldg(A.rp + v);
@@ -279,7 +303,7 @@ struct AppendBuf {
 
 // Queue the staged edges: their items are built here (kAppBuf / 32 per lane),
 // reserved with one atomic and written.
-template <bool Listed>
+template <int Mode>
 __device__ __forceinline__ void append_flush(const PeelArgs& A, int slot, int buf, AppendBuf& B,
                                              unsigned long long* nfront) {
     const unsigned lane = lane_id();
@@ -298,7 +322,7 @@ __device__ __forceinline__ void append_flush(const PeelArgs& A, int slot, int bu
 #pragma unroll
         for (int k = 0; k < kPer; k++) {
             const int i = (int)lane * kPer + k;
-            q[k] = i < B.n && make_item<Listed>(A, true, 1, B.e[i], it[k], dx[k]);
+            q[k] = i < B.n && make_item<Mode>(A, true, 1, B.e[i], it[k], dx[k]);
             if (q[k]) {
                 nq++;
                 sum += dx[k];
@@ -331,15 +355,15 @@ __device__ __forceinline__ void append_flush(const PeelArgs& A, int slot, int bu
 }
 
 // The same as a call (the level-change passes: several call sites, rare flushes).
-template <bool Listed>
+template <int Mode>
 __device__ __noinline__ void append_flush_call(const PeelArgs& A, int slot, int buf, AppendBuf& B,
                                                unsigned long long* nfront) {
-    append_flush<Listed>(A, slot, buf, B, nfront);
+    append_flush<Mode>(A, slot, buf, B, nfront);
 }
 
 // Stage up to two edges per lane (f, g of one triangle) for the round in
 // `slot`; cur_sup (the level, warp-uniform) <= 0 queues no item.
-template <bool Listed>
+template <int Mode>
 __device__ __forceinline__ void warp_append2_staged(const PeelArgs& A, int slot, int buf, bool wf, int32_t f,
                                                     bool wg, int32_t g, int32_t cur_sup, AppendBuf& B,
                                                     unsigned long long* nfront) {
@@ -350,7 +374,7 @@ __device__ __forceinline__ void warp_append2_staged(const PeelArgs& A, int slot,
     const int nq = (wf ? 1 : 0) + (wg ? 1 : 0);
     const int nincl = warp_incl_scan(nq);
     const int ntot = __shfl_sync(kFull, nincl, 31);
-    if (B.n + ntot > kAppBuf) append_flush<Listed>(A, slot, buf, B, nfront);
+    if (B.n + ntot > kAppBuf) append_flush<Mode>(A, slot, buf, B, nfront);
     int p = B.n + nincl - nq;
     if (wf) B.e[p++] = f;
     if (wg) B.e[p] = g;
@@ -360,7 +384,7 @@ __device__ __forceinline__ void warp_append2_staged(const PeelArgs& A, int slot,
 // Queue up to two edges per lane directly, with one reservation per warp step
 // (the search-mode sub-rounds: their steps are long and append rarely, and the
 // staging state would stay live across the binary searches).
-template <bool Listed>
+template <int Mode>
 __device__ __forceinline__ void warp_append2_direct(const PeelArgs& A, int slot, int buf, bool wf, int32_t f,
                                                     bool wg, int32_t g, int32_t cur_sup,
                                                     unsigned long long* nfront) {
@@ -370,8 +394,8 @@ __device__ __forceinline__ void warp_append2_direct(const PeelArgs& A, int slot,
     if (lane == 0) atomicAdd(nfront, (unsigned long long)(__popc(mf) + __popc(mg)));
     int4 itf, itg;
     long long dxf, dxg;
-    const bool qf = make_item<Listed>(A, wf, cur_sup, f, itf, dxf);
-    const bool qg = make_item<Listed>(A, wg, cur_sup, g, itg, dxg);
+    const bool qf = make_item<Mode>(A, wf, cur_sup, f, itf, dxf);
+    const bool qg = make_item<Mode>(A, wg, cur_sup, g, itg, dxg);
     const int nq = (qf ? 1 : 0) + (qg ? 1 : 0);
     if (__ballot_sync(kFull, nq > 0) == 0) return;
     const long long c = (qf ? dxf : 0) + (qg ? dxg : 0);
@@ -400,6 +424,7 @@ __device__ __forceinline__ void warp_append2_direct(const PeelArgs& A, int slot,
 
 // Stage the edges flagged by `want` (one per lane) for the round in `slot`.
 // cur_sup is the edge's support at marking time (0 => no alive triangle).
+template <int Search>
 __device__ __forceinline__ void warp_append_staged(const PeelArgs& A, bool listed, int slot, int buf, bool want,
                                                    int32_t e, int32_t cur_sup, AppendBuf& B,
                                                    unsigned long long* nfront) {
@@ -411,8 +436,8 @@ __device__ __forceinline__ void warp_append_staged(const PeelArgs& A, bool liste
     if (m == 0) return;
     const int ntot = __popc(m);
     if (B.n + ntot > kAppBuf) {
-        if (listed) append_flush_call<true>(A, slot, buf, B, nfront);
-        else append_flush_call<false>(A, slot, buf, B, nfront);
+        if (listed) append_flush_call<kListed>(A, slot, buf, B, nfront);
+        else append_flush_call<Search>(A, slot, buf, B, nfront);
     }
     if (st) B.e[B.n + __popc(m & lanemask_lt())] = e;
     B.n += ntot;
@@ -479,6 +504,8 @@ __device__ __forceinline__ void pass_start(const PeelArgs& A, int np) {
     }
 }
 
+// Search: the mode when the peel is not listed.
+template <int Search>
 __device__ __forceinline__ bool level_transition(const PeelArgs& A, bool listed, int r_next, int t, int& np,
                                               int32_t* l_out, int32_t* app_e, RoundBar& RB, RoundShared* RS) {
     const unsigned lane = lane_id();
@@ -563,17 +590,18 @@ __device__ __forceinline__ bool level_transition(const PeelArgs& A, bool listed,
                     A.rnd[e[u]] = r_next;
                     code_mark(A.code, e[u], sv[u] > 0 ? ((unsigned)r_next & 3u) : kCodeDead);
                 }
-                warp_append_staged(A, listed, slot, buf, want, e[u], sv[u], B, &A.ctl->pfe[np % 3]);
+                warp_append_staged<Search>(A, listed, slot, buf, want, e[u], sv[u], B, &A.ctl->pfe[np % 3]);
             }
             __syncthreads();  // s_tk / s_base are reused by the next tile
         }
-        if (listed) append_flush_call<true>(A, slot, buf, B, &A.ctl->pfe[np % 3]);
-        else append_flush_call<false>(A, slot, buf, B, &A.ctl->pfe[np % 3]);
+        if (listed) append_flush_call<kListed>(A, slot, buf, B, &A.ctl->pfe[np % 3]);
+        else append_flush_call<Search>(A, slot, buf, B, &A.ctl->pfe[np % 3]);
         pass_min(A, np, mloc);
     }
     np++;
     if (!round_barrier(A.ctl, RB, RS, r_next, &A.ctl->dmin[t & 1])) return false;
-    if (ld_cg_u64(&A.ctl->pfe[(np + 2) % 3]) > 0) {
+    RB.fe = ld_cg_u64(&A.ctl->pfe[(np + 2) % 3]);
+    if (RB.fe > 0) {
         *l_out = g;
         return true;
     }
@@ -598,14 +626,16 @@ __device__ __forceinline__ bool level_transition(const PeelArgs& A, bool listed,
                 A.rnd[e] = r_next;
                 code_mark(A.code, e, sv > 0 ? ((unsigned)r_next & 3u) : kCodeDead);
             }
-            warp_append_staged(A, listed, slot, buf, want, e, sv, B, &A.ctl->pfe[np % 3]);
+            warp_append_staged<Search>(A, listed, slot, buf, want, e, sv, B, &A.ctl->pfe[np % 3]);
         }
     }
-    if (listed) append_flush_call<true>(A, slot, buf, B, &A.ctl->pfe[np % 3]);
-    else append_flush_call<false>(A, slot, buf, B, &A.ctl->pfe[np % 3]);
+    if (listed) append_flush_call<kListed>(A, slot, buf, B, &A.ctl->pfe[np % 3]);
+    else append_flush_call<Search>(A, slot, buf, B, &A.ctl->pfe[np % 3]);
     pass_min(A, np, mloc);
     np++;
-    return round_barrier(A.ctl, RB, RS, r_next, &A.ctl->dmin[t & 1]);
+    if (!round_barrier(A.ctl, RB, RS, r_next, &A.ctl->dmin[t & 1])) return false;
+    RB.fe = ld_cg_u64(&A.ctl->pfe[(np + 2) % 3]);
+    return true;
 }
 
 // k-truss search (fixed level l): the frontier is every alive edge with
@@ -620,6 +650,7 @@ __device__ __forceinline__ bool level_transition(const PeelArgs& A, bool listed,
 constexpr unsigned long long kFixedItemCap = 1ull << 27;
 constexpr unsigned long long kFixedCandCap = 1ull << 35;
 
+template <int Search>
 __device__ __forceinline__ void warp_append_capped(const PeelArgs& A, bool listed, int slot, int buf, bool want,
                                                    int32_t e,
                                                    int32_t s, int r_next, unsigned long long* nfront) {
@@ -627,7 +658,7 @@ __device__ __forceinline__ void warp_append_capped(const PeelArgs& A, bool liste
     if (__ballot_sync(kFull, want) == 0) return;
     int4 it;
     long long dx;
-    const bool q = listed ? make_item<true>(A, want, s, e, it, dx) : make_item<false>(A, want, s, e, it, dx);
+    const bool q = listed ? make_item<kListed>(A, want, s, e, it, dx) : make_item<Search>(A, want, s, e, it, dx);
     const unsigned m = __ballot_sync(kFull, q);
     const long long c = q ? dx : 0;
     const long long incl = warp_incl_scan(c);
@@ -669,6 +700,7 @@ __device__ __forceinline__ void warp_append_capped(const PeelArgs& A, bool liste
 }
 
 // One collection pass for sub-round r_next; true when it took an edge.
+template <int Search>
 __device__ bool fixed_collect(const PeelArgs& A, bool listed, int32_t l, int r_next, int& np, RoundBar& RB,
                               RoundShared* RS) {
     const unsigned lane = lane_id();
@@ -685,11 +717,12 @@ __device__ bool fixed_collect(const PeelArgs& A, bool listed, int32_t l, int r_n
             s = __ldcg(A.live + e);
             want = ((cw >> ((unsigned)(e & 7) * 4u)) & 15u) == kCodeAlive && s <= l;
         }
-        warp_append_capped(A, listed, slot, buf, want, (int32_t)e, s, r_next, &A.ctl->pfe[np % 3]);
+        warp_append_capped<Search>(A, listed, slot, buf, want, (int32_t)e, s, r_next, &A.ctl->pfe[np % 3]);
     }
     np++;
     if (!round_barrier(A.ctl, RB, RS, r_next, &A.ctl->dmin[0])) return false;
-    return ld_cg_u64(&A.ctl->pfe[(np + 2) % 3]) > 0;
+    RB.fe = ld_cg_u64(&A.ctl->pfe[(np + 2) % 3]);
+    return RB.fe > 0;
 }
 
 // Item windows: slot cb lies in item i0 (first slot base0); items i0+1.. start
@@ -780,15 +813,30 @@ __device__ __forceinline__ void window_items(const long long* __restrict__ qb, c
 #endif
 constexpr int kWin = TDT_PEEL_WIN;  // 32-slot windows per peel step
 
+template <int Mode>
 __device__ __forceinline__ void search_slots(const PeelArgs& A, const int4 (&it)[kWin], const int (&tl)[kWin], int r,
-                                             bool (&tr)[kWin], int32_t (&f)[kWin], int32_t (&g)[kWin],
+                                             int cst, bool (&tr)[kWin], int32_t (&f)[kWin], int32_t (&g)[kWin],
                                              int32_t (&rf)[kWin], int32_t (&rg)[kWin]) {
+    // before the first compaction the rows are the graph's own
+    const bool whole = Mode != kCompact || cst == kWhole;
+    const int32_t* out_col = whole ? A.cols : A.out_col;
     int32_t w[kWin];
 #pragma unroll
     for (int h = 0; h < kWin; h++) {
         w[h] = f[h] = g[h] = 0;
         rf[h] = rg[h] = -2;
-        if (tr[h]) {
+        if (Mode == kCompact && tr[h]) {
+            const bool o = tl[h] < it[h].w;
+            const int i = o ? tl[h] : tl[h] - it[h].w;
+            // an item queued before the last compaction has the lengths of then
+            tr[h] = cst != kStale || i < __ldcg((o ? A.out_len : A.in_len) + it[h].y);
+            if (tr[h]) {
+                const int64_t k = __ldg((o ? A.rp : A.cp) + it[h].y) + i;
+                w[h] = __ldcg((o ? out_col : A.in_src) + k);
+                f[h] = o && whole ? (int32_t)k : __ldcg((o ? A.out_eid : A.in_eid) + k);
+                tr[h] = w[h] != it[h].z;
+            }
+        } else if (tr[h]) {
             if (tl[h] < it[h].w) {
                 f[h] = (int32_t)(__ldg(A.rp + it[h].y) + tl[h]);
                 w[h] = __ldg(A.cols + f[h]);
@@ -821,7 +869,7 @@ __device__ __forceinline__ void search_slots(const PeelArgs& A, const int4 (&it)
             const int32_t y = it[h].z, src = w[h] < y ? w[h] : y;
             key[h] = w[h] < y ? y : w[h];
             b[h] = __ldg(A.rp + src);
-            n[h] = (int)(__ldg(A.rp + src + 1) - b[h]);
+            n[h] = Mode == kCompact ? __ldcg(A.out_len + src) : (int)(__ldg(A.rp + src + 1) - b[h]);
         }
         tr[h] = n[h] > 0;
         any |= n[h] > 1;
@@ -831,7 +879,10 @@ __device__ __forceinline__ void search_slots(const PeelArgs& A, const int4 (&it)
         any = false;
         int32_t c[kWin];
 #pragma unroll
-        for (int h = 0; h < kWin; h++) c[h] = n[h] > 1 ? __ldg(A.cols + b[h] + (n[h] >> 1)) : INT32_MAX;
+        for (int h = 0; h < kWin; h++) {
+            c[h] = INT32_MAX;
+            if (n[h] > 1) c[h] = Mode == kCompact ? out_col[b[h] + (n[h] >> 1)] : __ldg(A.cols + b[h] + (n[h] >> 1));
+        }
 #pragma unroll
         for (int h = 0; h < kWin; h++) {
             const int half = n[h] >> 1;
@@ -841,10 +892,17 @@ __device__ __forceinline__ void search_slots(const PeelArgs& A, const int4 (&it)
         }
     }
 #pragma unroll
-    for (int h = 0; h < kWin; h++) tr[h] = tr[h] && __ldg(A.cols + b[h]) == key[h];
-#pragma unroll
     for (int h = 0; h < kWin; h++) {
         g[h] = (int32_t)b[h];
+        if (Mode == kCompact) {
+            if (tr[h] && !whole) g[h] = A.out_eid[b[h]];
+            tr[h] = tr[h] && out_col[b[h]] == key[h];
+        } else {
+            tr[h] = tr[h] && __ldg(A.cols + b[h]) == key[h];
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < kWin; h++) {
         x[h] = tr[h] ? __ldcg(A.code + (g[h] >> 3)) : 0u;
     }
 #pragma unroll
@@ -860,9 +918,10 @@ struct Pending {
     int32_t o[2 * kWin];
 };
 
-template <bool Listed>
+template <int Mode>
 __device__ __forceinline__ void settle(const PeelArgs& A, const Pending& P, int r, int32_t l, int nslot, int nbuf,
                                        AppendBuf& B, int32_t& dm) {
+    constexpr bool Listed = Mode == kListed;
     bool w[2 * kWin];
     // queued with an item when the level is above 0 (an edge without
     // triangles never appears in a list, so its code is never read)
@@ -879,10 +938,10 @@ __device__ __forceinline__ void settle(const PeelArgs& A, const Pending& P, int 
 #pragma unroll
     for (int h = 0; h < kWin; h++) {
         if (Listed)
-            warp_append2_staged<Listed>(A, nslot, nbuf, w[2 * h], P.e[2 * h], w[2 * h + 1], P.e[2 * h + 1], l, B,
+            warp_append2_staged<Mode>(A, nslot, nbuf, w[2 * h], P.e[2 * h], w[2 * h + 1], P.e[2 * h + 1], l, B,
                                         &A.ctl->fe[nslot]);
         else
-            warp_append2_direct<Listed>(A, nslot, nbuf, w[2 * h], P.e[2 * h], w[2 * h + 1], P.e[2 * h + 1], l,
+            warp_append2_direct<Mode>(A, nslot, nbuf, w[2 * h], P.e[2 * h], w[2 * h + 1], P.e[2 * h + 1], l,
                                         &A.ctl->fe[nslot]);
     }
 }
@@ -896,9 +955,10 @@ __device__ __forceinline__ void settle(const PeelArgs& A, const Pending& P, int 
 // window starts, records, list entry, codes, decrement.  With the counters
 // handed over by the barrier, peel of R-MAT scale 12 / 16 / 20 / 22: 2.58 /
 // 9.70 / 40.3 / 116.6 -> 1.72 / 7.32 / 33.6 / 104.2 ms.
-template <bool Listed>
+template <int Mode>
 __device__ __forceinline__ void lean_round(const PeelArgs& A, int r, int32_t l, int N, int T, int gwarp, int nwarps,
-                                           int32_t* ebuf, int* s_dmin) {
+                                           int32_t* ebuf, int* s_dmin, int cst) {
+    constexpr bool Listed = Mode == kListed;
     if (gwarp * kWarp >= T) return;
     const unsigned lane = lane_id();
     const unsigned le = lanemask_lt() | (1u << lane);
@@ -954,7 +1014,7 @@ __device__ __forceinline__ void lean_round(const PeelArgs& A, int r, int32_t l, 
             rf[0] = v[0] ? code_round(xf, fg.x, r) : -2;
             rg[0] = v[0] ? code_round(xg, fg.y, r) : -2;
         } else {
-            search_slots(A, it, tl, r, v, f, g, rf, rg);
+            search_slots<Mode>(A, it, tl, r, cst, v, f, g, rf, rg);
 #pragma unroll
             for (int h = 0; h < kL; h++)
                 if (!v[h]) rf[h] = -2;
@@ -984,12 +1044,12 @@ __device__ __forceinline__ void lean_round(const PeelArgs& A, int r, int32_t l, 
                 A.rnd[g[h]] = r + 1;
                 code_mark(A.code, g[h], cm);
             }
-            warp_append2_staged<Listed>(A, nslot, nbuf, wf, f[h], wg, g[h], l, B, &A.ctl->fe[nslot]);
+            warp_append2_staged<Mode>(A, nslot, nbuf, wf, f[h], wg, g[h], l, B, &A.ctl->fe[nslot]);
         }
     }
     dm = warp_min(dm);
     if (lane == 0 && dm != INT32_MAX) atomicMin(s_dmin, dm);
-    append_flush<Listed>(A, nslot, nbuf, B, &A.ctl->fe[nslot]);
+    append_flush<Mode>(A, nslot, nbuf, B, &A.ctl->fe[nslot]);
 }
 
 // One sub-round: warps gwarp = 0..nwarps-1 share the candidate slots of round r.
@@ -999,10 +1059,11 @@ __device__ __forceinline__ void lean_round(const PeelArgs& A, int r, int32_t l, 
 // the level changes): the kernel arguments are a __grid_constant__ parameter,
 // so no call passes a local copy of them, and no call frame is saved around
 // every sub-round.
-template <bool Listed>
+template <int Mode>
 __device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t l, unsigned long long packed,
                                               long long nprev, long long gwarp, long long nwarps, int* s_dmin,
-                                              int32_t* app_e) {
+                                              int32_t* app_e, int cst) {
+    constexpr bool Listed = Mode == kListed;
     const unsigned lane = lane_id();
     const unsigned le = lanemask_lt() | (1u << lane);
     int32_t dm = INT32_MAX;
@@ -1025,7 +1086,7 @@ __device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t 
         }
     }
     if (T <= nwarps * kWarp * (Listed ? kLeanWindows : kLeanSearch) && T <= (long long)kSlotIdx * kWarp) {
-        lean_round<Listed>(A, r, l, (int)N, (int)T, (int)gwarp, (int)nwarps, app_e + wib * kAppBuf, s_dmin);
+        lean_round<Mode>(A, r, l, (int)N, (int)T, (int)gwarp, (int)nwarps, app_e + wib * kAppBuf, s_dmin, cst);
         return;
     }
     // listed mode: each warp owns a contiguous range of candidate slots (a
@@ -1113,7 +1174,7 @@ __device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t 
                 }
             }
             // the previous step's decrement results, while these loads are in flight
-            settle<Listed>(A, P, r, l, nslot, nbuf, B, dm);
+            settle<Mode>(A, P, r, l, nslot, nbuf, B, dm);
 #pragma unroll
             for (int h = 0; h < kWin; h++) {
                 if (tr[h]) {
@@ -1128,8 +1189,8 @@ __device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t 
                 tl[h] = (int)(cb + h * kWarp + lane - bl[h]);
                 tr[h] = v[h];
             }
-            search_slots(A, it, tl, r, tr, f, g, rf, rg);
-            settle<Listed>(A, P, r, l, nslot, nbuf, B, dm);
+            search_slots<Mode>(A, it, tl, r, cst, tr, f, g, rf, rg);
+            settle<Mode>(A, P, r, l, nslot, nbuf, B, dm);
         }
         // a triangle is alive when both other edges are alive or peel in r or r+1;
         // which of f, g this lane decrements: the ownership rules above
@@ -1157,25 +1218,176 @@ __device__ __forceinline__ void process_round(const PeelArgs& A, int r, int32_t 
     }
     if (!dyn) break;
     }
-    settle<Listed>(A, P, r, l, nslot, nbuf, B, dm);
-    if (Listed) append_flush<Listed>(A, nslot, nbuf, B, &A.ctl->fe[nslot]);
+    settle<Mode>(A, P, r, l, nslot, nbuf, B, dm);
+    if (Listed) append_flush<Mode>(A, nslot, nbuf, B, &A.ctl->fe[nslot]);
     dm = warp_min(dm);
     if (lane == 0 && dm != INT32_MAX) atomicMin(s_dmin, dm);
+}
+
+// The search peel walks a peeled edge's neighbours, dead edges among them, and
+// they cost it a round-code load each.  Its rows are therefore compacted (order
+// and row starts kept, lengths shrunk; the first time into a copy, then in
+// place) whenever the alive edges have halved: every compaction reads what the
+// one before left, so all of them together read about twice the edges, and the
+// slots of a Chung-Lu graph fall from 3.1 to 1.1 a list entry (host model, 60 K
+// vertices).  Peel of one of 1 M vertices: 104 -> 69 ms, 3 ms of them in
+// compactions (a quarter off instead of half: 72 ms).
+__device__ __forceinline__ void compact_init(const PeelArgs& A) {
+    const int64_t nth = (int64_t)gridDim.x * kPeelBlock, tid = (int64_t)blockIdx.x * kPeelBlock + threadIdx.x;
+    for (int64_t u = tid; u < A.V; u += nth) {
+        A.out_len[u] = (int32_t)(__ldg(A.rp + u + 1) - __ldg(A.rp + u));
+        A.in_len[u] = (int32_t)(__ldg(A.cp + u + 1) - __ldg(A.cp + u));
+    }
+}
+
+constexpr long long kCompactMin = 4096;  // alive edges at the last compaction below which there is no next one
+constexpr int kCompactLong = 1024;  // rows longer than this are compacted by a block
+
+// An edge stays until its sub-round is over: alive, or marked for sub-round r.
+__device__ __forceinline__ bool compact_keep(const PeelArgs& A, int32_t e, int r) {
+    const unsigned c = (__ldcg(A.code + (e >> 3)) >> ((unsigned)(e & 7) * 4u)) & 15u;
+    return c == kCodeAlive || c == ((unsigned)r & 3u);
+}
+
+// One row's out- or in-edges by a warp or by the block, kCompactPer entries a
+// thread at a time; returns the new length.
+constexpr int kCompactPer = 4;
+
+template <bool Out, bool Block>
+__device__ __forceinline__ int compact_row(const PeelArgs& A, int64_t base, int len, int r, bool whole,
+                                           int* s_warp) {
+    const unsigned lane = lane_id();
+    const int wib = threadIdx.x / kWarp;
+    constexpr int kThr = Block ? kPeelBlock : kWarp;
+    constexpr int kPer = Block ? kCompactPer : 1;
+    const int tid = Block ? (int)threadIdx.x : (int)lane;
+    int32_t* ids = (Out ? A.out_col : A.in_src) + base;
+    int32_t* eids = (Out ? A.out_eid : A.in_eid) + base;
+    int n = 0;
+    for (int t = 0; t < len; t += kPer * kThr) {
+        int2 x[kPer];
+        bool keep[kPer];
+        unsigned m[kPer];
+#pragma unroll
+        for (int j = 0; j < kPer; j++) {
+            const int i = t + j * kThr + tid;
+            x[j] = make_int2(0, -1);
+            if (i < len) {
+                if (Out && whole) x[j] = make_int2(__ldg(A.cols + base + i), (int32_t)(base + i));
+                else x[j] = make_int2(__ldcg(ids + i), __ldcg(eids + i));
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kPer; j++) keep[j] = x[j].y >= 0 && compact_keep(A, x[j].y, r);
+#pragma unroll
+        for (int j = 0; j < kPer; j++) {
+            m[j] = __ballot_sync(kFull, keep[j]);
+            if (Block && lane == 0) s_warp[j * kPeelWarps + wib] = __popc(m[j]);
+        }
+        int all = __popc(m[0]), at = 0;
+        if (Block) {
+            __syncthreads();  // also: every entry of this tile has been read
+            all = 0;
+        }
+#pragma unroll
+        for (int j = 0; j < kPer; j++) {
+            if (Block) {
+                at = all;
+                for (int w = 0; w < kPeelWarps; w++) {
+                    const int c = s_warp[j * kPeelWarps + w];
+                    if (w < wib) at += c;
+                    all += c;
+                }
+            }
+            if (keep[j]) {
+                const int to = n + at + __popc(m[j] & lanemask_lt());
+                ids[to] = x[j].x;
+                eids[to] = x[j].y;
+            }
+        }
+        n += all;
+        if (Block) __syncthreads();
+        else __syncwarp();
+    }
+    return n;
+}
+
+// Drops the edges peeled before sub-round r from every row (a grid barrier
+// follows).  A block takes kPeelBlock rows at a time, a thread reading the
+// lengths of one: a warp compacts its 32 rows one after the other, then the
+// block the long ones.  The rows of a block lie far apart in rank: the hubs are
+// the top ranks, side by side.
+__device__ __forceinline__ void compact_rows(const PeelArgs& A, int r, bool whole, int* s_warp, int32_t* s_rows) {
+    __shared__ int s_n;
+    const unsigned lane = lane_id();
+    const int64_t stride = (A.V + kPeelBlock - 1) / kPeelBlock;
+    for (int64_t b = blockIdx.x; b < stride; b += gridDim.x) {
+        const int64_t u = b + threadIdx.x * stride;
+        int lo = 0, li = 0;
+        int64_t po = 0, pi = 0;
+        if (u < A.V) {
+            lo = __ldcg(A.out_len + u);
+            li = __ldcg(A.in_len + u);
+            po = __ldg(A.rp + u);
+            pi = __ldg(A.cp + u);
+        }
+        if (threadIdx.x == 0) s_n = 0;
+        __syncthreads();
+        if (lo > kCompactLong || li > kCompactLong) s_rows[atomicAdd(&s_n, 1)] = (int32_t)threadIdx.x;
+        unsigned m = __ballot_sync(kFull, lo > 0 && lo <= kCompactLong);
+        while (m) {
+            const int k = __ffs(m) - 1;
+            m &= m - 1;
+            const int n = compact_row<true, false>(A, __shfl_sync(kFull, po, k), __shfl_sync(kFull, lo, k), r, whole, nullptr);
+            if ((int)lane == k) A.out_len[u] = n;
+        }
+        m = __ballot_sync(kFull, li > 0 && li <= kCompactLong);
+        while (m) {
+            const int k = __ffs(m) - 1;
+            m &= m - 1;
+            const int n = compact_row<false, false>(A, __shfl_sync(kFull, pi, k), __shfl_sync(kFull, li, k), r, whole, nullptr);
+            if ((int)lane == k) A.in_len[u] = n;
+        }
+        __syncthreads();
+        const int rows = s_n;
+        for (int i = 0; i < rows; i++) {
+            const int64_t v = b + s_rows[i] * stride;
+            const int vo = __ldcg(A.out_len + v), vi = __ldcg(A.in_len + v);
+            __syncthreads();
+            // a length at or under the bound was settled by its warp
+            if (vo > kCompactLong) {
+                const int n = compact_row<true, true>(A, __ldg(A.rp + v), vo, r, whole, s_warp);
+                if (threadIdx.x == 0) A.out_len[v] = n;
+            }
+            if (vi > kCompactLong) {
+                const int n = compact_row<false, true>(A, __ldg(A.cp + v), vi, r, whole, s_warp);
+                if (threadIdx.x == 0) A.in_len[v] = n;
+            }
+        }
+        __syncthreads();
+    }
 }
 
 #ifndef TDT_PEEL_MINB
 #define TDT_PEEL_MINB 2
 #endif
 // A is a __grid_constant__ parameter: the helpers take it by reference and
-// read its fields from the parameter bank instead of a local copy.  Lists:
-// the caller gave a list tail, and whether the lists fit is decided on the
-// device; without a tail the search peel has a kernel, and its registers, of
-// its own (Chung-Lu, 1 M vertices: 121 -> 104 ms).
-template <bool Lists>
+// read its fields from the parameter bank instead of a local copy.
+// kListed: the caller gave a list tail, and whether the lists fit is decided on
+// the device (search otherwise).  Without a tail the search peels have kernels,
+// and their registers, of their own (Chung-Lu, 1 M vertices, without
+// compaction: 121 -> 104 ms).  A fixed level does not compact: most of its work
+// is its first sub-rounds (k = 10 / 100 at R-MAT scale 20 6.7 / 40.0 ms, with
+// compaction 7.0 / 41.7).
+template <int Mode>
 __global__ void __launch_bounds__(kPeelBlock, TDT_PEEL_MINB) peel_kernel(const __grid_constant__ PeelArgs A) {
     __shared__ int32_t s_app_e[kPeelWarps * kAppBuf];  // per-warp append staging
     __shared__ RoundShared s_round;
-    const bool listed = Lists && *(volatile int*)&A.ctl->listed != 0;
+    __shared__ int s_warp[kCompactPer * kPeelWarps];
+    const bool lists = *(volatile int*)&A.ctl->listed != 0;
+    const bool listed = Mode == kListed && lists;
+    if (Mode == kListed ? !lists && A.search_next : lists) return;
+    constexpr int kOther = Mode == kCompact ? kCompact : kSearch;
     const int wib = threadIdx.x / kWarp;
     const int64_t gwarp = (int64_t)blockIdx.x * kPeelWarps + wib;
     const int64_t nwarps = (int64_t)gridDim.x * kPeelWarps;
@@ -1190,16 +1402,24 @@ __global__ void __launch_bounds__(kPeelBlock, TDT_PEEL_MINB) peel_kernel(const _
     if (threadIdx.x == 0) s_round.dmin = INT32_MAX;
     RoundBar RB{gridDim.x, 0ull, 0ull};
     long long nprev = 0;  // items of the sub-round before
+    // compaction: edges alive now and at the last one
+    long long alive = A.E, alive_c = A.E;
+    int cst = kWhole;
+    if constexpr (Mode == kCompact) {
+        compact_init(A);
+        if (!round_barrier(A.ctl, RB, &s_round, 0, &A.ctl->dmin[0])) return;
+    }
     if (A.mode == 0) {
-        ok = level_transition(A, listed, 0, ntrans++, np, &l, s_app_e, RB, &s_round);
+        ok = level_transition<kOther>(A, listed, 0, ntrans++, np, &l, s_app_e, RB, &s_round);
     } else {
         l = A.fixed_level;
-        ok = fixed_collect(A, listed, l, 0, np, RB, &s_round);
+        ok = fixed_collect<kOther>(A, listed, l, 0, np, RB, &s_round);
     }
     if (!ok) {
         if (master) A.ctl->rounds = 0;
         return;
     }
+    alive -= (long long)RB.fe;
     uint64_t t_mark = globaltimer_ns();
     for (;;) {
         if (master) {
@@ -1209,8 +1429,9 @@ __global__ void __launch_bounds__(kPeelBlock, TDT_PEEL_MINB) peel_kernel(const _
             A.ctl->grab[(r + 2) & 3] = 0;
             if (globaltimer_ns() - t_start > A.deadline_ns) set_status(A.ctl, TDT_ERR_TIMEOUT);
         }
-        if (listed) process_round<true>(A, r, l, RB.q, nprev, gwarp, nwarps, &s_round.dmin, s_app_e);
-        else process_round<false>(A, r, l, RB.q, nprev, gwarp, nwarps, &s_round.dmin, s_app_e);
+        if (listed) process_round<kListed>(A, r, l, RB.q, nprev, gwarp, nwarps, &s_round.dmin, s_app_e, kWhole);
+        else process_round<kOther>(A, r, l, RB.q, nprev, gwarp, nwarps, &s_round.dmin, s_app_e, cst);
+        if (cst == kStale) cst = kFresh;
         nprev = (long long)(RB.q >> kCandBits);
         if (nprev > A.E) nprev = A.E;
         __syncthreads();
@@ -1231,19 +1452,29 @@ __global__ void __launch_bounds__(kPeelBlock, TDT_PEEL_MINB) peel_kernel(const _
         if (RB.fe == 0) {
             if (A.mode != 0) {
                 // k-truss search: the next batch of low-support edges, if any
-                if (!fixed_collect(A, listed, l, r + 1, np, RB, &s_round)) break;
+                if (!fixed_collect<kOther>(A, listed, l, r + 1, np, RB, &s_round)) break;
                 t_mark = globaltimer_ns();
                 r++;
+                alive -= (long long)RB.fe;
                 continue;
             }
             int32_t nl;
-            const bool more = level_transition(A, listed, r + 1, ntrans++, np, &nl, s_app_e, RB, &s_round);
+            const bool more = level_transition<kOther>(A, listed, r + 1, ntrans++, np, &nl, s_app_e, RB, &s_round);
             if (master) A.ctl->t_trans += globaltimer_ns() - t_b;
             if (!more) break;
             l = nl;
         }
         t_mark = globaltimer_ns();
         r++;
+        if constexpr (Mode == kCompact) {
+            alive -= (long long)RB.fe;
+            if (2 * alive <= alive_c && alive_c >= kCompactMin) {
+                compact_rows(A, r, cst == kWhole, s_warp, s_app_e);
+                alive_c = alive;
+                cst = kStale;
+                if (!round_barrier(A.ctl, RB, &s_round, r, &A.ctl->dmin[(ntrans + 1) & 1])) return;
+            }
+        }
     }
     if (master) {
         A.ctl->rounds = r + 1;
@@ -1449,6 +1680,8 @@ __global__ void stats_final_kernel(PeelCtl* ctl, int64_t* stats, int mode) {
 }
 
 // ------------------------------------------------------------------ host side
+constexpr int64_t kSearchNextEdges = 1 << 20;
+
 void prof_mark(int phase, cudaStream_t st);
 
 // Test hook: wall-clock budget of the next peel launches (<= 0: the default).
@@ -1705,6 +1938,12 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     A.code = L.code;
     TDT_CUDA(cudaMemsetAsync(L.code, 0xff, 4 * (size_t)(E / 8 + 1), st));
     A.off = L.off; A.lists = lists;
+    // the search peel's copy of the out-edges and the row lengths, in arrays
+    // that only the listing uses
+    A.out_col = reinterpret_cast<int32_t*>(L.off);
+    A.out_eid = A.out_col + E;
+    A.out_len = reinterpret_cast<int32_t*>(L.sbase);
+    A.in_len = L.indeg;
     A.alive[0] = L.alive[0]; A.alive[1] = L.alive[1];
     A.sidx[0] = L.sidx; A.sidx[1] = L.sidx + kSlotIdx;
     A.V = V; A.E = E; A.round_cap = E + 2;
@@ -1724,21 +1963,32 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     // 18.2 / 14.0 / 13.3, scale 20 61.4 / 40.2 / 34.1; Chung-Lu (1.5 M edges)
     // 10.6 / 9.6 / 9.8.  The search peel keeps every block: its slots are
     // binary searches.
-    void* kern = tail > 0 ? (void*)peel_kernel<true> : (void*)peel_kernel<false>;
-    int occ = 0;
-    TDT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kPeelBlock, 0));
-    if (occ < 1) {
-        set_error("peel kernel cannot be resident");
-        return TDT_ERR_UNSUPPORTED;
-    }
-    if (di.sms * occ > 4096) occ = 4096 / di.sms;
-    int nblk = di.sms * occ;
-    if (tail > 0 && E < (1ll << 20)) nblk = di.sms;
-    if (g_peel_half_sms > 0) nblk = (g_peel_half_sms * di.sms + 1) / 2;
-    if (nblk > di.sms * occ) nblk = di.sms * occ;
-    void* args[] = {&A};
-    TDT_CUDA(cudaLaunchCooperativeKernel(kern, dim3(nblk), dim3(kPeelBlock), args, 0, st));
-    note_launch();
+    // With a list tail the device decides whether the peel is listed.  A large
+    // graph whose lists do not fit then goes to the compacting search kernel,
+    // which follows (a launch that returns at once costs 4 us); a small one is
+    // searched in place.
+    A.search_next = mode == 0 && tail > 0 && E >= kSearchNextEdges;
+    auto launch_peel = [&](void* kern, bool lists_k) -> int {
+        int occ = 0;
+        TDT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kPeelBlock, 0));
+        if (occ < 1) {
+            set_error("peel kernel cannot be resident");
+            return TDT_ERR_UNSUPPORTED;
+        }
+        if (di.sms * occ > 4096) occ = 4096 / di.sms;
+        int nblk = di.sms * occ;
+        if (lists_k && E < (1ll << 20)) nblk = di.sms;
+        if (g_peel_half_sms > 0) nblk = (g_peel_half_sms * di.sms + 1) / 2;
+        if (nblk > di.sms * occ) nblk = di.sms * occ;
+        void* args[] = {&A};
+        TDT_CUDA(cudaLaunchCooperativeKernel(kern, dim3(nblk), dim3(kPeelBlock), args, 0, st));
+        note_launch();
+        return TDT_OK;
+    };
+    if (tail > 0) rc = launch_peel((void*)peel_kernel<kListed>, true);
+    if (rc == TDT_OK && (tail == 0 || A.search_next))
+        rc = launch_peel(mode == 0 ? (void*)peel_kernel<kCompact> : (void*)peel_kernel<kSearch>, false);
+    if (rc) return rc;
     prof_mark(3, st);
 
     if (mode == 0) {
