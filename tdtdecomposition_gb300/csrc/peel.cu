@@ -1517,24 +1517,82 @@ __global__ void validate_kernel(const int64_t* __restrict__ rp, const int32_t* _
     }
 }
 
-__global__ void indeg_kernel(const int32_t* __restrict__ rows, const int32_t* __restrict__ cols, int64_t E,
-                             int64_t V, int32_t* __restrict__ indeg, const PeelCtl* ctl) {
-    if (*(volatile const int*)&ctl->g.status != 0) return;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E;
-         e += (int64_t)gridDim.x * blockDim.x)
-        atomicAdd(indeg + cols[e], 1);
+// In-adjacency.  Ids are degree ranks, so most heads are among the top ids and
+// a hub's counter would take one atomic per in-edge, one after the other (7 to
+// 9 ns each).  A block counts the heads of its edges among the top kCscHot ids
+// in shared memory and adds each counter to the global one once; the fill then
+// reserves a run of the in-list per (block, top id) and takes places in it from
+// shared memory.  Both kernels at R-MAT scale 16 / 18 / 22: 145 us / 490 us /
+// 4.1 ms with an atomic per edge, 39 us / 93 us / 2.0 ms.  The in-lists come out
+// nearly in source order, and the walk that follows them fell from 1.10 to
+// 0.51 ms at scale 18, from 8.4 to 6.8 ms at scale 21.
+constexpr int kCscBlock = 512;
+constexpr int kCscHot = 8192;
+// Edges of a tile of the fill in a large graph: the places that the resident
+// blocks write at one time stay within L2 (scale 22: 3.37 ms with one share a
+// block, 2.85 with 65,536, 1.71 with 16,384, 1.66 with 4,096).
+constexpr int kCscTile = 8192;
+constexpr int kCscUnroll = 4;
+
+// f(e, cols[e]) over edges [e0, e1) by the block.
+template <class F>
+__device__ __forceinline__ void csc_edges(const int32_t* __restrict__ cols, int64_t e0, int64_t e1, F&& f) {
+    for (int64_t e = e0 + threadIdx.x; e < e1; e += kCscUnroll * kCscBlock) {
+        int32_t v[kCscUnroll];
+#pragma unroll
+        for (int k = 0; k < kCscUnroll; k++) v[k] = e + k * kCscBlock < e1 ? __ldg(cols + e + k * kCscBlock) : -1;
+#pragma unroll
+        for (int k = 0; k < kCscUnroll; k++)
+            if (v[k] >= 0) f(e + k * kCscBlock, v[k]);
+    }
 }
 
-__global__ void csc_fill_kernel(const int32_t* __restrict__ rows, const int32_t* __restrict__ cols, int64_t E,
-                                int64_t V, const int64_t* __restrict__ cp, int32_t* __restrict__ cursor,
-                                int32_t* __restrict__ in_src, int32_t* __restrict__ in_eid, const PeelCtl* ctl) {
+__global__ void __launch_bounds__(kCscBlock) indeg_kernel(const int32_t* __restrict__ cols, int64_t E, int64_t V,
+                                                          int32_t* __restrict__ indeg, const PeelCtl* ctl) {
+    __shared__ int32_t s_cnt[kCscHot];
     if (*(volatile const int*)&ctl->g.status != 0) return;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const int32_t u = rows[e], v = cols[e];
-        const int64_t pos = cp[v] + atomicAdd(cursor + v, 1);
-        in_src[pos] = u;
-        in_eid[pos] = (int32_t)e;
+    const int32_t hot0 = V > kCscHot ? (int32_t)(V - kCscHot) : 0;
+    const int hot = (int)(V - hot0);
+    for (int i = threadIdx.x; i < hot; i += kCscBlock) s_cnt[i] = 0;
+    __syncthreads();
+    const int64_t per = (E + gridDim.x - 1) / gridDim.x, e0 = blockIdx.x * per;
+    csc_edges(cols, e0, e0 + per < E ? e0 + per : E, [&](int64_t, int32_t v) {
+        if (v >= hot0) atomicAdd(s_cnt + (v - hot0), 1);
+        else atomicAdd(indeg + v, 1);
+    });
+    __syncthreads();
+    for (int i = threadIdx.x; i < hot; i += kCscBlock)
+        if (s_cnt[i]) atomicAdd(indeg + hot0 + i, s_cnt[i]);
+}
+
+__global__ void __launch_bounds__(kCscBlock) csc_fill_kernel(const int32_t* __restrict__ rows,
+                                                             const int32_t* __restrict__ cols, int64_t E, int64_t V,
+                                                             int64_t tile,
+                                                             const int64_t* __restrict__ cp,
+                                                             int32_t* __restrict__ cursor, int32_t* __restrict__ in_src,
+                                                             int32_t* __restrict__ in_eid, const PeelCtl* ctl) {
+    __shared__ int32_t s_cur[kCscHot];  // counts, then the next place of the block's run
+    if (*(volatile const int*)&ctl->g.status != 0) return;
+    const int32_t hot0 = V > kCscHot ? (int32_t)(V - kCscHot) : 0;
+    const int hot = (int)(V - hot0);
+    for (int64_t e0 = blockIdx.x * tile; e0 < E; e0 += gridDim.x * tile) {
+        const int64_t e1 = e0 + tile < E ? e0 + tile : E;
+        for (int i = threadIdx.x; i < hot; i += kCscBlock) s_cur[i] = 0;
+        __syncthreads();
+        csc_edges(cols, e0, e1, [&](int64_t, int32_t v) {
+            if (v >= hot0) atomicAdd(s_cur + (v - hot0), 1);
+        });
+        __syncthreads();
+        for (int i = threadIdx.x; i < hot; i += kCscBlock)
+            if (s_cur[i]) s_cur[i] = (int32_t)__ldg(cp + hot0 + i) + atomicAdd(cursor + hot0 + i, s_cur[i]);
+        __syncthreads();
+        csc_edges(cols, e0, e1, [&](int64_t e, int32_t v) {
+            const int32_t pos = v >= hot0 ? atomicAdd(s_cur + (v - hot0), 1)
+                                          : (int32_t)__ldg(cp + v) + atomicAdd(cursor + v, 1);
+            in_src[pos] = __ldg(rows + e);
+            in_eid[pos] = (int32_t)e;
+        });
+        __syncthreads();
     }
 }
 
@@ -1872,12 +1930,18 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     // in-adjacency (CSC) of the oriented graph: the walk's middle vertices, and
     // the peel without lists
     TDT_CUDA(cudaMemsetAsync(L.indeg, 0, 4 * (size_t)V, st));
-    indeg_kernel<<<g_e, tb, 0, st>>>(rows_use, cols, E, V, L.indeg, L.ctl);
+    // tiles of the in-adjacency build: at least one per resident block
+    const int64_t csc_blocks = (int64_t)di.sms * 4;
+    int64_t csc_tile = kCscTile;
+    while (csc_tile > 1024 && E < csc_tile * csc_blocks) csc_tile /= 2;
+    const int64_t csc_tiles = (E + csc_tile - 1) / csc_tile;
+    const unsigned g_csc = (unsigned)(csc_tiles < csc_blocks ? csc_tiles : csc_blocks);
+    indeg_kernel<<<g_csc, kCscBlock, 0, st>>>(cols, E, V, L.indeg, L.ctl);
     TDT_LAUNCH_CHECK("indeg");
     rc = exclusive_scan<int32_t, int64_t>(L.indeg, L.cp, V, L.cp + V, L.scan_ws, st);
     if (rc) return rc;
     TDT_CUDA(cudaMemsetAsync(L.indeg, 0, 4 * (size_t)V, st));
-    csc_fill_kernel<<<g_e, tb, 0, st>>>(rows_use, cols, E, V, L.cp, L.indeg, L.in_src, L.in_eid, L.ctl);
+    csc_fill_kernel<<<g_csc, kCscBlock, 0, st>>>(rows_use, cols, E, V, csc_tile, L.cp, L.indeg, L.in_src, L.in_eid, L.ctl);
     TDT_LAUNCH_CHECK("csc_fill");
     // The list tail: final lists grow from its start, the staging slots of the
     // one walk end at its end.
