@@ -1649,21 +1649,27 @@ __global__ void list_decide_kernel(const int64_t* __restrict__ off, const int64_
     ctl->rewalk_skip = !ok || compact;
 }
 
-__global__ void truss_out_kernel(const int32_t* __restrict__ rnd, const int32_t* __restrict__ round_level,
-                                 int64_t E, int32_t* __restrict__ truss, uint32_t* __restrict__ keys,
-                                 uint32_t* __restrict__ vals, PeelCtl* ctl) {
-    if (ctl->g.status != 0) return;
+// Truss numbers, and the digit totals of the sort by round.
+__global__ void __launch_bounds__(256) truss_out_kernel(const int32_t* __restrict__ rnd,
+                                                        const int32_t* __restrict__ round_level, int64_t E,
+                                                        int32_t* __restrict__ truss, int passes, uint32_t* hist,
+                                                        PeelCtl* ctl) {
+    __shared__ uint32_t s_hist[kMaxPasses * kRadix];
+    if (__syncthreads_or(*(volatile int*)&ctl->g.status != 0)) return;
+    const int run = radix_passes_run(passes, ctl->rounds);
+    DigitHist H{s_hist};
+    H.init(run);
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E;
          e += (int64_t)gridDim.x * blockDim.x) {
         const int32_t r = rnd[e];
+        H.add((uint32_t)r, run);
         if (r < 0) {  // every edge is peeled when the run completes
             atomicMax((int*)&ctl->g.status, (int)TDT_ERR_CAPACITY);
             continue;
         }
-        if (truss) truss[e] = round_level[r] + 2;
-        keys[e] = (uint32_t)r;
-        vals[e] = (uint32_t)e;
+        if (truss) truss[e] = __ldg(round_level + r) + 2;
     }
+    H.flush(run, hist);
 }
 
 // Number of sorted positions whose round has level <= lv (levels are
@@ -1678,12 +1684,17 @@ __device__ __forceinline__ int64_t count_level_le(const uint32_t* keys, int64_t 
     return lo;
 }
 
-__global__ void ptr_etruss_kernel(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ vals, int64_t E,
-                                  const int32_t* __restrict__ round_level, int32_t* __restrict__ ptr_truss,
+// k0 / v0: the buffer of the sort's first pass, k1 / v1 of its second.
+__global__ void ptr_etruss_kernel(const uint32_t* __restrict__ k0, const uint32_t* __restrict__ v0,
+                                  const uint32_t* __restrict__ k1, const uint32_t* __restrict__ v1, int passes,
+                                  int64_t E, const int32_t* __restrict__ round_level, int32_t* __restrict__ ptr_truss,
                                   int64_t ptr_cap, int32_t* __restrict__ e_truss, PeelCtl* ctl,
                                   int64_t* __restrict__ stats) {
     if (*(volatile int*)&ctl->g.status != 0) return;
     const long long rounds = ctl->rounds;
+    const bool first = radix_passes_run(passes, rounds) & 1;
+    const uint32_t* keys = first ? k0 : k1;
+    const uint32_t* vals = first ? v0 : v1;
     const int32_t L = rounds > 0 ? round_level[rounds - 1] : 0;
     const int64_t n0 = rounds > 0 ? count_level_le(keys, E, round_level, 0) : E;
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1871,7 +1882,7 @@ Layout carve(void* ws, int64_t V, int64_t E) {
     L.code = (unsigned*)c.take(4 * (e / 8 + 1));
     size_t scan_b = scan_scratch_bytes((int64_t)(e > v ? e : v) + 1);
     L.scan_ws = c.take(scan_b);
-    L.sort_ws = c.take(radix_sort_scratch_bytes((int64_t)e));
+    L.sort_ws = c.take(radix_scratch(nullptr, (int64_t)e, 4).bytes);
     L.total = c.off + 256;
     return L;
 }
@@ -1938,7 +1949,7 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     const unsigned g_csc = (unsigned)(csc_tiles < csc_blocks ? csc_tiles : csc_blocks);
     indeg_kernel<<<g_csc, kCscBlock, 0, st>>>(cols, E, V, L.indeg, L.ctl);
     TDT_LAUNCH_CHECK("indeg");
-    rc = exclusive_scan<int32_t, int64_t>(L.indeg, L.cp, V, L.cp + V, L.scan_ws, st);
+    rc = exclusive_scan<int32_t, int64_t>(L.indeg, L.cp, V, L.cp + V, L.scan_ws, &L.ctl->g.status, st);
     if (rc) return rc;
     TDT_CUDA(cudaMemsetAsync(L.indeg, 0, 4 * (size_t)V, st));
     csc_fill_kernel<<<g_csc, kCscBlock, 0, st>>>(rows_use, cols, E, V, csc_tile, L.cp, L.indeg, L.in_src, L.in_eid, L.ctl);
@@ -1953,7 +1964,7 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     if (tail > 0) {
         rc = launch_stage_rows(rp, V, L.sbase, &L.ctl->g.status, st);
         if (rc) return rc;
-        rc = exclusive_scan<int64_t, int64_t>(L.sbase, L.sbase, V, L.sbase + V, L.scan_ws, st);
+        rc = exclusive_scan<int64_t, int64_t>(L.sbase, L.sbase, V, L.sbase + V, L.scan_ws, &L.ctl->g.status, st);
         if (rc) return rc;
         stage_decide_kernel<<<1, 1, 0, st>>>(L.sbase, V, tail, L.ctl);
         TDT_LAUNCH_CHECK("stage_decide");
@@ -1977,7 +1988,7 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     }
     // per-edge triangle lists in the workspace tail when 24 T bytes fit
     if (tail > 0) {
-        rc = exclusive_scan<int32_t, int64_t>(L.sup, L.off, E, L.off + E, L.scan_ws, st);
+        rc = exclusive_scan<int32_t, int64_t>(L.sup, L.off, E, L.off + E, L.scan_ws, &L.ctl->g.status, st);
         if (rc) return rc;
         list_decide_kernel<<<1, 1, 0, st>>>(L.off, L.sbase, E, V, tail, L.ctl);
         TDT_LAUNCH_CHECK("list_decide");
@@ -2056,23 +2067,23 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     prof_mark(3, st);
 
     if (mode == 0) {
-        // outputs: truss numbers, then e_truss / ptr_truss from a stable sort by round
-        uint32_t* keys = reinterpret_cast<uint32_t*>(L.qi[0]);
-        uint32_t* vals = keys + E;
-        uint32_t* keys_alt = reinterpret_cast<uint32_t*>(L.qi[1]);
-        uint32_t* vals_alt = keys_alt + E;
-        truss_out_kernel<<<g_e, tb, 0, st>>>(L.rnd, L.round_level, E, truss, keys, vals, L.ctl);
+        // outputs: truss numbers, then e_truss / ptr_truss from a stable sort of
+        // the edges by round (as many passes as the rounds have digits)
+        uint32_t* k0 = reinterpret_cast<uint32_t*>(L.qi[0]);
+        uint32_t* v0 = k0 + E;
+        uint32_t* k1 = reinterpret_cast<uint32_t*>(L.qi[1]);
+        uint32_t* v1 = k1 + E;
+        int passes = 1;
+        while (passes < 4 && ((int64_t)1 << (8 * passes)) < E + 2) passes++;
+        const RadixScratch R = radix_scratch(L.sort_ws, E, passes);
+        TDT_CUDA(cudaMemsetAsync(R.hist, 0, R.bytes, st));
+        truss_out_kernel<<<g_e, tb, 0, st>>>(L.rnd, L.round_level, E, truss, passes, R.hist, L.ctl);
         TDT_LAUNCH_CHECK("truss_out");
-        const uint32_t* sk = keys;
-        const uint32_t* sv = vals;
-        int bits = 8;
-        while (bits < 32 && ((int64_t)1 << bits) < E + 2) bits += 8;
-        bool in_alt = false;
-        rc = radix_sort_pairs<uint32_t>(keys, vals, keys_alt, vals_alt, E, 0, bits, L.sort_ws, &in_alt, st);
+        rc = radix_sort<uint32_t, true>(reinterpret_cast<const uint32_t*>(L.rnd), k0, k1, v0, v1, E, passes, R, nullptr,
+                                        &L.ctl->rounds, &L.ctl->g.status, st);
         if (rc) return rc;
-        if (in_alt) { sk = keys_alt; sv = vals_alt; }
-        ptr_etruss_kernel<<<g_e, tb, 0, st>>>(sk, sv, E, L.round_level, ptr_truss, ptr_cap, e_truss, L.ctl,
-                                               stats);
+        ptr_etruss_kernel<<<g_e, tb, 0, st>>>(k0, v0, k1, v1, passes, E, L.round_level, ptr_truss, ptr_cap, e_truss,
+                                              L.ctl, stats);
         TDT_LAUNCH_CHECK("ptr_etruss");
         stats_final_kernel<<<1, 1, 0, st>>>(L.ctl, stats, 0);
         TDT_LAUNCH_CHECK("stats_final");

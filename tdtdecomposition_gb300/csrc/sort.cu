@@ -1,12 +1,11 @@
 // Device-wide exclusive scan and stable LSD radix sort (8-bit digits).
 //
-// Scan: reduce -> scan of block totals -> scan with offsets (three launches).
-// Radix sort pass: (1) per-tile digit histogram, (2) exclusive scan of the
-// digit-major histogram table, (3) per-tile stable ranking with
-// __match_any_sync (warp multisplit), staging in shared memory and coalesced
-// scatter.  Keys are stable across passes, so sorting (key, value) pairs
-// whose values arrive in ascending order gives ascending values per key.
-#include "common.cuh"
+// Both are single-pass: a tile publishes its totals and finds its start by
+// looking back over the tiles before it (tiles are handed out in order, so the
+// tiles waited for are running).  The scan is one launch instead of three; a
+// sort pass is one launch instead of five, and reads its keys once instead of
+// twice, with no digit table of all tiles to scan between.  A pass over 67 M
+// 64-bit keys: 600 -> 400 us (bound: 16 bytes a key, 160 us).
 #include "sort.cuh"
 
 namespace tdt {
@@ -36,244 +35,236 @@ __device__ __forceinline__ T block_excl_scan(T v, T* s_warp, T* total) {
 }
 
 template <class TI, class TO>
-__global__ void __launch_bounds__(kScanBlock) scan_reduce_kernel(const TI* __restrict__ in, int64_t n,
-                                                                 TO* __restrict__ partial) {
+__global__ void __launch_bounds__(kScanBlock) scan_kernel(const TI* in, int64_t n, TO* out, TO* total_out,
+                                                          unsigned long long* words, unsigned* next, int* status) {
+    using W = TileWord<unsigned long long>;
     __shared__ TO s_warp[33];
-    int64_t base = (int64_t)blockIdx.x * kScanTile;
-    TO sum = 0;
-#pragma unroll
-    for (int k = 0; k < kScanItems; k++) {
-        int64_t i = base + (int64_t)k * kScanBlock + threadIdx.x;
-        if (i < n) sum += (TO)in[i];
-    }
-    TO tot;
-    block_excl_scan<TO>(sum, s_warp, &tot);
-    if (threadIdx.x == 0) partial[blockIdx.x] = tot;
-}
-
-template <class TO>
-__global__ void __launch_bounds__(kScanBlock) scan_partials_kernel(TO* partial, int64_t nb) {
-    __shared__ TO s_warp[33];
-    TO carry = 0;
-    for (int64_t b0 = 0; b0 < nb; b0 += kScanBlock) {
-        int64_t i = b0 + threadIdx.x;
-        TO v = i < nb ? partial[i] : TO(0);
-        TO tot;
-        TO ex = block_excl_scan<TO>(v, s_warp, &tot);
-        if (i < nb) partial[i] = carry + ex;
-        carry += tot;
-    }
-}
-
-template <class TI, class TO>
-__global__ void __launch_bounds__(kScanBlock) scan_final_kernel(const TI* __restrict__ in, int64_t n,
-                                                                const TO* __restrict__ partial,
-                                                                TO* __restrict__ out, TO* total_out) {
-    __shared__ TO s_warp[33];
-    const int64_t base = (int64_t)blockIdx.x * kScanTile;
-    // blocked arrangement: thread t owns items base + t*kScanItems ...
+    __shared__ unsigned s_tile;
+    __shared__ unsigned long long s_before;
+    if (threadIdx.x == 0) s_tile = atomicAdd(next, 1u);
+    __syncthreads();
+    const int64_t tile = s_tile;
+    const int64_t base = tile * kScanTile + (int64_t)threadIdx.x * kScanItems;
     TO v[kScanItems];
     TO sum = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        int64_t i = base + (int64_t)threadIdx.x * kScanItems + k;
-        v[k] = i < n ? (TO)in[i] : TO(0);
+        v[k] = base + k < n ? (TO)in[base + k] : TO(0);
         sum += v[k];
     }
     TO tot;
-    TO run = partial[blockIdx.x] + block_excl_scan<TO>(sum, s_warp, &tot);
+    TO run = block_excl_scan<TO>(sum, s_warp, &tot);
+    if (threadIdx.x < kWarp) {
+        if (threadIdx.x == 0)
+            *(volatile unsigned long long*)(words + tile) =
+                (tile == 0 ? W::kInclusive : W::kAggregate) | (unsigned long long)tot;
+        const unsigned long long before = warp_look_back(words, tile, status);
+        if (threadIdx.x == 0) {
+            if (tile > 0)
+                *(volatile unsigned long long*)(words + tile) =
+                    W::kInclusive | ((before + (unsigned long long)tot) & W::kValue);
+            s_before = before;
+        }
+    }
+    __syncthreads();
+    run += (TO)s_before;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        int64_t i = base + (int64_t)threadIdx.x * kScanItems + k;
-        if (i < n) out[i] = run;
+        if (base + k < n) out[base + k] = run;
         run += v[k];
     }
-    if (total_out && blockIdx.x == gridDim.x - 1 && threadIdx.x == kScanBlock - 1) *total_out = run;
+    if (total_out && tile == (int64_t)gridDim.x - 1 && threadIdx.x == kScanBlock - 1) *total_out = run;
 }
 
 size_t scan_scratch_bytes(int64_t n) {
-    int64_t nb = (n + kScanTile - 1) / kScanTile;
+    const int64_t nb = (n + kScanTile - 1) / kScanTile;
     return (size_t)(nb + 1) * 8 + 256;
 }
 
-// out[i] = sum(in[0..i)), and *total_out (device, may be null) = sum(in).
-// `in` and `out` may alias.
 template <class TI, class TO>
-int exclusive_scan(const TI* in, TO* out, int64_t n, TO* total_out, void* scratch, cudaStream_t st) {
+int exclusive_scan(const TI* in, TO* out, int64_t n, TO* total_out, void* scratch, int* status, cudaStream_t st) {
     if (n <= 0) {
         if (total_out) TDT_CUDA(cudaMemsetAsync(total_out, 0, sizeof(TO), st));
         return TDT_OK;
     }
-    int64_t nb = (n + kScanTile - 1) / kScanTile;
-    TO* partial = reinterpret_cast<TO*>(scratch);
-    scan_reduce_kernel<TI, TO><<<(unsigned)nb, kScanBlock, 0, st>>>(in, n, partial);
-    TDT_LAUNCH_CHECK("scan_reduce");
-    scan_partials_kernel<TO><<<1, kScanBlock, 0, st>>>(partial, nb);
-    TDT_LAUNCH_CHECK("scan_partials");
-    scan_final_kernel<TI, TO><<<(unsigned)nb, kScanBlock, 0, st>>>(in, n, partial, out, total_out);
-    TDT_LAUNCH_CHECK("scan_final");
+    const int64_t nb = (n + kScanTile - 1) / kScanTile;
+    unsigned long long* words = reinterpret_cast<unsigned long long*>(scratch);
+    TDT_CUDA(cudaMemsetAsync(words, 0, (size_t)(nb + 1) * 8, st));
+    scan_kernel<TI, TO><<<(unsigned)nb, kScanBlock, 0, st>>>(in, n, out, total_out, words,
+                                                            reinterpret_cast<unsigned*>(words + nb), status);
+    TDT_LAUNCH_CHECK("scan");
     return TDT_OK;
 }
 
-template int exclusive_scan<int32_t, int64_t>(const int32_t*, int64_t*, int64_t, int64_t*, void*, cudaStream_t);
-template int exclusive_scan<int64_t, int64_t>(const int64_t*, int64_t*, int64_t, int64_t*, void*, cudaStream_t);
-template int exclusive_scan<uint32_t, uint32_t>(const uint32_t*, uint32_t*, int64_t, uint32_t*, void*,
-                                                cudaStream_t);
-template int exclusive_scan<int32_t, int32_t>(const int32_t*, int32_t*, int64_t, int32_t*, void*, cudaStream_t);
+template int exclusive_scan<int32_t, int64_t>(const int32_t*, int64_t*, int64_t, int64_t*, void*, int*, cudaStream_t);
+template int exclusive_scan<int64_t, int64_t>(const int64_t*, int64_t*, int64_t, int64_t*, void*, int*, cudaStream_t);
 
 // ------------------------------------------------------------------ radix sort
-constexpr int kSortBlock = 256;
+constexpr int kSortBlock = 256;   // one thread per digit
 constexpr int kSortWarps = kSortBlock / kWarp;
-constexpr int kRadix = 256;
-// keys per thread: the staging tile (keys + values) stays within 48 KB static smem
-template <class K>
-struct SortCfg {
-    static constexpr int items = sizeof(K) == 8 ? 8 : 16;
-    static constexpr int tile = kSortBlock * items;  // 2048 (64-bit) or 4096 (32-bit) keys
-};
+static_assert(kSortBlock == kRadix, "one thread per digit");
+// Keys per thread, blocks per SM and tiles looked back on at a time (67 M draws
+// / 65,536 draws preprocessed: 7.62 ms / 312 us with 12, 5, 4; 7.53 / 352 with
+// 16, 4, 4; 8.38 / 317 with 8, 6, 4; 8.26 / 362 with 16, 4, 1).
+constexpr int kSortItems = 12;
+constexpr int kSortMinBlocks = 5;
+constexpr int kBack = 4;
+constexpr int kSortTile = kSortBlock * kSortItems;
+// counts fit 30 bits below this many keys
+constexpr int64_t kWideKeys = 1ll << 30;
 
-template <class K>
-__global__ void __launch_bounds__(kSortBlock) radix_hist_kernel(const K* __restrict__ keys, int64_t n,
-                                                                int shift, uint32_t* __restrict__ hist,
-                                                                int64_t ntiles) {
-    __shared__ uint32_t s_h[kRadix];
-    for (int i = threadIdx.x; i < kRadix; i += kSortBlock) s_h[i] = 0;
-    __syncthreads();
-    constexpr int kSortItems = SortCfg<K>::items;
-    const int64_t base = (int64_t)blockIdx.x * SortCfg<K>::tile;
-#pragma unroll 4
-    for (int k = 0; k < kSortItems; k++) {
-        int64_t i = base + (int64_t)k * kSortBlock + threadIdx.x;
-        if (i < n) atomicAdd(&s_h[(unsigned)((keys[i] >> shift) & 0xff)], 1u);
-    }
-    __syncthreads();
-    for (int d = threadIdx.x; d < kRadix; d += kSortBlock) hist[(int64_t)d * ntiles + blockIdx.x] = s_h[d];
-}
-
-template <class K, bool kHasVals>
-__global__ void __launch_bounds__(kSortBlock) radix_scatter_kernel(
+template <class K, class S, bool kVals, bool kIota>
+__global__ void __launch_bounds__(kSortBlock, kSortMinBlocks) radix_pass_kernel(
     const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, K* __restrict__ keys_out,
-    uint32_t* __restrict__ vals_out, int64_t n, int shift, const uint32_t* __restrict__ hist_scan,
-    int64_t ntiles) {
-    constexpr int kSortItems = SortCfg<K>::items;
-    constexpr int kSortTile = SortCfg<K>::tile;
-    __shared__ uint32_t s_wcnt[kSortWarps][kRadix];
-    __shared__ uint32_t s_tile_start[kRadix];
-    __shared__ uint32_t s_warp_tmp[33];
-    __shared__ K s_keys[kSortTile];
-    __shared__ uint32_t s_vals[kHasVals ? kSortTile : 1];
+    uint32_t* __restrict__ vals_out, int64_t n, int pass, const uint32_t* __restrict__ hist,
+    uint32_t* tile_next, S* words, const uint32_t* n_dev, const long long* max_dev, int* status) {
+    using W = TileWord<S>;
+    if (max_dev && pass > 0 && (*max_dev >> (8 * pass)) == 0) return;
+    if (n_dev) n = *n_dev < n ? (int64_t)*n_dev : n;
+    extern __shared__ __align__(16) unsigned char smem[];
+    K* s_keys = reinterpret_cast<K*>(smem);
+    uint32_t* s_vals = reinterpret_cast<uint32_t*>(smem + sizeof(K) * kSortTile);
+    __shared__ uint32_t s_wcnt[kSortWarps][kRadix];  // per warp: counts, then first places in the tile
+    __shared__ uint32_t s_to[kRadix];      // first place of the digit in the output minus that in the tile (mod 2^32)
+    __shared__ uint32_t s_tmp[33];
+    __shared__ unsigned s_tile;
     const int w = threadIdx.x / kWarp;
     const unsigned lane = lane_id();
+    const int shift = 8 * pass;
+    if (threadIdx.x == 0) s_tile = atomicAdd(tile_next, 1u);
     for (int i = lane; i < kRadix; i += kWarp) s_wcnt[w][i] = 0;
-    __syncwarp();
-    const int64_t base = (int64_t)blockIdx.x * kSortTile;
-    // warp w owns the contiguous sub-tile [w*kSortItems*32, (w+1)*kSortItems*32)
+    __syncthreads();
+    const int64_t tile = s_tile;
+    const int64_t base = tile * kSortTile;
+    if (base >= n) return;
+    // warp w owns the contiguous sub-tile of kSortItems * 32 keys; ranks among
+    // its keys of the same digit
     K key[kSortItems];
-    uint32_t val[kSortItems];
-    uint32_t rank[kSortItems];
+    uint32_t val[kVals ? kSortItems : 1];
+    uint16_t rank[kSortItems];
+    const int64_t mine = base + (int64_t)w * (kSortItems * kWarp) + lane;
 #pragma unroll
     for (int it = 0; it < kSortItems; it++) {
-        const int64_t i = base + (int64_t)w * (kSortItems * kWarp) + it * kWarp + lane;
-        const bool ok = i < n;
-        key[it] = ok ? keys_in[i] : K(0);
-        if (kHasVals) val[it] = ok ? vals_in[i] : 0u;
+        const int64_t i = mine + it * kWarp;
+        key[it] = i < n ? keys_in[i] : K(0);
+        if (kVals) val[it] = kIota ? (uint32_t)i : (i < n ? vals_in[i] : 0u);
+    }
+    // the first lane of a step's equal digits counts them in the warp's row, and
+    // all of them rank from its result
+#pragma unroll
+    for (int it = 0; it < kSortItems; it++) {
+        const bool ok = mine + it * kWarp < n;
         const unsigned d = ok ? (unsigned)((key[it] >> shift) & 0xff) : (unsigned)kRadix;
         const unsigned peers = __match_any_sync(kFull, d);
-        const unsigned leader = __ffs(peers) - 1;
+        const int first = __ffs(peers) - 1;
         uint32_t pre = 0;
-        if (ok) pre = s_wcnt[w][d];
+        if (ok && (int)lane == first) pre = atomicAdd(&s_wcnt[w][d], (uint32_t)__popc(peers));
+        rank[it] = (uint16_t)(__shfl_sync(kFull, pre, first) + __popc(peers & lanemask_lt()));
         __syncwarp();
-        if (ok && lane == leader) s_wcnt[w][d] = pre + __popc(peers);
-        __syncwarp();
-        rank[it] = ok ? pre + __popc(peers & lanemask_lt()) : 0xffffffffu;
     }
     __syncthreads();
-    // per digit: exclusive offsets across warps, then across digits
-    uint32_t tile_cnt = 0;
-    if (threadIdx.x < kRadix) {
-        const int d = threadIdx.x;
-        uint32_t run = 0;
+    const int d = threadIdx.x;
+    uint32_t cnt = 0;
 #pragma unroll
-        for (int ww = 0; ww < kSortWarps; ww++) {
-            uint32_t c = s_wcnt[ww][d];
-            s_wcnt[ww][d] = run;
-            run += c;
-        }
-        tile_cnt = run;
+    for (int ww = 0; ww < kSortWarps; ww++) cnt += s_wcnt[ww][d];
+    S* mine_w = words + tile * kRadix + d;
+    *(volatile S*)mine_w = (tile == 0 ? W::kInclusive : W::kAggregate) | (S)cnt;
+    // the digit's first place in the tile, for each warp, and in the output
+    const uint32_t start = block_excl_scan<uint32_t>(cnt, s_tmp, nullptr);
+    uint32_t run = start;
+#pragma unroll
+    for (int ww = 0; ww < kSortWarps; ww++) {
+        const uint32_t c = s_wcnt[ww][d];
+        s_wcnt[ww][d] = run;
+        run += c;
     }
-    uint32_t tot;
-    uint32_t start = block_excl_scan<uint32_t>(tile_cnt, s_warp_tmp, &tot);
-    if (threadIdx.x < kRadix) s_tile_start[threadIdx.x] = start;
-    __syncthreads();
+    const uint32_t digit0 = block_excl_scan<uint32_t>(__ldg(hist + d), s_tmp, nullptr);
 #pragma unroll
     for (int it = 0; it < kSortItems; it++) {
-        if (rank[it] != 0xffffffffu) {
-            const unsigned d = (unsigned)((key[it] >> shift) & 0xff);
-            const uint32_t p = s_tile_start[d] + s_wcnt[w][d] + rank[it];
+        if (mine + it * kWarp < n) {
+            const uint32_t p = s_wcnt[w][(unsigned)((key[it] >> shift) & 0xff)] + rank[it];
             s_keys[p] = key[it];
-            if (kHasVals) s_vals[p] = val[it];
+            if (kVals) s_vals[p] = val[it];
         }
     }
+    S before = 0;
+    if (tile > 0) {
+        // the rows of words of the tiles before, kBack of them in flight
+        bool more = true;
+        for (int64_t t = tile - 1; more && t >= 0; t -= kBack) {
+            S x[kBack];
+#pragma unroll
+            for (int j = 0; j < kBack; j++) x[j] = t - j >= 0 ? *(const volatile S*)(words + (t - j) * kRadix + d) : S(0);
+#pragma unroll
+            for (int j = 0; j < kBack; j++) {
+                if (!more || t - j < 0) continue;
+                if (x[j] == 0) x[j] = tile_word_wait(words + (t - j) * kRadix + d, status);
+                before += x[j] & W::kValue;
+                more = (x[j] & W::kInclusive) == 0;
+            }
+        }
+        *(volatile S*)mine_w = W::kInclusive | ((before + (S)cnt) & W::kValue);
+    }
+    s_to[d] = digit0 + (uint32_t)before - start;
     __syncthreads();
-    const int64_t tile_n = min((int64_t)kSortTile, n - base);
+    const int tile_n = (int)(n - base < kSortTile ? n - base : kSortTile);
     for (int i = threadIdx.x; i < tile_n; i += kSortBlock) {
         const K k = s_keys[i];
-        const unsigned d = (unsigned)((k >> shift) & 0xff);
-        const int64_t g = (int64_t)hist_scan[(int64_t)d * ntiles + blockIdx.x] + (i - s_tile_start[d]);
-        keys_out[g] = k;
-        if (kHasVals) vals_out[g] = s_vals[i];
+        const uint32_t g = s_to[(unsigned)((k >> shift) & 0xff)] + (uint32_t)i;
+        if (g < n) {
+            keys_out[g] = k;
+            if (kVals) vals_out[g] = s_vals[i];
+        }
     }
 }
 
-size_t radix_sort_scratch_bytes(int64_t n) {
-    int64_t ntiles = (n + SortCfg<uint32_t>::tile - 1) / SortCfg<uint32_t>::tile;
-    int64_t ntiles64 = (n + SortCfg<uint64_t>::tile - 1) / SortCfg<uint64_t>::tile;
-    if (ntiles64 > ntiles) ntiles = ntiles64;
-    int64_t hn = ntiles * kRadix;
-    return (size_t)hn * 4 + scan_scratch_bytes(hn) + 512;
+RadixScratch radix_scratch(void* base, int64_t n, int passes) {
+    const size_t ntiles = (size_t)((n + kSortTile - 1) / kSortTile);
+    const size_t head = ((size_t)kMaxPasses * kRadix + kMaxPasses) * 4 + 224;  // a multiple of 256
+    const size_t word = n < kWideKeys ? 4 : 8;
+    RadixScratch R;
+    R.hist = reinterpret_cast<uint32_t*>(base);
+    R.tile_next = base ? R.hist + kMaxPasses * kRadix : nullptr;
+    R.words = base ? (void*)(reinterpret_cast<char*>(base) + head) : nullptr;
+    R.bytes = head + (size_t)passes * ntiles * kRadix * word;
+    return R;
 }
 
-// Stable sort of (keys, vals) by key bits [begin_bit, end_bit).  Ping-pongs
-// between (keys, vals) and (keys_alt, vals_alt); the result ends in the pair
-// returned through *result_in_alt.  vals may be null (keys only).
-template <class K>
-int radix_sort_pairs(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, int64_t n,
-                     int begin_bit, int end_bit, void* scratch, bool* result_in_alt, cudaStream_t st) {
-    *result_in_alt = false;
-    if (n <= 1) return TDT_OK;
-    TDT_CHECK_ARG(n < (int64_t)UINT32_MAX, "radix sort of %lld keys exceeds 32-bit ranks", (long long)n);
-    const int64_t ntiles = (n + SortCfg<K>::tile - 1) / SortCfg<K>::tile;
-    const int64_t hn = ntiles * kRadix;
-    uint32_t* hist = reinterpret_cast<uint32_t*>(scratch);
-    void* scan_ws = reinterpret_cast<char*>(scratch) + ((hn * 4 + 255) / 256) * 256;
-    K* src_k = keys;
-    uint32_t* src_v = vals;
-    K* dst_k = keys_alt;
-    uint32_t* dst_v = vals_alt;
-    bool alt = false;
-    for (int shift = begin_bit; shift < end_bit; shift += 8) {
-        radix_hist_kernel<K><<<(unsigned)ntiles, kSortBlock, 0, st>>>(src_k, n, shift, hist, ntiles);
-        TDT_LAUNCH_CHECK("radix_hist");
-        int rc = exclusive_scan<uint32_t, uint32_t>(hist, hist, hn, nullptr, scan_ws, st);
-        if (rc) return rc;
-        if (vals)
-            radix_scatter_kernel<K, true><<<(unsigned)ntiles, kSortBlock, 0, st>>>(
-                src_k, src_v, dst_k, dst_v, n, shift, hist, ntiles);
-        else
-            radix_scatter_kernel<K, false><<<(unsigned)ntiles, kSortBlock, 0, st>>>(
-                src_k, nullptr, dst_k, nullptr, n, shift, hist, ntiles);
-        TDT_LAUNCH_CHECK("radix_scatter");
-        K* tk = src_k; src_k = dst_k; dst_k = tk;
-        uint32_t* tv = src_v; src_v = dst_v; dst_v = tv;
-        alt = !alt;
+template <class K, class S, bool kVals>
+static int radix_passes(const K* in, K* b0, K* b1, uint32_t* v0, uint32_t* v1, int64_t n, int passes,
+                        const RadixScratch& R, const uint32_t* n_dev, const long long* max_dev, int* status,
+                        cudaStream_t st) {
+    const int64_t ntiles = (n + kSortTile - 1) / kSortTile;
+    const int smem = (int)(sizeof(K) + (kVals ? 4 : 0)) * kSortTile;
+    S* words = reinterpret_cast<S*>(R.words);
+    for (int p = 0; p < passes; p++) {
+        auto kern = kVals && p == 0 ? radix_pass_kernel<K, S, kVals, true> : radix_pass_kernel<K, S, kVals, false>;
+        TDT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        const K* kin = p == 0 ? in : (p & 1) ? b0 : b1;
+        const uint32_t* vin = (p & 1) ? v0 : v1;
+        kern<<<(unsigned)ntiles, kSortBlock, smem, st>>>(kin, vin, (p & 1) ? b1 : b0, (p & 1) ? v1 : v0, n, p,
+                                                        R.hist + p * kRadix, R.tile_next + p,
+                                                        words + (size_t)p * ntiles * kRadix, n_dev, max_dev, status);
+        TDT_LAUNCH_CHECK("radix_pass");
     }
-    *result_in_alt = alt;
     return TDT_OK;
 }
 
-template int radix_sort_pairs<uint32_t>(uint32_t*, uint32_t*, uint32_t*, uint32_t*, int64_t, int, int, void*,
-                                        bool*, cudaStream_t);
-template int radix_sort_pairs<uint64_t>(uint64_t*, uint32_t*, uint64_t*, uint32_t*, int64_t, int, int, void*,
-                                        bool*, cudaStream_t);
+template <class K, bool kVals>
+int radix_sort(const K* in, K* b0, K* b1, uint32_t* v0, uint32_t* v1, int64_t n, int passes, const RadixScratch& R,
+               const uint32_t* n_dev, const long long* max_dev, int* status, cudaStream_t st) {
+    if (n <= 0) return TDT_OK;
+    TDT_CHECK_ARG(n < (int64_t)UINT32_MAX, "radix sort of %lld keys exceeds 32-bit ranks", (long long)n);
+    TDT_CHECK_ARG(passes >= 1 && passes <= kMaxPasses, "%d radix passes", passes);
+    return n < kWideKeys
+               ? radix_passes<K, uint32_t, kVals>(in, b0, b1, v0, v1, n, passes, R, n_dev, max_dev, status, st)
+               : radix_passes<K, unsigned long long, kVals>(in, b0, b1, v0, v1, n, passes, R, n_dev, max_dev, status,
+                                                            st);
+}
+
+template int radix_sort<uint32_t, true>(const uint32_t*, uint32_t*, uint32_t*, uint32_t*, uint32_t*, int64_t, int,
+                                        const RadixScratch&, const uint32_t*, const long long*, int*, cudaStream_t);
+template int radix_sort<uint64_t, false>(const uint64_t*, uint64_t*, uint64_t*, uint32_t*, uint32_t*, int64_t, int,
+                                         const RadixScratch&, const uint32_t*, const long long*, int*, cudaStream_t);
 
 }  // namespace tdt

@@ -4,15 +4,113 @@
 #include <stdint.h>
 #include <stddef.h>
 
+#include "common.cuh"
+
 namespace tdt {
 
-size_t scan_scratch_bytes(int64_t n);
-template <class TI, class TO>
-int exclusive_scan(const TI* in, TO* out, int64_t n, TO* total_out, void* scratch, cudaStream_t st);
+// ------------------------------------------------------------------ look-back
+// A tile's status word: its aggregate, then its inclusive prefix, in the low
+// bits under two flag bits.  Words are zero before the pass.
+template <class S>
+struct TileWord {
+    static constexpr S kAggregate = S(1) << (8 * sizeof(S) - 2);
+    static constexpr S kInclusive = S(2) << (8 * sizeof(S) - 2);
+    static constexpr S kValue = kAggregate - 1;
+};
 
-size_t radix_sort_scratch_bytes(int64_t n);
-template <class K>
-int radix_sort_pairs(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, int64_t n, int begin_bit,
-                     int end_bit, void* scratch, bool* result_in_alt, cudaStream_t st);
+// Wait limit of a look-back on a tile that has not published (tiles are handed
+// out in order, so the awaited block is running); past it the waiter records
+// TDT_ERR_TIMEOUT and goes on, and the caller's result is rejected.
+constexpr uint64_t kLookBackTimeoutNs = 2ull * 1000ull * 1000ull * 1000ull;
+
+template <class S>
+__device__ __forceinline__ S tile_word_wait(const S* p, int* status) {
+    S w = *(const volatile S*)p;
+    if (w) return w;
+    const uint64_t t0 = globaltimer_ns();
+    for (unsigned spins = 1;; spins++) {
+        w = *(const volatile S*)p;
+        if (w) return w;
+        if ((spins & 63u) == 0 && globaltimer_ns() - t0 > kLookBackTimeoutNs) {
+            if (status) atomicMax(status, (int)TDT_ERR_TIMEOUT);
+            return TileWord<S>::kInclusive;
+        }
+    }
+}
+
+// Sum of the tiles before `tile`, by one whole warp: 32 predecessors at a time
+// (words[t] is tile t's).  Lane 0 has published the tile's aggregate.
+template <class S>
+__device__ __forceinline__ S warp_look_back(const S* words, int64_t tile, int* status) {
+    using W = TileWord<S>;
+    S sum = 0;
+    for (int64_t t = tile - 1; t >= 0; t -= kWarp) {
+        const int64_t mine = t - (int64_t)lane_id();
+        const S w = mine >= 0 ? tile_word_wait(words + mine, status) : W::kInclusive;
+        const unsigned inc = __ballot_sync(kFull, (w & W::kInclusive) != 0);
+        const int last = inc ? __ffs(inc) - 1 : kWarp - 1;  // nearest inclusive prefix
+        sum += warp_sum((int)lane_id() <= last ? (S)(w & W::kValue) : S(0));
+        if (inc) break;
+    }
+    return sum;
+}
+
+size_t scan_scratch_bytes(int64_t n);
+// out[i] = sum(in[0..i)), and *total_out (device, may be null) = sum(in).  in
+// and out may alias.  status: receives TDT_ERR_TIMEOUT (may be null).
+template <class TI, class TO>
+int exclusive_scan(const TI* in, TO* out, int64_t n, TO* total_out, void* scratch, int* status, cudaStream_t st);
+
+// ------------------------------------------------------------------ radix sort
+// Stable LSD sort by 8-bit digits, one launch per pass: the digit totals of
+// every pass come from the kernel that makes the keys (DigitHist), and a tile
+// finds where its digits go by looking back over the tiles before it, so a
+// pass reads and writes each key once.
+constexpr int kRadix = 256;
+constexpr int kMaxPasses = 8;
+
+// Scratch of one sort, zeroed by radix_zero before the key kernel runs.
+struct RadixScratch {
+    uint32_t* hist;        // [passes][256]
+    uint32_t* tile_next;   // [passes]
+    void* words;           // [passes][tiles][256]
+    size_t bytes;          // of the whole, from hist on
+};
+RadixScratch radix_scratch(void* base, int64_t n, int passes);  // base may be null (sizes only)
+
+// Digit totals of a key kernel's keys: init, add per key, flush by the block.
+struct DigitHist {
+    uint32_t* s;           // shared memory, kMaxPasses * kRadix words
+    __device__ __forceinline__ void init(int passes) {
+        for (int i = threadIdx.x; i < passes * kRadix; i += blockDim.x) s[i] = 0u;
+        __syncthreads();
+    }
+    template <class K>
+    __device__ __forceinline__ void add(K key, int passes) {
+        for (int p = 0; p < passes; p++) atomicAdd(s + p * kRadix + (unsigned)((key >> (8 * p)) & 0xff), 1u);
+    }
+    __device__ __forceinline__ void flush(int passes, uint32_t* hist) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < passes * kRadix; i += blockDim.x)
+            if (s[i]) atomicAdd(hist + i, s[i]);
+    }
+};
+
+// Sorts n keys by their low 8 * passes bits.  in may be another array than the
+// two that the passes alternate between (pass 0 writes b0, pass 1 b1, ...); the
+// sorted keys are in radix_result.  vals: with kVals the values are the keys'
+// indices at first.  n_dev (may be null): the number of keys, at most n, read on
+// the device.  max_dev (may be null): passes above the highest set digit of
+// *max_dev do nothing, and the result is in the buffer of the last pass that
+// ran (radix_passes_run).
+template <class K, bool kVals>
+int radix_sort(const K* in, K* b0, K* b1, uint32_t* v0, uint32_t* v1, int64_t n, int passes, const RadixScratch& R,
+               const uint32_t* n_dev, const long long* max_dev, int* status, cudaStream_t st);
+
+__host__ __device__ inline int radix_passes_run(int passes, long long max_key) {
+    int p = 1;
+    while (p < passes && (max_key >> (8 * p)) != 0) p++;
+    return p;
+}
 
 }  // namespace tdt
