@@ -72,6 +72,7 @@ struct PeelCtl {
     // processing, and level transitions; diagnostic only
     unsigned long long t_proc, t_wait, t_trans, t_total;
     unsigned long long grab[4];    // slot cursor of search-mode sub-round r, at r & 3
+    unsigned done;                 // blocks of a triangle count that finished
 };
 
 // How the peel finds an edge's triangles: in its list, by search in the graph's
@@ -1483,18 +1484,17 @@ __global__ void __launch_bounds__(kPeelBlock, TDT_PEEL_MINB) peel_kernel(const _
 }
 
 // ------------------------------------------------------------------ setup / output kernels
-__global__ void rows_from_rp_kernel(const int64_t* __restrict__ rp, int64_t V, int32_t* __restrict__ rows) {
-    const unsigned lane = lane_id();
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t u = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; u < V; u += nw) {
-        const int64_t b = rp[u], e = rp[u + 1];
-        for (int64_t i = b + lane; i < e; i += kWarp) rows[i] = (int32_t)u;
-    }
-}
-
 // Input validation, before any kernel indexes through the graph:
 // row_ptr[0] == 0, row_ptr[V] == E, non-decreasing; rows[e] is the row that
 // owns position e; u < v < V; columns strictly increasing within a row.
+__device__ __forceinline__ int validate_edge(const int32_t* __restrict__ cols, int64_t e, int64_t u, int64_t b,
+                                             int64_t en, int64_t V) {
+    const int32_t v = cols[e];
+    if (u < 0 || u >= V || v >= V || u >= v) return TDT_ERR_NOT_ORIENTED;
+    if (e < b || e >= en) return TDT_ERR_INVALID;
+    return e + 1 < en && cols[e + 1] <= v ? TDT_ERR_INVALID : TDT_OK;
+}
+
 __global__ void validate_kernel(const int64_t* __restrict__ rp, const int32_t* __restrict__ rows,
                                 const int32_t* __restrict__ cols, int64_t E, int64_t V, PeelCtl* ctl) {
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -1503,17 +1503,32 @@ __global__ void validate_kernel(const int64_t* __restrict__ rp, const int32_t* _
     for (int64_t u = tid; u < V; u += nth)
         if (rp[u] > rp[u + 1]) atomicMax(&ctl->g.status, (int)TDT_ERR_INVALID);
     for (int64_t e = tid; e < E; e += nth) {
-        const int32_t u = rows[e], v = cols[e];
-        if (u < 0 || u >= V || v >= V || u >= v) {
-            atomicMax(&ctl->g.status, (int)TDT_ERR_NOT_ORIENTED);
-            continue;
-        }
+        const int32_t u = rows[e];
+        const bool in = u >= 0 && u < V;
+        const int err = validate_edge(cols, e, u, in ? rp[u] : 0, in ? rp[u + 1] : 0, V);
+        if (err) atomicMax(&ctl->g.status, err);
+    }
+}
+
+// The same when the caller gave no rows: a warp per row writes them, inside
+// [0, E) whatever row_ptr says.
+__global__ void validate_rows_kernel(const int64_t* __restrict__ rp, int32_t* __restrict__ rows,
+                                     const int32_t* __restrict__ cols, int64_t E, int64_t V, PeelCtl* ctl) {
+    const unsigned lane = lane_id();
+    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    if (tid == 0 && (rp[0] != 0 || rp[V] != E)) atomicMax(&ctl->g.status, (int)TDT_ERR_INVALID);
+    for (int64_t u = tid >> 5; u < V; u += nw) {
         const int64_t b = rp[u], en = rp[u + 1];
-        if (e < b || e >= en) {
+        if (b > en || b < 0 || en > E) {
             atomicMax(&ctl->g.status, (int)TDT_ERR_INVALID);
             continue;
         }
-        if (e + 1 < en && cols[e + 1] <= v) atomicMax(&ctl->g.status, (int)TDT_ERR_INVALID);
+        for (int64_t e = b + lane; e < en; e += kWarp) {
+            rows[e] = (int32_t)u;
+            const int err = validate_edge(cols, e, u, b, en, V);
+            if (err) atomicMax(&ctl->g.status, err);
+        }
     }
 }
 
@@ -1565,11 +1580,12 @@ __global__ void __launch_bounds__(kCscBlock) indeg_kernel(const int32_t* __restr
         if (s_cnt[i]) atomicAdd(indeg + hot0 + i, s_cnt[i]);
 }
 
+// left: the in-degrees, counted down to zero as the in-lists fill from their ends.
 __global__ void __launch_bounds__(kCscBlock) csc_fill_kernel(const int32_t* __restrict__ rows,
                                                              const int32_t* __restrict__ cols, int64_t E, int64_t V,
                                                              int64_t tile,
                                                              const int64_t* __restrict__ cp,
-                                                             int32_t* __restrict__ cursor, int32_t* __restrict__ in_src,
+                                                             int32_t* __restrict__ left, int32_t* __restrict__ in_src,
                                                              int32_t* __restrict__ in_eid, const PeelCtl* ctl) {
     __shared__ int32_t s_cur[kCscHot];  // counts, then the next place of the block's run
     if (*(volatile const int*)&ctl->g.status != 0) return;
@@ -1584,11 +1600,12 @@ __global__ void __launch_bounds__(kCscBlock) csc_fill_kernel(const int32_t* __re
         });
         __syncthreads();
         for (int i = threadIdx.x; i < hot; i += kCscBlock)
-            if (s_cur[i]) s_cur[i] = (int32_t)__ldg(cp + hot0 + i) + atomicAdd(cursor + hot0 + i, s_cur[i]);
+            if (s_cur[i])
+                s_cur[i] = (int32_t)__ldg(cp + hot0 + i) + atomicSub(left + hot0 + i, s_cur[i]) - s_cur[i];
         __syncthreads();
         csc_edges(cols, e0, e1, [&](int64_t e, int32_t v) {
             const int32_t pos = v >= hot0 ? atomicAdd(s_cur + (v - hot0), 1)
-                                          : (int32_t)__ldg(cp + v) + atomicAdd(cursor + v, 1);
+                                          : (int32_t)__ldg(cp + v) + atomicSub(left + v, 1) - 1;
             in_src[pos] = __ldg(rows + e);
             in_eid[pos] = (int32_t)e;
         });
@@ -1596,27 +1613,33 @@ __global__ void __launch_bounds__(kCscBlock) csc_fill_kernel(const int32_t* __re
     }
 }
 
-// sup = cA + cB + cC (the role counts of the support pass), edge state =
-// {sup, alive}, triangle total.
+// sup = cA + cB + cC (the role counts of the walk) and the triangle total; for
+// a peel also the edge state (live = sup, no sub-round, code alive).  A count
+// (live null) ends here: sup is the caller's array or null, and the last block
+// writes the stats.
 __global__ void init_state_kernel(const int32_t* __restrict__ cA, const int32_t* __restrict__ cB,
                                   const int32_t* __restrict__ cC, int32_t* __restrict__ sup,
-                                  int32_t* __restrict__ live, int32_t* __restrict__ rnd, int64_t E,
-                                  PeelCtl* ctl) {
+                                  int32_t* __restrict__ live, int32_t* __restrict__ rnd,
+                                  unsigned* __restrict__ code, int64_t E, PeelCtl* ctl, int64_t* __restrict__ stats) {
     __shared__ long long s_part[32];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         for (int i = 0; i < 3; i++) ctl->mgt[i] = INT32_MAX;
         ctl->dmin[0] = INT32_MAX;
         ctl->dmin[1] = INT32_MAX;
     }
+    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, nth = (int64_t)gridDim.x * blockDim.x;
     long long acc = 0;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E;
-         e += (int64_t)gridDim.x * blockDim.x) {
+    for (int64_t e = tid; e < E; e += nth) {
         const int32_t s = cA[e] + cB[e] + cC[e];
-        sup[e] = s;
-        live[e] = s;
-        rnd[e] = -1;
+        if (sup) sup[e] = s;
+        if (live) {
+            live[e] = s;
+            rnd[e] = -1;
+        }
         acc += s;
     }
+    if (code)
+        for (int64_t i = tid; i < E / 8 + 1; i += nth) code[i] = ~0u;
     acc = warp_sum(acc);
     if (lane_id() == 0) s_part[threadIdx.x / kWarp] = acc;
     __syncthreads();
@@ -1624,14 +1647,15 @@ __global__ void init_state_kernel(const int32_t* __restrict__ cA, const int32_t*
         long long b = 0;
         for (int i = 0; i < (int)(blockDim.x / kWarp); i++) b += s_part[i];
         atomicAdd((unsigned long long*)&ctl->triangles, (unsigned long long)b);
+        if (!live) {
+            __threadfence();
+            if (atomicAdd(&ctl->done, 1u) == gridDim.x - 1) {
+                for (int i = 0; i < TDT_STAT_COUNT; i++) stats[i] = 0;
+                stats[TDT_STAT_STATUS] = *(volatile int*)&ctl->g.status;
+                stats[TDT_STAT_TRIANGLES] = (long long)atomicAdd((unsigned long long*)&ctl->triangles, 0ull) / 3;
+            }
+        }
     }
-}
-
-// One walk that counts and lists when the staging slots fit the list tail,
-// else a walk that only counts.
-__global__ void stage_decide_kernel(const int64_t* __restrict__ sbase, int64_t V, unsigned long long tail_bytes,
-                                    PeelCtl* ctl) {
-    ctl->stage_skip = !(ctl->g.status == 0 && (unsigned long long)sbase[V] <= tail_bytes / 8);
 }
 
 // Lists fit when 8 bytes x (3T = off[E]) fit the list tail.  After the one
@@ -1690,7 +1714,11 @@ __global__ void ptr_etruss_kernel(const uint32_t* __restrict__ k0, const uint32_
                                   int64_t E, const int32_t* __restrict__ round_level, int32_t* __restrict__ ptr_truss,
                                   int64_t ptr_cap, int32_t* __restrict__ e_truss, PeelCtl* ctl,
                                   int64_t* __restrict__ stats) {
-    if (*(volatile int*)&ctl->g.status != 0) return;
+    if (*(volatile int*)&ctl->g.status != 0) {  // before this kernel, or its own: then thread 0 goes on
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+            for (int i = 0; i < TDT_STAT_COUNT; i++) stats[i] = 0;
+        return;
+    }
     const long long rounds = ctl->rounds;
     const bool first = radix_passes_run(passes, rounds) & 1;
     const uint32_t* keys = first ? k0 : k1;
@@ -1738,9 +1766,14 @@ __global__ void ktruss_out_kernel(const int32_t* __restrict__ rnd, int64_t E, ui
     }
 }
 
+// The stats words that ptr_etruss_kernel leaves (mode 0), or all.
 __global__ void stats_final_kernel(PeelCtl* ctl, int64_t* stats, int mode) {
-    stats[TDT_STAT_STATUS] = ctl->g.status;
+    const int st = ctl->g.status;
+    if (mode != 0)
+        for (int i = 0; i < TDT_STAT_COUNT; i++) stats[i] = 0;
+    stats[TDT_STAT_STATUS] = st;
     stats[TDT_STAT_LISTED] = ctl->listed ? (ctl->compact_skip ? 1 : 2) : 0;
+    stats[TDT_STAT_ALIVE] = 0;
     if (mode != 0) {
         stats[TDT_STAT_ALIVE] = (long long)ctl->alive;
         stats[TDT_STAT_ROUNDS] = ctl->rounds;
@@ -1804,11 +1837,10 @@ int test_barrier_timeout(void* ws, long long limit_ns, cudaStream_t st) {
     return status;
 }
 
-int launch_stage_rows(const int64_t* rp, int64_t nv, int64_t* slots, const int* status, cudaStream_t st);
 int launch_walk_count(const int64_t* rp, const int32_t* cols, const int64_t* cp, const int32_t* in_src,
                       const int32_t* in_eid, int64_t nv, int64_t ne, int32_t* cA, int32_t* cB, int32_t* cC,
-                      const int64_t* sbase, int2* stage_end, const int* stage_skip, int32_t* runA, void* units,
-                      void* ctl, int* status, cudaStream_t st);
+                      const int64_t* sbase, int2* stage_end, unsigned long long stage_slots, int* stage_skip,
+                      int32_t* runA, void* units, void* ctl, int* status, cudaStream_t st);
 int launch_walk_list(const int64_t* rp, const int32_t* cols, const int64_t* cp, const int32_t* in_src,
                      const int32_t* in_eid, int64_t nv, int64_t ne, const int64_t* off, int32_t* cA, int2* lists,
                      int32_t* runA, void* units, void* ctl, const int* gate, int* status, cudaStream_t st);
@@ -1850,8 +1882,11 @@ struct Layout {
     int32_t* sidx;
     int32_t* alive[2];
     unsigned* code;
-    void* scan_ws;
+    void* scan_cp;
+    void* scan_sb;
+    void* scan_off;
     void* sort_ws;
+    size_t zero_peel, zero_sort;
     size_t total;
 };
 
@@ -1859,10 +1894,19 @@ Layout carve(void* ws, int64_t V, int64_t E) {
     Carver c{reinterpret_cast<char*>(ws)};
     Layout L;
     const size_t e = (size_t)(E > 0 ? E : 1), v = (size_t)(V > 0 ? V : 1);
+    // zeroed at the start of a run, in one go: up to zero_peel for every mode,
+    // up to zero_sort for a decomposition
     L.ctl = (PeelCtl*)c.take(4096);
     L.sup_ctl = c.take(256);
-    L.rows_d = (int32_t*)c.take(4 * e);
+    L.scan_cp = c.take(scan_scratch_bytes((int64_t)v));
+    L.scan_sb = c.take(scan_scratch_bytes((int64_t)v));
+    L.scan_off = c.take(scan_scratch_bytes((int64_t)e));
     L.indeg = (int32_t*)c.take(4 * v);
+    L.qi[0] = (int4*)c.take(16 * e);
+    L.zero_peel = c.off;
+    L.sort_ws = c.take(radix_scratch(nullptr, (int64_t)e, 4).bytes);
+    L.zero_sort = c.off;
+    L.rows_d = (int32_t*)c.take(4 * e);
     L.cp = (int64_t*)c.take(8 * (v + 1));
     L.in_src = (int32_t*)c.take(4 * e);
     L.in_eid = (int32_t*)c.take(4 * e);
@@ -1870,7 +1914,8 @@ Layout carve(void* ws, int64_t V, int64_t E) {
     L.live = (int32_t*)c.take(4 * e);
     L.rnd = (int32_t*)c.take(4 * e);
     L.round_level = (int32_t*)c.take(4 * (e + 2));
-    for (int b = 0; b < 3; b++) {
+    L.qb[0] = (long long*)c.take(8 * e);
+    for (int b = 1; b < 3; b++) {
         L.qi[b] = (int4*)c.take(16 * e);
         L.qb[b] = (long long*)c.take(8 * e);
     }
@@ -1880,9 +1925,6 @@ Layout carve(void* ws, int64_t V, int64_t E) {
     L.alive[0] = (int32_t*)c.take(4 * e);
     L.alive[1] = (int32_t*)c.take(4 * e);
     L.code = (unsigned*)c.take(4 * (e / 8 + 1));
-    size_t scan_b = scan_scratch_bytes((int64_t)(e > v ? e : v) + 1);
-    L.scan_ws = c.take(scan_b);
-    L.sort_ws = c.take(radix_scratch(nullptr, (int64_t)e, 4).bytes);
     L.total = c.off + 256;
     return L;
 }
@@ -1911,9 +1953,9 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     int rc = device_info(&di);
     if (rc) return rc;
     Layout L = carve(ws, V, E);
-    TDT_CUDA(cudaMemsetAsync(L.ctl, 0, 4096, st));
-    TDT_CUDA(cudaMemsetAsync(stats, 0, sizeof(int64_t) * TDT_STAT_COUNT, st));
+    TDT_CUDA(cudaMemsetAsync(ws, 0, E == 0 ? 4096 : mode == 0 ? L.zero_sort : L.zero_peel, st));
     if (E == 0) {
+        TDT_CUDA(cudaMemsetAsync(stats, 0, sizeof(int64_t) * TDT_STAT_COUNT, st));
         if (mode == 0) {
             if (ptr_truss && ptr_cap >= 1) TDT_CUDA(cudaMemsetAsync(ptr_truss, 0, 4, st));
             int64_t h[TDT_STAT_COUNT] = {0, 2, 1, 0, 0, 0, 0, 0};
@@ -1925,13 +1967,11 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     }
     const int tb = 256;
     const unsigned g_e = grid_for(E, tb, di.sms, 8);
-    const int32_t* rows_use = rows;
-    if (!rows_use) {
-        rows_from_rp_kernel<<<grid_for(V * 32, tb, di.sms, 8), tb, 0, st>>>(rp, V, L.rows_d);
-        TDT_LAUNCH_CHECK("rows_from_rp");
-        rows_use = L.rows_d;
-    }
-    validate_kernel<<<g_e, tb, 0, st>>>(rp, rows_use, cols, E, V, L.ctl);
+    const int32_t* rows_use = rows ? rows : L.rows_d;
+    if (rows)
+        validate_kernel<<<g_e, tb, 0, st>>>(rp, rows, cols, E, V, L.ctl);
+    else
+        validate_rows_kernel<<<grid_for(V * 32, tb, di.sms, 8), tb, 0, st>>>(rp, L.rows_d, cols, E, V, L.ctl);
     TDT_LAUNCH_CHECK("validate");
     // cA, cB, cC (role counts) live in the first queue buffer until the peel starts
     int32_t* cA = reinterpret_cast<int32_t*>(L.qi[0]);
@@ -1940,7 +1980,6 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     prof_mark(0, st);
     // in-adjacency (CSC) of the oriented graph: the walk's middle vertices, and
     // the peel without lists
-    TDT_CUDA(cudaMemsetAsync(L.indeg, 0, 4 * (size_t)V, st));
     // tiles of the in-adjacency build: at least one per resident block
     const int64_t csc_blocks = (int64_t)di.sms * 4;
     int64_t csc_tile = kCscTile;
@@ -1949,9 +1988,8 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     const unsigned g_csc = (unsigned)(csc_tiles < csc_blocks ? csc_tiles : csc_blocks);
     indeg_kernel<<<g_csc, kCscBlock, 0, st>>>(cols, E, V, L.indeg, L.ctl);
     TDT_LAUNCH_CHECK("indeg");
-    rc = exclusive_scan<int32_t, int64_t>(L.indeg, L.cp, V, L.cp + V, L.scan_ws, &L.ctl->g.status, st);
+    rc = exclusive_scan(L.indeg, L.cp, V, L.cp + V, L.scan_cp, &L.ctl->g.status, st);
     if (rc) return rc;
-    TDT_CUDA(cudaMemsetAsync(L.indeg, 0, 4 * (size_t)V, st));
     csc_fill_kernel<<<g_csc, kCscBlock, 0, st>>>(rows_use, cols, E, V, csc_tile, L.cp, L.indeg, L.in_src, L.in_eid, L.ctl);
     TDT_LAUNCH_CHECK("csc_fill");
     // The list tail: final lists grow from its start, the staging slots of the
@@ -1962,33 +2000,28 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     int2* lists = reinterpret_cast<int2*>(reinterpret_cast<char*>(ws) + list_base);
     int2* stage_end = lists + tail / 8;
     if (tail > 0) {
-        rc = launch_stage_rows(rp, V, L.sbase, &L.ctl->g.status, st);
+        rc = scan_stage_slots(rp, L.sbase, V, L.sbase + V, L.scan_sb, &L.ctl->g.status, st);
         if (rc) return rc;
-        rc = exclusive_scan<int64_t, int64_t>(L.sbase, L.sbase, V, L.sbase + V, L.scan_ws, &L.ctl->g.status, st);
-        if (rc) return rc;
-        stage_decide_kernel<<<1, 1, 0, st>>>(L.sbase, V, tail, L.ctl);
-        TDT_LAUNCH_CHECK("stage_decide");
     }
     // the walk: counts, and the role-A entries when they can be staged (skipped
     // on the device when validation failed); the plan of its units stays for
     // the list walk
-    TDT_CUDA(cudaMemsetAsync(cA, 0, 16 * (size_t)E, st));  // cA, cB, cC and the distribution's counters
     rc = launch_walk_count(rp, cols, L.cp, L.in_src, L.in_eid, V, E, cA, cB, cC, tail > 0 ? L.sbase : nullptr,
-                           stage_end, &L.ctl->stage_skip, L.alive[0], L.qi[2], L.sup_ctl, &L.ctl->g.status, st);
+                           stage_end, tail / 8, &L.ctl->stage_skip, L.alive[0], L.qi[2], L.sup_ctl,
+                           &L.ctl->g.status, st);
     if (rc) return rc;
-    init_state_kernel<<<g_e, tb, 0, st>>>(cA, cB, cC, L.sup, L.live, L.rnd, E, L.ctl);
+    const bool peel = mode != 2;
+    init_state_kernel<<<g_e, tb, 0, st>>>(cA, cB, cC, peel ? L.sup : support_out, peel ? L.live : nullptr, L.rnd,
+                                          peel ? L.code : nullptr, E, L.ctl, stats);
     TDT_LAUNCH_CHECK("init_state");
     prof_mark(1, st);
     if (mode == 2) {
-        if (support_out) TDT_CUDA(cudaMemcpyAsync(support_out, L.sup, 4 * (size_t)E, cudaMemcpyDeviceToDevice, st));
-        stats_final_kernel<<<1, 1, 0, st>>>(L.ctl, stats, 1);
-        TDT_LAUNCH_CHECK("stats_final");
         for (int ph = 2; ph <= 4; ph++) prof_mark(ph, st);
         return TDT_OK;
     }
     // per-edge triangle lists in the workspace tail when 24 T bytes fit
     if (tail > 0) {
-        rc = exclusive_scan<int32_t, int64_t>(L.sup, L.off, E, L.off + E, L.scan_ws, &L.ctl->g.status, st);
+        rc = exclusive_scan(L.sup, L.off, E, L.off + E, L.scan_off, &L.ctl->g.status, st);
         if (rc) return rc;
         list_decide_kernel<<<1, 1, 0, st>>>(L.off, L.sbase, E, V, tail, L.ctl);
         TDT_LAUNCH_CHECK("list_decide");
@@ -2011,7 +2044,6 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
         A.qb[b] = L.qb[b];
     }
     A.code = L.code;
-    TDT_CUDA(cudaMemsetAsync(L.code, 0xff, 4 * (size_t)(E / 8 + 1), st));
     A.off = L.off; A.lists = lists;
     // the search peel's copy of the out-edges and the row lengths, in arrays
     // that only the listing uses
@@ -2076,7 +2108,6 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
         int passes = 1;
         while (passes < 4 && ((int64_t)1 << (8 * passes)) < E + 2) passes++;
         const RadixScratch R = radix_scratch(L.sort_ws, E, passes);
-        TDT_CUDA(cudaMemsetAsync(R.hist, 0, R.bytes, st));
         truss_out_kernel<<<g_e, tb, 0, st>>>(L.rnd, L.round_level, E, truss, passes, R.hist, L.ctl);
         TDT_LAUNCH_CHECK("truss_out");
         rc = radix_sort<uint32_t, true>(reinterpret_cast<const uint32_t*>(L.rnd), k0, k1, v0, v1, E, passes, R, nullptr,

@@ -34,10 +34,28 @@ __device__ __forceinline__ T block_excl_scan(T v, T* s_warp, T* total) {
     return res;
 }
 
-template <class TI, class TO>
-__global__ void __launch_bounds__(kScanBlock) scan_kernel(const TI* in, int64_t n, TO* out, TO* total_out,
+// What a scan adds up.
+template <class TI>
+struct ScanArray {
+    const TI* in;
+    __device__ __forceinline__ int64_t operator()(int64_t i) const { return (int64_t)in[i]; }
+};
+// Staging slots of row i of a CSR (d (d - 1) / 2 for d entries; 0 once an error
+// is known).
+struct ScanStageSlots {
+    const int64_t* rp;
+    const int* status;
+    __device__ __forceinline__ int64_t operator()(int64_t i) const {
+        const int64_t d = rp[i + 1] - rp[i];
+        return *(volatile const int*)status == 0 && d > 1 ? d * (d - 1) / 2 : 0;
+    }
+};
+
+template <class In>
+__global__ void __launch_bounds__(kScanBlock) scan_kernel(In in, int64_t n, int64_t* out, int64_t* total_out,
                                                           unsigned long long* words, unsigned* next, int* status) {
     using W = TileWord<unsigned long long>;
+    using TO = int64_t;
     __shared__ TO s_warp[33];
     __shared__ unsigned s_tile;
     __shared__ unsigned long long s_before;
@@ -49,7 +67,7 @@ __global__ void __launch_bounds__(kScanBlock) scan_kernel(const TI* in, int64_t 
     TO sum = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        v[k] = base + k < n ? (TO)in[base + k] : TO(0);
+        v[k] = base + k < n ? in(base + k) : TO(0);
         sum += v[k];
     }
     TO tot;
@@ -81,23 +99,29 @@ size_t scan_scratch_bytes(int64_t n) {
     return (size_t)(nb + 1) * 8 + 256;
 }
 
-template <class TI, class TO>
-int exclusive_scan(const TI* in, TO* out, int64_t n, TO* total_out, void* scratch, int* status, cudaStream_t st) {
+template <class In>
+static int run_scan(In in, int64_t* out, int64_t n, int64_t* total_out, void* scratch, int* status, cudaStream_t st) {
     if (n <= 0) {
-        if (total_out) TDT_CUDA(cudaMemsetAsync(total_out, 0, sizeof(TO), st));
+        if (total_out) TDT_CUDA(cudaMemsetAsync(total_out, 0, sizeof(int64_t), st));
         return TDT_OK;
     }
     const int64_t nb = (n + kScanTile - 1) / kScanTile;
     unsigned long long* words = reinterpret_cast<unsigned long long*>(scratch);
-    TDT_CUDA(cudaMemsetAsync(words, 0, (size_t)(nb + 1) * 8, st));
-    scan_kernel<TI, TO><<<(unsigned)nb, kScanBlock, 0, st>>>(in, n, out, total_out, words,
-                                                            reinterpret_cast<unsigned*>(words + nb), status);
+    scan_kernel<In><<<(unsigned)nb, kScanBlock, 0, st>>>(in, n, out, total_out, words,
+                                                        reinterpret_cast<unsigned*>(words + nb), status);
     TDT_LAUNCH_CHECK("scan");
     return TDT_OK;
 }
 
-template int exclusive_scan<int32_t, int64_t>(const int32_t*, int64_t*, int64_t, int64_t*, void*, int*, cudaStream_t);
-template int exclusive_scan<int64_t, int64_t>(const int64_t*, int64_t*, int64_t, int64_t*, void*, int*, cudaStream_t);
+int exclusive_scan(const int32_t* in, int64_t* out, int64_t n, int64_t* total_out, void* scratch, int* status,
+                   cudaStream_t st) {
+    return run_scan(ScanArray<int32_t>{in}, out, n, total_out, scratch, status, st);
+}
+
+int scan_stage_slots(const int64_t* rp, int64_t* out, int64_t nv, int64_t* total_out, void* scratch, int* status,
+                     cudaStream_t st) {
+    return run_scan(ScanStageSlots{rp, status}, out, nv, total_out, scratch, status, st);
+}
 
 // ------------------------------------------------------------------ radix sort
 constexpr int kSortBlock = 256;   // one thread per digit

@@ -56,10 +56,13 @@ __device__ __forceinline__ S warp_look_back(const S* words, int64_t tile, int* s
 }
 
 size_t scan_scratch_bytes(int64_t n);
-// out[i] = sum(in[0..i)), and *total_out (device, may be null) = sum(in).  in
-// and out may alias.  status: receives TDT_ERR_TIMEOUT (may be null).
-template <class TI, class TO>
-int exclusive_scan(const TI* in, TO* out, int64_t n, TO* total_out, void* scratch, int* status, cudaStream_t st);
+// out[i] = sum(in[0..i)), and *total_out (device, may be null) = sum(in).
+// scratch: zeroed by the caller.  status: receives TDT_ERR_TIMEOUT.
+int exclusive_scan(const int32_t* in, int64_t* out, int64_t n, int64_t* total_out, void* scratch, int* status,
+                   cudaStream_t st);
+// The same over the staging slots of the rows of a CSR (walk.cu).
+int scan_stage_slots(const int64_t* rp, int64_t* out, int64_t nv, int64_t* total_out, void* scratch, int* status,
+                     cudaStream_t st);
 
 // ------------------------------------------------------------------ radix sort
 // Stable LSD sort by 8-bit digits, one launch per pass: the digit totals of
@@ -69,7 +72,7 @@ int exclusive_scan(const TI* in, TO* out, int64_t n, TO* total_out, void* scratc
 constexpr int kRadix = 256;
 constexpr int kMaxPasses = 8;
 
-// Scratch of one sort, zeroed by radix_zero before the key kernel runs.
+// Scratch of one sort, zeroed by the caller before the key kernel runs.
 struct RadixScratch {
     uint32_t* hist;        // [passes][256]
     uint32_t* tile_next;   // [passes]

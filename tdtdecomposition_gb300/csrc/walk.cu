@@ -107,7 +107,7 @@ struct WalkArgs {
     const int2* units;          // block rows: {v, part}
     int* status;
     const int* gate;            // non-zero: skip
-    const int* stage_skip;      // kWalkCount: non-zero: count only
+    const int* stage_skip;      // kWalkCount: non-zero: count only (written by the plan)
     int warp_cap;
     int light_in;
     int row_cap;
@@ -147,7 +147,10 @@ __device__ __forceinline__ bool is_block_row(int64_t dout, int64_t din, int warp
 // over rows with in-edges is at most E), and the hubs, the rows of several.
 __global__ void walk_plan_kernel(const int64_t* __restrict__ rp, const int64_t* __restrict__ cp, int64_t nv,
                                  int warp_cap, int light_in, int2* __restrict__ units,
-                                 int32_t* __restrict__ hubs, WalkCtl* ctl, const int* status) {
+                                 int32_t* __restrict__ hubs, const int64_t* __restrict__ sbase,
+                                 unsigned long long stage_slots, int* stage_skip, WalkCtl* ctl, const int* status) {
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        *stage_skip = !(*(volatile const int*)status == 0 && sbase && (unsigned long long)sbase[nv] <= stage_slots);
     if (*(volatile const int*)status != 0) return;
     const unsigned lane = lane_id();
     const int64_t nth = (int64_t)gridDim.x * blockDim.x;
@@ -923,16 +926,6 @@ __global__ void __launch_bounds__(kDsBlock, 4) distribute_kernel(const __grid_co
     }
 }
 
-// Staging slots of each row (their exclusive scan gives sbase).
-__global__ void stage_rows_kernel(const int64_t* __restrict__ rp, int64_t nv, int64_t* __restrict__ slots,
-                                  const int* status) {
-    const bool ok = *(volatile const int*)status == 0;
-    for (int64_t u = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; u < nv; u += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t d = rp[u + 1] - rp[u];
-        slots[u] = ok && d > 1 ? d * (d - 1) / 2 : 0;
-    }
-}
-
 template <int M>
 static int launch_walk(WalkArgs A, WalkCtl* ctl, cudaStream_t st) {
     DeviceInfo di;
@@ -977,36 +970,25 @@ static WalkArgs walk_args(const int64_t* rp, const int32_t* cols, const int64_t*
     return A;
 }
 
-// Staging slots of every row: slots[0..nv), to be scanned into sbase.
-int launch_stage_rows(const int64_t* rp, int64_t nv, int64_t* slots, const int* status, cudaStream_t st) {
-    if (nv <= 0) return TDT_OK;
-    DeviceInfo di;
-    int rc = device_info(&di);
-    if (rc) return rc;
-    stage_rows_kernel<<<grid_for(nv, 256, di.sms, 8), 256, 0, st>>>(rp, nv, slots, status);
-    TDT_LAUNCH_CHECK("stage_rows");
-    return TDT_OK;
-}
-
-// Plan and count walk: role counts of every edge (cA, cB, cC zeroed by the
-// caller) and, with sbase and *stage_skip == 0, the role-A entries in their
-// staging slots, which end at stage_end.  units: 16 E bytes of scratch that stays as
+// Plan and count walk: role counts of every edge and, when sbase (else null)
+// needs no more than stage_slots, the role-A entries in their staging slots,
+// which end at stage_end; *stage_skip receives the choice.  cA, cB, cC and ctl
+// are zeroed by the caller.  units: 16 E bytes of scratch that stays as
 // the list walk's plan; runA: int32[E] scratch; ctl: 256 bytes.
 int launch_walk_count(const int64_t* rp, const int32_t* cols, const int64_t* cp, const int32_t* in_src,
                       const int32_t* in_eid, int64_t nv, int64_t ne, int32_t* cA, int32_t* cB, int32_t* cC,
-                      const int64_t* sbase, int2* stage_end, const int* stage_skip, int32_t* runA, void* units,
-                      void* ctl, int* status, cudaStream_t st) {
+                      const int64_t* sbase, int2* stage_end, unsigned long long stage_slots, int* stage_skip,
+                      int32_t* runA, void* units, void* ctl, int* status, cudaStream_t st) {
     if (nv <= 0) return TDT_OK;
     DeviceInfo di;
     int rc = device_info(&di);
     if (rc) return rc;
-    TDT_CUDA(cudaMemsetAsync(ctl, 0, sizeof(WalkCtl), st));
     int wc = 0, hc = 0;
     support_caps(&wc, &hc);
     const int warp_cap = wc > 0 && wc < kLightCap ? wc : kLightCap;
     walk_plan_kernel<<<grid_for(nv, 256, di.sms, 8), 256, 0, st>>>(rp, cp, nv, warp_cap,
                                                                   ne < kLightInEdges ? kLightInSmall : kLightInLarge,
-                                                                  reinterpret_cast<int2*>(units), hub_list(units, ne),
+                                                                  reinterpret_cast<int2*>(units), hub_list(units, ne), sbase, stage_slots, stage_skip,
                                                                   reinterpret_cast<WalkCtl*>(ctl), status);
     TDT_LAUNCH_CHECK("walk_plan");
     WalkArgs A = walk_args(rp, cols, cp, in_src, in_eid, nv, ne, cA, cB, cC, units, status, status);

@@ -147,7 +147,7 @@ def truss_decompose(graph, workspace=None, stream=None, sync=True, lists="auto",
     e_truss = torch.empty(max(E, 1), dtype=torch.int32, device=dev)
     cap = E + 2
     ptr = torch.empty(cap, dtype=torch.int32, device=dev)
-    stats = torch.zeros(STAT_COUNT, dtype=torch.int64, device=dev)
+    stats = torch.empty(STAT_COUNT, dtype=torch.int64, device=dev)
     need = L.tdt_decompose_workspace_bytes(V, E)
     wso = _ws_for(dev, workspace)
     base = (need + 255) // 256 * 256
@@ -177,7 +177,7 @@ def ktruss_search(graph, k, workspace=None, stream=None, lists="auto"):
     dev = cols.device
     V, E = rp.shape[0] - 1, cols.shape[0]
     mask = torch.empty(E, dtype=torch.bool, device=dev)
-    stats = torch.zeros(STAT_COUNT, dtype=torch.int64, device=dev)
+    stats = torch.empty(STAT_COUNT, dtype=torch.int64, device=dev)
     wso = _ws_for(dev, workspace)
     base = (L.tdt_decompose_workspace_bytes(V, E) + 255) // 256 * 256
     tail = _list_bytes(wso, cols, rp, lists, base, rows)
@@ -194,7 +194,7 @@ def ktruss_search(graph, k, workspace=None, stream=None, lists="auto"):
 def triangle_count_arrays(cols, rp, ws):
     L = _lib.load()
     V, E = rp.shape[0] - 1, cols.shape[0]
-    stats = torch.zeros(STAT_COUNT, dtype=torch.int64, device=cols.device)
+    stats = torch.empty(STAT_COUNT, dtype=torch.int64, device=cols.device)
     buf = ws.get(L.tdt_decompose_workspace_bytes(V, E))
     with torch.cuda.device(cols.device):
         rc = L.tdt_triangle_count(cols.data_ptr(), rp.data_ptr(), V, E, None, stats.data_ptr(), buf.data_ptr(),
@@ -212,7 +212,7 @@ def triangle_count(graph, workspace=None, stream=None, return_support=False):
     dev = cols.device
     V, E = rp.shape[0] - 1, cols.shape[0]
     support = torch.empty(E, dtype=torch.int32, device=dev) if return_support else None
-    stats = torch.zeros(STAT_COUNT, dtype=torch.int64, device=dev)
+    stats = torch.empty(STAT_COUNT, dtype=torch.int64, device=dev)
     ws = _ws_for(dev, workspace).get(L.tdt_decompose_workspace_bytes(V, E))
     s = (stream or torch.cuda.current_stream(dev)).cuda_stream
     with torch.cuda.device(cols.device):
