@@ -36,7 +36,6 @@ constexpr int kSupWarps = kSupBlock / kWarp;
 constexpr int kSupMinBlocks = TDT_SUP_MINB;    // resident blocks per SM (3: registers <= 42)
 constexpr int kSupSmemBytes = 64 * 1024;       // dynamic shared memory per block
 constexpr int kVertexBatch = 2;                // light vertices per turn below the top quarter of ids
-constexpr int kHeavyChunk = 16;                // vertices scanned per heavy grab
 constexpr int kQueue = 64;                     // candidate queue entries per warp
 
 // Light rows: one warp, a 4 KB slice of the block buffer:
@@ -382,18 +381,29 @@ __device__ __forceinline__ void flush_row(const RowState& R, const SupArgs& A, i
         if (R.cnt[i]) atomicAdd(A.out + R.bu + i, (int32_t)R.cnt[i]);
 }
 
-// Static round-robin schedule (no scratch at all).  kVec: the wedge walk loads
-// 16-byte chunks of cols (walk_group_vec).
+// Schedule, without scratch memory: the rows are dealt out to the blocks, row
+// after row, because rows next to each other cost alike (ids are degree ranks);
+// the warps of a block take its light rows from a counter in shared memory.
+// Against chunks of 16 rows next to each other (SMs active 55 % of the time):
+// R-MAT scale 18 (3.8 M edges) 2.68 -> 1.34 ms, 20 (15.7 M) 9.9 -> 8.1, 300 K
+// Chung-Lu vertices 1.23 -> 1.07.  Rows shared by the blocks of a cluster,
+// from a counter in its first block: clusters of 2 / 4 / 8 1.33 / 1.36 / 1.47 ms
+// at scale 18.  The rest is the walk: its bitmap tests and the wedge loads.
+//
+// kVec: the wedge walk loads 16-byte chunks of cols (walk_group_vec).
 template <bool kVec>
 __global__ void __launch_bounds__(kSupBlock, kSupMinBlocks) support_kernel(OutRows G, SupArgs A) {
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ int32_t s_list[kHeavyChunk];
+    __shared__ int32_t s_list[kSupBlock];
     __shared__ int32_t s_wsum[2][kSupWarps + 1];
     __shared__ int s_n;
+    __shared__ unsigned s_light;
     const int wib = threadIdx.x / kWarp;
     const unsigned lane = lane_id();
     const int64_t nv = G.nv;
-    const long long nchunks = (nv + kHeavyChunk - 1) / kHeavyChunk;
+    const int64_t step = gridDim.x, first = blockIdx.x;
+    const int64_t mine = first < nv ? (nv - first + step - 1) / step : 0;  // rows first, first + step, ..
+    if (threadIdx.x == 0) s_light = 0;
     const int warp_cap = A.warp_cap;
     const int heavy_cap = A.heavy_cap;
 
@@ -410,12 +420,13 @@ __global__ void __launch_bounds__(kSupBlock, kSupMinBlocks) support_kernel(OutRo
         Q.pos = reinterpret_cast<int32_t*>(smem + kHvQueues + wib * 8 * kQueue);
         Q.vi = Q.pos + kQueue;
         Q.n = 0;
-        for (long long c = blockIdx.x; c < nchunks; c += gridDim.x) {
+        for (int64_t k0 = 0; k0 < mine; k0 += kSupBlock) {
             if (threadIdx.x == 0) s_n = 0;
             __syncthreads();
-            for (int k = threadIdx.x; k < kHeavyChunk; k += kSupBlock) {
-                const long long u = c * kHeavyChunk + k;
-                if (u < nv && G.end(u) - G.begin(u) > warp_cap) s_list[atomicAdd(&s_n, 1)] = (int32_t)u;
+            const int64_t k = k0 + threadIdx.x;
+            if (k < mine) {
+                const int64_t u = first + k * step;
+                if (G.end(u) - G.begin(u) > warp_cap) s_list[atomicAdd(&s_n, 1)] = (int32_t)u;
             }
             __syncthreads();
             const int nh = s_n;
@@ -507,8 +518,8 @@ __global__ void __launch_bounds__(kSupBlock, kSupMinBlocks) support_kernel(OutRo
         }
     }
 
-    // ---- phase 2: rows with 2 <= d+(u) <= warp_cap, one warp per row, taken
-    // in batches from the top ids (highest degree rank) down
+    // ---- phase 2: rows with 2 <= d+(u) <= warp_cap, one warp per row
+    __syncthreads();
     unsigned char* sl = smem + wib * kSliceBytes;
     int32_t* l_su = reinterpret_cast<int32_t*>(sl + kSlSu);
     uint32_t* l_cnt = reinterpret_cast<uint32_t*>(sl + kSlCnt);
@@ -522,21 +533,22 @@ __global__ void __launch_bounds__(kSupBlock, kSupMinBlocks) support_kernel(OutRo
     Q.pos = reinterpret_cast<int32_t*>(sl + kSlQ);
     Q.vi = Q.pos + kQueue;
     Q.n = 0;
-    const long long gw = (long long)blockIdx.x * kSupWarps + wib;
-    const long long nw = (long long)gridDim.x * kSupWarps;
     // rows are taken from the top id down: the top quarter of the ids (the
     // rows whose out-neighbours have the longest lists) one row per turn, the
     // rest kVertexBatch rows per turn, so no warp is left with a long batch
     // while the others idle
-    const unsigned long long t1 = ((unsigned long long)nv + 3) / 4;
-    for (long long it = 0;; it++) {
-        const unsigned long long t = (unsigned long long)(gw + it * nw);
-        const unsigned long long b = t < t1 ? t : t1 + (t - t1) * kVertexBatch;
+    const int64_t t1 = (mine + 3) / 4;
+    for (;;) {
+        unsigned g = 0;
+        if (lane == 0) g = atomicAdd(&s_light, 1u);
+        const int64_t t = __shfl_sync(kFull, g, 0);
+        const int64_t b = t < t1 ? t : t1 + (t - t1) * kVertexBatch;
         const int nq = t < t1 ? 1 : kVertexBatch;
-        if ((long long)b >= nv) break;
+        if (b >= mine) break;
         for (int q = 0; q < nq; q++) {
-            const long long uu = nv - 1 - ((long long)b + q);
-            if (uu < 0) break;
+            const int64_t k = mine - 1 - (b + q);
+            if (k < 0) break;
+            const int64_t uu = first + k * step;
             const int32_t bu = G.begin(uu);
             const int d = (int)(G.end(uu) - bu);
             if (d < 2 || d > warp_cap) continue;
