@@ -1,78 +1,25 @@
 // Drop-in `trusstensor` operators (myhpu_extension.cpp:572-593) for sm_103a.
 //
 // The reference runs one thread per (edge, tile) and walks a two-pointer merge
-// of the two out-lists with scalar loads (kernel.cu:28-685).  Here one warp
-// owns one edge: the shorter of the two out-lists is hashed into a per-warp
-// shared-memory table (128 keys per pass) and the longer list is streamed
-// through it with coalesced loads, 32 columns per step.  Matching on column
-// values instead of merging keeps the operators exact on lists that carry the
-// reference's -1 sentinels (peeled edges are overwritten with -1 in place,
-// singlegpu_truss.py:118), where a binary search would not be.
+// of the two out-lists with scalar loads (kernel.cu:28-685).  Here a warp takes
+// a group of edges and streams their N+(v) through a shared-memory table of
+// N+(u) (walk_edges).  Matching on column values instead of merging keeps the
+// operators exact on lists that carry the reference's -1 sentinels (peeled
+// edges are overwritten with -1 in place, singlegpu_truss.py:118), where a
+// binary search would not be.
 //
 // Tiling (n_cut): tile j of vertex v is [row_ptr[v*n_cut+j], row_ptr[v*n_cut+j+1])
 // and tiles partition a row by column value (csr_to_tilingcsr,
 // singlegpu_truss.py:160-169), so the union over tiles of the per-tile
-// intersections is the intersection of the whole rows; each warp intersects
-// whole rows [row_ptr[v*n_cut], row_ptr[v*n_cut+n_cut]).
+// intersections is the intersection of the whole rows
+// [row_ptr[v*n_cut], row_ptr[v*n_cut+n_cut]).
 #include "common.cuh"
 
 namespace tdt {
 
-constexpr int kHashSlots = 256;   // per warp, power of two
-constexpr int kHashChunk = 128;   // keys per pass (load factor 1/2)
 constexpr int kOpsBlock = 256;    // 8 warps
+constexpr int kOpsMinBlocks = 5;  // resident blocks of the edge walks (shared memory)
 constexpr int32_t kEmpty = INT32_MIN;
-
-__device__ __forceinline__ unsigned hash_slot(int32_t key) {
-    return ((unsigned)key * 2654435761u) >> (32 - 8);  // 8 = log2(kHashSlots)
-}
-
-// Intersects cols[a0,a1) and cols[b0,b1) (sorted apart from -1 holes) and calls
-// on_match(pa, pb) for every pair of positions holding the same column >= 0.
-// All 32 lanes must call it together.
-template <class F>
-__device__ __forceinline__ void warp_intersect_hash(const int32_t* __restrict__ cols, int64_t a0,
-                                                    int64_t a1, int64_t b0, int64_t b1,
-                                                    int32_t* hkey, int32_t* hpos, F&& on_match) {
-    const unsigned lane = lane_id();
-    const int64_t la = a1 - a0, lb = b1 - b0;
-    if (la <= 0 || lb <= 0) return;
-    const bool a_short = la <= lb;
-    const int64_t s0 = a_short ? a0 : b0, s1 = a_short ? a1 : b1;
-    const int64_t l0 = a_short ? b0 : a0, l1 = a_short ? b1 : a1;
-    for (int64_t c = s0; c < s1; c += kHashChunk) {
-        const int64_t ce = min(c + (int64_t)kHashChunk, s1);
-        for (int i = lane; i < kHashSlots; i += kWarp) hkey[i] = kEmpty;
-        __syncwarp();
-        for (int64_t i = c + lane; i < ce; i += kWarp) {
-            int32_t key = __ldg(cols + i);
-            if (key < 0) continue;
-            unsigned h = hash_slot(key);
-            for (int probe = 0; probe < kHashSlots; probe++) {
-                int32_t old = atomicCAS(&hkey[h], kEmpty, key);
-                if (old == kEmpty) { hpos[h] = (int32_t)(i - c); break; }
-                h = (h + 1) & (kHashSlots - 1);
-            }
-        }
-        __syncwarp();
-        for (int64_t j = l0 + lane; j < l1; j += kWarp) {
-            int32_t x = __ldg(cols + j);
-            if (x < 0) continue;
-            unsigned h = hash_slot(x);
-            for (int probe = 0; probe < kHashSlots; probe++) {
-                int32_t k = hkey[h];
-                if (k == kEmpty) break;
-                if (k == x) {
-                    int64_t sp = c + hpos[h];
-                    if (a_short) on_match(sp, j); else on_match(j, sp);
-                    break;
-                }
-                h = (h + 1) & (kHashSlots - 1);
-            }
-        }
-        __syncwarp();
-    }
-}
 
 // Row ranges are clamped to [0, n_edges] so a malformed row_ptr cannot move an
 // access outside the per-edge arrays.
@@ -89,6 +36,202 @@ struct RowView {
         return e < b ? b : e;
     }
 };
+
+// ------------------------------------------------------------------ triangles of a list of edges
+// For every edge (u, v) of a list, the columns that N+(u) and N+(v) share: the
+// walk of the peel-update and k-truss operators.  A warp takes a group of list
+// entries.  Edges of a group with the same u (neighbours in the list, as edges
+// are stored by source) share one hash table of N+(u) in shared memory, with a
+// bitmap of eight bits per slot in front of it; the rows N+(v) of these edges,
+// widened to the aligned 16-byte chunks that hold them, form one flat space of
+// chunks, walked 32 a step (the owner of a lane's chunk comes from one
+// OR-reduction of the row starts inside the step).  A chunk that holds an entry
+// is mapped as a whole, so any alignment of cols will do.  Most entries miss the
+// bitmap; the others go to a queue and are looked up 32 at a time.  Rows of more
+// than kWalkKeys keys are staged in pieces.
+//
+// Bound by issuing the tests.  One edge at a time, its shorter list hashed and
+// the longer one streamed, the update of 0.87 M of 1.86 M edges (R-MAT scale 17,
+// 109 M entries of N+(v)) took 540 us; in groups 416, with the counts of N+(u)
+// kept in shared memory 431, in chunks of four columns 302 (2.4 M edges of a
+// Chung-Lu graph 1,161 -> 564, the saturating support of all of scale 17
+// 1,748 -> 770).  Tables of 128 keys and more blocks per SM: 317.
+constexpr int kWalkKeys = 256;                 // keys per pass, load factor <= 1/2
+constexpr int kWalkSlots = 2 * kWalkKeys;
+constexpr int kWalkMinLog2 = 6;
+constexpr int kWalkQueue = 64;                 // a push adds up to 32 to at most 31
+
+struct EdgeWalkShared {
+    int32_t key[kWalkSlots];
+    uint32_t bm[kWalkSlots / 4];
+    uint4 row[kWarp];                          // N+(v) by place in the run: first chunk, begin, end, group lane
+    uint2 queue[kWalkQueue];                   // ring: column, place in the run and offset in N+(v)
+    uint32_t start[kWarp];                     // first chunk again
+    int32_t cnt[kWarp];                        // by group lane
+    uint32_t hits[kWalkKeys / 2];              // of each staged key, 16 bits
+    uint16_t pos[kWalkSlots];                  // key index, and the flag of its edge in bit 15
+};
+
+// list(i): the edge of entry i, or -1.  mark(e): flag of an edge.  hit(me, pa,
+// mb): a common column, at position pa of N+(v) and an edge of u with flag mb;
+// bit 0 of the result counts it for the entry's edge, bit 1 for the edge of u.
+// row(pb, count) and done(e, count), count > 0: the counts of the edges of u,
+// once per staged piece, and of the entries.
+template <class List, class Mark, class Hit, class Row, class Done>
+__device__ __forceinline__ void walk_edges(const int32_t* __restrict__ rows, const int32_t* __restrict__ cols,
+                                           const RowView& rv, int64_t n, int group, EdgeWalkShared& S, List&& list,
+                                           Mark&& mark, Hit&& hit, Row&& row, Done&& done) {
+    const unsigned lane = lane_id(), lt = lanemask_lt();
+    // chunk c of the flat space of positions + shift holds positions 4 c - shift .. + 3
+    const unsigned shift = (unsigned)((uintptr_t)cols >> 2) & 3u;
+    const int4* __restrict__ cols4 = reinterpret_cast<const int4*>(cols - shift);
+    const int64_t nw = (int64_t)gridDim.x * (kOpsBlock / kWarp);
+    for (int64_t g = blockIdx.x * (int64_t)(kOpsBlock / kWarp) + threadIdx.x / kWarp; g * group < n; g += nw) {
+        const int64_t i = g * group + lane;
+        int64_t e = -1;
+        int32_t u = -1, bv = 0, lv = 0;
+        bool me = false;
+        if ((int)lane < group && i < n) {
+            e = list(i);
+            if (e >= 0 && e < rv.n_edges) {
+                u = __ldg(rows + e);
+                const int32_t v = __ldg(cols + e);
+                if (rv.valid(u) && rv.valid(v)) {  // a sentinel edge has no triangles
+                    bv = (int32_t)rv.begin(v);
+                    lv = (int32_t)(rv.end(v) - bv);
+                    me = mark(e);
+                }
+            }
+        }
+        S.cnt[lane] = 0;
+        const unsigned marked = __ballot_sync(kFull, me);
+        const bool wide = __any_sync(kFull, lv >= (1 << 26));  // 32 of them might overflow a start
+        unsigned todo = __ballot_sync(kFull, lv > 0);
+        while (todo) {
+            const int first = __ffs(todo) - 1;
+            const int32_t ur = __shfl_sync(kFull, u, first);
+            const unsigned run = wide ? 1u << first : __ballot_sync(kFull, u == ur) & todo;
+            todo &= ~run;
+            const bool mine = (run >> lane) & 1u;
+            const unsigned lo = (unsigned)bv + shift, hi = lo + (unsigned)lv;
+            const int32_t len = mine ? (int32_t)(((hi + 3) >> 2) - (lo >> 2)) : 0;
+            const int32_t incl = warp_incl_scan(len);
+            const unsigned total = (unsigned)__shfl_sync(kFull, incl, 31);
+            if (mine) {
+                const int k = __popc(run & lt);
+                S.start[k] = (unsigned)(incl - len);
+                S.row[k] = make_uint4((unsigned)(incl - len), lo, hi, lane);
+            }
+            const int nrun = __popc(run);
+            const int off_shift = wide ? 0 : 5;  // a wide row is alone in its run
+            const int64_t bu = rv.begin(ur), eu = rv.end(ur);
+            for (int64_t c = bu; c < eu; c += kWalkKeys) {
+                const int d = (int)(eu - c < kWalkKeys ? eu - c : kWalkKeys);
+                int lg = 33 - __clz(d);  // 2 d rounded up to a power of two, or the next one
+                if (2 * d == 1 << (lg - 1)) lg--;
+                lg = lg < kWalkMinLog2 ? kWalkMinLog2 : lg;
+                const unsigned slots = 1u << lg;
+                for (unsigned k = lane; k < slots / 4; k += kWarp) {
+                    reinterpret_cast<int4*>(S.key)[k] = make_int4(kEmpty, kEmpty, kEmpty, kEmpty);
+                    S.bm[k] = 0u;
+                }
+                for (int k = lane; k < (d + 1) / 2; k += kWarp) S.hits[k] = 0u;
+                __syncwarp();
+                for (int k = lane; k < d; k += kWarp) {
+                    const int32_t key = __ldg(cols + c + k);
+                    if (key < 0) continue;
+                    const unsigned h = (unsigned)key * 2654435761u;
+                    const unsigned bit = h >> (29 - lg);
+                    atomicOr(S.bm + (bit >> 5), 1u << (bit & 31));
+                    unsigned slot = h >> (32 - lg);
+                    while (atomicCAS(&S.key[slot], kEmpty, key) != kEmpty) slot = (slot + 1) & (slots - 1);
+                    S.pos[slot] = (uint16_t)(k | (mark(c + k) ? 0x8000 : 0));
+                }
+                __syncwarp();
+                int ob = 0, nq = 0;
+                unsigned head = 0;
+                // look up m queue entries, one per lane
+                auto resolve = [&](int m) {
+                    __syncwarp();
+                    if ((int)lane < m) {
+                        const uint2 q = S.queue[(head + lane) & (kWalkQueue - 1)];
+                        const int32_t x = (int32_t)q.x;
+                        const uint4 r = S.row[wide ? 0u : q.y & 31u];
+                        unsigned slot = (q.x * 2654435761u) >> (32 - lg);
+                        int32_t k = S.key[slot];
+                        while (k != x && k != kEmpty) {
+                            slot = (slot + 1) & (slots - 1);
+                            k = S.key[slot];
+                        }
+                        if (k == x) {
+                            const unsigned kb = S.pos[slot], at = kb & 0x7fffu;
+                            const int64_t pa = (int64_t)r.y + (q.y >> off_shift) - shift;
+                            const unsigned c2 = hit((marked >> r.w) & 1u, pa, (bool)(kb >> 15));
+                            if (c2 & 1u) atomicAdd(&S.cnt[r.w], 1);
+                            if (c2 & 2u) atomicAdd(&S.hits[at >> 1], 1u << (16 * (at & 1u)));
+                        }
+                    }
+                    __syncwarp();
+                    head += m;
+                    nq -= m;
+                };
+                for (unsigned base = 0; base < total; base += kWarp) {
+                    // row starts inside (base, base + 32): each is > base, and at most 31 fit
+                    const int k = ob + 1 + (int)lane;
+                    const unsigned B = k < nrun ? S.start[k] : ~0u;
+                    const unsigned ahead = B - base;
+                    const unsigned mk = __reduce_or_sync(kFull, ahead < (unsigned)kWarp ? 1u << ahead : 0u);
+                    const int nb = __popc(mk);
+                    const unsigned Bn = __shfl_sync(kFull, B, nb);
+                    unsigned cm = 0, ent = 0;
+                    int4 x4 = make_int4(0, 0, 0, 0);
+                    if (base + lane < total) {
+                        const int o = ob + __popc(mk & (lt | (1u << lane)));
+                        const uint4 r = S.row[o];
+                        const unsigned c4 = (r.y >> 2) + (base + lane - r.x), p0 = c4 << 2;
+                        x4 = __ldg(cols4 + c4);
+                        // every column is tested (a hashed index stays inside the
+                        // bitmap); holes and entries outside the row are masked after
+                        auto test = [&](int32_t x) {
+                            const unsigned b = ((unsigned)x * 2654435761u) >> (29 - lg);
+                            return (S.bm[b >> 5] >> (b & 31)) & 1u;
+                        };
+                        cm = test(x4.x) | test(x4.y) << 1 | test(x4.z) << 2 | test(x4.w) << 3;
+                        if (p0 < r.y) cm &= 0xFu << (r.y - p0);
+                        if (p0 + 4 > r.z) cm &= 0xFu >> (p0 + 4 - r.z);
+                        ent = ((p0 - r.y) << off_shift) + (unsigned)o;
+                    }
+                    ob += nb + (Bn == base + kWarp ? 1 : 0);
+                    const int32_t xs[4] = {x4.x, x4.y, x4.z, x4.w};
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const bool cand = ((cm >> q) & 1u) && xs[q] >= 0;
+                        const unsigned m = __ballot_sync(kFull, cand);
+                        if (cand)
+                            S.queue[(head + nq + __popc(m & lt)) & (kWalkQueue - 1)] =
+                                make_uint2((unsigned)xs[q], ent + ((unsigned)q << off_shift));
+                        nq += __popc(m);
+                        if (nq >= kWarp) resolve(kWarp);
+                    }
+                }
+                if (nq > 0) resolve(nq);
+                __syncwarp();
+                for (int k = lane; k < d; k += kWarp) {
+                    const int32_t count = (int32_t)((S.hits[k >> 1] >> (16 * (k & 1))) & 0xffffu);
+                    if (count > 0) row(c + k, count);
+                }
+                __syncwarp();
+            }
+        }
+        const int32_t count = S.cnt[lane];
+        if (count > 0) done(e, count);
+        __syncwarp();
+    }
+}
+
+// Entries a warp takes at a time: as many as leave every warp of the grid
+// kWalkTurns groups, at most a warp's width; 4 or 8 turns measured the same.
+constexpr int kWalkTurns = 2;
 
 // ------------------------------------------------------------------ segment_add
 // kernel.cu:5-26: one thread per row.
@@ -171,69 +314,44 @@ struct AffectArgs {
     uint8_t* in_win;
     int32_t* buff_index;
     int32_t* buf_size;
+    int group;
 };
 
 // kernel.cu:144-191/:407-456 (kAffectDeleted), :220-273/:492-547 (kAffectNot),
-// :302-370/:578-648 (kAffectNotWin).  One warp per affected edge.
+// :302-370/:578-648 (kAffectNotWin).
 template <int MODE>
-__global__ void __launch_bounds__(kOpsBlock) affect_kernel(AffectArgs A) {
-    __shared__ int32_t s_key[kOpsBlock / kWarp][kHashSlots];
-    __shared__ int32_t s_pos[kOpsBlock / kWarp][kHashSlots];
-    const int wib = threadIdx.x / kWarp;
-    const unsigned lane = lane_id();
-    const int64_t nw = (int64_t)gridDim.x * (kOpsBlock / kWarp);
-    for (int64_t i = blockIdx.x * (int64_t)(kOpsBlock / kWarp) + wib; i < A.n_affect; i += nw) {
-        const int64_t e = __ldg(A.e_affect + i);
-        if (e < 0 || e >= A.rv.n_edges) continue;
-        const int32_t u = __ldg(A.rows + e), v = __ldg(A.cols + e);
-        if (!A.rv.valid(u) || !A.rv.valid(v)) continue;  // a sentinel edge has no triangles
-        const bool me = A.mark[e] != 0;
-        int32_t count = 0;
-        warp_intersect_hash(A.cols, A.rv.begin(v), A.rv.end(v), A.rv.begin(u), A.rv.end(u),
-                            s_key[wib], s_pos[wib], [&](int64_t pa, int64_t pb) {
-            const bool ma = A.mark[pa] != 0, mb = A.mark[pb] != 0;
-            if (MODE == kAffectDeleted) {
-                if (me || ma || mb) {
-                    if (*(volatile int32_t*)(A.out + pa) > A.l) { atomicSub(A.out + pa, 1); A.n_mark[pa] = 1; }
-                    if (*(volatile int32_t*)(A.out + pb) > A.l) { atomicSub(A.out + pb, 1); A.n_mark[pb] = 1; }
-                    if (!me) count++;
-                }
-            } else {
-                if (!(me && ma && mb)) {
-                    const int64_t wedge[2] = {pa, pb};
-#pragma unroll
-                    for (int q = 0; q < 2; q++) {
-                        const int64_t x = wedge[q];
-                        if (*(volatile int32_t*)(A.out + x) > A.l) {
-                            int32_t t = atomicSub(A.out + x, 1);
-                            if (t - 1 == A.l) A.n_mark[x] = 1;
-                            if (MODE == kAffectNotWin && t == A.windows_high) {
-                                A.in_win[x] = 1;
-                                const int32_t slot = atomicAdd(A.buf_size, 1);
-                                if (slot >= 0 && slot < A.rv.n_edges) A.buff_index[slot] = (int32_t)x;
-                            }
-                        }
-                    }
-                    if (me) count++;
-                }
-            }
+__global__ void __launch_bounds__(kOpsBlock, kOpsMinBlocks) affect_kernel(AffectArgs A) {
+    __shared__ __align__(16) EdgeWalkShared s[kOpsBlock / kWarp];
+    auto in_window = [&](int64_t x) {
+        A.in_win[x] = 1;
+        const int32_t slot = atomicAdd(A.buf_size, 1);
+        if (slot >= 0 && slot < A.rv.n_edges) A.buff_index[slot] = (int32_t)x;
+    };
+    auto lower = [&](int64_t x, int32_t by) {
+        const int32_t t = atomicSub(A.out + x, by);
+        if (MODE == kAffectDeleted || (t > A.l && t - by <= A.l)) A.n_mark[x] = 1;
+        if (MODE == kAffectNotWin && t >= A.windows_high && t - by < A.windows_high) in_window(x);
+    };
+    walk_edges(
+        A.rows, A.cols, A.rv, A.n_affect, A.group, s[threadIdx.x / kWarp],
+        [&](int64_t i) { return (int64_t)__ldg(A.e_affect + i); }, [&](int64_t e) { return A.mark[e] != 0; },
+        [&](bool me, int64_t pa, bool mb) {
+            const bool ma = A.mark[pa] != 0;
+            const int32_t now = *(volatile int32_t*)(A.out + pa);
+            if (MODE == kAffectDeleted ? !(me || ma || mb) : me && ma && mb) return 0u;
+            if (now > A.l) lower(pa, 1);
+            return (MODE == kAffectDeleted ? !me : me) ? 3u : 2u;
+        },
+        [&](int64_t pb, int32_t count) {
+            // as far as one after the other would: a value falls while it is above l
+            const int32_t now = *(volatile int32_t*)(A.out + pb);
+            if (now > A.l) lower(pb, (int32_t)min((int64_t)count, (int64_t)now - A.l));
+        },
+        [&](int64_t e, int32_t count) {
+            int32_t t = atomicSub(A.out + e, count);
+            if (MODE == kAffectDeleted || t - count <= A.l) A.n_mark[e] = 1;
+            if (MODE == kAffectNotWin && t - count < A.windows_high && t >= A.windows_high) in_window(e);
         });
-        count = warp_sum(count);
-        if (lane == 0 && count > 0) {
-            if (MODE == kAffectDeleted) {
-                atomicSub(A.out + e, count);
-                A.n_mark[e] = 1;
-            } else {
-                int32_t t = atomicSub(A.out + e, count);
-                if (t - count <= A.l) A.n_mark[e] = 1;
-                if (MODE == kAffectNotWin && t - count < A.windows_high && t >= A.windows_high) {
-                    A.in_win[e] = 1;
-                    const int32_t slot = atomicAdd(A.buf_size, 1);
-                    if (slot >= 0 && slot < A.rv.n_edges) A.buff_index[slot] = (int32_t)e;
-                }
-            }
-        }
-    }
 }
 
 // ------------------------------------------------------------------ k-truss search operators
@@ -245,63 +363,56 @@ struct EdgeOpArgs {
     int32_t k;
     const uint8_t* mark;
     int32_t* out;
+    int group;
 };
 
 // ktruss_cuda.py:121-200: support saturating at k.
-__global__ void __launch_bounds__(kOpsBlock) support_k_kernel(EdgeOpArgs A) {
-    __shared__ int32_t s_key[kOpsBlock / kWarp][kHashSlots];
-    __shared__ int32_t s_pos[kOpsBlock / kWarp][kHashSlots];
-    const int wib = threadIdx.x / kWarp;
-    const unsigned lane = lane_id();
-    const int64_t nw = (int64_t)gridDim.x * (kOpsBlock / kWarp);
-    for (int64_t i = blockIdx.x * (int64_t)(kOpsBlock / kWarp) + wib; i < A.n_edges; i += nw) {
-        const int32_t u = __ldg(A.rows + i), v = __ldg(A.cols + i);
-        if (!A.rv.valid(u) || !A.rv.valid(v)) continue;
-        int32_t count = 0;
-        warp_intersect_hash(A.cols, A.rv.begin(v), A.rv.end(v), A.rv.begin(u), A.rv.end(u),
-                            s_key[wib], s_pos[wib], [&](int64_t pa, int64_t pb) {
+__global__ void __launch_bounds__(kOpsBlock, kOpsMinBlocks) support_k_kernel(EdgeOpArgs A) {
+    __shared__ __align__(16) EdgeWalkShared s[kOpsBlock / kWarp];
+    walk_edges(
+        A.rows, A.cols, A.rv, A.n_edges, A.group, s[threadIdx.x / kWarp], [](int64_t i) { return i; },
+        [](int64_t) { return false; },
+        [&](bool, int64_t pa, bool) {
             if (*(volatile int32_t*)(A.out + pa) < A.k) atomicAdd(A.out + pa, 1);
-            if (*(volatile int32_t*)(A.out + pb) < A.k) atomicAdd(A.out + pb, 1);
-            count++;
+            return 3u;
+        },
+        [&](int64_t pb, int32_t count) {
+            const int32_t now = *(volatile int32_t*)(A.out + pb);
+            if (now < A.k) atomicAdd(A.out + pb, (int32_t)min((int64_t)count, (int64_t)A.k - now));
+        },
+        [&](int64_t e, int32_t count) {
+            if (*(volatile int32_t*)(A.out + e) < A.k) atomicAdd(A.out + e, count);
         });
-        count = warp_sum(count);
-        if (lane == 0 && count > 0 && *(volatile int32_t*)(A.out + i) < A.k) atomicAdd(A.out + i, count);
-    }
 }
 
 // ktruss_cuda.py:201-286: unconditional decrements on an extracted subgraph.
-__global__ void __launch_bounds__(kOpsBlock) sub_affect_kernel(EdgeOpArgs A) {
-    __shared__ int32_t s_key[kOpsBlock / kWarp][kHashSlots];
-    __shared__ int32_t s_pos[kOpsBlock / kWarp][kHashSlots];
-    const int wib = threadIdx.x / kWarp;
-    const unsigned lane = lane_id();
-    const int64_t nw = (int64_t)gridDim.x * (kOpsBlock / kWarp);
-    for (int64_t i = blockIdx.x * (int64_t)(kOpsBlock / kWarp) + wib; i < A.n_edges; i += nw) {
-        const int32_t u = __ldg(A.rows + i), v = __ldg(A.cols + i);
-        if (!A.rv.valid(u) || !A.rv.valid(v)) continue;
-        const bool mi = A.mark[i] != 0;
-        int32_t count = 0;
-        warp_intersect_hash(A.cols, A.rv.begin(v), A.rv.end(v), A.rv.begin(u), A.rv.end(u),
-                            s_key[wib], s_pos[wib], [&](int64_t pa, int64_t pb) {
-            const bool ma = A.mark[pa] != 0, mb = A.mark[pb] != 0;
-            if (mi || ma || mb) {
-                if (!ma) atomicSub(A.out + pa, 1);
-                if (!mb) atomicSub(A.out + pb, 1);
-                if (!mi) count++;
-            }
-        });
-        count = warp_sum(count);
-        if (lane == 0 && count > 0) atomicSub(A.out + i, count);
-    }
+__global__ void __launch_bounds__(kOpsBlock, kOpsMinBlocks) sub_affect_kernel(EdgeOpArgs A) {
+    __shared__ __align__(16) EdgeWalkShared s[kOpsBlock / kWarp];
+    walk_edges(
+        A.rows, A.cols, A.rv, A.n_edges, A.group, s[threadIdx.x / kWarp], [](int64_t i) { return i; },
+        [&](int64_t e) { return A.mark[e] != 0; },
+        [&](bool me, int64_t pa, bool mb) {
+            const bool ma = A.mark[pa] != 0;
+            if (!(me || ma || mb)) return 0u;
+            if (!ma) atomicSub(A.out + pa, 1);
+            return (me ? 0u : 1u) | (mb ? 0u : 2u);
+        },
+        [&](int64_t pb, int32_t count) { atomicSub(A.out + pb, count); },
+        [&](int64_t e, int32_t count) { atomicSub(A.out + e, count); });
 }
 
 // ------------------------------------------------------------------ host launchers
-static int ops_grid(int64_t warps_needed) {
+// Grid of a walk over n list entries, and the entries a warp takes at a time.
+static int walk_grid(int64_t n, int* group) {
     DeviceInfo di;
     if (device_info(&di) != TDT_OK) return -1;
-    int64_t blocks = (warps_needed + (kOpsBlock / kWarp) - 1) / (kOpsBlock / kWarp);
-    int64_t cap = (int64_t)di.sms * 8;
-    if (blocks < 1) blocks = 1;
+    const int64_t warps = (int64_t)di.sms * kOpsMinBlocks * (kOpsBlock / kWarp);
+    int64_t per = n / (warps * kWalkTurns);
+    if (per < 1) per = 1;
+    if (per > kWarp) per = kWarp;
+    *group = (int)per;
+    const int64_t groups = (n + per - 1) / per;
+    const int64_t blocks = (groups + kOpsBlock / kWarp - 1) / (kOpsBlock / kWarp), cap = (int64_t)di.sms * kOpsMinBlocks;
     return (int)(blocks < cap ? blocks : cap);
 }
 
@@ -357,8 +468,8 @@ int launch_affect(int mode, const int32_t* e_affect, int64_t n_affect, const int
     TDT_CHECK_ARG(e_affect && rows && cols && rp && mark && n_mark && out, "null pointer");
     if (mode == kAffectNotWin) TDT_CHECK_ARG(in_win && buff_index && buf_size, "null window buffer");
     AffectArgs A{e_affect, n_affect, rows, cols, RowView{rp, n_cut, (row_ptr_len - 1) / n_cut, n_edges},
-                 mark, l, n_mark, out, windows_high, in_win, buff_index, buf_size};
-    int g = ops_grid(n_affect);
+                 mark, l, n_mark, out, windows_high, in_win, buff_index, buf_size, 0};
+    int g = walk_grid(n_affect, &A.group);
     if (g < 0) return TDT_ERR_CUDA;
     switch (mode) {
         case kAffectDeleted: affect_kernel<kAffectDeleted><<<g, kOpsBlock, 0, st>>>(A); break;
@@ -376,8 +487,8 @@ int launch_support_k(const int32_t* rows, const int32_t* cols, const int32_t* rp
     TDT_CHECK_ARG(n_edges >= 0, "negative size");
     if (n_edges == 0) return TDT_OK;
     TDT_CHECK_ARG(rows && cols && rp && out, "null pointer");
-    EdgeOpArgs A{rows, cols, RowView{rp, n_cut, (row_ptr_len - 1) / n_cut, n_edges}, n_edges, k, nullptr, out};
-    int g = ops_grid(n_edges);
+    EdgeOpArgs A{rows, cols, RowView{rp, n_cut, (row_ptr_len - 1) / n_cut, n_edges}, n_edges, k, nullptr, out, 0};
+    int g = walk_grid(n_edges, &A.group);
     if (g < 0) return TDT_ERR_CUDA;
     support_k_kernel<<<g, kOpsBlock, 0, st>>>(A);
     TDT_LAUNCH_CHECK("support_k");
@@ -392,8 +503,8 @@ int launch_sub_affect(const int32_t* rows, const int32_t* cols, const int32_t* r
     TDT_CHECK_ARG(n_edges >= 0, "negative size");
     if (n_edges == 0) return TDT_OK;
     TDT_CHECK_ARG(rows && cols && rp && mark && out, "null pointer");
-    EdgeOpArgs A{rows, cols, RowView{rp, n_cut, (row_ptr_len - 1) / n_cut, n_edges}, n_edges, 0, mark, out};
-    int g = ops_grid(n_edges);
+    EdgeOpArgs A{rows, cols, RowView{rp, n_cut, (row_ptr_len - 1) / n_cut, n_edges}, n_edges, 0, mark, out, 0};
+    int g = walk_grid(n_edges, &A.group);
     if (g < 0) return TDT_ERR_CUDA;
     sub_affect_kernel<<<g, kOpsBlock, 0, st>>>(A);
     TDT_LAUNCH_CHECK("sub_affect");
