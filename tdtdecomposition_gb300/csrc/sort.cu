@@ -127,27 +127,31 @@ int scan_stage_slots(const int64_t* rp, int64_t* out, int64_t nv, int64_t* total
 constexpr int kSortBlock = 256;   // one thread per digit
 constexpr int kSortWarps = kSortBlock / kWarp;
 static_assert(kSortBlock == kRadix, "one thread per digit");
-// Keys per thread, blocks per SM and tiles looked back on at a time (67 M draws
-// / 65,536 draws preprocessed: 7.62 ms / 312 us with 12, 5, 4; 7.53 / 352 with
-// 16, 4, 4; 8.38 / 317 with 8, 6, 4; 8.26 / 362 with 16, 4, 1).
-constexpr int kSortItems = 12;
-constexpr int kSortMinBlocks = 5;
-constexpr int kBack = 4;
-constexpr int kSortTile = kSortBlock * kSortItems;
+// Keys per thread: 16 leave four blocks per SM, long runs of a digit and few
+// look-backs; a sort of few tiles is a chain of latencies, so its tiles are
+// smaller (65,536 / 0.8 M / 67 M draws preprocessed: 318 us / 390 us / 6.77 ms
+// with 12, 326 / 406 / 6.26 with 16, 24 at three blocks per SM 332 us / 6.17 ms).
+constexpr int kSortItems = 16, kSortSmallItems = 12;
+constexpr int64_t kSortSmall = 1 << 20;
+constexpr int kSortBatch = 4;          // steps ranked together
+static_assert(kSortItems % kSortBatch == 0 && kSortSmallItems % kSortBatch == 0, "whole batches");
+constexpr int kBack = 4;               // tiles looked back on at a time
+static int64_t sort_tile(int64_t n) { return (int64_t)kSortBlock * (n < kSortSmall ? kSortSmallItems : kSortItems); }
 // counts fit 30 bits below this many keys
 constexpr int64_t kWideKeys = 1ll << 30;
 
-template <class K, class S, bool kVals, bool kIota>
-__global__ void __launch_bounds__(kSortBlock, kSortMinBlocks) radix_pass_kernel(
+template <class K, class S, bool kVals, bool kIota, int kItems>
+__global__ void __launch_bounds__(kSortBlock, 4) radix_pass_kernel(
     const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, K* __restrict__ keys_out,
     uint32_t* __restrict__ vals_out, int64_t n, int pass, const uint32_t* __restrict__ hist,
     uint32_t* tile_next, S* words, const uint32_t* n_dev, const long long* max_dev, int* status) {
     using W = TileWord<S>;
+    constexpr int kTile = kSortBlock * kItems;
     if (max_dev && pass > 0 && (*max_dev >> (8 * pass)) == 0) return;
     if (n_dev) n = *n_dev < n ? (int64_t)*n_dev : n;
     extern __shared__ __align__(16) unsigned char smem[];
     K* s_keys = reinterpret_cast<K*>(smem);
-    uint32_t* s_vals = reinterpret_cast<uint32_t*>(smem + sizeof(K) * kSortTile);
+    uint32_t* s_vals = reinterpret_cast<uint32_t*>(smem + sizeof(K) * kTile);
     __shared__ uint32_t s_wcnt[kSortWarps][kRadix];  // per warp: counts, then first places in the tile
     __shared__ uint32_t s_to[kRadix];      // first place of the digit in the output minus that in the tile (mod 2^32)
     __shared__ uint32_t s_tmp[33];
@@ -159,32 +163,52 @@ __global__ void __launch_bounds__(kSortBlock, kSortMinBlocks) radix_pass_kernel(
     for (int i = lane; i < kRadix; i += kWarp) s_wcnt[w][i] = 0;
     __syncthreads();
     const int64_t tile = s_tile;
-    const int64_t base = tile * kSortTile;
+    const int64_t base = tile * kTile;
     if (base >= n) return;
-    // warp w owns the contiguous sub-tile of kSortItems * 32 keys; ranks among
+    // warp w owns the contiguous sub-tile of kItems * 32 keys; ranks among
     // its keys of the same digit
-    K key[kSortItems];
-    uint32_t val[kVals ? kSortItems : 1];
-    uint16_t rank[kSortItems];
-    const int64_t mine = base + (int64_t)w * (kSortItems * kWarp) + lane;
+    K key[kItems];
+    uint32_t val[kVals ? kItems : 1];
+    uint16_t rank[kItems];
+    const int64_t mine = base + (int64_t)w * (kItems * kWarp) + lane;
 #pragma unroll
-    for (int it = 0; it < kSortItems; it++) {
+    for (int it = 0; it < kItems; it++) {
         const int64_t i = mine + it * kWarp;
-        key[it] = i < n ? keys_in[i] : K(0);
+        key[it] = i < n ? keys_in[i] : ~K(0);
         if (kVals) val[it] = kIota ? (uint32_t)i : (i < n ? vals_in[i] : 0u);
     }
-    // the first lane of a step's equal digits counts them in the warp's row, and
-    // all of them rank from its result
+    // The first lane of a step's equal digits counts them in the warp's row, and
+    // all of them rank from its result, kSortBatch steps at a time.  The equal
+    // digits come from eight ballots: __match_any_sync takes a turn per distinct
+    // value and held the passes over random digits at 0.58 ms, over skewed ones at
+    // 0.36 (67 M keys; preprocessing 7.70 -> 6.77 ms with the ballots, 6.97 with
+    // lane masks OR-ed in shared memory).  Keys past the end have the last digit
+    // and the last places, which are not written.
 #pragma unroll
-    for (int it = 0; it < kSortItems; it++) {
-        const bool ok = mine + it * kWarp < n;
-        const unsigned d = ok ? (unsigned)((key[it] >> shift) & 0xff) : (unsigned)kRadix;
-        const unsigned peers = __match_any_sync(kFull, d);
-        const int first = __ffs(peers) - 1;
-        uint32_t pre = 0;
-        if (ok && (int)lane == first) pre = atomicAdd(&s_wcnt[w][d], (uint32_t)__popc(peers));
-        rank[it] = (uint16_t)(__shfl_sync(kFull, pre, first) + __popc(peers & lanemask_lt()));
-        __syncwarp();
+    for (int b0 = 0; b0 < kItems; b0 += kSortBatch) {
+        unsigned peers[kSortBatch];
+        uint32_t pre[kSortBatch];
+#pragma unroll
+        for (int j = 0; j < kSortBatch; j++) {
+            const unsigned d = (unsigned)((key[b0 + j] >> shift) & 0xff);
+            peers[j] = kFull;
+#pragma unroll
+            for (int b = 0; b < 8; b++) {
+                const bool p = (d >> b) & 1u;
+                const unsigned v = __ballot_sync(kFull, p);
+                peers[j] &= p ? v : ~v;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kSortBatch; j++) {
+            const unsigned d = (unsigned)((key[b0 + j] >> shift) & 0xff);
+            pre[j] = 0;
+            if ((peers[j] & lanemask_lt()) == 0) pre[j] = atomicAdd(&s_wcnt[w][d], (uint32_t)__popc(peers[j]));
+            __syncwarp();
+        }
+#pragma unroll
+        for (int j = 0; j < kSortBatch; j++)
+            rank[b0 + j] = (uint16_t)(__shfl_sync(kFull, pre[j], __ffs(peers[j]) - 1) + __popc(peers[j] & lanemask_lt()));
     }
     __syncthreads();
     const int d = threadIdx.x;
@@ -204,12 +228,10 @@ __global__ void __launch_bounds__(kSortBlock, kSortMinBlocks) radix_pass_kernel(
     }
     const uint32_t digit0 = block_excl_scan<uint32_t>(__ldg(hist + d), s_tmp, nullptr);
 #pragma unroll
-    for (int it = 0; it < kSortItems; it++) {
-        if (mine + it * kWarp < n) {
-            const uint32_t p = s_wcnt[w][(unsigned)((key[it] >> shift) & 0xff)] + rank[it];
-            s_keys[p] = key[it];
-            if (kVals) s_vals[p] = val[it];
-        }
+    for (int it = 0; it < kItems; it++) {
+        const uint32_t p = s_wcnt[w][(unsigned)((key[it] >> shift) & 0xff)] + rank[it];
+        s_keys[p] = key[it];
+        if (kVals) s_vals[p] = val[it];
     }
     S before = 0;
     if (tile > 0) {
@@ -231,7 +253,7 @@ __global__ void __launch_bounds__(kSortBlock, kSortMinBlocks) radix_pass_kernel(
     }
     s_to[d] = digit0 + (uint32_t)before - start;
     __syncthreads();
-    const int tile_n = (int)(n - base < kSortTile ? n - base : kSortTile);
+    const int tile_n = (int)(n - base < kTile ? n - base : kTile);
     for (int i = threadIdx.x; i < tile_n; i += kSortBlock) {
         const K k = s_keys[i];
         const uint32_t g = s_to[(unsigned)((k >> shift) & 0xff)] + (uint32_t)i;
@@ -243,7 +265,7 @@ __global__ void __launch_bounds__(kSortBlock, kSortMinBlocks) radix_pass_kernel(
 }
 
 RadixScratch radix_scratch(void* base, int64_t n, int passes) {
-    const size_t ntiles = (size_t)((n + kSortTile - 1) / kSortTile);
+    const size_t ntiles = (size_t)((n + sort_tile(n) - 1) / sort_tile(n));
     const size_t head = ((size_t)kMaxPasses * kRadix + kMaxPasses) * 4 + 224;  // a multiple of 256
     const size_t word = n < kWideKeys ? 4 : 8;
     RadixScratch R;
@@ -254,15 +276,17 @@ RadixScratch radix_scratch(void* base, int64_t n, int passes) {
     return R;
 }
 
-template <class K, class S, bool kVals>
+template <class K, class S, bool kVals, int kItems>
 static int radix_passes(const K* in, K* b0, K* b1, uint32_t* v0, uint32_t* v1, int64_t n, int passes,
                         const RadixScratch& R, const uint32_t* n_dev, const long long* max_dev, int* status,
                         cudaStream_t st) {
-    const int64_t ntiles = (n + kSortTile - 1) / kSortTile;
-    const int smem = (int)(sizeof(K) + (kVals ? 4 : 0)) * kSortTile;
+    constexpr int kTile = kSortBlock * kItems;
+    const int64_t ntiles = (n + kTile - 1) / kTile;
+    const int smem = (int)(sizeof(K) + (kVals ? 4 : 0)) * kTile;
     S* words = reinterpret_cast<S*>(R.words);
     for (int p = 0; p < passes; p++) {
-        auto kern = kVals && p == 0 ? radix_pass_kernel<K, S, kVals, true> : radix_pass_kernel<K, S, kVals, false>;
+        auto kern = kVals && p == 0 ? radix_pass_kernel<K, S, kVals, true, kItems>
+                                       : radix_pass_kernel<K, S, kVals, false, kItems>;
         TDT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         const K* kin = p == 0 ? in : (p & 1) ? b0 : b1;
         const uint32_t* vin = (p & 1) ? v0 : v1;
@@ -280,10 +304,10 @@ int radix_sort(const K* in, K* b0, K* b1, uint32_t* v0, uint32_t* v1, int64_t n,
     if (n <= 0) return TDT_OK;
     TDT_CHECK_ARG(n < (int64_t)UINT32_MAX, "radix sort of %lld keys exceeds 32-bit ranks", (long long)n);
     TDT_CHECK_ARG(passes >= 1 && passes <= kMaxPasses, "%d radix passes", passes);
-    return n < kWideKeys
-               ? radix_passes<K, uint32_t, kVals>(in, b0, b1, v0, v1, n, passes, R, n_dev, max_dev, status, st)
-               : radix_passes<K, unsigned long long, kVals>(in, b0, b1, v0, v1, n, passes, R, n_dev, max_dev, status,
-                                                            st);
+    auto run = n < kSortSmall  ? radix_passes<K, uint32_t, kVals, kSortSmallItems>
+               : n < kWideKeys ? radix_passes<K, uint32_t, kVals, kSortItems>
+                               : radix_passes<K, unsigned long long, kVals, kSortItems>;
+    return run(in, b0, b1, v0, v1, n, passes, R, n_dev, max_dev, status, st);
 }
 
 template int radix_sort<uint32_t, true>(const uint32_t*, uint32_t*, uint32_t*, uint32_t*, uint32_t*, int64_t, int,

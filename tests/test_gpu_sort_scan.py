@@ -78,3 +78,10 @@ def test_peel_order_tile_edges(pairs):
                                  rows=torch.as_tensor(rows).cuda()))
     assert r.kmax == kmax and np.array_equal(r.e_truss.cpu().numpy(), et)
     assert np.array_equal(r.ptr_truss.cpu().numpy(), pt) and np.array_equal(r.truss.cpu().numpy(), truss)
+
+
+@pytest.mark.parametrize("m", [(1 << 20) - 1, 1 << 20, (1 << 20) + 1, (1 << 20) + 4095, (1 << 20) + 4097])
+def test_preprocess_large_tiles(m):
+    """Draws around the size from which the sort takes its larger tiles."""
+    rng = np.random.default_rng(m)
+    _check(rng.integers(0, 300, m), rng.integers(0, 60000, m))
