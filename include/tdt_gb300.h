@@ -146,6 +146,12 @@ int tdt_segment_add(const int32_t *col_indices, int64_t num_values, const int32_
 int tdt_segment_max(const int32_t *values, int64_t num_values, const int64_t *offsets,
                     int64_t num_segments, int64_t *output, tdt_stream_t stream);
 
+/* Largest value of two arrays (no counterpart in the reference; it sizes
+ * tdt_preprocess's id space): output[0] = max(a[0:na], b[0:nb]).  Of two empty
+ * arrays, or of values that are all below -2139062144, it is -2139062144. */
+int tdt_max_id(const int32_t *a, int64_t na, const int32_t *b, int64_t nb, int32_t *output,
+               tdt_stream_t stream);
+
 /* segment_isin2 (myhpu_extension.cpp:24-34; kernel.cu:28-79) and
  * segment_isin2tile (myhpu_extension.cpp:43-56; kernel.cu:81-141):
  * output[i] += number of triangles containing edge i (its support).

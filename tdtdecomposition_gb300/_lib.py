@@ -38,6 +38,7 @@ _SIGS = [
     ("tdt_test_barrier_timeout", ctypes.c_int, [c_ptr, ctypes.c_longlong, c_ptr]),
     ("tdt_segment_add", ctypes.c_int, [c_ptr, c_i64, c_ptr, c_ptr, c_i64, c_ptr]),
     ("tdt_segment_max", ctypes.c_int, [c_ptr, c_i64, c_ptr, c_i64, c_ptr, c_ptr]),
+    ("tdt_max_id", ctypes.c_int, [c_ptr, c_i64, c_ptr, c_i64, c_ptr, c_ptr]),
     ("tdt_segment_isin2", ctypes.c_int, [c_ptr, c_ptr, c_ptr, c_i64, c_ptr, c_i64, c_ptr]),
     ("tdt_segment_isin2tile", ctypes.c_int, [c_ptr, c_ptr, c_ptr, c_i64, c_i32, c_ptr, c_i64, c_ptr]),
     ("tdt_sub_all_affected_support", ctypes.c_int,

@@ -107,6 +107,7 @@ int device_info(DeviceInfo* out) {
 // ops.cu
 int launch_segment_add(const int32_t*, const int32_t*, int32_t*, int64_t, int64_t, cudaStream_t);
 int launch_segment_max(const int32_t*, const int64_t*, int64_t, int64_t, int64_t*, cudaStream_t);
+int launch_max_id(const int32_t* a, int64_t na, const int32_t* b, int64_t nb, int32_t* out, cudaStream_t st);
 int launch_affect(int mode, const int32_t*, int64_t, const int32_t*, const int32_t*, const int32_t*, int64_t,
                   int32_t, const uint8_t*, int32_t, uint8_t*, int32_t*, int32_t, uint8_t*, int32_t*, int32_t*,
                   int64_t, cudaStream_t);
@@ -226,6 +227,10 @@ API int tdt_segment_add(const int32_t* col_indices, int64_t num_values, const in
 API int tdt_segment_max(const int32_t* values, int64_t num_values, const int64_t* offsets, int64_t num_segments,
                         int64_t* output, tdt_stream_t stream) {
     return launch_segment_max(values, offsets, num_segments, num_values, output, (cudaStream_t)stream);
+}
+
+API int tdt_max_id(const int32_t* a, int64_t na, const int32_t* b, int64_t nb, int32_t* output, tdt_stream_t stream) {
+    return launch_max_id(a, na, b, nb, output, (cudaStream_t)stream);
 }
 
 API int tdt_segment_isin2(const int32_t* a_rows, const int32_t* b_col_indices, const int32_t* b_row_ptr,

@@ -17,6 +17,18 @@ from . import _lib
 from .graph import CSRCOO
 
 
+def _max_id(a, b=None):
+    if b is not None and (b.device != a.device or b.numel() == 0):
+        raise RuntimeError("src and dst must be non-empty and on one device")
+    out = torch.empty(1, dtype=torch.int32, device=a.device)
+    with torch.cuda.device(a.device):
+        rc = _lib.load().tdt_max_id(a.data_ptr(), a.numel(), b.data_ptr() if b is not None else None,
+                                    b.numel() if b is not None else 0, out.data_ptr(),
+                                    torch.cuda.current_stream(a.device).cuda_stream)
+    _lib.check(rc, "tdt_max_id")
+    return out.item()
+
+
 def preprocess_edges(src, dst, vertex_group=None, num_ids=None, workspace=None):
     """src, dst: int32 CUDA tensors of the raw edge list (ids >= 0).  Returns
     (CSRCOO with int64 row_ptr, vertices: int32 original id of each rank),
@@ -35,11 +47,11 @@ def preprocess_edges(src, dst, vertex_group=None, num_ids=None, workspace=None):
     dev = src.device
     m = src.numel()
     if num_ids is None:
-        num_ids = int(torch.maximum(src.max(), dst.max())) + 1 if m else 0
+        num_ids = _max_id(src, dst) + 1 if m else 0
     ng = 0
     if vertex_group is not None:
         vertex_group = vertex_group.to(torch.int32).contiguous()
-        ng = int(vertex_group.max()) + 1 if vertex_group.numel() else 1
+        ng = _max_id(vertex_group) + 1 if vertex_group.numel() else 1
         if vertex_group.numel() < num_ids:
             raise ValueError("vertex_group must hold one entry per vertex id")
     rows = torch.empty(max(m, 1), dtype=torch.int32, device=dev)
@@ -56,10 +68,10 @@ def preprocess_edges(src, dst, vertex_group=None, num_ids=None, workspace=None):
                               rows.data_ptr(), cols.data_ptr(), rp.data_ptr(), verts.data_ptr(), counts.data_ptr(),
                               ws.data_ptr(), ws.numel(), torch.cuda.current_stream(dev).cuda_stream)
     _lib.check(rc, "tdt_preprocess")
-    E, V, st = (int(x) for x in counts.cpu())
+    E, V, st = counts.tolist()
     if st != 0:
         raise _lib.TdtError(st, "tdt_preprocess", "vertex id outside [0, num_ids)")
-    g = CSRCOO(columns=cols[:E], row_ptr=rp[:V + 1].clone(), rows=rows[:E])
+    g = CSRCOO(columns=cols[:E], row_ptr=rp if V == num_ids else rp[:V + 1].clone(), rows=rows[:E])
     return g, verts[:V]
 
 

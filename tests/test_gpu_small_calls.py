@@ -67,3 +67,16 @@ def test_malformed_is_refused(name, rp, c):
             call()
     stats = T.truss_decompose(g, lists=False, sync=False)[3].cpu()
     assert int(stats[T.STAT_STATUS]) != 0 and int(stats[1:].abs().sum()) == 0
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 255, 256, 257, 100003, 3000001])
+def test_max_id(n):
+    from tdtdecomposition_gb300.preprocess import _max_id
+    rng = np.random.default_rng(n)
+    a, b = rng.integers(0, 1 << 31, n, dtype=np.int64).astype(np.int32), rng.integers(0, 1 << 30, n + 5).astype(np.int32)
+    a[rng.integers(n)] = (1 << 31) - 1 if n % 2 else 7
+    ca, cb = torch.as_tensor(a).cuda(), torch.as_tensor(b).cuda()
+    assert _max_id(ca, cb) == max(int(a.max()), int(b.max()))
+    assert _max_id(ca[n - 1:]) == int(a[-1])
+    with pytest.raises(RuntimeError):
+        _max_id(ca, ca[:0])
