@@ -89,6 +89,8 @@ def _list_bytes(ws, cols, rp, lists, base, rows=None):
     need = 24 * T + 256
     if lists is True:
         return need + S
+    if ws.buf is not None and base + need + S <= ws.buf.numel():
+        return need + S  # the workspace holds it already: nothing to ask the driver for
     free, _ = torch.cuda.mem_get_info(cols.device)
     have = free + (ws.buf.numel() if ws.buf is not None else 0) - base
     if need + S <= STAGE_BUDGET_FRACTION * have:
@@ -163,10 +165,10 @@ def truss_decompose(graph, workspace=None, stream=None, sync=True, lists="auto",
     _lib.check(rc, "tdt_truss_decompose")
     if not sync:
         return truss, e_truss, ptr, stats
-    sh = stats.cpu()
+    sh = stats.tolist()
     _check_stats(sh, "tdt_truss_decompose")
-    return TrussResult(truss, e_truss[: int(sh[STAT_NETRUSS])], ptr[: int(sh[STAT_NPTR])], int(sh[STAT_KMAX]),
-                       int(sh[STAT_TRIANGLES]), int(sh[STAT_ROUNDS]), bool(sh[STAT_LISTED]), int(sh[STAT_LISTED]))
+    return TrussResult(truss, e_truss[: sh[STAT_NETRUSS]], ptr[: sh[STAT_NPTR]], sh[STAT_KMAX],
+                       sh[STAT_TRIANGLES], sh[STAT_ROUNDS], bool(sh[STAT_LISTED]), sh[STAT_LISTED])
 
 
 def ktruss_search(graph, k, workspace=None, stream=None, lists="auto"):
@@ -187,7 +189,7 @@ def ktruss_search(graph, k, workspace=None, stream=None, lists="auto"):
         rc = L.tdt_ktruss_search(rows.data_ptr() if rows is not None else None, cols.data_ptr(), rp.data_ptr(), V, E,
                                  int(k), mask.data_ptr(), stats.data_ptr(), ws.data_ptr(), base + tail, s)
     _lib.check(rc, "tdt_ktruss_search")
-    _check_stats(stats.cpu(), "tdt_ktruss_search")
+    _check_stats(stats.tolist(), "tdt_ktruss_search")
     return mask
 
 
@@ -200,9 +202,9 @@ def triangle_count_arrays(cols, rp, ws):
         rc = L.tdt_triangle_count(cols.data_ptr(), rp.data_ptr(), V, E, None, stats.data_ptr(), buf.data_ptr(),
                                   buf.numel(), torch.cuda.current_stream(cols.device).cuda_stream)
     _lib.check(rc, "tdt_triangle_count")
-    sh = stats.cpu()
+    sh = stats.tolist()
     _check_stats(sh, "tdt_triangle_count")
-    return int(sh[STAT_TRIANGLES])
+    return sh[STAT_TRIANGLES]
 
 
 def triangle_count(graph, workspace=None, stream=None, return_support=False):
@@ -220,9 +222,9 @@ def triangle_count(graph, workspace=None, stream=None, return_support=False):
                                   support.data_ptr() if support is not None else None,
                                   stats.data_ptr(), ws.data_ptr(), ws.numel(), s)
     _lib.check(rc, "tdt_triangle_count")
-    sh = stats.cpu()
+    sh = stats.tolist()
     _check_stats(sh, "tdt_triangle_count")
-    T = int(sh[STAT_TRIANGLES])
+    T = sh[STAT_TRIANGLES]
     return (T, support) if return_support else T
 
 
