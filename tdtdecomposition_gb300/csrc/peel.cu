@@ -72,7 +72,7 @@ struct PeelCtl {
     // processing, and level transitions; diagnostic only
     unsigned long long t_proc, t_wait, t_trans, t_total;
     unsigned long long grab[4];    // slot cursor of search-mode sub-round r, at r & 3
-    unsigned done;                 // blocks of a triangle count that finished
+    unsigned done;                 // blocks of a counting last kernel that finished
 };
 
 // How the peel finds an edge's triangles: in its list, by search in the graph's
@@ -1658,21 +1658,6 @@ __global__ void init_state_kernel(const int32_t* __restrict__ cA, const int32_t*
     }
 }
 
-// Lists fit when 8 bytes x (3T = off[E]) fit the list tail.  After the one
-// walk the role-A entries are moved from the staging slots (at the end of the
-// tail) when both fit side by side; otherwise, when the lists alone fit, a
-// second walk writes them; otherwise the peel searches.
-__global__ void list_decide_kernel(const int64_t* __restrict__ off, const int64_t* __restrict__ sbase, int64_t E,
-                                   int64_t V, unsigned long long tail_bytes, PeelCtl* ctl) {
-    const unsigned long long need = (unsigned long long)off[E], slots = tail_bytes / 8;
-    const int ok = ctl->g.status == 0 && need <= slots;
-    const int compact = ok && !ctl->stage_skip && need <= slots - (unsigned long long)sbase[V];
-    ctl->listed = ok;
-    ctl->list_skip = !ok;
-    ctl->compact_skip = !compact;
-    ctl->rewalk_skip = !ok || compact;
-}
-
 // Truss numbers, and the digit totals of the sort by round.
 __global__ void __launch_bounds__(256) truss_out_kernel(const int32_t* __restrict__ rnd,
                                                         const int32_t* __restrict__ round_level, int64_t E,
@@ -1696,27 +1681,40 @@ __global__ void __launch_bounds__(256) truss_out_kernel(const int32_t* __restric
     H.flush(run, hist);
 }
 
-// Number of sorted positions whose round has level <= lv (levels are
-// non-decreasing in round order).
+// Number of sorted positions whose round has level <= lv: the first round above
+// it (levels do not fall from round to round), then its first position.
 __device__ __forceinline__ int64_t count_level_le(const uint32_t* keys, int64_t E, const int32_t* round_level,
-                                                  int32_t lv) {
-    int64_t lo = 0, hi = E;
+                                                  int64_t rounds, int32_t lv) {
+    int64_t lo = 0, hi = rounds;
     while (lo < hi) {
-        int64_t mid = (lo + hi) >> 1;
-        if (round_level[keys[mid]] <= lv) lo = mid + 1; else hi = mid;
+        const int64_t mid = (lo + hi) >> 1;
+        if (__ldg(round_level + mid) <= lv) lo = mid + 1; else hi = mid;
+    }
+    const int64_t r = lo;
+    for (lo = 0, hi = E; lo < hi;) {
+        const int64_t mid = (lo + hi) >> 1;
+        if ((int64_t)__ldg(keys + mid) < r) lo = mid + 1; else hi = mid;
     }
     return lo;
 }
 
-// k0 / v0: the buffer of the sort's first pass, k1 / v1 of its second.
+// Stats words of a finished peel (how it found the triangles).
+__device__ __forceinline__ void write_stats(const PeelCtl* ctl, int64_t* stats, int status) {
+    for (int i = 0; i < TDT_STAT_COUNT; i++) stats[i] = 0;
+    stats[TDT_STAT_STATUS] = status;
+    stats[TDT_STAT_LISTED] = ctl->listed ? (ctl->compact_skip ? 1 : 2) : 0;
+}
+
 __global__ void ptr_etruss_kernel(const uint32_t* __restrict__ k0, const uint32_t* __restrict__ v0,
                                   const uint32_t* __restrict__ k1, const uint32_t* __restrict__ v1, int passes,
                                   int64_t E, const int32_t* __restrict__ round_level, int32_t* __restrict__ ptr_truss,
                                   int64_t ptr_cap, int32_t* __restrict__ e_truss, PeelCtl* ctl,
                                   int64_t* __restrict__ stats) {
-    if (*(volatile int*)&ctl->g.status != 0) {  // before this kernel, or its own: then thread 0 goes on
-        if (blockIdx.x == 0 && threadIdx.x == 0)
-            for (int i = 0; i < TDT_STAT_COUNT; i++) stats[i] = 0;
+    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t nth = (int64_t)gridDim.x * blockDim.x;
+    const int status = *(volatile int*)&ctl->g.status;
+    if (status != 0) {  // of an earlier kernel, or thread 0's of this one
+        if (tid == 0) write_stats(ctl, stats, status);
         return;
     }
     const long long rounds = ctl->rounds;
@@ -1724,20 +1722,20 @@ __global__ void ptr_etruss_kernel(const uint32_t* __restrict__ k0, const uint32_
     const uint32_t* keys = first ? k0 : k1;
     const uint32_t* vals = first ? v0 : v1;
     const int32_t L = rounds > 0 ? round_level[rounds - 1] : 0;
-    const int64_t n0 = rounds > 0 ? count_level_le(keys, E, round_level, 0) : E;
-    const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t nth = (int64_t)gridDim.x * blockDim.x;
+    const int64_t n0 = rounds > 0 ? count_level_le(keys, E, round_level, rounds, 0) : E;
     if (ptr_truss) {
         if ((int64_t)L + 1 > ptr_cap) {
             if (tid == 0) atomicMax(&ctl->g.status, (int)TDT_ERR_CAPACITY);
         } else {
             for (int64_t i = tid; i <= L; i += nth)
-                ptr_truss[i] = (int32_t)((i == 0 ? n0 : count_level_le(keys, E, round_level, (int32_t)i)) - n0);
+                ptr_truss[i] = (int32_t)((i == 0 ? n0 : count_level_le(keys, E, round_level, rounds, (int32_t)i)) -
+                                         n0);
         }
     }
     if (e_truss)
         for (int64_t p = n0 + tid; p < E; p += nth) e_truss[p - n0] = (int32_t)vals[p];
     if (tid == 0) {
+        write_stats(ctl, stats, ptr_truss && (int64_t)L + 1 > ptr_cap ? TDT_ERR_CAPACITY : TDT_OK);
         stats[TDT_STAT_KMAX] = (long long)L + 2;
         stats[TDT_STAT_NPTR] = (long long)L + 1;
         stats[TDT_STAT_ROUNDS] = rounds;
@@ -1746,8 +1744,9 @@ __global__ void ptr_etruss_kernel(const uint32_t* __restrict__ k0, const uint32_
     }
 }
 
+// Membership; the last block writes the stats.
 __global__ void ktruss_out_kernel(const int32_t* __restrict__ rnd, int64_t E, uint8_t* __restrict__ in_k,
-                                  PeelCtl* ctl) {
+                                  PeelCtl* ctl, int64_t* __restrict__ stats) {
     __shared__ unsigned long long s_part[32];
     unsigned long long acc = 0;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < E;
@@ -1763,21 +1762,13 @@ __global__ void ktruss_out_kernel(const int32_t* __restrict__ rnd, int64_t E, ui
         unsigned long long b = 0;
         for (int i = 0; i < (int)(blockDim.x / kWarp); i++) b += s_part[i];
         atomicAdd(&ctl->alive, b);
-    }
-}
-
-// The stats words that ptr_etruss_kernel leaves (mode 0), or all.
-__global__ void stats_final_kernel(PeelCtl* ctl, int64_t* stats, int mode) {
-    const int st = ctl->g.status;
-    if (mode != 0)
-        for (int i = 0; i < TDT_STAT_COUNT; i++) stats[i] = 0;
-    stats[TDT_STAT_STATUS] = st;
-    stats[TDT_STAT_LISTED] = ctl->listed ? (ctl->compact_skip ? 1 : 2) : 0;
-    stats[TDT_STAT_ALIVE] = 0;
-    if (mode != 0) {
-        stats[TDT_STAT_ALIVE] = (long long)ctl->alive;
-        stats[TDT_STAT_ROUNDS] = ctl->rounds;
-        stats[TDT_STAT_TRIANGLES] = ctl->triangles / 3;
+        __threadfence();
+        if (atomicAdd(&ctl->done, 1u) == gridDim.x - 1) {
+            write_stats(ctl, stats, *(volatile int*)&ctl->g.status);
+            stats[TDT_STAT_ALIVE] = (long long)atomicAdd(&ctl->alive, 0ull);
+            stats[TDT_STAT_ROUNDS] = ctl->rounds;
+            stats[TDT_STAT_TRIANGLES] = ctl->triangles / 3;
+        }
     }
 }
 
@@ -1977,6 +1968,13 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     int32_t* cA = reinterpret_cast<int32_t*>(L.qi[0]);
     int32_t* cB = cA + E;
     int32_t* cC = cB + E;
+    // The list tail: final lists grow from its start, the staging slots of the
+    // one walk end at its end.
+    const size_t list_base = (need + 255) & ~(size_t)255;
+    const unsigned long long tail =
+        mode != 2 && ws_bytes > list_base ? (unsigned long long)(ws_bytes - list_base) : 0ull;
+    int2* lists = reinterpret_cast<int2*>(reinterpret_cast<char*>(ws) + list_base);
+    int2* stage_end = lists + tail / 8;
     prof_mark(0, st);
     // in-adjacency (CSC) of the oriented graph: the walk's middle vertices, and
     // the peel without lists
@@ -1988,21 +1986,11 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     const unsigned g_csc = (unsigned)(csc_tiles < csc_blocks ? csc_tiles : csc_blocks);
     indeg_kernel<<<g_csc, kCscBlock, 0, st>>>(cols, E, V, L.indeg, L.ctl);
     TDT_LAUNCH_CHECK("indeg");
-    rc = exclusive_scan(L.indeg, L.cp, V, L.cp + V, L.scan_cp, &L.ctl->g.status, st);
+    rc = tail > 0 ? scan_rows(L.indeg, L.cp, L.scan_cp, rp, L.sbase, L.scan_sb, V, &L.ctl->g.status, st)
+                  : exclusive_scan(L.indeg, L.cp, V, L.cp + V, L.scan_cp, &L.ctl->g.status, st);
     if (rc) return rc;
     csc_fill_kernel<<<g_csc, kCscBlock, 0, st>>>(rows_use, cols, E, V, csc_tile, L.cp, L.indeg, L.in_src, L.in_eid, L.ctl);
     TDT_LAUNCH_CHECK("csc_fill");
-    // The list tail: final lists grow from its start, the staging slots of the
-    // one walk end at its end.
-    const size_t list_base = (need + 255) & ~(size_t)255;
-    const unsigned long long tail =
-        mode != 2 && ws_bytes > list_base ? (unsigned long long)(ws_bytes - list_base) : 0ull;
-    int2* lists = reinterpret_cast<int2*>(reinterpret_cast<char*>(ws) + list_base);
-    int2* stage_end = lists + tail / 8;
-    if (tail > 0) {
-        rc = scan_stage_slots(rp, L.sbase, V, L.sbase + V, L.scan_sb, &L.ctl->g.status, st);
-        if (rc) return rc;
-    }
     // the walk: counts, and the role-A entries when they can be staged (skipped
     // on the device when validation failed); the plan of its units stays for
     // the list walk
@@ -2021,10 +2009,10 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     }
     // per-edge triangle lists in the workspace tail when 24 T bytes fit
     if (tail > 0) {
-        rc = exclusive_scan(L.sup, L.off, E, L.off + E, L.scan_off, &L.ctl->g.status, st);
+        const ListDecision D{L.sbase + V, tail, &L.ctl->stage_skip, &L.ctl->listed, &L.ctl->list_skip,
+                             &L.ctl->compact_skip, &L.ctl->rewalk_skip};
+        rc = scan_lists(L.sup, L.off, E, L.scan_off, D, &L.ctl->g.status, st);
         if (rc) return rc;
-        list_decide_kernel<<<1, 1, 0, st>>>(L.off, L.sbase, E, V, tail, L.ctl);
-        TDT_LAUNCH_CHECK("list_decide");
         // second walk, when the lists fit but not beside the staging slots
         rc = launch_walk_list(rp, cols, L.cp, L.in_src, L.in_eid, V, E, L.off, cA, lists, L.alive[0], L.qi[2],
                               L.sup_ctl, &L.ctl->rewalk_skip, &L.ctl->g.status, st);
@@ -2116,13 +2104,9 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
         ptr_etruss_kernel<<<g_e, tb, 0, st>>>(k0, v0, k1, v1, passes, E, L.round_level, ptr_truss, ptr_cap, e_truss,
                                               L.ctl, stats);
         TDT_LAUNCH_CHECK("ptr_etruss");
-        stats_final_kernel<<<1, 1, 0, st>>>(L.ctl, stats, 0);
-        TDT_LAUNCH_CHECK("stats_final");
     } else {
-        ktruss_out_kernel<<<g_e, tb, 0, st>>>(L.rnd, E, in_k, L.ctl);
+        ktruss_out_kernel<<<g_e, tb, 0, st>>>(L.rnd, E, in_k, L.ctl, stats);
         TDT_LAUNCH_CHECK("ktruss_out");
-        stats_final_kernel<<<1, 1, 0, st>>>(L.ctl, stats, 1);
-        TDT_LAUNCH_CHECK("stats_final");
     }
     prof_mark(4, st);
     return TDT_OK;

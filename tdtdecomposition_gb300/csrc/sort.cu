@@ -52,34 +52,45 @@ struct ScanStageSlots {
 };
 
 template <class In>
-__global__ void __launch_bounds__(kScanBlock) scan_kernel(In in, int64_t n, int64_t* out, int64_t* total_out,
-                                                          unsigned long long* words, unsigned* next, int* status) {
+struct ScanJob {
+    In in;
+    int64_t n;
+    int64_t* out;
+    int64_t* total;
+    unsigned long long* words;
+    unsigned* next;
+    int64_t tiles;
+};
+
+// One tile of a job; done(total) is called by one thread of the last tile.
+template <class In, class Done>
+__device__ __forceinline__ void scan_tile(const ScanJob<In>& J, int* status, Done&& done) {
     using W = TileWord<unsigned long long>;
     using TO = int64_t;
     __shared__ TO s_warp[33];
     __shared__ unsigned s_tile;
     __shared__ unsigned long long s_before;
-    if (threadIdx.x == 0) s_tile = atomicAdd(next, 1u);
+    if (threadIdx.x == 0) s_tile = atomicAdd(J.next, 1u);
     __syncthreads();
-    const int64_t tile = s_tile;
+    const int64_t tile = s_tile, n = J.n;
     const int64_t base = tile * kScanTile + (int64_t)threadIdx.x * kScanItems;
     TO v[kScanItems];
     TO sum = 0;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        v[k] = base + k < n ? in(base + k) : TO(0);
+        v[k] = base + k < n ? J.in(base + k) : TO(0);
         sum += v[k];
     }
     TO tot;
     TO run = block_excl_scan<TO>(sum, s_warp, &tot);
     if (threadIdx.x < kWarp) {
         if (threadIdx.x == 0)
-            *(volatile unsigned long long*)(words + tile) =
+            *(volatile unsigned long long*)(J.words + tile) =
                 (tile == 0 ? W::kInclusive : W::kAggregate) | (unsigned long long)tot;
-        const unsigned long long before = warp_look_back(words, tile, status);
+        const unsigned long long before = warp_look_back(J.words, tile, status);
         if (threadIdx.x == 0) {
             if (tile > 0)
-                *(volatile unsigned long long*)(words + tile) =
+                *(volatile unsigned long long*)(J.words + tile) =
                     W::kInclusive | ((before + (unsigned long long)tot) & W::kValue);
             s_before = before;
         }
@@ -88,10 +99,39 @@ __global__ void __launch_bounds__(kScanBlock) scan_kernel(In in, int64_t n, int6
     run += (TO)s_before;
 #pragma unroll
     for (int k = 0; k < kScanItems; k++) {
-        if (base + k < n) out[base + k] = run;
+        if (base + k < n) J.out[base + k] = run;
         run += v[k];
     }
-    if (total_out && tile == (int64_t)gridDim.x - 1 && threadIdx.x == kScanBlock - 1) *total_out = run;
+    if (tile == J.tiles - 1 && threadIdx.x == kScanBlock - 1) {
+        if (J.total) *J.total = run;
+        done(run);
+    }
+}
+
+__global__ void __launch_bounds__(kScanBlock) scan_kernel(ScanJob<ScanArray<int32_t>> J, int* status) {
+    scan_tile(J, status, [](int64_t) {});
+}
+
+// The in-adjacency's offsets and the rows' staging slots, tiles of both in one
+// launch (a launch and 5 us of a small call).
+__global__ void __launch_bounds__(kScanBlock) scan_rows_kernel(ScanJob<ScanArray<int32_t>> J,
+                                                               ScanJob<ScanStageSlots> K, int* status) {
+    if (blockIdx.x < J.tiles) scan_tile(J, status, [](int64_t) {});
+    else scan_tile(K, status, [](int64_t) {});
+}
+
+// The lists' offsets, and whether there are lists.
+__global__ void __launch_bounds__(kScanBlock) scan_lists_kernel(ScanJob<ScanArray<int32_t>> J, ListDecision D,
+                                                                int* status) {
+    scan_tile(J, status, [&](int64_t need) {
+        const unsigned long long slots = D.tail_bytes / 8;
+        const int ok = *(volatile int*)status == 0 && (unsigned long long)need <= slots;
+        const int compact = ok && !*D.stage_skip && (unsigned long long)need <= slots - (unsigned long long)*D.staged;
+        *D.listed = ok;
+        *D.list_skip = !ok;
+        *D.compact_skip = !compact;
+        *D.rewalk_skip = !ok || compact;
+    });
 }
 
 size_t scan_scratch_bytes(int64_t n) {
@@ -100,27 +140,45 @@ size_t scan_scratch_bytes(int64_t n) {
 }
 
 template <class In>
-static int run_scan(In in, int64_t* out, int64_t n, int64_t* total_out, void* scratch, int* status, cudaStream_t st) {
-    if (n <= 0) {
-        if (total_out) TDT_CUDA(cudaMemsetAsync(total_out, 0, sizeof(int64_t), st));
-        return TDT_OK;
-    }
+static ScanJob<In> scan_job(In in, int64_t* out, int64_t n, int64_t* total, void* scratch) {
     const int64_t nb = (n + kScanTile - 1) / kScanTile;
     unsigned long long* words = reinterpret_cast<unsigned long long*>(scratch);
-    scan_kernel<In><<<(unsigned)nb, kScanBlock, 0, st>>>(in, n, out, total_out, words,
-                                                        reinterpret_cast<unsigned*>(words + nb), status);
+    return {in, n, out, total, words, reinterpret_cast<unsigned*>(words + nb), nb};
+}
+
+int exclusive_scan(const int32_t* in, int64_t* out, int64_t n, int64_t* total, void* scratch, int* status,
+                   cudaStream_t st) {
+    if (n <= 0) {
+        if (total) TDT_CUDA(cudaMemsetAsync(total, 0, sizeof(int64_t), st));
+        return TDT_OK;
+    }
+    const auto J = scan_job(ScanArray<int32_t>{in}, out, n, total, scratch);
+    scan_kernel<<<(unsigned)J.tiles, kScanBlock, 0, st>>>(J, status);
     TDT_LAUNCH_CHECK("scan");
     return TDT_OK;
 }
 
-int exclusive_scan(const int32_t* in, int64_t* out, int64_t n, int64_t* total_out, void* scratch, int* status,
-                   cudaStream_t st) {
-    return run_scan(ScanArray<int32_t>{in}, out, n, total_out, scratch, status, st);
+int scan_rows(const int32_t* in, int64_t* out, void* scratch, const int64_t* rp, int64_t* slots, void* slots_scratch,
+              int64_t nv, int* status, cudaStream_t st) {
+    if (nv <= 0) {
+        TDT_CUDA(cudaMemsetAsync(out, 0, sizeof(int64_t), st));
+        TDT_CUDA(cudaMemsetAsync(slots, 0, sizeof(int64_t), st));
+        return TDT_OK;
+    }
+    const auto J = scan_job(ScanArray<int32_t>{in}, out, nv, out + nv, scratch);
+    const auto K = scan_job(ScanStageSlots{rp, status}, slots, nv, slots + nv, slots_scratch);
+    scan_rows_kernel<<<(unsigned)(J.tiles + K.tiles), kScanBlock, 0, st>>>(J, K, status);
+    TDT_LAUNCH_CHECK("scan_rows");
+    return TDT_OK;
 }
 
-int scan_stage_slots(const int64_t* rp, int64_t* out, int64_t nv, int64_t* total_out, void* scratch, int* status,
-                     cudaStream_t st) {
-    return run_scan(ScanStageSlots{rp, status}, out, nv, total_out, scratch, status, st);
+int scan_lists(const int32_t* in, int64_t* out, int64_t n, void* scratch, const ListDecision& D, int* status,
+               cudaStream_t st) {
+    TDT_CHECK_ARG(n > 0, "no lists");
+    const auto J = scan_job(ScanArray<int32_t>{in}, out, n, out + n, scratch);
+    scan_lists_kernel<<<(unsigned)J.tiles, kScanBlock, 0, st>>>(J, D, status);
+    TDT_LAUNCH_CHECK("scan_lists");
+    return TDT_OK;
 }
 
 // ------------------------------------------------------------------ radix sort

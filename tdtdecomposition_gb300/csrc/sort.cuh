@@ -56,13 +56,28 @@ __device__ __forceinline__ S warp_look_back(const S* words, int64_t tile, int* s
 }
 
 size_t scan_scratch_bytes(int64_t n);
-// out[i] = sum(in[0..i)), and *total_out (device, may be null) = sum(in).
-// scratch: zeroed by the caller.  status: receives TDT_ERR_TIMEOUT.
-int exclusive_scan(const int32_t* in, int64_t* out, int64_t n, int64_t* total_out, void* scratch, int* status,
+// Scratch is zeroed by the caller; status receives TDT_ERR_TIMEOUT.
+// out[i] = sum(in[0..i)), and *total (device, may be null) = sum(in).
+int exclusive_scan(const int32_t* in, int64_t* out, int64_t n, int64_t* total, void* scratch, int* status,
                    cudaStream_t st);
-// The same over the staging slots of the rows of a CSR (walk.cu).
-int scan_stage_slots(const int64_t* rp, int64_t* out, int64_t nv, int64_t* total_out, void* scratch, int* status,
-                     cudaStream_t st);
+// The same over one int32 per vertex (out: nv + 1), and over the staging slots
+// of the rows of a CSR (slots: nv + 1; walk.cu).
+int scan_rows(const int32_t* in, int64_t* out, void* scratch, const int64_t* rp, int64_t* slots, void* slots_scratch,
+              int64_t nv, int* status, cudaStream_t st);
+// The same over n > 0 list lengths (out: n + 1), and the choice it leaves: lists
+// when their 8-byte entries fit the tail, from the staging slots when they fit
+// beside those.
+struct ListDecision {
+    const int64_t* staged;         // staging slots in all
+    unsigned long long tail_bytes;
+    const int* stage_skip;         // non-zero: nothing was staged
+    int* listed;
+    int* list_skip;
+    int* compact_skip;
+    int* rewalk_skip;
+};
+int scan_lists(const int32_t* in, int64_t* out, int64_t n, void* scratch, const ListDecision& D, int* status,
+               cudaStream_t st);
 
 // ------------------------------------------------------------------ radix sort
 // Stable LSD sort by 8-bit digits, one launch per pass: the digit totals of
