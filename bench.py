@@ -447,7 +447,7 @@ def bench_reference_gpu(dev, g, ws, flow_scale=18, reps=3):
     return {"image": "myhpu_extension_kernel.cu compiled unmodified for sm_103a",
             "support_pass": {"workload": "the benchmark graph (E=%d), n_cut = 2" % g.num_edges,
                              "reference_kernel": "checkElementsTwoPtrTile (K3)", "reference_ms": t_ref,
-                             "ours_kernel": "support_kernel (count walk, tdt_triangle_count)", "ours_ms": t_ours,
+                             "ours_kernel": "walk_kernel (count walk, tdt_triangle_count)", "ours_ms": t_ours,
                              "speedup": t_ref / t_ours, "same_support": same},
             "flow": {"workload": "R-MAT scale %d, edge factor 16, seed 1 (V=%d, E=%d)" % (flow_scale, V, E),
                      "reference": "singlegpu_truss.k_truss flow over the reference kernels (n_cut = 2)",
@@ -896,10 +896,10 @@ def main_ours(args):
     ach = B_dec / (ms_step / 1e3) / 1e9
     phases_ms = {"support": t_sup, "listing": t_list, "peel": t_peel, "outputs": t_post}
     per_kernel = {
-        "support_kernel": {"ms": round(t_sup, 4), "algorithmic_bytes": B_sup,
+        "support phase (in-adjacency, walk)": {"ms": round(t_sup, 4), "algorithmic_bytes": B_sup,
                            "achieved_gbs": round(B_sup / (t_sup / 1e3) / 1e9, 1),
                            "traffic": mt["support"] if mt else None},
-        "reenumeration (listing + transpose + peel kernels)": {
+        "reenumeration (distribution + peel kernels)": {
             "ms": round(t_list + t_peel, 4), "algorithmic_bytes": B_sup,
             "achieved_gbs": round(B_sup / ((t_list + t_peel) / 1e3) / 1e9, 1),
             "traffic": (mt["listing"] + mt["peel"]) if mt else None},

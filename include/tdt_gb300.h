@@ -385,11 +385,10 @@ enum tdt_stat_index {
  * per-edge triangle lists: when 24 * T bytes fit there (T = triangle count),
  * the peel reads each peeled edge's triangles from its list; otherwise it
  * finds them by binary search in the adjacency.  When the tail also holds the
- * staging area of the one walk (8 bytes per slot of the per-edge bounds
- * min(d+(u)-i-1, d+(v)) + min(i, d-(v)-1), edge (u,v) at position i of row
- * u), one walk counts the triangles and writes the lists; otherwise a
- * count-only walk runs first and a second walk writes them.  Results are
- * identical every way. */
+ * staging area of the one walk (8 bytes per slot, d+(u)-i-1 slots for the edge
+ * at position i of row u), one walk counts the triangles and stages what the
+ * lists are made from; otherwise a count-only walk runs first and a second
+ * walk writes it.  Results are identical every way. */
 size_t tdt_decompose_workspace_bytes(int64_t num_vertices, int64_t num_edges);
 
 /* Full truss decomposition: the single-call replacement of the `--cuda` flow

@@ -1,12 +1,11 @@
 """Autotuner of the work split and launch shape.
 
-The support and listing kernels give a row to one warp when its out-degree is
-at most `warp_cap`, to a whole block (shared-memory staged, pairs spread
-evenly over 512 threads) when it is at most `heavy_cap`, and search it in
-place beyond that; their wedge walk reads one column per lane or 16-byte
-chunks of four (`vec`); the peel reads triangles from per-edge lists or
-searches for them (`lists`), on a persistent grid of `peel_grid` half-SM
-units (0: the size heuristic).  Which choice is fastest depends on the
+The triangle walk gives a row to one warp when its out-degree is at most
+`warp_cap` (and it has few in-edges), to a whole block otherwise, in column
+chunks of `heavy_cap` entries; `vec` is the wedge width of the drop-in support
+operator (the whole-path walk always reads 16-byte chunks of four columns);
+the peel reads triangles from per-edge lists or searches for them (`lists`),
+on a persistent grid of `peel_grid` half-SM units (0: the size heuristic).  Which choice is fastest depends on the
 degree profile and size of the workload, so the tuner times the candidates
 on the workload itself (CUDA events, after one warm-up run each), one
 dimension at a time from the defaults (a coordinate search: the split, then
