@@ -14,8 +14,10 @@ outputs) of that graph.
 * roofline: algorithmic bytes over CUDA-event time: a decomposition moves
          B_dec = 2 B_sup (B_sup = 4W + 28E + 4(V+1), W = sum over edges of
          d+(u)+d+(v)): the support pass, then one re-enumeration of each
-         edge's triangles (listing + peel); DRAM traffic per decomposition
-         from one ncu capture of this workload sits beside it;
+         edge's triangles (listing + peel).  B_sup counts the merge of both
+         rows of every edge; the walk tests fewer wedges, so a support phase
+         can read above the peak.  DRAM traffic from an ncu capture sits
+         beside it;
 * cpu_baseline: the oracle port of the reference's CPU flow (OpenMP, all host
          cores) on a bounded R-MAT sample.
 
@@ -747,22 +749,15 @@ def bench_served_small(dev, srv, num_graphs=4096, rate=20000.0):
 # ---------------------------------------------------------------- GPU arm
 # DRAM bytes per triangle of each phase of a decomposition (the sum of
 # dram__bytes_read.sum + dram__bytes_write.sum over the phase's kernels), from
-# a one-pass ncu capture of the main launches of one R-MAT scale-20
+# an ncu capture of the main launches of one R-MAT scale-20
 # decomposition (T = 423,980,669) of this build.  The lists, the staging area
 # and the peel's slots all grow with T, so a phase's traffic at another size
 # is its rate x T.  Reported beside the algorithmic bytes, never used for them.
-TRAFFIC_PER_TRIANGLE = {"support": 41.2, "listing": 66.4, "peel": 46.6}
-TRAFFIC_SOURCE = ("ncu one-pass capture (dram__bytes_read.sum + dram__bytes_write.sum) of one R-MAT scale-20 "
-                  "decomposition, scaled per triangle")
-# The same DRAM bytes per decomposition of R-MAT scale 22, edge factor 16,
-# from one-kernel, one-launch, one-pass captures of the main kernels at that
-# size (the one walk 130.8 GB, compaction 82.7 GB, transpose 56.0 GB, peel
-# 121.3 GB; the in-adjacency and bounds kernels scaled from scale 20): at
-# this size the peel's supports no longer fit in L2, so its rate per
-# triangle is higher than at scale 20.
-TRAFFIC_BY_WORKLOAD = {(22, 16): {"support": 133.1e9, "listing": 138.7e9, "peel": 121.3e9}}
-TRAFFIC_SOURCE_BY_WORKLOAD = ("ncu one-kernel, one-launch, one-pass captures (dram__bytes_read.sum + "
-                              "dram__bytes_write.sum) of the main kernels of one decomposition of this workload")
+TRAFFIC_PER_TRIANGLE = {"support": 25.4, "listing": 60.1, "peel": 48.5}
+TRAFFIC_SOURCE = ("ncu capture (dram__bytes_read.sum + dram__bytes_write.sum) of one R-MAT scale-20 "
+                  "decomposition, scaled per triangle; at scale 22, where the supports no longer fit in L2, "
+                  "the peel moves more than that")
+
 
 
 def main_ours(args):
@@ -887,8 +882,8 @@ def main_ours(args):
     t_sup, t_list, t_peel, t_post = (phases[k] / n for k in range(4))
     # the decomposition's algorithmic bytes B_dec = 2 B_sup: the support pass,
     # then one re-enumeration of each edge's triangles (listing + peel)
-    mt = TRAFFIC_BY_WORKLOAD.get((scale, ef)) or {k: v * res.triangles for k, v in TRAFFIC_PER_TRIANGLE.items()}
-    traffic_src = TRAFFIC_SOURCE_BY_WORKLOAD if (scale, ef) in TRAFFIC_BY_WORKLOAD else TRAFFIC_SOURCE
+    mt = {k: v * res.triangles for k, v in TRAFFIC_PER_TRIANGLE.items()}
+    traffic_src = TRAFFIC_SOURCE
     if res.listing != 2:
         # the captures behind these figures are of the one-walk listed path
         mt, traffic_src = None, "not captured for this path"
