@@ -139,6 +139,9 @@ struct RoundShared {
     unsigned long long q, fe;
     int ok;
     int dmin;                    // smallest decrement result of the block's sub-round
+    // level changes: edges alive, the alive list's length and which of the two it is (-1: every edge id)
+    long long alive, nlist;
+    int list;
 };
 
 __device__ __forceinline__ void red_release_add(unsigned long long* p, unsigned long long v) {
@@ -446,16 +449,16 @@ __device__ __forceinline__ void warp_append_staged(const PeelArgs& A, bool liste
 
 // Level changes (decomposition mode).  Level change t starts level L_t =
 // min support over the alive edges and queues F = alive edges with support
-// L_t.  The alive edges live in a compacted list (list t&1 is the input of
-// change t, all edge ids at t = 0).
+// L_t.  The alive edges lie among the entries of a list, every edge id at
+// first, rewritten from one array into the other when enough of it has died.
 //
 // One streaming pass usually suffices: a lower bound g of L_t is known before
 // the pass (0 at t = 0; afterwards the minimum support above L_{t-1} seen at
 // change t-1, lowered by every decrement result above L_{t-1} during level
-// L_{t-1}).  The pass compacts the survivors into list (t+1)&1, queues the
-// alive edges with support == g, and takes the minimum support above g.  If
+// L_{t-1}).  The pass may rewrite the list, queues the alive edges with
+// support == g, and takes the minimum support above g.  If
 // anything was queued, L_t = g.  Otherwise L_t = that minimum, and one more
-// pass over the compacted list queues its frontier (3 of 307 level changes
+// pass over the list queues its frontier (3 of 307 level changes
 // at R-MAT scale 22; a side list of the supports just above g, written by
 // every first pass for that case, cost the level changes 3 ms there).  Every
 // pass k ends with a grid barrier and writes its minimum and queued count to
@@ -472,6 +475,14 @@ __device__ __forceinline__ void fold_min(int* dst, int32_t v) {
 }
 
 __device__ __forceinline__ void pass_min(const PeelArgs& A, int np, int32_t v) { fold_min(&A.ctl->mgt[np % 3], v); }
+
+// A level change rewrites the alive list only when a kListSlack-th of it has
+// died; until then its dead entries cost a code word each, and until the first
+// rewrite the list is every edge id and is not read at all.  Level changes are
+// bound by these passes on large graphs: rewritten every time 19.1 ms at R-MAT
+// scale 22 (546 levels), 5.7 at 20, 0.99 at 16; now 14.2, 4.7 and 0.83 (a third
+// instead of an eighth: 14.7, 4.7, 0.81).
+constexpr int kListSlack = 8;
 
 // Level-change passes stream the alive list in steps of kStep x 32 entries per
 // warp: the gathers of a step are in flight together and the step reserves its
@@ -512,11 +523,12 @@ __device__ __forceinline__ bool level_transition(const PeelArgs& A, bool listed,
     const unsigned lane = lane_id();
     const long long gw = (long long)blockIdx.x * kPeelWarps + threadIdx.x / kWarp;
     const long long nw = (long long)gridDim.x * kPeelWarps;
-    const int p = t & 1;
     const bool first = t == 0;
-    const int32_t* cur = A.alive[p];
-    int32_t* nxt = A.alive[p ^ 1];
-    const long long ncur = first ? A.E : (long long)__ldcg(&A.ctl->cnt[(t + 2) % 3]);
+    const int p = RS->list;
+    const int32_t* cur = p < 0 ? nullptr : A.alive[p];
+    int32_t* nxt = A.alive[p < 0 ? 0 : p ^ 1];
+    const long long ncur = RS->nlist;
+    const bool write = RS->alive < ncur - ncur / kListSlack;
     int32_t g = 0;
     if (!first) {
         const int32_t a = *(volatile int*)&A.ctl->mgt[(np + 2) % 3];
@@ -549,7 +561,7 @@ __device__ __forceinline__ bool level_transition(const PeelArgs& A, bool listed,
             for (int u = 0; u < kStep; u++) {
                 const long long i = base + u * kWarp + lane;
                 e[u] = 0;
-                if (i < ncur) e[u] = first ? (int32_t)i : __ldcg(cur + i);
+                if (i < ncur) e[u] = cur ? __ldcg(cur + i) : (int32_t)i;
             }
 #pragma unroll
             for (int u = 0; u < kStep; u++) {
@@ -572,20 +584,27 @@ __device__ __forceinline__ bool level_transition(const PeelArgs& A, bool listed,
                 nk += __popc(km[u]);
                 if (keep[u] && sv[u] > g) mloc = sv[u] < mloc ? sv[u] : mloc;
             }
-            if (lane == 0) s_tk[wib] = nk;
-            __syncthreads();
-            if (wib == 0) {
+            if (write) {
+                if (lane == 0) s_tk[wib] = nk;
+                __syncthreads();
+            }
+            if (write && wib == 0) {
                 const int a = lane < kPeelWarps ? s_tk[lane] : 0;
                 const int ai = warp_incl_scan(a);
                 if (lane == kPeelWarps - 1) s_base = ai ? atomicAdd(ocnt, (unsigned long long)ai) : 0ull;
                 if (lane < kPeelWarps) s_tk[lane] = ai - a;
             }
-            __syncthreads();
-            unsigned long long ok = s_base + (unsigned long long)s_tk[wib];
+            unsigned long long ok = 0;
+            if (write) {
+                __syncthreads();
+                ok = s_base + (unsigned long long)s_tk[wib];
+            }
 #pragma unroll
             for (int u = 0; u < kStep; u++) {
-                if (keep[u]) nxt[ok + __popc(km[u] & lt)] = e[u];
-                ok += __popc(km[u]);
+                if (write) {
+                    if (keep[u]) nxt[ok + __popc(km[u] & lt)] = e[u];
+                    ok += __popc(km[u]);
+                }
                 const bool want = keep[u] && sv[u] == g;
                 if (want) {
                     A.rnd[e[u]] = r_next;
@@ -593,7 +612,7 @@ __device__ __forceinline__ bool level_transition(const PeelArgs& A, bool listed,
                 }
                 warp_append_staged<Search>(A, listed, slot, buf, want, e[u], sv[u], B, &A.ctl->pfe[np % 3]);
             }
-            __syncthreads();  // s_tk / s_base are reused by the next tile
+            if (write) __syncthreads();  // s_tk / s_base are reused by the next tile
         }
         if (listed) append_flush_call<kListed>(A, slot, buf, B, &A.ctl->pfe[np % 3]);
         else append_flush_call<Search>(A, slot, buf, B, &A.ctl->pfe[np % 3]);
@@ -602,6 +621,10 @@ __device__ __forceinline__ bool level_transition(const PeelArgs& A, bool listed,
     np++;
     if (!round_barrier(A.ctl, RB, RS, r_next, &A.ctl->dmin[t & 1])) return false;
     RB.fe = ld_cg_u64(&A.ctl->pfe[(np + 2) % 3]);
+    if (write && threadIdx.x == 0) {  // every thread has read the state, and reads it again after other barriers
+        RS->list = p < 0 ? 0 : p ^ 1;
+        RS->nlist = (long long)__ldcg(&A.ctl->cnt[t % 3]);
+    }
     if (RB.fe > 0) {
         *l_out = g;
         return true;
@@ -612,16 +635,17 @@ __device__ __forceinline__ bool level_transition(const PeelArgs& A, bool listed,
     pass_start(A, np);
     int32_t mloc = INT32_MAX;
     {
-        // pass 2: one more pass over the compacted list
-        const long long n2 = (long long)__ldcg(&A.ctl->cnt[t % 3]);
+        // pass 2: one more pass over the list
+        const long long n2 = write ? (long long)__ldcg(&A.ctl->cnt[t % 3]) : ncur;
         for (long long base = gw * kWarp; base < n2; base += nw * kWarp) {
             const long long i = base + lane;
             int32_t e = 0, sv = INT32_MAX;
             if (i < n2) {
-                e = __ldcg(nxt + i);
-                sv = __ldcg(A.live + e);
+                e = write ? __ldcg(nxt + i) : cur ? __ldcg(cur + i) : (int32_t)i;
+                const unsigned cw = __ldcg(A.code + (e >> 3));
+                if (((cw >> ((unsigned)(e & 7) * 4u)) & 15u) == kCodeAlive) sv = __ldcg(A.live + e);
             }
-            const bool want = i < n2 && sv == m;
+            const bool want = sv == m;  // m < INT32_MAX
             if (!want && sv > m) mloc = sv < mloc ? sv : mloc;
             if (want) {
                 A.rnd[e] = r_next;
@@ -1400,7 +1424,12 @@ __global__ void __launch_bounds__(kPeelBlock, TDT_PEEL_MINB) peel_kernel(const _
     int32_t l = 0;
     int ntrans = 0, np = 0;
     bool ok;
-    if (threadIdx.x == 0) s_round.dmin = INT32_MAX;
+    if (threadIdx.x == 0) {
+        s_round.dmin = INT32_MAX;
+        s_round.alive = s_round.nlist = A.E;
+        s_round.list = -1;
+    }
+    __syncthreads();
     RoundBar RB{gridDim.x, 0ull, 0ull};
     long long nprev = 0;  // items of the sub-round before
     // compaction: edges alive now and at the last one
@@ -1421,6 +1450,7 @@ __global__ void __launch_bounds__(kPeelBlock, TDT_PEEL_MINB) peel_kernel(const _
         return;
     }
     alive -= (long long)RB.fe;
+    if (threadIdx.x == 0) s_round.alive -= (long long)RB.fe;
     uint64_t t_mark = globaltimer_ns();
     for (;;) {
         if (master) {
@@ -1465,6 +1495,7 @@ __global__ void __launch_bounds__(kPeelBlock, TDT_PEEL_MINB) peel_kernel(const _
             if (!more) break;
             l = nl;
         }
+        if (threadIdx.x == 0) s_round.alive -= (long long)RB.fe;
         t_mark = globaltimer_ns();
         r++;
         if constexpr (Mode == kCompact) {
