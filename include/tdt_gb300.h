@@ -122,6 +122,12 @@ void tdt_set_ktruss_batch_caps(long long items, long long cands);
  * equal range per warp (default 2^20; lower values take the dynamic split on
  * small graphs).  <= 0 restores the default.  Results do not depend on it. */
 void tdt_set_peel_dynamic_min(long long slots);
+
+/* Testing knob of the scans' and sorts' look-back waits: a wait of longer than
+ * ns for a tile before it gives up, and the call's status is TDT_ERR_TIMEOUT
+ * (default 2 s).  <= 0 restores the default.  Affects calls launched
+ * afterwards from any thread. */
+void tdt_set_lookback_limit_ns(long long ns);
 int tdt_test_barrier_timeout(void *workspace, long long limit_ns, cudaStream_t stream);
 
 /* =====================================================================
@@ -357,8 +363,9 @@ int tdt_peeling_direct_tile_oi(const int32_t *e_curr, int64_t n_curr, const int3
  * ranges.  Inputs: src/dst int32[num_draws] with ids in [0, num_ids).
  * Outputs: rows/cols int32[num_draws] (first E_out used), row_ptr
  * int64[num_ids+1] (first V_out+1 used), vertices int32[num_ids] (original id
- * of each rank), counts int64[3] = {E_out, V_out, status} (device).  No host
- * synchronisation inside. */
+ * of each rank), counts int64[3] = {E_out, V_out, status} (device; TDT_ERR_INVALID:
+ * an id outside [0, num_ids), TDT_ERR_TIMEOUT: a device wait ran out and the
+ * outputs are not to be used).  No host synchronisation inside. */
 size_t tdt_preprocess_workspace_bytes(int64_t num_draws, int64_t num_ids);
 int tdt_preprocess(const int32_t *src, const int32_t *dst, int64_t num_draws, int64_t num_ids,
                    const int32_t *vertex_group, int32_t num_groups, int32_t *rows, int32_t *cols,

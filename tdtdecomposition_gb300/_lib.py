@@ -35,6 +35,7 @@ _SIGS = [
     ("tdt_set_peel_deadline_ns", None, [ctypes.c_longlong]),
     ("tdt_set_ktruss_batch_caps", None, [ctypes.c_longlong, ctypes.c_longlong]),
     ("tdt_set_peel_dynamic_min", None, [ctypes.c_longlong]),
+    ("tdt_set_lookback_limit_ns", None, [ctypes.c_longlong]),
     ("tdt_test_barrier_timeout", ctypes.c_int, [c_ptr, ctypes.c_longlong, c_ptr]),
     ("tdt_segment_add", ctypes.c_int, [c_ptr, c_i64, c_ptr, c_ptr, c_i64, c_ptr]),
     ("tdt_segment_max", ctypes.c_int, [c_ptr, c_i64, c_ptr, c_i64, c_ptr, c_ptr]),
@@ -95,6 +96,9 @@ _SIGS = [
     ("tdt_ktruss_search", ctypes.c_int,
      [c_ptr, c_ptr, c_ptr, c_i64, c_i64, c_i32, c_ptr, c_ptr, c_ptr, c_size, c_ptr]),
 ]
+
+
+ERR_INVALID, ERR_TIMEOUT = 1, 4  # tdt_status
 
 
 class TdtError(RuntimeError):

@@ -127,6 +127,7 @@ void set_peel_grid(int half_sms);
 void set_peel_deadline(long long ns);
 void set_fixed_caps(long long items, long long cands);
 void set_peel_dyn_min(long long slots);
+void set_look_back_limit(long long ns);
 int peel_clock(const void* ws, long long* ns, cudaStream_t st);
 int test_barrier_timeout(void* ws, long long limit_ns, cudaStream_t st);
 int launch_support_accum_i32(const int32_t* rp, int32_t stride, const int32_t* cols, int64_t nv, int64_t ne,
@@ -174,6 +175,7 @@ API void tdt_set_peel_grid(int half_sms) { set_peel_grid(half_sms); }
 API void tdt_set_peel_deadline_ns(long long ns) { set_peel_deadline(ns); }
 API void tdt_set_ktruss_batch_caps(long long items, long long cands) { set_fixed_caps(items, cands); }
 API void tdt_set_peel_dynamic_min(long long slots) { set_peel_dyn_min(slots); }
+API void tdt_set_lookback_limit_ns(long long ns) { set_look_back_limit(ns); }
 API int tdt_peel_clock(const void* workspace, long long* ns, cudaStream_t stream) {
     return peel_clock(workspace, ns, stream);
 }

@@ -18,6 +18,8 @@
 //      every id, vertices[rank]
 //   4. relabel + orient each edge -> (lo << B) | hi, radix sort
 //   5. rows / cols, and row_ptr from the places where the row changes
+// Ids that come out of a sort are bounded before they index: a sort whose wait
+// ran out leaves keys that are none (sort.cuh).
 // Each sort's digit totals are taken by the kernel that makes its keys.  67 M /
 // 65,536 draws: 10.6 ms / 560 us in 108 / 73 launches with five launches a sort
 // pass and an atomic per degree and row count, 7.6 ms / 312 us in 29 / 21.
@@ -72,9 +74,10 @@ struct UniqueCtl {
 };
 
 __global__ void __launch_bounds__(kPpBlock) pp_unique(const uint64_t* __restrict__ keys, int64_t m,
-                                                      uint64_t sentinel, int B, uint64_t* __restrict__ ukeys,
+                                                      uint64_t sentinel, int B, uint32_t num_ids,
+                                                      uint64_t* __restrict__ ukeys,
                                                       int32_t* __restrict__ deg, unsigned long long* words,
-                                                      UniqueCtl* ctl, int* status) {
+                                                      UniqueCtl* ctl, LookBack L) {
     using W = TileWord<unsigned long long>;
     __shared__ int32_t s_id[kUqTable];
     __shared__ int32_t s_n[kUqTable];
@@ -124,7 +127,7 @@ __global__ void __launch_bounds__(kPpBlock) pp_unique(const uint64_t* __restrict
         }
         if (w == 0) {
             if (lane == 0) *(volatile unsigned long long*)(words + tile) = (tile == 0 ? W::kInclusive : W::kAggregate) | tot;
-            const unsigned long long before = warp_look_back(words, tile, status);
+            const unsigned long long before = warp_look_back(words, tile, L);
             if (lane == 0) {
                 if (tile > 0) *(volatile unsigned long long*)(words + tile) = W::kInclusive | (before + tot);
                 s_before = before;
@@ -144,9 +147,9 @@ __global__ void __launch_bounds__(kPpBlock) pp_unique(const uint64_t* __restrict
             const unsigned run = ((after & (0u - after)) - 1u) & ~lt;  // from a head to before the next
             if ((heads >> lane) & 1u) {
                 const int c = __popc(f[it] & run);
-                if (c) atomicAdd(deg + lo, c);
+                if (c && (uint32_t)lo < num_ids) atomicAdd(deg + lo, c);
             }
-            if (mine) {
+            if (mine && (uint32_t)hi < num_ids) {
                 const unsigned h = ((unsigned)hi * 2654435761u) >> 21;
                 int32_t id = *(volatile int32_t*)(s_id + h);
                 if (id == -1) id = atomicCAS(s_id + h, -1, hi);
@@ -198,6 +201,7 @@ __global__ void pp_ranks(const uint64_t* __restrict__ vkeys, int64_t num_ids, in
         const uint64_t k = vkeys[p];
         if (k == ~0ull) continue;
         const int32_t id = (int32_t)(k & mask);
+        if (id >= num_ids) continue;
         rank[id] = (int32_t)p;
         vertices[p] = id;
         if (p + 1 == num_ids || vkeys[p + 1] == ~0ull) *vcount = (unsigned long long)(p + 1);
@@ -208,7 +212,8 @@ __global__ void pp_ranks(const uint64_t* __restrict__ vkeys, int64_t num_ids, in
 __global__ void __launch_bounds__(kPpBlock) pp_relabel(const uint64_t* __restrict__ ukeys,
                                                        const uint32_t* __restrict__ e_out, int B,
                                                        const int32_t* __restrict__ rank,
-                                                       uint64_t* __restrict__ keys2, int passes, uint32_t* hist) {
+                                                       uint64_t* __restrict__ keys2, uint64_t num_ids, int passes,
+                                                       uint32_t* hist) {
     __shared__ uint32_t s_hist[kMaxPasses * kRadix];
     DigitHist H{s_hist};
     H.init(passes);
@@ -216,8 +221,12 @@ __global__ void __launch_bounds__(kPpBlock) pp_relabel(const uint64_t* __restric
     const int64_t eo = (int64_t)*e_out;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < eo; i += (int64_t)gridDim.x * blockDim.x) {
         const uint64_t k = ukeys[i];
-        const uint64_t a = (uint64_t)rank[k >> B], b = (uint64_t)rank[k & mask];
-        const uint64_t k2 = ((a < b ? a : b) << B) | (a < b ? b : a);
+        const uint64_t lo = k >> B, hi = k & mask;
+        uint64_t k2 = 0;
+        if (lo < num_ids && hi < num_ids) {
+            const uint64_t a = (uint64_t)rank[lo], b = (uint64_t)rank[hi];
+            k2 = ((a < b ? a : b) << B) | (a < b ? b : a);
+        }
         keys2[i] = k2;
         H.add(k2, passes);
     }
@@ -243,6 +252,7 @@ __global__ void pp_emit(const uint64_t* __restrict__ keys2, const uint32_t* __re
             cols[i] = (int32_t)(k & mask);
             r1 = (int64_t)r + 1;
             r0 = i == 0 ? 0 : (int64_t)(keys2[i - 1] >> B) + 1;
+            if (r < 0 || r >= num_ids) r0 = r1;
         }
         if (r1 - r0 <= 8)
             for (int64_t r = r0; r < r1; r++) row_ptr[r] = i;
@@ -387,7 +397,7 @@ int run_preprocess(const int32_t* src, const int32_t* dst, int64_t m, int64_t nu
     int per_sm = 0;
     TDT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pp_unique, kPpBlock, 0));
     pp_unique<<<grid_for(m, kUqTile, di.sms, per_sm > 0 ? per_sm : 1), kPpBlock, 0, st>>>(
-        sk, m, sentinel, B, uk, L.deg, L.uwords, L.uniq, L.status);
+        sk, m, sentinel, B, (uint32_t)num_ids, uk, L.deg, L.uwords, L.uniq, look_back(L.status));
     TDT_LAUNCH_CHECK("pp_unique");
     const uint32_t* e_out = &L.uniq->e_out;
     // 3. rank vertices by (group, degree, id); absent ids carry ~0, which stays
@@ -401,7 +411,7 @@ int run_preprocess(const int32_t* src, const int32_t* dst, int64_t m, int64_t nu
                                                               L.vcount);
     TDT_LAUNCH_CHECK("pp_ranks");
     // 4. relabel + orient, sort by (row, col); the sorted draw keys are no longer needed
-    pp_relabel<<<g_m, tb, 0, st>>>(uk, e_out, B, L.rank, sk, pe, L.s2.hist);
+    pp_relabel<<<g_m, tb, 0, st>>>(uk, e_out, B, L.rank, sk, (uint64_t)num_ids, pe, L.s2.hist);
     TDT_LAUNCH_CHECK("pp_relabel");
     rc = radix_sort<uint64_t, false>(sk, uk, sk, nullptr, nullptr, m, pe, L.s2, e_out, nullptr, L.status, st);
     if (rc) return rc;

@@ -11,6 +11,13 @@
 
 namespace tdt {
 
+// Test knob: wait limit of the look-backs launched next (<= 0: the default).
+static long long g_look_back_limit_ns = 0;
+void set_look_back_limit(long long ns) { g_look_back_limit_ns = ns; }
+LookBack look_back(int* status) {
+    return {status, g_look_back_limit_ns > 0 ? (unsigned long long)g_look_back_limit_ns : kLookBackTimeoutNs};
+}
+
 constexpr int kScanBlock = 512;
 constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanBlock * kScanItems;
@@ -65,7 +72,7 @@ struct ScanJob {
 
 // One tile of a job; done(total) is called by one thread of the last tile.
 template <class In, class Done>
-__device__ __forceinline__ void scan_tile(const ScanJob<In>& J, int* status, Done&& done) {
+__device__ __forceinline__ void scan_tile(const ScanJob<In>& J, const LookBack& L, Done&& done) {
     using W = TileWord<unsigned long long>;
     using TO = int64_t;
     __shared__ TO s_warp[33];
@@ -88,7 +95,7 @@ __device__ __forceinline__ void scan_tile(const ScanJob<In>& J, int* status, Don
         if (threadIdx.x == 0)
             *(volatile unsigned long long*)(J.words + tile) =
                 (tile == 0 ? W::kInclusive : W::kAggregate) | (unsigned long long)tot;
-        const unsigned long long before = warp_look_back(J.words, tile, status);
+        const unsigned long long before = warp_look_back(J.words, tile, L);
         if (threadIdx.x == 0) {
             if (tile > 0)
                 *(volatile unsigned long long*)(J.words + tile) =
@@ -109,24 +116,24 @@ __device__ __forceinline__ void scan_tile(const ScanJob<In>& J, int* status, Don
     }
 }
 
-__global__ void __launch_bounds__(kScanBlock) scan_kernel(ScanJob<ScanArray<int32_t>> J, int* status) {
-    scan_tile(J, status, [](int64_t) {});
+__global__ void __launch_bounds__(kScanBlock) scan_kernel(ScanJob<ScanArray<int32_t>> J, LookBack L) {
+    scan_tile(J, L, [](int64_t) {});
 }
 
 // The in-adjacency's offsets and the rows' staging slots, tiles of both in one
 // launch (a launch and 5 us of a small call).
 __global__ void __launch_bounds__(kScanBlock) scan_rows_kernel(ScanJob<ScanArray<int32_t>> J,
-                                                               ScanJob<ScanStageSlots> K, int* status) {
-    if (blockIdx.x < J.tiles) scan_tile(J, status, [](int64_t) {});
-    else scan_tile(K, status, [](int64_t) {});
+                                                               ScanJob<ScanStageSlots> K, LookBack L) {
+    if (blockIdx.x < J.tiles) scan_tile(J, L, [](int64_t) {});
+    else scan_tile(K, L, [](int64_t) {});
 }
 
 // The lists' offsets, and whether there are lists.
 __global__ void __launch_bounds__(kScanBlock) scan_lists_kernel(ScanJob<ScanArray<int32_t>> J, ListDecision D,
-                                                                int* status) {
-    scan_tile(J, status, [&](int64_t need) {
+                                                                LookBack L) {
+    scan_tile(J, L, [&](int64_t need) {
         const unsigned long long slots = D.tail_bytes / 8;
-        const int ok = *(volatile int*)status == 0 && (unsigned long long)need <= slots;
+        const int ok = *(volatile int*)L.status == 0 && (unsigned long long)need <= slots;
         const int compact = ok && !*D.stage_skip && (unsigned long long)need <= slots - (unsigned long long)*D.staged;
         *D.listed = ok;
         *D.list_skip = !ok;
@@ -154,7 +161,7 @@ int exclusive_scan(const int32_t* in, int64_t* out, int64_t n, int64_t* total, v
         return TDT_OK;
     }
     const auto J = scan_job(ScanArray<int32_t>{in}, out, n, total, scratch);
-    scan_kernel<<<(unsigned)J.tiles, kScanBlock, 0, st>>>(J, status);
+    scan_kernel<<<(unsigned)J.tiles, kScanBlock, 0, st>>>(J, look_back(status));
     TDT_LAUNCH_CHECK("scan");
     return TDT_OK;
 }
@@ -168,7 +175,7 @@ int scan_rows(const int32_t* in, int64_t* out, void* scratch, const int64_t* rp,
     }
     const auto J = scan_job(ScanArray<int32_t>{in}, out, nv, out + nv, scratch);
     const auto K = scan_job(ScanStageSlots{rp, status}, slots, nv, slots + nv, slots_scratch);
-    scan_rows_kernel<<<(unsigned)(J.tiles + K.tiles), kScanBlock, 0, st>>>(J, K, status);
+    scan_rows_kernel<<<(unsigned)(J.tiles + K.tiles), kScanBlock, 0, st>>>(J, K, look_back(status));
     TDT_LAUNCH_CHECK("scan_rows");
     return TDT_OK;
 }
@@ -177,7 +184,7 @@ int scan_lists(const int32_t* in, int64_t* out, int64_t n, void* scratch, const 
                cudaStream_t st) {
     TDT_CHECK_ARG(n > 0, "no lists");
     const auto J = scan_job(ScanArray<int32_t>{in}, out, n, out + n, scratch);
-    scan_lists_kernel<<<(unsigned)J.tiles, kScanBlock, 0, st>>>(J, D, status);
+    scan_lists_kernel<<<(unsigned)J.tiles, kScanBlock, 0, st>>>(J, D, look_back(status));
     TDT_LAUNCH_CHECK("scan_lists");
     return TDT_OK;
 }
@@ -203,7 +210,7 @@ template <class K, class S, bool kVals, bool kIota, int kItems>
 __global__ void __launch_bounds__(kSortBlock, 4) radix_pass_kernel(
     const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, K* __restrict__ keys_out,
     uint32_t* __restrict__ vals_out, int64_t n, int pass, const uint32_t* __restrict__ hist,
-    uint32_t* tile_next, S* words, const uint32_t* n_dev, const long long* max_dev, int* status) {
+    uint32_t* tile_next, S* words, const uint32_t* n_dev, const long long* max_dev, LookBack L) {
     using W = TileWord<S>;
     constexpr int kTile = kSortBlock * kItems;
     if (max_dev && pass > 0 && (*max_dev >> (8 * pass)) == 0) return;
@@ -303,7 +310,7 @@ __global__ void __launch_bounds__(kSortBlock, 4) radix_pass_kernel(
 #pragma unroll
             for (int j = 0; j < kBack; j++) {
                 if (!more || t - j < 0) continue;
-                if (x[j] == 0) x[j] = tile_word_wait(words + (t - j) * kRadix + d, status);
+                if (x[j] == 0) x[j] = tile_word_wait(words + (t - j) * kRadix + d, L);
                 before += x[j] & W::kValue;
                 more = (x[j] & W::kInclusive) == 0;
             }
@@ -351,7 +358,8 @@ static int radix_passes(const K* in, K* b0, K* b1, uint32_t* v0, uint32_t* v1, i
         const uint32_t* vin = (p & 1) ? v0 : v1;
         kern<<<(unsigned)ntiles, kSortBlock, smem, st>>>(kin, vin, (p & 1) ? b1 : b0, (p & 1) ? v1 : v0, n, p,
                                                         R.hist + p * kRadix, R.tile_next + p,
-                                                        words + (size_t)p * ntiles * kRadix, n_dev, max_dev, status);
+                                                        words + (size_t)p * ntiles * kRadix, n_dev, max_dev,
+                                                        look_back(status));
         TDT_LAUNCH_CHECK("radix_pass");
     }
     return TDT_OK;

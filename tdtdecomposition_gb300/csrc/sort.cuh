@@ -20,19 +20,34 @@ struct TileWord {
 
 // Wait limit of a look-back on a tile that has not published (tiles are handed
 // out in order, so the awaited block is running); past it the waiter records
-// TDT_ERR_TIMEOUT and goes on, and the caller's result is rejected.
+// TDT_ERR_TIMEOUT and goes on with a prefix that is too small, so its results
+// stay inside their arrays but leave places unwritten.  Kernels that index by
+// such results bound them, or do not start (look_back_failed), and the caller's
+// result is rejected.
 constexpr uint64_t kLookBackTimeoutNs = 2ull * 1000ull * 1000ull * 1000ull;
 
+struct LookBack {
+    int* status;
+    unsigned long long limit_ns;
+};
+LookBack look_back(int* status);  // with the limit in force (tdt_set_lookback_limit_ns)
+
+// A wait of an earlier kernel ran out.  The same for every thread: where it is
+// true no block of the kernel that asks goes on to raise the status.
+__device__ __forceinline__ bool look_back_failed(const int* status) {
+    return *(const volatile int*)status == (int)TDT_ERR_TIMEOUT;
+}
+
 template <class S>
-__device__ __forceinline__ S tile_word_wait(const S* p, int* status) {
+__device__ __forceinline__ S tile_word_wait(const S* p, const LookBack& L) {
     S w = *(const volatile S*)p;
     if (w) return w;
     const uint64_t t0 = globaltimer_ns();
     for (unsigned spins = 1;; spins++) {
         w = *(const volatile S*)p;
         if (w) return w;
-        if ((spins & 63u) == 0 && globaltimer_ns() - t0 > kLookBackTimeoutNs) {
-            if (status) atomicMax(status, (int)TDT_ERR_TIMEOUT);
+        if ((spins & 7u) == 1u && globaltimer_ns() - t0 > L.limit_ns) {
+            atomicMax(L.status, (int)TDT_ERR_TIMEOUT);
             return TileWord<S>::kInclusive;
         }
     }
@@ -41,12 +56,12 @@ __device__ __forceinline__ S tile_word_wait(const S* p, int* status) {
 // Sum of the tiles before `tile`, by one whole warp: 32 predecessors at a time
 // (words[t] is tile t's).  Lane 0 has published the tile's aggregate.
 template <class S>
-__device__ __forceinline__ S warp_look_back(const S* words, int64_t tile, int* status) {
+__device__ __forceinline__ S warp_look_back(const S* words, int64_t tile, const LookBack& L) {
     using W = TileWord<S>;
     S sum = 0;
     for (int64_t t = tile - 1; t >= 0; t -= kWarp) {
         const int64_t mine = t - (int64_t)lane_id();
-        const S w = mine >= 0 ? tile_word_wait(words + mine, status) : W::kInclusive;
+        const S w = mine >= 0 ? tile_word_wait(words + mine, L) : W::kInclusive;
         const unsigned inc = __ballot_sync(kFull, (w & W::kInclusive) != 0);
         const int last = inc ? __ffs(inc) - 1 : kWarp - 1;  // nearest inclusive prefix
         sum += warp_sum((int)lane_id() <= last ? (S)(w & W::kValue) : S(0));

@@ -48,6 +48,7 @@
 // 9.4 ms.  The walk issues 2.6 instructions a cycle per SM (scale 20: 4.1 ms,
 // DRAM 29 %); the regrouping moves 13 GB in 4 ms per role.
 #include "common.cuh"
+#include "sort.cuh"
 
 namespace tdt {
 
@@ -424,7 +425,8 @@ __global__ void __launch_bounds__(kWkBlock, kWkMinBlocks) walk_kernel(const __gr
     __shared__ int s_wsum[kWkWarps];
     __shared__ unsigned long long s_unit;
     __shared__ int s_next;
-    if (A.gate && *(volatile const int*)A.gate != 0) return;
+    const bool failed = M == kWalkList && look_back_failed(A.status);  // the offsets are not the scan's
+    if ((A.gate && *(volatile const int*)A.gate != 0) || failed) return;
     const int wib = threadIdx.x / kWarp;
     const unsigned lane = lane_id();
     const unsigned sh = (unsigned)(((uintptr_t)A.cols & 15u) >> 2);
@@ -651,7 +653,8 @@ __global__ void __launch_bounds__(kDsBlock, 4) distribute_kernel(const __grid_co
     __shared__ int64_t s_F[RoleC ? 1 : kDsBlock];  // role B: where the staged role-A entries go
     __shared__ int32_t s_wsum[2][kDsWarps];
     __shared__ unsigned long long s_win;
-    if (A.gate && *(volatile const int*)A.gate != 0) return;
+    const bool failed = look_back_failed(A.status);  // the offsets are not the scan's
+    if ((A.gate && *(volatile const int*)A.gate != 0) || failed) return;
     const int wib = threadIdx.x / kWarp;
     const unsigned lane = lane_id();
     const unsigned lt = lanemask_lt(), le = lt | (1u << lane);

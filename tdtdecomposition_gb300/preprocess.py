@@ -29,6 +29,12 @@ def _max_id(a, b=None):
     return out.item()
 
 
+def _check_status(st):
+    if st != 0:
+        raise _lib.TdtError(st, "tdt_preprocess",
+                            "vertex id outside [0, num_ids)" if st == _lib.ERR_INVALID else "reported by the device")
+
+
 def preprocess_edges(src, dst, vertex_group=None, num_ids=None, workspace=None):
     """src, dst: int32 CUDA tensors of the raw edge list (ids >= 0).  Returns
     (CSRCOO with int64 row_ptr, vertices: int32 original id of each rank),
@@ -69,8 +75,7 @@ def preprocess_edges(src, dst, vertex_group=None, num_ids=None, workspace=None):
                               ws.data_ptr(), ws.numel(), torch.cuda.current_stream(dev).cuda_stream)
     _lib.check(rc, "tdt_preprocess")
     E, V, st = counts.tolist()
-    if st != 0:
-        raise _lib.TdtError(st, "tdt_preprocess", "vertex id outside [0, num_ids)")
+    _check_status(st)
     g = CSRCOO(columns=cols[:E], row_ptr=rp if V == num_ids else rp[:V + 1].clone(), rows=rows[:E])
     return g, verts[:V]
 
