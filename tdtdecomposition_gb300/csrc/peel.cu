@@ -1313,6 +1313,8 @@ __device__ __forceinline__ int compact_row(const PeelArgs& A, int64_t base, int 
         if (Block) {
             __syncthreads();  // also: every entry of this tile has been read
             all = 0;
+        } else {
+            __syncwarp();  // the same: a vote orders no memory
         }
 #pragma unroll
         for (int j = 0; j < kPer; j++) {
