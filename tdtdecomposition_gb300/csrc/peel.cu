@@ -1538,7 +1538,8 @@ __global__ void validate_kernel(const int64_t* __restrict__ rp, const int32_t* _
     for (int64_t e = tid; e < E; e += nth) {
         const int32_t u = rows[e];
         const bool in = u >= 0 && u < V;
-        const int err = validate_edge(cols, e, u, in ? rp[u] : 0, in ? rp[u + 1] : 0, V);
+        const int64_t en = in ? rp[u + 1] : 0;
+        const int err = validate_edge(cols, e, u, in ? rp[u] : 0, en < E ? en : E, V);  // cols ends at E
         if (err) atomicMax(&ctl->g.status, err);
     }
 }
