@@ -104,7 +104,7 @@ void tdt_set_peel_grid(int half_sms);
  * has no bounded waits).  tdt_set_peel_deadline_ns: wall-clock budget of the
  * peel launches that follow (<= 0 restores the default of 120 s); a run past
  * it stops between sub-rounds with TDT_ERR_TIMEOUT in its stats.
- * tdt_test_barrier_timeout: launches 8 blocks at a grid barrier that one of
+ * tdt_test_barrier_timeout: launches 8 blocks at the peel's barrier, which one of
  * them never reaches; the others give up after limit_ns (1 ms .. 2 s) and the
  * call returns the device status, TDT_ERR_TIMEOUT.  workspace: >= 4096 bytes
  * of device memory.  Blocks the calling thread until the kernel ends. */

@@ -120,13 +120,12 @@ __device__ __forceinline__ Off find_sorted(const int32_t* __restrict__ cols, Off
 }
 
 // ------------------------------------------------------------------ grid barrier
-// Control block shared by the persistent kernels (device memory, zeroed by the
-// host before a launch).  One 64-bit arrival counter that only grows: barrier
-// k of a launch is complete when it reaches k x nblocks, so the last block to
-// arrive releases the others with its own increment (no reset, no second
-// word to publish).  Bit 63 of the same word aborts the run: a waiter sees it
-// in the value it polls and an arriving block in the value its increment
-// returns, with no extra load on the barrier's path.
+// Control block of the persistent kernels' barrier (round_barrier, peel.cu; device
+// memory, zeroed by the host before a launch).  One 64-bit arrival counter that
+// only grows: barrier k of a launch is complete when it reaches k x nblocks, so
+// the last block to arrive releases the others with its own increment (no
+// reset, no second word to publish).  Bit 63 of the same word aborts the run: a
+// waiter sees it in the value it polls, with no extra load on the barrier's path.
 struct GridCtl {
     unsigned long long arrive;
     unsigned pad0[62];
@@ -151,50 +150,5 @@ __device__ __forceinline__ void grid_abort(GridCtl* ctl) { atomicOr(&ctl->arrive
 // Wait limit of one grid barrier.  A barrier that does not complete within it
 // sets GridCtl::status = TDT_ERR_TIMEOUT and every block leaves its loop.
 constexpr uint64_t kBarrierTimeoutNs = 20ull * 1000ull * 1000ull * 1000ull;
-
-// Barrier over all blocks of a cooperative launch.  Returns false when the
-// run is being aborted (timeout or an error elsewhere).
-__device__ __forceinline__ bool grid_barrier(GridCtl* ctl, unsigned nblocks,
-                                             uint64_t limit_ns = kBarrierTimeoutNs) {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        __threadfence();  // the block's writes before its arrival
-        const unsigned long long old = atomicAdd(&ctl->arrive, 1ull);
-        if (old & kGridAbortBit) {
-            ok = 0;
-        } else {
-            const unsigned long long target = (old / nblocks + 1) * nblocks;
-            if (old + 1 != target) {
-                // one load per spin; the clock every 32 spins, and a short
-                // sleep once the wait is long
-                const uint64_t t0 = globaltimer_ns();
-                unsigned spins = 0;
-                for (;;) {
-                    const unsigned long long v = ld_acquire_u64(&ctl->arrive);
-                    if (v & kGridAbortBit) {
-                        ok = 0;
-                        break;
-                    }
-                    if (v >= target) break;
-                    if ((++spins & 31u) == 0) {
-                        if (globaltimer_ns() - t0 > limit_ns) {
-                            atomicMax(&ctl->status, (int)TDT_ERR_TIMEOUT);
-                            grid_abort(ctl);
-                            ok = 0;
-                            break;
-                        }
-                        if (spins > 4096) __nanosleep(200);
-                    }
-                }
-            }
-        }
-        __threadfence();  // the other blocks' writes before this block's next reads
-        s_ok = ok;
-    }
-    __syncthreads();
-    return s_ok != 0;
-}
 
 }  // namespace tdt

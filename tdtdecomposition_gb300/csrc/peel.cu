@@ -150,8 +150,10 @@ __device__ __forceinline__ void red_release_add(unsigned long long* p, unsigned 
 
 // Barrier over all blocks; next: the round whose counters are wanted.  dmin:
 // where the block's smallest decrement result goes (reset for the next
-// sub-round).  False when the run is being aborted.
-__device__ __forceinline__ bool round_barrier(PeelCtl* ctl, RoundBar& B, RoundShared* S, int next, int* dmin) {
+// sub-round).  A wait of more than limit_ns sets TDT_ERR_TIMEOUT and aborts the
+// run.  False when the run is being aborted.
+__device__ __forceinline__ bool round_barrier(PeelCtl* ctl, RoundBar& B, RoundShared* S, int next, int* dmin,
+                                              uint64_t limit_ns = kBarrierTimeoutNs) {
     __syncthreads();
     if (threadIdx.x == 0) {
         int ok = 1;
@@ -170,7 +172,7 @@ __device__ __forceinline__ bool round_barrier(PeelCtl* ctl, RoundBar& B, RoundSh
             }
             if (v >= B.target) break;
             if ((++spins & 31u) == 0) {
-                if (globaltimer_ns() - t0 > kBarrierTimeoutNs) {
+                if (globaltimer_ns() - t0 > limit_ns) {
                     atomicMax(&ctl->g.status, (int)TDT_ERR_TIMEOUT);
                     grid_abort(&ctl->g);
                     ok = 0;
@@ -1841,23 +1843,28 @@ void set_fixed_caps(long long items, long long cands) {
     g_fixed_cand_cap = cands;
 }
 
-// A grid barrier that one block never reaches: the others wait limit_ns, then
-// leave with TDT_ERR_TIMEOUT in ctl->status (the test of the bounded waits).
-__global__ void barrier_probe_kernel(GridCtl* ctl, unsigned long long limit_ns) {
+// The peel's barrier with one block that never reaches it: the others wait
+// limit_ns, then leave with TDT_ERR_TIMEOUT in the status (the test of the
+// bounded waits).
+__global__ void barrier_probe_kernel(PeelCtl* ctl, unsigned long long limit_ns) {
+    __shared__ RoundShared s_round;
     if (blockIdx.x == 0) return;
-    grid_barrier(ctl, gridDim.x, limit_ns);
+    if (threadIdx.x == 0) s_round.dmin = INT32_MAX;
+    RoundBar RB{gridDim.x, 0ull, 0ull};
+    round_barrier(ctl, RB, &s_round, 0, &ctl->dmin[0], limit_ns);
 }
 
 int test_barrier_timeout(void* ws, long long limit_ns, cudaStream_t st) {
     TDT_CHECK_ARG(ws != nullptr, "null workspace");
     TDT_CHECK_ARG(limit_ns >= 1000000ll && limit_ns <= 2000000000ll, "limit %lld ns outside [1 ms, 2 s]",
                   limit_ns);
-    GridCtl* ctl = reinterpret_cast<GridCtl*>(ws);
-    TDT_CUDA(cudaMemsetAsync(ctl, 0, sizeof(GridCtl), st));
+    static_assert(sizeof(PeelCtl) <= 4096, "the probe's workspace");
+    PeelCtl* ctl = reinterpret_cast<PeelCtl*>(ws);
+    TDT_CUDA(cudaMemsetAsync(ctl, 0, sizeof(PeelCtl), st));
     barrier_probe_kernel<<<8, 32, 0, st>>>(ctl, (unsigned long long)limit_ns);
     TDT_LAUNCH_CHECK("barrier_probe");
     int status = 0;
-    TDT_CUDA(cudaMemcpyAsync(&status, &ctl->status, sizeof(int), cudaMemcpyDeviceToHost, st));
+    TDT_CUDA(cudaMemcpyAsync(&status, &ctl->g.status, sizeof(int), cudaMemcpyDeviceToHost, st));
     TDT_CUDA(cudaStreamSynchronize(st));
     return status;
 }
