@@ -1872,10 +1872,10 @@ int test_barrier_timeout(void* ws, long long limit_ns, cudaStream_t st) {
 int launch_walk_count(const int64_t* rp, const int32_t* cols, const int64_t* cp, const int32_t* in_src,
                       const int32_t* in_eid, int64_t nv, int64_t ne, int32_t* cA, int32_t* cB, int32_t* cC,
                       const int64_t* sbase, int2* stage_end, unsigned long long stage_slots, int* stage_skip,
-                      int32_t* runA, void* units, void* ctl, int* status, cudaStream_t st);
+                      int32_t* runA, void* units, void* longs, void* ctl, int* status, cudaStream_t st);
 int launch_walk_list(const int64_t* rp, const int32_t* cols, const int64_t* cp, const int32_t* in_src,
                      const int32_t* in_eid, int64_t nv, int64_t ne, const int64_t* off, int32_t* cA, int2* lists,
-                     int32_t* runA, void* units, void* ctl, const int* gate, int* status, cudaStream_t st);
+                     int32_t* runA, void* units, void* longs, void* ctl, const int* gate, int* status, cudaStream_t st);
 int launch_distribute(const int64_t* rp, const int32_t* cols, const int32_t* rows, const int64_t* cp,
                       const int32_t* in_eid, int64_t nv, int64_t ne, const int64_t* off, const int32_t* cA,
                       const int32_t* cB, const int64_t* sbase, const int2* stage_end, const int* stage_skip,
@@ -2036,7 +2036,7 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     // on the device when validation failed); the plan of its units stays for
     // the list walk
     rc = launch_walk_count(rp, cols, L.cp, L.in_src, L.in_eid, V, E, cA, cB, cC, tail > 0 ? L.sbase : nullptr,
-                           stage_end, tail / 8, &L.ctl->stage_skip, L.alive[0], L.qi[2], L.sup_ctl,
+                           stage_end, tail / 8, &L.ctl->stage_skip, L.alive[0], L.qi[2], L.qi[1], L.sup_ctl,
                            &L.ctl->g.status, st);
     if (rc) return rc;
     const bool peel = mode != 2;
@@ -2056,7 +2056,7 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
         if (rc) return rc;
         // second walk, when the lists fit but not beside the staging slots
         rc = launch_walk_list(rp, cols, L.cp, L.in_src, L.in_eid, V, E, L.off, cA, lists, L.alive[0], L.qi[2],
-                              L.sup_ctl, &L.ctl->rewalk_skip, &L.ctl->g.status, st);
+                              L.qi[1], L.sup_ctl, &L.ctl->rewalk_skip, &L.ctl->g.status, st);
         if (rc) return rc;
         rc = launch_distribute(rp, cols, rows_use, L.cp, L.in_eid, V, E, L.off, cA, cB, L.sbase, stage_end,
                                &L.ctl->compact_skip, lists, reinterpret_cast<uint32_t*>(cC + E), L.qi[2], L.sup_ctl, &L.ctl->list_skip, &L.ctl->g.status, st);

@@ -24,6 +24,8 @@
 //   many, or with more than warp_cap out-edges, to a block (2^16 bits) whose
 //   warps take its in-edges 32 at a time.  The in-edges of a hub are split
 //   into parts of kPart, each a unit of its own.
+// * A tail far longer than the row is not streamed: the row's entries are
+//   searched in it, at the end of the warp's work (walk_long_tails).
 // * The tails of 32 in-edges form one flat space of 16-byte chunks of cols: a
 //   lane loads four columns per step and the owning in-edge of each lane's
 //   chunk comes from one OR-reduction over the group's starts.
@@ -105,6 +107,7 @@ struct WalkArgs {
     const int64_t* off;         // kWalkList: list offsets int64[E+1]
     int2* out;                  // kWalkCount: end of the staging slots; kWalkList: the lists
     int32_t* runA;              // role-A entries so far of rows walked in column chunks
+    int2* longs;                // 2 E: runs of in-edges with long tails (see push_long_tails)
     const int2* units;          // block rows: {v, part}
     int* status;
     const int* gate;            // non-zero: skip
@@ -120,6 +123,7 @@ struct WalkCtl {
     unsigned long long light_next[2];
     unsigned long long dist_next[2];  // and of the role-B and role-C passes
     unsigned long long dist_done;     // blocks that finished the role-C pass
+    unsigned long long longs_next[2]; // places of WalkArgs::longs in use, of the count and the list walk
 };
 
 // First staging slot of the role-A entries of the edge at position i of a row
@@ -183,14 +187,31 @@ struct WalkRow {
     uint32_t span;              // last id - first id
     uint32_t mask;
     bool exact;                 // span + 1 fits the bitmap (bit span + 1 stays clear: ids outside the row go there)
+    uint32_t limit;             // entries of the longest tail that is streamed through it
     bool parts;                 // other units walk this row too
     bool chunked, more;         // the row is walked in column chunks; this is not its first
 };
 
+// A tail may be far longer than the row it is streamed through: v of few
+// out-edges behind a source u of many, as in orders that are not degree ranks (the
+// wheel of 200 K vertices with its hub at id 0 streams 20 G entries, 28 ms of
+// support phase).  Past kLongTail entries and kLongRatio times the row's, the
+// row's entries are searched in the tail instead (that wheel: 0.15 ms), so the
+// walk stays within a factor of the rows' lengths.  Support phase with ratios 8 /
+// 32 / 128, and none: R-MAT scale 16 in id order 1.6 / 2.2 / 3.0 / 2.8 ms, with a
+// hub joined to all of it 1.7 / 2.4 / 2.9 / 7.1, scale 18 in id order 24 / 26 /
+// 31 / 35; degree ranks at scale 18 0.66 with any; tails of 128 or 2,048 instead
+// of 512 within 5 %.
+constexpr uint32_t kLongTail = 512, kLongRatio = 8;
+__device__ __forceinline__ uint32_t tail_limit(uint32_t dout) {
+    return dout > UINT32_MAX / kLongRatio ? UINT32_MAX : max(kLongTail, kLongRatio * dout);
+}
+
 __device__ __forceinline__ WalkRow row_init(const WalkArgs& A, unsigned char* bm, unsigned char* cnt,
-                                            unsigned char* perm, int log2bits, int64_t e0, int d, bool chunked,
+                                            unsigned char* perm, int log2bits, int64_t e0, int d, int64_t dout,
                                             bool more, bool parts) {
     WalkRow R;
+    R.limit = tail_limit((uint32_t)dout);
     R.bm = reinterpret_cast<uint32_t*>(bm);
     R.cnt = reinterpret_cast<uint32_t*>(cnt);
     R.perm = perm;
@@ -200,7 +221,7 @@ __device__ __forceinline__ WalkRow row_init(const WalkArgs& A, unsigned char* bm
     R.span = (uint32_t)(__ldg(A.cols + e0 + d - 1) - R.wb);
     R.mask = (1u << log2bits) - 1u;
     R.exact = R.span < R.mask;
-    R.chunked = chunked;
+    R.chunked = dout > d;
     R.more = more;
     R.parts = parts;
     return R;
@@ -237,12 +258,102 @@ __device__ __forceinline__ int row_find(const WalkArgs& A, const WalkRow& R, uin
     return p < 0 ? -1 : (int)(p - R.e0);
 }
 
+constexpr uint32_t kNoRun = UINT32_MAX;
+
 // This warp's group of up to 32 in-edges.
 struct WalkGroup {
+    uint32_t* longs;            // the warp's last run of in-edges with long tails (kNoRun: none)
     int4* ge;                   // per non-empty tail: {first chunk, begin, end, 0} (positions in colsA)
     int64_t* off;               // listing: slot of the in-edge's first role-A entry
     uint32_t* cnt;              // role-A entries found (listing: starts at the entries of earlier chunks)
 };
+
+// First slot of the role-A entries of in-edge eid, an edge of row u = [beg, end).
+template <int M>
+__device__ __forceinline__ int64_t role_a_slot(const WalkArgs& A, int32_t eid, int32_t u, int64_t beg, int64_t end) {
+    return M == kWalkList ? __ldg(A.off + eid) : stage_slot(__ldg(A.sbase + u), end - beg, eid - beg);
+}
+
+// Role-A entries of an in-edge found so far (all of them unless its row is
+// walked in chunks).
+template <int M>
+__device__ __forceinline__ void role_a_done(const WalkArgs& A, int32_t eid, uint32_t c, bool chunked) {
+    if (chunked) A.runA[eid] = (int32_t)c;
+    if (M == kWalkCount) A.cA[eid] = (int32_t)c;
+    else if (!chunked && c != (uint32_t)__ldg(A.cA + eid)) atomicMax(A.status, (int)TDT_ERR_CAPACITY);
+}
+
+// In-edges with long tails, one per lane where its bit of m is set, are left for
+// the end of the warp's work: a run of entries {edge, source} behind a header
+// {the warp's run before, entries}.  (Searched on the spot they cost the walk
+// of 512 Barabasi-Albert graphs 8 %: registers around a call that never came.)
+template <int M>
+__device__ __forceinline__ void push_long_tails(const WalkArgs& A, const WalkGroup& Q, WalkCtl* ctl, unsigned m,
+                                                int32_t eid, int32_t u) {
+    const unsigned lane = lane_id();
+    unsigned long long at = 0;
+    if (lane == 0) {
+        at = atomicAdd(&ctl->longs_next[M], 1ull + __popc(m));
+        A.longs[at] = make_int2((int)*Q.longs, __popc(m));
+        *Q.longs = (uint32_t)at;
+    }
+    at = __shfl_sync(kFull, at, 0);
+    if ((m >> lane) & 1u) A.longs[at + 1 + __popc(m & lanemask_lt())] = make_int2(eid, u);
+}
+
+// The runs of a warp.  The entries of the rows N+(v), of a run's in-edges (u,v)
+// as one flat space, are searched in the tails.  The rows' own counts have been
+// flushed by this block.
+template <int M>
+__device__ __forceinline__ void walk_long_tails(const WalkArgs& A, const WalkGroup& Q, bool list, int2* out0,
+                                                int64_t cap) {
+    const unsigned lane = lane_id();
+    __syncwarp();
+    for (uint32_t run = *Q.longs; run != kNoRun;) {
+        const int2 head = __ldcg(A.longs + (int64_t)run);
+        int32_t eid = 0, n = 0;
+        int64_t end = 0, e0 = 0;
+        if ((int)lane < head.y) {
+            const int2 x = __ldcg(A.longs + (int64_t)run + 1 + lane);
+            eid = x.x;
+            const int32_t v = __ldg(A.cols + eid);
+            e0 = __ldg(A.rp + v);
+            n = (int32_t)(__ldg(A.rp + v + 1) - e0);
+            end = __ldg(A.rp + x.y + 1);
+            if (list) Q.off[lane] = role_a_slot<M>(A, eid, x.y, __ldg(A.rp + x.y), end);
+            Q.cnt[lane] = 0u;
+        }
+        __syncwarp();
+        // a run's rows are of different v, or of one and its tails, longer than they, of different u
+        const int32_t incl = warp_incl_scan(n);
+        const int32_t total = __shfl_sync(kFull, incl, 31), S = incl - n;
+        for (int32_t b = 0; b < total; b += kWarp) {
+            const int32_t at = b + (int32_t)lane;
+            int own = 0;  // last lane with S <= at
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1)
+                if (__shfl_sync(kFull, S, own + step) <= at) own += step;
+            const int64_t e = __shfl_sync(kFull, e0, own) + (at - __shfl_sync(kFull, S, own));
+            const int64_t lo = (int64_t)__shfl_sync(kFull, eid, own) + 1, hi = __shfl_sync(kFull, end, own);
+            if (at >= total) continue;
+            const int64_t p = find_sorted<int64_t>(A.cols, lo, hi, __ldg(A.cols + e));
+            if (p < 0) continue;
+            if (M == kWalkCount) {
+                atomicAdd(A.cB + p, 1);
+                atomicAdd(A.cC + e, 1);
+            }
+            const uint32_t old = atomicAdd(Q.cnt + own, 1u);
+            if (list) {
+                const int64_t to = Q.off[own] + old;
+                if (to < cap) out0[to] = make_int2((int32_t)p, (int32_t)e);
+            }
+        }
+        __syncwarp();
+        if ((int)lane < head.y) role_a_done<M>(A, eid, Q.cnt[lane], false);
+        __syncwarp();
+        run = (uint32_t)head.x;
+    }
+}
 
 // One in-edge per lane, at position k of the in-adjacency (k < 0: none), of
 // the staged row or, Kind = kRowTiny, each of its own row cols[e0, e0 + d).
@@ -252,29 +363,31 @@ enum RowKind { kRowExact = 0, kRowHashed = 1, kRowTiny = 2 };
 
 template <int M, int Kind>
 __device__ __forceinline__ void walk_in_edges(const WalkArgs& A, const WalkRow& R, const WalkGroup& Q,
-                                              const int4* __restrict__ cols4, unsigned sh, bool list, int2* out0,
-                                              int64_t cap, int64_t k, int64_t e0, int d) {
+                                              WalkCtl* ctl, const int4* __restrict__ cols4, unsigned sh, bool list,
+                                              int2* out0, int64_t cap, int64_t k, int64_t e0, int d) {
     const unsigned lane = lane_id();
     const unsigned lt = lanemask_lt(), le = lt | (1u << lane);
     constexpr bool Exact = Kind == kRowExact;
     int32_t eid = 0, units = 0;
     unsigned lo = 0, hi = 0;
     int64_t slot = 0;
-    if (k >= 0) {
-        const int32_t u = __ldg(A.in_src + k);
-        eid = __ldg(A.in_eid + k);
-        const int64_t end = __ldg(A.rp + u + 1);
-        lo = (unsigned)eid + 1u + sh;
-        hi = (unsigned)end + sh;
-        if (hi > lo) {
-            units = (int32_t)(((hi + 3u) >> 2) - (lo >> 2));
-            if (M == kWalkList) {
-                slot = __ldg(A.off + eid);
-            } else if (list) {
-                const int64_t beg = __ldg(A.rp + u);
-                slot = stage_slot(__ldg(A.sbase + u), end - beg, eid - beg);
+    {
+        bool far = false;
+        int32_t u = 0;
+        if (k >= 0) {
+            u = __ldg(A.in_src + k);
+            eid = __ldg(A.in_eid + k);
+            const int64_t end = __ldg(A.rp + u + 1);
+            lo = (unsigned)eid + 1u + sh;
+            hi = (unsigned)end + sh;
+            if (hi > lo) {
+                far = hi - lo > (Kind == kRowTiny ? tail_limit((uint32_t)d) : R.limit);
+                if (!far) units = (int32_t)(((hi + 3u) >> 2) - (lo >> 2));
+                if (list) slot = role_a_slot<M>(A, eid, u, __ldg(A.rp + u), end);
             }
         }
+        const unsigned m = __ballot_sync(kFull, far);
+        if (m && !(Kind != kRowTiny && R.more)) push_long_tails<M>(A, Q, ctl, m, eid, u);
     }
     const unsigned nem = __ballot_sync(kFull, units > 0);
     if (nem == 0) return;
@@ -398,13 +511,7 @@ __device__ __forceinline__ void walk_in_edges(const WalkArgs& A, const WalkRow& 
         ob += nb + (Bn == base + kWarp ? 1 : 0);
         __syncwarp();
     }
-    if (units > 0) {
-        const uint32_t c = Q.cnt[ci];
-        const bool chunked = Kind != kRowTiny && R.chunked;
-        if (chunked) A.runA[eid] = (int32_t)c;
-        if (M == kWalkCount) A.cA[eid] = (int32_t)c;
-        else if (!chunked && c != (uint32_t)__ldg(A.cA + eid)) atomicMax(A.status, (int)TDT_ERR_CAPACITY);
-    }
+    if (units > 0) role_a_done<M>(A, eid, Q.cnt[ci], Kind != kRowTiny && R.chunked);
     __syncwarp();
 }
 
@@ -425,6 +532,7 @@ __global__ void __launch_bounds__(kWkBlock, kWkMinBlocks) walk_kernel(const __gr
     __shared__ int s_wsum[kWkWarps];
     __shared__ unsigned long long s_unit;
     __shared__ int s_next;
+    __shared__ uint32_t s_longs[kWkWarps];
     const bool failed = M == kWalkList && look_back_failed(A.status);  // the offsets are not the scan's
     if ((A.gate && *(volatile const int*)A.gate != 0) || failed) return;
     const int wib = threadIdx.x / kWarp;
@@ -437,9 +545,12 @@ __global__ void __launch_bounds__(kWkBlock, kWkMinBlocks) walk_kernel(const __gr
     int2* out0 = M == kWalkList ? A.out : A.out - cap;
     unsigned char* gs = smem + kWkRowBytes + wib * kGrpBytes;
     WalkGroup Q;
+    Q.longs = s_longs + wib;
     Q.ge = reinterpret_cast<int4*>(gs);
     Q.off = reinterpret_cast<int64_t*>(gs + 16 * kWarp);
     Q.cnt = reinterpret_cast<uint32_t*>(gs + 24 * kWarp);
+
+    if (lane == 0) s_longs[wib] = kNoRun;
 
     // ---- block rows
     const unsigned long long nunits = ctl->nunits;
@@ -453,10 +564,10 @@ __global__ void __launch_bounds__(kWkBlock, kWkMinBlocks) walk_kernel(const __gr
         const int64_t r0 = __ldg(A.rp + v), r1 = __ldg(A.rp + v + 1);
         const int64_t i0 = __ldg(A.cp + v), i1 = __ldg(A.cp + v + 1);
         const int64_t ka = i0 + (int64_t)un.y * kPart, kb = ka + kPart < i1 ? ka + kPart : i1;
-        const bool parts = i1 - i0 > kPart, chunked = r1 - r0 > A.row_cap;
+        const bool parts = i1 - i0 > kPart;
         for (int64_t c0 = r0; c0 < r1; c0 += A.row_cap) {
             const int d = (int)(r1 - c0 < A.row_cap ? r1 - c0 : A.row_cap);
-            WalkRow R = row_init(A, smem + kWkBm, smem + kWkCnt, nullptr, kHeavyLog2, c0, d, chunked, c0 > r0, parts);
+            WalkRow R = row_init(A, smem + kWkBm, smem + kWkCnt, nullptr, kHeavyLog2, c0, d, r1 - r0, c0 > r0, parts);
             const int nw = row_words(R);
             for (int i = threadIdx.x; i < nw; i += kWkBlock) R.bm[i] = 0u;
             if (threadIdx.x == 0) s_next = 0;
@@ -487,8 +598,8 @@ __global__ void __launch_bounds__(kWkBlock, kWkMinBlocks) walk_kernel(const __gr
                 nx = __shfl_sync(kFull, nx, 0);
                 if (ka + nx >= kb) break;
                 const int64_t k = ka + nx + lane < kb ? ka + nx + lane : -1;
-                if (R.exact) walk_in_edges<M, kRowExact>(A, R, Q, cols4, sh, list, out0, cap, k, 0, 0);
-                else walk_in_edges<M, kRowHashed>(A, R, Q, cols4, sh, list, out0, cap, k, 0, 0);
+                if (R.exact) walk_in_edges<M, kRowExact>(A, R, Q, ctl, cols4, sh, list, out0, cap, k, 0, 0);
+                else walk_in_edges<M, kRowHashed>(A, R, Q, ctl, cols4, sh, list, out0, cap, k, 0, 0);
             }
             __syncthreads();
             if (M == kWalkCount) row_flush(A, R, threadIdx.x, kWkBlock);
@@ -537,7 +648,7 @@ __global__ void __launch_bounds__(kWkBlock, kWkMinBlocks) walk_kernel(const __gr
                 const int64_t k = __shfl_sync(kFull, i0, own) + (at - __shfl_sync(kFull, ts, own));
                 const int64_t e0 = __shfl_sync(kFull, r0, own);
                 const int dr = __shfl_sync(kFull, d, own);
-                walk_in_edges<M, kRowTiny>(A, WalkRow{}, Q, cols4, sh, list, out0, cap, at < ttotal ? k : -1, e0, dr);
+                walk_in_edges<M, kRowTiny>(A, WalkRow{}, Q, ctl, cols4, sh, list, out0, cap, at < ttotal ? k : -1, e0, dr);
             }
         }
         unsigned todo = __ballot_sync(kFull, d > 0 && !tiny);
@@ -546,7 +657,7 @@ __global__ void __launch_bounds__(kWkBlock, kWkMinBlocks) walk_kernel(const __gr
             todo &= todo - 1;
             const int64_t e0 = __shfl_sync(kFull, r0, src), k0 = __shfl_sync(kFull, i0, src);
             const int dr = __shfl_sync(kFull, d, src), dk = __shfl_sync(kFull, din, src);
-            WalkRow R = row_init(A, sl + kLtBm, sl + kLtCnt, sl + kLtPerm, kLightLog2, e0, dr, false, false, false);
+            WalkRow R = row_init(A, sl + kLtBm, sl + kLtCnt, sl + kLtPerm, kLightLog2, e0, dr, dr, false, false);
             const int nw = row_words(R);
             for (int i = lane; i < nw; i += kWarp) R.bm[i] = 0u;
             __syncwarp();
@@ -564,7 +675,7 @@ __global__ void __launch_bounds__(kWkBlock, kWkMinBlocks) walk_kernel(const __gr
             __syncwarp();
             if (R.exact) {
                 for (int k = lane; k - (int)lane < dk; k += kWarp)
-                    walk_in_edges<M, kRowExact>(A, R, Q, cols4, sh, list, out0, cap, k < dk ? k0 + k : -1, 0, 0);
+                    walk_in_edges<M, kRowExact>(A, R, Q, ctl, cols4, sh, list, out0, cap, k < dk ? k0 + k : -1, 0, 0);
             } else {
                 for (int i = lane; i < dr; i += kWarp) {
                     const uint32_t x = (uint32_t)(__ldg(A.cols + e0 + i) - R.wb) & R.mask;
@@ -572,12 +683,13 @@ __global__ void __launch_bounds__(kWkBlock, kWkMinBlocks) walk_kernel(const __gr
                 }
                 __syncwarp();
                 for (int k = lane; k - (int)lane < dk; k += kWarp)
-                    walk_in_edges<M, kRowHashed>(A, R, Q, cols4, sh, list, out0, cap, k < dk ? k0 + k : -1, 0, 0);
+                    walk_in_edges<M, kRowHashed>(A, R, Q, ctl, cols4, sh, list, out0, cap, k < dk ? k0 + k : -1, 0, 0);
             }
             if (M == kWalkCount) row_flush(A, R, lane, kWarp);
             __syncwarp();
         }
     }
+    walk_long_tails<M>(A, Q, list, out0, cap);
 }
 
 // Roles B and C from the role-A entries (eB, eC) of eA = (u,v):
@@ -977,11 +1089,12 @@ static WalkArgs walk_args(const int64_t* rp, const int32_t* cols, const int64_t*
 // needs no more than stage_slots, the role-A entries in their staging slots,
 // which end at stage_end; *stage_skip receives the choice.  cA, cB, cC and ctl
 // are zeroed by the caller.  units: 16 E bytes of scratch that stays as
-// the list walk's plan; runA: int32[E] scratch; ctl: 256 bytes.
+// the list walk's plan; runA: int32[E] and longs: 16 E bytes of scratch; ctl:
+// 256 bytes.
 int launch_walk_count(const int64_t* rp, const int32_t* cols, const int64_t* cp, const int32_t* in_src,
                       const int32_t* in_eid, int64_t nv, int64_t ne, int32_t* cA, int32_t* cB, int32_t* cC,
                       const int64_t* sbase, int2* stage_end, unsigned long long stage_slots, int* stage_skip,
-                      int32_t* runA, void* units, void* ctl, int* status, cudaStream_t st) {
+                      int32_t* runA, void* units, void* longs, void* ctl, int* status, cudaStream_t st) {
     if (nv <= 0) return TDT_OK;
     DeviceInfo di;
     int rc = device_info(&di);
@@ -999,6 +1112,7 @@ int launch_walk_count(const int64_t* rp, const int32_t* cols, const int64_t* cp,
     A.out = stage_end;
     A.stage_skip = stage_skip;
     A.runA = runA;
+    A.longs = reinterpret_cast<int2*>(longs);
     return launch_walk<kWalkCount>(A, reinterpret_cast<WalkCtl*>(ctl), st);
 }
 
@@ -1006,12 +1120,14 @@ int launch_walk_count(const int64_t* rp, const int32_t* cols, const int64_t* cp,
 // same plan (skipped on the device when *gate != 0).
 int launch_walk_list(const int64_t* rp, const int32_t* cols, const int64_t* cp, const int32_t* in_src,
                      const int32_t* in_eid, int64_t nv, int64_t ne, const int64_t* off, int32_t* cA, int2* lists,
-                     int32_t* runA, void* units, void* ctl, const int* gate, int* status, cudaStream_t st) {
+                     int32_t* runA, void* units, void* longs, void* ctl, const int* gate, int* status,
+                     cudaStream_t st) {
     if (nv <= 0) return TDT_OK;
     WalkArgs A = walk_args(rp, cols, cp, in_src, in_eid, nv, ne, cA, nullptr, nullptr, units, gate, status);
     A.off = off;
     A.out = lists;
     A.runA = runA;
+    A.longs = reinterpret_cast<int2*>(longs);
     return launch_walk<kWalkList>(A, reinterpret_cast<WalkCtl*>(ctl), st);
 }
 
