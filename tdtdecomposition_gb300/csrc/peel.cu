@@ -1522,12 +1522,16 @@ __global__ void __launch_bounds__(kPeelBlock, TDT_PEEL_MINB) peel_kernel(const _
 // Input validation, before any kernel indexes through the graph:
 // row_ptr[0] == 0, row_ptr[V] == E, non-decreasing; rows[e] is the row that
 // owns position e; u < v < V; columns strictly increasing within a row.
-__device__ __forceinline__ int validate_edge(const int32_t* __restrict__ cols, int64_t e, int64_t u, int64_t b,
-                                             int64_t en, int64_t V) {
-    const int32_t v = cols[e];
+__device__ __forceinline__ int validate_edge(int32_t v, int32_t next, int64_t e, int64_t u, int64_t b, int64_t en,
+                                             int64_t V) {
     if (u < 0 || u >= V || v >= V || u >= v) return TDT_ERR_NOT_ORIENTED;
     if (e < b || e >= en) return TDT_ERR_INVALID;
-    return e + 1 < en && cols[e + 1] <= v ? TDT_ERR_INVALID : TDT_OK;
+    return e + 1 < en && next <= v ? TDT_ERR_INVALID : TDT_OK;
+}
+
+// The column after edge e in a row that ends at en.
+__device__ __forceinline__ int32_t next_col(const int32_t* __restrict__ cols, int64_t e, int64_t en) {
+    return e + 1 < en ? cols[e + 1] : 0;
 }
 
 __global__ void validate_kernel(const int64_t* __restrict__ rp, const int32_t* __restrict__ rows,
@@ -1540,19 +1544,32 @@ __global__ void validate_kernel(const int64_t* __restrict__ rp, const int32_t* _
     for (int64_t e = tid; e < E; e += nth) {
         const int32_t u = rows[e];
         const bool in = u >= 0 && u < V;
-        const int64_t en = in ? rp[u + 1] : 0;
-        const int err = validate_edge(cols, e, u, in ? rp[u] : 0, en < E ? en : E, V);  // cols ends at E
+        const int64_t end = in ? rp[u + 1] : 0, en = end < E ? end : E;  // cols ends at E
+        const int err = validate_edge(cols[e], next_col(cols, e, en), e, u, in ? rp[u] : 0, en, V);
         if (err) atomicMax(&ctl->g.status, err);
     }
 }
 
 // The same when the caller gave no rows: a warp per row writes them, inside
-// [0, E) whatever row_ptr says.
-__global__ void validate_rows_kernel(const int64_t* __restrict__ rp, int32_t* __restrict__ rows,
-                                     const int32_t* __restrict__ cols, int64_t E, int64_t V, PeelCtl* ctl) {
+// [0, E) whatever row_ptr says.  Rows of more than kValLong edges wait in shared
+// memory for the whole block, with kValUnroll edges a thread in flight: degree
+// ranks have few of them, but a low hub's row in one warp is a chain of loads
+// (a row of 2 M edges: 39 ms in a warp, 1.8 in a block).  Eight blocks per SM: the
+// short rows wait for loads too (validation of scale 21 0.13 ms longer at six).
+constexpr int kValBlock = 256;
+constexpr int kValLong = 2048, kValList = 64, kValUnroll = 4;
+
+__global__ void __launch_bounds__(kValBlock, 8) validate_rows_kernel(const int64_t* __restrict__ rp,
+                                                                  int32_t* __restrict__ rows,
+                                                                  const int32_t* __restrict__ cols, int64_t E,
+                                                                  int64_t V, PeelCtl* ctl) {
+    __shared__ int32_t s_long[kValList];
+    __shared__ int s_n;
     const unsigned lane = lane_id();
     const int64_t tid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
     if (tid == 0 && (rp[0] != 0 || rp[V] != E)) atomicMax(&ctl->g.status, (int)TDT_ERR_INVALID);
     for (int64_t u = tid >> 5; u < V; u += nw) {
         const int64_t b = rp[u], en = rp[u + 1];
@@ -1560,9 +1577,42 @@ __global__ void validate_rows_kernel(const int64_t* __restrict__ rp, int32_t* __
             atomicMax(&ctl->g.status, (int)TDT_ERR_INVALID);
             continue;
         }
+        if (en - b > kValLong) {
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&s_n, 1);
+            at = __shfl_sync(kFull, at, 0);
+            if (at < kValList) {
+                if (lane == 0) s_long[at] = (int32_t)u;
+                continue;
+            }
+        }
         for (int64_t e = b + lane; e < en; e += kWarp) {
             rows[e] = (int32_t)u;
-            const int err = validate_edge(cols, e, u, b, en, V);
+            const int err = validate_edge(cols[e], next_col(cols, e, en), e, u, b, en, V);
+            if (err) atomicMax(&ctl->g.status, err);
+        }
+    }
+    __syncthreads();
+    const int n = s_n < kValList ? s_n : kValList;
+    for (int i = 0; i < n; i++) {
+        const int64_t u = s_long[i], b = rp[u], en = rp[u + 1];
+        for (int64_t e0 = b + threadIdx.x; e0 < en; e0 += kValUnroll * kValBlock) {
+            int32_t v[kValUnroll], next[kValUnroll];
+#pragma unroll
+            for (int k = 0; k < kValUnroll; k++) {
+                const int64_t e = e0 + k * kValBlock;
+                v[k] = e < en ? cols[e] : 0;
+                next[k] = next_col(cols, e, en);
+            }
+            int err = TDT_OK;
+#pragma unroll
+            for (int k = 0; k < kValUnroll; k++) {
+                const int64_t e = e0 + k * kValBlock;
+                if (e < en) {
+                    rows[e] = (int32_t)u;
+                    err = max(err, validate_edge(v[k], next[k], e, u, b, en, V));
+                }
+            }
             if (err) atomicMax(&ctl->g.status, err);
         }
     }
@@ -2003,7 +2053,7 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     if (rows)
         validate_kernel<<<g_e, tb, 0, st>>>(rp, rows, cols, E, V, L.ctl);
     else
-        validate_rows_kernel<<<grid_for(V * 32, tb, di.sms, 8), tb, 0, st>>>(rp, L.rows_d, cols, E, V, L.ctl);
+        validate_rows_kernel<<<grid_for(V * 32, kValBlock, di.sms, 8), kValBlock, 0, st>>>(rp, L.rows_d, cols, E, V, L.ctl);
     TDT_LAUNCH_CHECK("validate");
     // cA, cB, cC (role counts) live in the first queue buffer until the peel starts
     int32_t* cA = reinterpret_cast<int32_t*>(L.qi[0]);
