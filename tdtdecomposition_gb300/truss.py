@@ -55,6 +55,11 @@ LIST_BUDGET_FRACTION = 0.6
 # lists plus the one walk's staging area (which is dead memory once the lists
 # are packed) may take more of the free memory
 STAGE_BUDGET_FRACTION = 0.75
+# and at most this many times the bytes of the rest of the workspace: orders that
+# are degree ranks need 0.4 to 1.0 times as much, R-MAT scale 18 in id order 9.5
+# (one walk 51 ms, two 70), a wheel of 200 K vertices with its hub at id 0 1,100
+# times (160 GB)
+STAGE_RATIO = 16
 
 
 def stage_bytes(cols, rp, rows=None):
@@ -73,7 +78,9 @@ def _list_bytes(ws, cols, rp, lists, base, rows=None):
     plus, when that fits too, the staging area of the one-walk pass (which
     then counts and lists in one walk instead of two).  lists:
     True/False/"auto" ("auto" keeps lists whenever they fit: the listed peel
-    is the faster one at every size, from 10 K edges up)."""
+    is the faster one at every size, from 10 K edges up; True always keeps
+    them, and takes the second walk where there is no room for the first's
+    staging)."""
     if lists is False:
         return 0
     key = _graph_key(cols, rp)
@@ -87,15 +94,17 @@ def _list_bytes(ws, cols, rp, lists, base, rows=None):
         S = stage_bytes(cols, rp, rows)
         ws.triangles[sk] = S
     need = 24 * T + 256
-    if lists is True:
-        return need + S
-    if ws.buf is not None and base + need + S <= ws.buf.numel():
+    if S > STAGE_RATIO * (base + need):
+        S = None
+    elif ws.buf is not None and base + need + S <= ws.buf.numel():
         return need + S  # the workspace holds it already: nothing to ask the driver for
+    if lists is True and S is None:
+        return need
     free, _ = torch.cuda.mem_get_info(cols.device)
     have = free + (ws.buf.numel() if ws.buf is not None else 0) - base
-    if need + S <= STAGE_BUDGET_FRACTION * have:
+    if S is not None and need + S <= (1.0 if lists is True else STAGE_BUDGET_FRACTION) * have:
         return need + S
-    return need if need <= LIST_BUDGET_FRACTION * have else 0
+    return need if lists is True or need <= LIST_BUDGET_FRACTION * have else 0
 
 
 _default_ws = {}
