@@ -32,8 +32,11 @@ class TrussResult(NamedTuple):
 class Workspace:
     """Device scratch reused across calls (grown on demand, torch-allocated).
 
-    It also remembers the triangle count of the graphs it has served, so that
-    later calls on the same graph can size the per-edge triangle lists."""
+    It also remembers how many triangles a graph of E edges and V vertices last
+    had, so that the next call on one of that size can ask for its lists without
+    a counting pass.  That sizes the list tail and nothing else: the device
+    keeps lists exactly when they fit, and a call that reads its result back
+    corrects the count."""
 
     def __init__(self, device=None):
         self.device = torch.device(device) if device is not None else torch.device("cuda")
@@ -48,7 +51,7 @@ class Workspace:
 
 
 def _graph_key(cols, rp):
-    return (cols.data_ptr(), cols.shape[0], rp.shape[0])
+    return (cols.shape[0], rp.shape[0])
 
 
 LIST_BUDGET_FRACTION = 0.6
@@ -72,7 +75,7 @@ def stage_bytes(cols, rp, rows=None):
     return 4 * int((d * (d - 1)).sum())
 
 
-def _list_bytes(ws, cols, rp, lists, base, rows=None):
+def _list_bytes(ws, cols, rp, lists, base, rows=None, count=False):
     """Bytes for the workspace's list tail, or 0 to let the peel search the
     adjacency instead: the per-edge triangle lists (24 bytes per triangle)
     plus, when that fits too, the staging area of the one-walk pass (which
@@ -80,10 +83,30 @@ def _list_bytes(ws, cols, rp, lists, base, rows=None):
     True/False/"auto" ("auto" keeps lists whenever they fit: the listed peel
     is the faster one at every size, from 10 K edges up; True always keeps
     them, and takes the second walk where there is no room for the first's
-    staging)."""
+    staging).  What the workspace has beyond that is offered too.  count: take
+    no count of an earlier graph of this size."""
     if lists is False:
         return 0
+    tail = _list_need(ws, cols, rp, lists, base, rows, count)
+    return max(tail, ws.buf.numel() - base) if tail and ws.buf is not None else tail
+
+
+def _learn(ws, cols, rp, stats, tail):
+    """The triangle count of a finished run, for the next graph of this size."""
     key = _graph_key(cols, rp)
+    if key in ws.triangles:
+        ws.triangles[key] = T = stats[STAT_TRIANGLES]
+        S = ws.triangles.get(("stage",) + key)
+        if stats[STAT_LISTED] == 1 and S is not None and 24 * T + 256 + S <= tail:
+            # this graph has more slots: room for them, and for the next one's
+            ws.triangles[("stage",) + key] = stage_bytes(cols, rp) * 17 // 16
+
+
+def _list_need(ws, cols, rp, lists, base, rows, count):
+    key = _graph_key(cols, rp)
+    if count:
+        ws.triangles.pop(key, None)
+        ws.triangles.pop(("stage",) + key, None)
     T = ws.triangles.get(key)
     if T is None:
         T = triangle_count_arrays(cols, rp, ws)
@@ -145,8 +168,11 @@ def truss_decompose(graph, workspace=None, stream=None, sync=True, lists="auto",
     """Full truss decomposition (singlegpu_truss.py:67-158 + :38-45).
 
     lists: "auto" keeps per-edge triangle lists in the workspace when they fit
-    in LIST_BUDGET_FRACTION of the free device memory (the first call on a
-    graph then counts its triangles first), True always, False never.
+    in LIST_BUDGET_FRACTION of the free device memory, True always, False
+    never.  The first call with "auto" or True on a graph of a size that the
+    workspace has not served counts the triangles first; later ones size the
+    lists by the last graph of that size, and with True (and sync) run once
+    more when that was too little.
     list_budget (bytes): instead, give the lists a fixed workspace tail and
     let the device decide (lists when 24 T bytes fit, else the search peel),
     with no counting pass."""
@@ -162,20 +188,29 @@ def truss_decompose(graph, workspace=None, stream=None, sync=True, lists="auto",
     need = L.tdt_decompose_workspace_bytes(V, E)
     wso = _ws_for(dev, workspace)
     base = (need + 255) // 256 * 256
-    tail = int(list_budget) if list_budget is not None else _list_bytes(wso, cols, rp, lists, base, rows)
-    ws = wso.get(base + tail)
     s = (stream or torch.cuda.current_stream(dev)).cuda_stream
-    # pass the requested size, not the (possibly larger, shared) buffer: the
-    # device keeps lists exactly when the tail it is given holds them
-    with torch.cuda.device(cols.device):
-        rc = L.tdt_truss_decompose(rows.data_ptr() if rows is not None else None, cols.data_ptr(), rp.data_ptr(), V, E,
-                                   truss.data_ptr(), e_truss.data_ptr(), ptr.data_ptr(), cap, stats.data_ptr(),
-                                   ws.data_ptr(), base + tail, s)
-    _lib.check(rc, "tdt_truss_decompose")
-    if not sync:
-        return truss, e_truss, ptr, stats
-    sh = stats.tolist()
-    _check_stats(sh, "tdt_truss_decompose")
+    tail = -1
+    while True:
+        asked = int(list_budget) if list_budget is not None else _list_bytes(wso, cols, rp, lists, base, rows)
+        if asked <= tail:
+            break
+        tail = asked
+        ws = wso.get(base + tail)
+        # the device keeps lists exactly when the tail it is given holds them
+        with torch.cuda.device(cols.device):
+            rc = L.tdt_truss_decompose(rows.data_ptr() if rows is not None else None, cols.data_ptr(), rp.data_ptr(),
+                                       V, E, truss.data_ptr(), e_truss.data_ptr(), ptr.data_ptr(), cap,
+                                       stats.data_ptr(), ws.data_ptr(), base + tail, s)
+        _lib.check(rc, "tdt_truss_decompose")
+        if not sync:
+            return truss, e_truss, ptr, stats
+        sh = stats.tolist()
+        _check_stats(sh, "tdt_truss_decompose")
+        if list_budget is not None:
+            break
+        _learn(wso, cols, rp, sh, tail)
+        if lists is not True or sh[STAT_LISTED] or E == 0:
+            break
     return TrussResult(truss, e_truss[: sh[STAT_NETRUSS]], ptr[: sh[STAT_NPTR]], sh[STAT_KMAX],
                        sh[STAT_TRIANGLES], sh[STAT_ROUNDS], bool(sh[STAT_LISTED]), sh[STAT_LISTED])
 
@@ -198,7 +233,9 @@ def ktruss_search(graph, k, workspace=None, stream=None, lists="auto"):
         rc = L.tdt_ktruss_search(rows.data_ptr() if rows is not None else None, cols.data_ptr(), rp.data_ptr(), V, E,
                                  int(k), mask.data_ptr(), stats.data_ptr(), ws.data_ptr(), base + tail, s)
     _lib.check(rc, "tdt_ktruss_search")
-    _check_stats(stats.tolist(), "tdt_ktruss_search")
+    sh = stats.tolist()
+    _check_stats(sh, "tdt_ktruss_search")
+    _learn(wso, cols, rp, sh, tail)
     return mask
 
 
