@@ -2,16 +2,18 @@
 
 The triangle walk gives a row to one warp when its out-degree is at most
 `warp_cap` (and it has few in-edges), to a whole block otherwise, in column
-chunks of `heavy_cap` entries; `vec` is the wedge width of the drop-in support
-operator (the whole-path walk always reads 16-byte chunks of four columns);
-the peel reads triangles from per-edge lists or searches for them (`lists`),
-on a persistent grid of `peel_grid` half-SM units (0: the size heuristic).  Which choice is fastest depends on the
-degree profile and size of the workload, so the tuner times the candidates
-on the workload itself (CUDA events, after one warm-up run each), one
-dimension at a time from the defaults (a coordinate search: the split, then
-the lists, the peel grid and the walk width), and caches the winner per
-workload signature (edge count and out-degree profile, bucketed).  Results
-do not depend on any of these choices."""
+chunks of `heavy_cap` entries; the peel reads triangles from per-edge lists or
+searches for them (`lists`), on a persistent grid of `peel_grid` half-SM units
+(0: the size heuristic).  Which choice is fastest depends on the degree profile
+and size of the workload, so the tuner times the candidates on the workload
+itself (CUDA events, after one warm-up run each), one dimension at a time from
+the defaults (a coordinate search: the split, then the lists and the peel
+grid), and caches the winner per workload signature (edge count and out-degree
+profile, bucketed).  Results do not depend on any of these choices.
+
+`vec`, the wedge width of the drop-in support operator, is not among them: a
+decomposition always reads 16-byte chunks of four columns, so it cannot tell
+the widths apart.  A Config carries the first of `vec_options`."""
 import math
 
 import torch
@@ -88,19 +90,13 @@ def tune(graph, workspace=None, lists_options=(True, False), candidates=CANDIDAT
         return timed[cfg]
 
     best = Config(candidates[0][0], candidates[0][1], lists_options[0], peel_grids[0], vec_options[0])
-    dims = [
-        [Config(wc, hc, best.lists, best.peel_grid, best.vec) for wc, hc in candidates],
-        None, None, None,
-    ]
-    for d in range(4):
+    for d in range(3):
         if d == 0:
-            opts = dims[0]
+            opts = [Config(wc, hc, best.lists, best.peel_grid, best.vec) for wc, hc in candidates]
         elif d == 1:
             opts = [Config(best.warp_cap, best.heavy_cap, li, best.peel_grid, best.vec) for li in lists_options]
-        elif d == 2:
-            opts = [Config(best.warp_cap, best.heavy_cap, best.lists, pg, best.vec) for pg in peel_grids]
         else:
-            opts = [Config(best.warp_cap, best.heavy_cap, best.lists, best.peel_grid, v) for v in vec_options]
+            opts = [Config(best.warp_cap, best.heavy_cap, best.lists, pg, best.vec) for pg in peel_grids]
         best = min(opts, key=cost)
     _cache[key] = best
     apply(best)
