@@ -107,7 +107,7 @@ struct WalkArgs {
     const int64_t* off;         // kWalkList: list offsets int64[E+1]
     int2* out;                  // kWalkCount: end of the staging slots; kWalkList: the lists
     int32_t* runA;              // role-A entries so far of rows walked in column chunks
-    int2* longs;                // 2 E: runs of in-edges with long tails (see push_long_tails)
+    uint32_t* longs;            // per in-edge with a long tail: the lane's one before it (walk_long_tails)
     const int2* units;          // block rows: {v, part}
     int* status;
     const int* gate;            // non-zero: skip
@@ -123,7 +123,6 @@ struct WalkCtl {
     unsigned long long light_next[2];
     unsigned long long dist_next[2];  // and of the role-B and role-C passes
     unsigned long long dist_done;     // blocks that finished the role-C pass
-    unsigned long long longs_next[2]; // places of WalkArgs::longs in use, of the count and the list walk
 };
 
 // First staging slot of the role-A entries of the edge at position i of a row
@@ -196,13 +195,15 @@ struct WalkRow {
 // out-edges behind a source u of many, as in orders that are not degree ranks (the
 // wheel of 200 K vertices with its hub at id 0 streams 20 G entries, 28 ms of
 // support phase).  Past kLongTail entries and kLongRatio times the row's, the
-// row's entries are searched in the tail instead (that wheel: 0.15 ms), so the
-// walk stays within a factor of the rows' lengths.  Support phase with ratios 8 /
-// 32 / 128, and none: R-MAT scale 16 in id order 1.6 / 2.2 / 3.0 / 2.8 ms, with a
-// hub joined to all of it 1.7 / 2.4 / 2.9 / 7.1, scale 18 in id order 24 / 26 /
-// 31 / 35; degree ranks at scale 18 0.66 with any; tails of 128 or 2,048 instead
-// of 512 within 5 %.
-constexpr uint32_t kLongTail = 512, kLongRatio = 8;
+// row's entries are searched in the tail instead (that wheel: 0.12 ms), so the
+// walk stays within a factor of the rows' lengths.  Support phase streaming all
+// of a tail / with ratios 32, 8 and 4: R-MAT scale 16 in id order 2.8 / 2.2, 1.6,
+// 1.3 ms, with a hub joined to all of it 7.1 / 2.4, 1.7, 1.4; scale 18 in id
+// order 35 / 26, 22, 21.  Tails of 512 instead of 128: a complete bipartite
+// graph of 2 x 3,000 with a path on one side 2.8 instead of 1.9 (all streamed 2.8).  Degree
+// ranks do not notice: scale 18 0.65 with any, scale 21 and 512 Barabasi-Albert
+// graphs within 1 %.
+constexpr uint32_t kLongTail = 128, kLongRatio = 4;
 __device__ __forceinline__ uint32_t tail_limit(uint32_t dout) {
     return dout > UINT32_MAX / kLongRatio ? UINT32_MAX : max(kLongTail, kLongRatio * dout);
 }
@@ -258,11 +259,11 @@ __device__ __forceinline__ int row_find(const WalkArgs& A, const WalkRow& R, uin
     return p < 0 ? -1 : (int)(p - R.e0);
 }
 
-constexpr uint32_t kNoRun = UINT32_MAX;
+constexpr uint32_t kNoEdge = UINT32_MAX;
 
 // This warp's group of up to 32 in-edges.
 struct WalkGroup {
-    uint32_t* longs;            // the warp's last run of in-edges with long tails (kNoRun: none)
+    uint32_t* longs;            // per lane: its last in-edge with a long tail (kNoEdge: none)
     int4* ge;                   // per non-empty tail: {first chunk, begin, end, 0} (positions in colsA)
     int64_t* off;               // listing: slot of the in-edge's first role-A entry
     uint32_t* cnt;              // role-A entries found (listing: starts at the entries of earlier chunks)
@@ -283,48 +284,36 @@ __device__ __forceinline__ void role_a_done(const WalkArgs& A, int32_t eid, uint
     else if (!chunked && c != (uint32_t)__ldg(A.cA + eid)) atomicMax(A.status, (int)TDT_ERR_CAPACITY);
 }
 
-// In-edges with long tails, one per lane where its bit of m is set, are left for
-// the end of the warp's work: a run of entries {edge, source} behind a header
-// {the warp's run before, entries}.  (Searched on the spot they cost the walk
-// of 512 Barabasi-Albert graphs 8 %: registers around a call that never came.)
-template <int M>
-__device__ __forceinline__ void push_long_tails(const WalkArgs& A, const WalkGroup& Q, WalkCtl* ctl, unsigned m,
-                                                int32_t eid, int32_t u) {
-    const unsigned lane = lane_id();
-    unsigned long long at = 0;
-    if (lane == 0) {
-        at = atomicAdd(&ctl->longs_next[M], 1ull + __popc(m));
-        A.longs[at] = make_int2((int)*Q.longs, __popc(m));
-        *Q.longs = (uint32_t)at;
-    }
-    at = __shfl_sync(kFull, at, 0);
-    if ((m >> lane) & 1u) A.longs[at + 1 + __popc(m & lanemask_lt())] = make_int2(eid, u);
-}
-
-// The runs of a warp.  The entries of the rows N+(v), of a run's in-edges (u,v)
-// as one flat space, are searched in the tails.  The rows' own counts have been
-// flushed by this block.
+// The in-edges with long tails that each lane of a warp left for the end of the
+// warp's work, a list through longs from the last one.  The entries of their
+// rows N+(v), of 32 in-edges (u,v) as one flat space, are searched in the tails.
+// The rows' own counts have been flushed by this block.  (Searched on the spot they
+// cost the walk of 512 Barabasi-Albert graphs 8 %: registers around a call that
+// never came.)
 template <int M>
 __device__ __forceinline__ void walk_long_tails(const WalkArgs& A, const WalkGroup& Q, bool list, int2* out0,
                                                 int64_t cap) {
     const unsigned lane = lane_id();
     __syncwarp();
-    for (uint32_t run = *Q.longs; run != kNoRun;) {
-        const int2 head = __ldcg(A.longs + (int64_t)run);
+    uint32_t k = Q.longs[lane];
+    Q.longs[lane] = kNoEdge;
+    while (__any_sync(kFull, k != kNoEdge)) {
         int32_t eid = 0, n = 0;
         int64_t end = 0, e0 = 0;
-        if ((int)lane < head.y) {
-            const int2 x = __ldcg(A.longs + (int64_t)run + 1 + lane);
-            eid = x.x;
+        const bool mine = k != kNoEdge;
+        if (mine) {
+            const int32_t u = __ldg(A.in_src + k);
+            eid = __ldg(A.in_eid + k);
+            k = A.longs[k];
             const int32_t v = __ldg(A.cols + eid);
             e0 = __ldg(A.rp + v);
             n = (int32_t)(__ldg(A.rp + v + 1) - e0);
-            end = __ldg(A.rp + x.y + 1);
-            if (list) Q.off[lane] = role_a_slot<M>(A, eid, x.y, __ldg(A.rp + x.y), end);
+            end = __ldg(A.rp + u + 1);
+            if (list) Q.off[lane] = role_a_slot<M>(A, eid, u, __ldg(A.rp + u), end);
             Q.cnt[lane] = 0u;
         }
         __syncwarp();
-        // a run's rows are of different v, or of one and its tails, longer than they, of different u
+        // pairs (u,v) differ and a tail is longer than its row: at most E in all
         const int32_t incl = warp_incl_scan(n);
         const int32_t total = __shfl_sync(kFull, incl, 31), S = incl - n;
         for (int32_t b = 0; b < total; b += kWarp) {
@@ -349,9 +338,8 @@ __device__ __forceinline__ void walk_long_tails(const WalkArgs& A, const WalkGro
             }
         }
         __syncwarp();
-        if ((int)lane < head.y) role_a_done<M>(A, eid, Q.cnt[lane], false);
+        if (mine) role_a_done<M>(A, eid, Q.cnt[lane], false);
         __syncwarp();
-        run = (uint32_t)head.x;
     }
 }
 
@@ -363,31 +351,29 @@ enum RowKind { kRowExact = 0, kRowHashed = 1, kRowTiny = 2 };
 
 template <int M, int Kind>
 __device__ __forceinline__ void walk_in_edges(const WalkArgs& A, const WalkRow& R, const WalkGroup& Q,
-                                              WalkCtl* ctl, const int4* __restrict__ cols4, unsigned sh, bool list,
-                                              int2* out0, int64_t cap, int64_t k, int64_t e0, int d) {
+                                              const int4* __restrict__ cols4, unsigned sh, bool list, int2* out0,
+                                              int64_t cap, int64_t k, int64_t e0, int d) {
     const unsigned lane = lane_id();
     const unsigned lt = lanemask_lt(), le = lt | (1u << lane);
     constexpr bool Exact = Kind == kRowExact;
     int32_t eid = 0, units = 0;
     unsigned lo = 0, hi = 0;
     int64_t slot = 0;
-    {
-        bool far = false;
-        int32_t u = 0;
-        if (k >= 0) {
-            u = __ldg(A.in_src + k);
-            eid = __ldg(A.in_eid + k);
-            const int64_t end = __ldg(A.rp + u + 1);
-            lo = (unsigned)eid + 1u + sh;
-            hi = (unsigned)end + sh;
-            if (hi > lo) {
-                far = hi - lo > (Kind == kRowTiny ? tail_limit((uint32_t)d) : R.limit);
-                if (!far) units = (int32_t)(((hi + 3u) >> 2) - (lo >> 2));
+    if (k >= 0) {
+        const int32_t u = __ldg(A.in_src + k);
+        eid = __ldg(A.in_eid + k);
+        const int64_t end = __ldg(A.rp + u + 1);
+        lo = (unsigned)eid + 1u + sh;
+        hi = (unsigned)end + sh;
+        if (hi > lo) {
+            if (hi - lo <= (Kind == kRowTiny ? tail_limit((uint32_t)d) : R.limit)) {
+                units = (int32_t)(((hi + 3u) >> 2) - (lo >> 2));
                 if (list) slot = role_a_slot<M>(A, eid, u, __ldg(A.rp + u), end);
+            } else if (Kind == kRowTiny || !R.more) {
+                A.longs[k] = Q.longs[lane];
+                Q.longs[lane] = (uint32_t)k;
             }
         }
-        const unsigned m = __ballot_sync(kFull, far);
-        if (m && !(Kind != kRowTiny && R.more)) push_long_tails<M>(A, Q, ctl, m, eid, u);
     }
     const unsigned nem = __ballot_sync(kFull, units > 0);
     if (nem == 0) return;
@@ -532,7 +518,7 @@ __global__ void __launch_bounds__(kWkBlock, kWkMinBlocks) walk_kernel(const __gr
     __shared__ int s_wsum[kWkWarps];
     __shared__ unsigned long long s_unit;
     __shared__ int s_next;
-    __shared__ uint32_t s_longs[kWkWarps];
+    __shared__ uint32_t s_longs[kWkBlock];
     const bool failed = M == kWalkList && look_back_failed(A.status);  // the offsets are not the scan's
     if ((A.gate && *(volatile const int*)A.gate != 0) || failed) return;
     const int wib = threadIdx.x / kWarp;
@@ -545,151 +531,156 @@ __global__ void __launch_bounds__(kWkBlock, kWkMinBlocks) walk_kernel(const __gr
     int2* out0 = M == kWalkList ? A.out : A.out - cap;
     unsigned char* gs = smem + kWkRowBytes + wib * kGrpBytes;
     WalkGroup Q;
-    Q.longs = s_longs + wib;
+    Q.longs = s_longs + wib * kWarp;
     Q.ge = reinterpret_cast<int4*>(gs);
     Q.off = reinterpret_cast<int64_t*>(gs + 16 * kWarp);
     Q.cnt = reinterpret_cast<uint32_t*>(gs + 24 * kWarp);
 
-    if (lane == 0) s_longs[wib] = kNoRun;
+    Q.longs[lane] = kNoEdge;
 
-    // ---- block rows
+    // ---- block rows, a unit a turn, and the warp rows in the last one.  Each turn
+    // ends with the searches it left: a block that only left them would take the
+    // most units.
     const unsigned long long nunits = ctl->nunits;
     for (;;) {
         if (threadIdx.x == 0) s_unit = atomicAdd(&ctl->unit_next[M], 1ull);
         __syncthreads();
         const unsigned long long ui = s_unit;
-        if (ui >= nunits) break;
-        const int2 un = __ldg(A.units + ui);
-        const int64_t v = un.x;
-        const int64_t r0 = __ldg(A.rp + v), r1 = __ldg(A.rp + v + 1);
-        const int64_t i0 = __ldg(A.cp + v), i1 = __ldg(A.cp + v + 1);
-        const int64_t ka = i0 + (int64_t)un.y * kPart, kb = ka + kPart < i1 ? ka + kPart : i1;
-        const bool parts = i1 - i0 > kPart;
-        for (int64_t c0 = r0; c0 < r1; c0 += A.row_cap) {
-            const int d = (int)(r1 - c0 < A.row_cap ? r1 - c0 : A.row_cap);
-            WalkRow R = row_init(A, smem + kWkBm, smem + kWkCnt, nullptr, kHeavyLog2, c0, d, r1 - r0, c0 > r0, parts);
-            const int nw = row_words(R);
-            for (int i = threadIdx.x; i < nw; i += kWkBlock) R.bm[i] = 0u;
-            if (threadIdx.x == 0) s_next = 0;
-            __syncthreads();
-            row_fill(A, R, threadIdx.x, kWkBlock);
-            __syncthreads();
-            if (R.exact) {
-                // running counts: each thread's run of words, then a block scan
-                const int per = (nw + kWkBlock - 1) / kWkBlock;
-                const int a = threadIdx.x * per, b = a + per < nw ? a + per : nw;
-                int s = 0;
-                for (int i = a; i < b; i++) s += __popc(R.bm[i]);
-                const int incl = warp_incl_scan(s);
-                if (lane == 31) s_wsum[wib] = incl;
+        const bool last = ui >= nunits;
+        if (!last) {
+            const int2 un = __ldg(A.units + ui);
+            const int64_t v = un.x;
+            const int64_t r0 = __ldg(A.rp + v), r1 = __ldg(A.rp + v + 1);
+            const int64_t i0 = __ldg(A.cp + v), i1 = __ldg(A.cp + v + 1);
+            const int64_t ka = i0 + (int64_t)un.y * kPart, kb = ka + kPart < i1 ? ka + kPart : i1;
+            const bool parts = i1 - i0 > kPart;
+            for (int64_t c0 = r0; c0 < r1; c0 += A.row_cap) {
+                const int d = (int)(r1 - c0 < A.row_cap ? r1 - c0 : A.row_cap);
+                WalkRow R = row_init(A, smem + kWkBm, smem + kWkCnt, nullptr, kHeavyLog2, c0, d, r1 - r0, c0 > r0, parts);
+                const int nw = row_words(R);
+                for (int i = threadIdx.x; i < nw; i += kWkBlock) R.bm[i] = 0u;
+                if (threadIdx.x == 0) s_next = 0;
                 __syncthreads();
-                int run = incl - s;
-                for (int i = 0; i < wib; i++) run += s_wsum[i];
-                for (int i = a; i < b; i++) {
-                    const uint32_t word = R.bm[i];
-                    R.bm[i] = word | ((uint32_t)run << 16);
-                    run += __popc(word);
+                row_fill(A, R, threadIdx.x, kWkBlock);
+                __syncthreads();
+                if (R.exact) {
+                    // running counts: each thread's run of words, then a block scan
+                    const int per = (nw + kWkBlock - 1) / kWkBlock;
+                    const int a = threadIdx.x * per, b = a + per < nw ? a + per : nw;
+                    int s = 0;
+                    for (int i = a; i < b; i++) s += __popc(R.bm[i]);
+                    const int incl = warp_incl_scan(s);
+                    if (lane == 31) s_wsum[wib] = incl;
+                    __syncthreads();
+                    int run = incl - s;
+                    for (int i = 0; i < wib; i++) run += s_wsum[i];
+                    for (int i = a; i < b; i++) {
+                        const uint32_t word = R.bm[i];
+                        R.bm[i] = word | ((uint32_t)run << 16);
+                        run += __popc(word);
+                    }
+                    __syncthreads();
+                }
+                for (;;) {
+                    int nx = 0;
+                    if (lane == 0) nx = atomicAdd(&s_next, kWarp);
+                    nx = __shfl_sync(kFull, nx, 0);
+                    if (ka + nx >= kb) break;
+                    const int64_t k = ka + nx + lane < kb ? ka + nx + lane : -1;
+                    if (R.exact) walk_in_edges<M, kRowExact>(A, R, Q, cols4, sh, list, out0, cap, k, 0, 0);
+                    else walk_in_edges<M, kRowHashed>(A, R, Q, cols4, sh, list, out0, cap, k, 0, 0);
                 }
                 __syncthreads();
+                if (M == kWalkCount) row_flush(A, R, threadIdx.x, kWkBlock);
+                __syncthreads();
             }
+        } else {
+            // ---- warp rows from the top rank down, one lane per row finding those
+            // with work: two at a time in the top quarter, where most of the work is
+            // (a long batch there left one warp running alone), then light_batch
+            const unsigned long long t1 = ((unsigned long long)A.nv + 3) / 4;
+            unsigned char* sl = smem + wib * kLtBytes;
             for (;;) {
-                int nx = 0;
-                if (lane == 0) nx = atomicAdd(&s_next, kWarp);
-                nx = __shfl_sync(kFull, nx, 0);
-                if (ka + nx >= kb) break;
-                const int64_t k = ka + nx + lane < kb ? ka + nx + lane : -1;
-                if (R.exact) walk_in_edges<M, kRowExact>(A, R, Q, ctl, cols4, sh, list, out0, cap, k, 0, 0);
-                else walk_in_edges<M, kRowHashed>(A, R, Q, ctl, cols4, sh, list, out0, cap, k, 0, 0);
-            }
-            __syncthreads();
-            if (M == kWalkCount) row_flush(A, R, threadIdx.x, kWkBlock);
-            __syncthreads();
-        }
-    }
-
-    // ---- warp rows from the top rank down, one lane per row finding those
-    // with work: two at a time in the top quarter, where most of the work is
-    // (a long batch there left one warp running alone), then light_batch
-    const unsigned long long t1 = ((unsigned long long)A.nv + 3) / 4;
-    unsigned char* sl = smem + wib * kLtBytes;
-    for (;;) {
-        unsigned long long t = 0;
-        if (lane == 0) t = atomicAdd(&ctl->light_next[M], 1ull);
-        t = __shfl_sync(kFull, t, 0);
-        const unsigned long long g1 = (t1 + kTopBatch - 1) / kTopBatch;
-        const int batch = t < g1 ? kTopBatch : light_batch;
-        const unsigned long long first = t < g1 ? t * kTopBatch : g1 * kTopBatch + (t - g1) * (unsigned)light_batch;
-        if (first >= (unsigned long long)A.nv) break;
-        const int64_t mine = A.nv - 1 - (int64_t)first - (int64_t)lane;
-        int64_t r0 = 0, i0 = 0;
-        int d = 0, din = 0;
-        if ((int)lane < batch && mine >= 0) {
-            r0 = __ldg(A.rp + mine);
-            i0 = __ldg(A.cp + mine);
-            const int64_t dout = __ldg(A.rp + mine + 1) - r0, di = __ldg(A.cp + mine + 1) - i0;
-            if (dout > 0 && di > 0 && !is_block_row(dout, di, A.warp_cap, A.light_in)) {
-                d = (int)dout;
-                din = (int)di;
-            }
-        }
-        // tiny rows: their in-edges, 32 at a time
-        const bool tiny = d > 0 && is_tiny_row(d, din);
-        if (__ballot_sync(kFull, tiny)) {
-            const int tn = tiny ? din : 0;
-            const int tincl = warp_incl_scan(tn);
-            const int ttotal = __shfl_sync(kFull, tincl, 31);
-            const int ts = tincl - tn;
-            for (int b = 0; b < ttotal; b += kWarp) {
-                const int at = b + (int)lane;
-                int own = 0;  // last lane with ts <= at
-#pragma unroll
-                for (int step = 16; step > 0; step >>= 1)
-                    if (__shfl_sync(kFull, ts, own + step) <= at) own += step;
-                const int64_t k = __shfl_sync(kFull, i0, own) + (at - __shfl_sync(kFull, ts, own));
-                const int64_t e0 = __shfl_sync(kFull, r0, own);
-                const int dr = __shfl_sync(kFull, d, own);
-                walk_in_edges<M, kRowTiny>(A, WalkRow{}, Q, ctl, cols4, sh, list, out0, cap, at < ttotal ? k : -1, e0, dr);
-            }
-        }
-        unsigned todo = __ballot_sync(kFull, d > 0 && !tiny);
-        while (todo) {
-            const int src = __ffs(todo) - 1;
-            todo &= todo - 1;
-            const int64_t e0 = __shfl_sync(kFull, r0, src), k0 = __shfl_sync(kFull, i0, src);
-            const int dr = __shfl_sync(kFull, d, src), dk = __shfl_sync(kFull, din, src);
-            WalkRow R = row_init(A, sl + kLtBm, sl + kLtCnt, sl + kLtPerm, kLightLog2, e0, dr, dr, false, false);
-            const int nw = row_words(R);
-            for (int i = lane; i < nw; i += kWarp) R.bm[i] = 0u;
-            __syncwarp();
-            row_fill(A, R, lane, kWarp);
-            __syncwarp();
-            int run = 0;
-            for (int b = 0; b < nw; b += kWarp) {
-                const int i = b + (int)lane;
-                const uint32_t word = i < nw ? R.bm[i] : 0u;
-                const int s = __popc(word);
-                const int incl = warp_incl_scan(s);
-                if (i < nw) R.bm[i] = word | ((uint32_t)(run + incl - s) << 16);
-                run += __shfl_sync(kFull, incl, 31);
-            }
-            __syncwarp();
-            if (R.exact) {
-                for (int k = lane; k - (int)lane < dk; k += kWarp)
-                    walk_in_edges<M, kRowExact>(A, R, Q, ctl, cols4, sh, list, out0, cap, k < dk ? k0 + k : -1, 0, 0);
-            } else {
-                for (int i = lane; i < dr; i += kWarp) {
-                    const uint32_t x = (uint32_t)(__ldg(A.cols + e0 + i) - R.wb) & R.mask;
-                    R.perm[word_rank(R.bm[x >> 4], x)] = (uint8_t)i;
+                unsigned long long t = 0;
+                if (lane == 0) t = atomicAdd(&ctl->light_next[M], 1ull);
+                t = __shfl_sync(kFull, t, 0);
+                const unsigned long long g1 = (t1 + kTopBatch - 1) / kTopBatch;
+                const int batch = t < g1 ? kTopBatch : light_batch;
+                const unsigned long long first = t < g1 ? t * kTopBatch : g1 * kTopBatch + (t - g1) * (unsigned)light_batch;
+                if (first >= (unsigned long long)A.nv) break;
+                const int64_t mine = A.nv - 1 - (int64_t)first - (int64_t)lane;
+                int64_t r0 = 0, i0 = 0;
+                int d = 0, din = 0;
+                if ((int)lane < batch && mine >= 0) {
+                    r0 = __ldg(A.rp + mine);
+                    i0 = __ldg(A.cp + mine);
+                    const int64_t dout = __ldg(A.rp + mine + 1) - r0, di = __ldg(A.cp + mine + 1) - i0;
+                    if (dout > 0 && di > 0 && !is_block_row(dout, di, A.warp_cap, A.light_in)) {
+                        d = (int)dout;
+                        din = (int)di;
+                    }
                 }
-                __syncwarp();
-                for (int k = lane; k - (int)lane < dk; k += kWarp)
-                    walk_in_edges<M, kRowHashed>(A, R, Q, ctl, cols4, sh, list, out0, cap, k < dk ? k0 + k : -1, 0, 0);
+                // tiny rows: their in-edges, 32 at a time
+                const bool tiny = d > 0 && is_tiny_row(d, din);
+                if (__ballot_sync(kFull, tiny)) {
+                    const int tn = tiny ? din : 0;
+                    const int tincl = warp_incl_scan(tn);
+                    const int ttotal = __shfl_sync(kFull, tincl, 31);
+                    const int ts = tincl - tn;
+                    for (int b = 0; b < ttotal; b += kWarp) {
+                        const int at = b + (int)lane;
+                        int own = 0;  // last lane with ts <= at
+        #pragma unroll
+                        for (int step = 16; step > 0; step >>= 1)
+                            if (__shfl_sync(kFull, ts, own + step) <= at) own += step;
+                        const int64_t k = __shfl_sync(kFull, i0, own) + (at - __shfl_sync(kFull, ts, own));
+                        const int64_t e0 = __shfl_sync(kFull, r0, own);
+                        const int dr = __shfl_sync(kFull, d, own);
+                        walk_in_edges<M, kRowTiny>(A, WalkRow{}, Q, cols4, sh, list, out0, cap, at < ttotal ? k : -1, e0, dr);
+                    }
+                }
+                unsigned todo = __ballot_sync(kFull, d > 0 && !tiny);
+                while (todo) {
+                    const int src = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    const int64_t e0 = __shfl_sync(kFull, r0, src), k0 = __shfl_sync(kFull, i0, src);
+                    const int dr = __shfl_sync(kFull, d, src), dk = __shfl_sync(kFull, din, src);
+                    WalkRow R = row_init(A, sl + kLtBm, sl + kLtCnt, sl + kLtPerm, kLightLog2, e0, dr, dr, false, false);
+                    const int nw = row_words(R);
+                    for (int i = lane; i < nw; i += kWarp) R.bm[i] = 0u;
+                    __syncwarp();
+                    row_fill(A, R, lane, kWarp);
+                    __syncwarp();
+                    int run = 0;
+                    for (int b = 0; b < nw; b += kWarp) {
+                        const int i = b + (int)lane;
+                        const uint32_t word = i < nw ? R.bm[i] : 0u;
+                        const int s = __popc(word);
+                        const int incl = warp_incl_scan(s);
+                        if (i < nw) R.bm[i] = word | ((uint32_t)(run + incl - s) << 16);
+                        run += __shfl_sync(kFull, incl, 31);
+                    }
+                    __syncwarp();
+                    if (R.exact) {
+                        for (int k = lane; k - (int)lane < dk; k += kWarp)
+                            walk_in_edges<M, kRowExact>(A, R, Q, cols4, sh, list, out0, cap, k < dk ? k0 + k : -1, 0, 0);
+                    } else {
+                        for (int i = lane; i < dr; i += kWarp) {
+                            const uint32_t x = (uint32_t)(__ldg(A.cols + e0 + i) - R.wb) & R.mask;
+                            R.perm[word_rank(R.bm[x >> 4], x)] = (uint8_t)i;
+                        }
+                        __syncwarp();
+                        for (int k = lane; k - (int)lane < dk; k += kWarp)
+                            walk_in_edges<M, kRowHashed>(A, R, Q, cols4, sh, list, out0, cap, k < dk ? k0 + k : -1, 0, 0);
+                    }
+                    if (M == kWalkCount) row_flush(A, R, lane, kWarp);
+                    __syncwarp();
+                }
             }
-            if (M == kWalkCount) row_flush(A, R, lane, kWarp);
-            __syncwarp();
         }
+        walk_long_tails<M>(A, Q, list, out0, cap);
+        if (last) break;
     }
-    walk_long_tails<M>(A, Q, list, out0, cap);
 }
 
 // Roles B and C from the role-A entries (eB, eC) of eA = (u,v):
@@ -1089,8 +1080,8 @@ static WalkArgs walk_args(const int64_t* rp, const int32_t* cols, const int64_t*
 // needs no more than stage_slots, the role-A entries in their staging slots,
 // which end at stage_end; *stage_skip receives the choice.  cA, cB, cC and ctl
 // are zeroed by the caller.  units: 16 E bytes of scratch that stays as
-// the list walk's plan; runA: int32[E] and longs: 16 E bytes of scratch; ctl:
-// 256 bytes.
+// the list walk's plan; runA: int32[E] and longs: uint32[E] scratch; ctl: 256
+// bytes.
 int launch_walk_count(const int64_t* rp, const int32_t* cols, const int64_t* cp, const int32_t* in_src,
                       const int32_t* in_eid, int64_t nv, int64_t ne, int32_t* cA, int32_t* cB, int32_t* cC,
                       const int64_t* sbase, int2* stage_end, unsigned long long stage_slots, int* stage_skip,
@@ -1112,7 +1103,7 @@ int launch_walk_count(const int64_t* rp, const int32_t* cols, const int64_t* cp,
     A.out = stage_end;
     A.stage_skip = stage_skip;
     A.runA = runA;
-    A.longs = reinterpret_cast<int2*>(longs);
+    A.longs = reinterpret_cast<uint32_t*>(longs);
     return launch_walk<kWalkCount>(A, reinterpret_cast<WalkCtl*>(ctl), st);
 }
 
@@ -1127,7 +1118,7 @@ int launch_walk_list(const int64_t* rp, const int32_t* cols, const int64_t* cp, 
     A.off = off;
     A.out = lists;
     A.runA = runA;
-    A.longs = reinterpret_cast<int2*>(longs);
+    A.longs = reinterpret_cast<uint32_t*>(longs);
     return launch_walk<kWalkList>(A, reinterpret_cast<WalkCtl*>(ctl), st);
 }
 

@@ -41,17 +41,25 @@ def _tail(n, d):
     return np.concatenate([np.stack([np.zeros_like(i), i], 1), np.stack([np.ones(d, np.int64), i[n - d:]], 1)])
 
 
+def _bipartite(n):
+    """n x n joined, and a path through the second half: block rows of one entry."""
+    a, b = np.meshgrid(np.arange(n), n + np.arange(n))
+    i = n + np.arange(n - 1)
+    return np.concatenate([np.stack([a.ravel(), b.ravel()], 1), np.stack([i, i + 1], 1)])
+
+
 GRAPHS = {
     "wheel": (lambda: _wheel(12000), 12000),
     "hubs": (lambda: _hubs(6000, 40, 30000, 1), 6040),       # several runs a warp, rows of all kinds
     "hubs_dense": (lambda: _hubs(9000, 3, 400000, 2), 9003),  # block rows with long tails
-    "tail_512": (lambda: _tail(513, 2), 514),                 # the longest tail that is streamed
-    "tail_513": (lambda: _tail(514, 2), 515),
-    "ratio_at": (lambda: _tail(8 * 80 + 1, 80), 8 * 80 + 2),
-    "ratio_past": (lambda: _tail(8 * 80 + 2, 80), 8 * 80 + 3),
-    "warp_row": (lambda: _tail(8 * 256 + 2, 256), 8 * 256 + 3),
-    "block_row": (lambda: _tail(8 * 257 + 2, 257), 8 * 257 + 3),
-    "chunked_row": (lambda: _tail(8 * 5000 + 2, 5000), 8 * 5000 + 3),
+    "tail_128": (lambda: _tail(129, 2), 130),                 # the longest tail that is streamed
+    "tail_129": (lambda: _tail(130, 2), 131),
+    "ratio_at": (lambda: _tail(4 * 80 + 1, 80), 4 * 80 + 2),
+    "ratio_past": (lambda: _tail(4 * 80 + 2, 80), 4 * 80 + 3),
+    "warp_row": (lambda: _tail(4 * 256 + 2, 256), 4 * 256 + 3),
+    "block_row": (lambda: _tail(4 * 257 + 2, 257), 4 * 257 + 3),
+    "chunked_row": (lambda: _tail(4 * 5000 + 2, 5000), 4 * 5000 + 3),
+    "bipartite": (lambda: _bipartite(300), 600),
 }
 
 
