@@ -60,11 +60,10 @@ constexpr int kWalkKeys = 256;                 // keys per pass, load factor <= 
 constexpr int kWalkSlots = 2 * kWalkKeys;
 constexpr int kWalkMinLog2 = 6;
 constexpr int kWalkQueue = 64;                 // a push adds up to 32 to at most 31
-// A key of a simple graph is hit once per entry of a run, 32 times at most; rows
-// with copies of a column hit it more often, and the lane whose hit makes a count
-// of kHitsFull hands those on (up to 31 others count on meanwhile).  The update
-// of R-MAT scale 17 283 -> 285 us; handed on every 65,408 entries instead, 286.
-constexpr unsigned kHitsFull = 0x8000u;
+// Chunks of a run that is walked in groups: should all its entries be copies of one
+// column, the count of their key fits 16 bits.
+constexpr unsigned kWalkChunks = 65536 / 4 - 1;
+constexpr int kLongRow = 512, kLongRatio = 2;
 
 struct EdgeWalkShared {
     int32_t key[kWalkSlots];
@@ -73,15 +72,133 @@ struct EdgeWalkShared {
     uint2 queue[kWalkQueue];                   // ring: column, place in the run and offset in N+(v)
     uint32_t start[kWarp];                     // first chunk again
     int32_t cnt[kWarp];                        // by group lane
-    uint32_t hits[kWalkKeys / 2];              // of each staged key, 16 bits (kHitsFull of them are handed on)
+    uint32_t hits[kWalkKeys / 2];              // of each staged key, 16 bits
     uint16_t pos[kWalkSlots];                  // key index, and the flag of its edge in bit 15
 };
+
+// A table of up to kWalkKeys keys: log2 of its slots.
+__device__ __forceinline__ int walk_table_log2(int d) {
+    int lg = 33 - __clz(d);  // 2 d rounded up to a power of two, or the next one
+    if (2 * d == 1 << (lg - 1)) lg--;
+    return lg < kWalkMinLog2 ? kWalkMinLog2 : lg;
+}
+
+// A run whose N+(u) = [bu, eu) is long and kLongRatio times as long as its rows
+// together (orders that are not degree ranks: a hub that ranks low), or one row
+// past kWalkChunks: the keys of the rows are staged, piece by piece, each with its
+// place in their flat space, and N+(u) is streamed.  Staged in pieces itself,
+// such a row was streamed through once per 256 of its own keys.  Wheel of 200 K
+// vertices, hub at id 0, update of 100 / 40,000 edges: 3.6 / 8.1 -> 1.1 / 2.5 ms
+// (one edge at a time, the shorter row hashed: 1.5 / 4.5); 96 K vertices in
+// cliques of 12 under such a hub 1.7 / 2.0 -> 0.53 / 0.78.  Longer rows or larger
+// ratios as the line (1,024, 4,096; 8) measured the same.  In a turn of its own
+// over the warp's groups: in the loop above it cost the update of R-MAT scale 17
+// 1.8 %, as a call 10.
+template <class Mark, class Hit, class Row>
+__device__ __forceinline__ void walk_long_run(const int32_t* __restrict__ cols, EdgeWalkShared& S, unsigned run,
+                                              int32_t bv, int32_t lv, unsigned marked, int64_t bu, int64_t eu,
+                                              Mark&& mark, Hit&& hit, Row&& row) {
+    const unsigned lane = lane_id(), lt = lanemask_lt();
+    const unsigned shift = (unsigned)((uintptr_t)cols >> 2) & 3u;
+    const int4* __restrict__ cols4 = reinterpret_cast<const int4*>(cols - shift);
+    const bool mine = (run >> lane) & 1u;
+    const unsigned incl = warp_incl_scan(mine ? (unsigned)lv : 0u);  // rows of different heads, or one: below 2^31
+    const unsigned keys = __shfl_sync(kFull, incl, 31);
+    const int places = __popc(run);
+    if (mine) {  // by place in the run: keys before the row's, its first edge, its group lane
+        const int k = __popc(run & lt);
+        S.start[k] = incl - (unsigned)lv;
+        S.row[k] = make_uint4(0u, (unsigned)bv, 0u, lane);
+    }
+    __syncwarp();
+    auto place_of = [&](unsigned f) {
+        int o = 0;
+#pragma unroll
+        for (int step = kWarp / 2; step > 0; step >>= 1)
+            if (o + step < places && S.start[o + step] <= f) o += step;
+        return o;
+    };
+    const unsigned ulo = (unsigned)bu + shift, uhi = (unsigned)eu + shift;
+    const unsigned b0 = ulo >> 2, b1 = (uhi + 3) >> 2;
+    for (unsigned c = 0; c < keys; c += kWalkKeys) {
+        const int d = (int)(keys - c < kWalkKeys ? keys - c : kWalkKeys);
+        const int lg = walk_table_log2(d);
+        const unsigned slots = 1u << lg;
+        for (unsigned k = lane; k < slots / 4; k += kWarp) {
+            reinterpret_cast<int4*>(S.key)[k] = make_int4(kEmpty, kEmpty, kEmpty, kEmpty);
+            S.bm[k] = 0u;
+        }
+        __syncwarp();
+        for (int k = lane; k < d; k += kWarp) {
+            const int o = place_of(c + k);
+            const int32_t key = __ldg(cols + (int64_t)S.row[o].y + (c + k - S.start[o]));
+            if (key < 0) continue;
+            const unsigned h = (unsigned)key * 2654435761u;
+            const unsigned bit = h >> (29 - lg);
+            atomicOr(S.bm + (bit >> 5), 1u << (bit & 31));
+            unsigned slot = h >> (32 - lg);
+            while (atomicCAS(&S.key[slot], kEmpty, key) != kEmpty) slot = (slot + 1) & (slots - 1);
+            S.pos[slot] = (uint16_t)k;
+        }
+        __syncwarp();
+        int nq = 0;
+        // look up the last m queue entries, one per lane: a key may be of several rows
+        auto resolve = [&](int m) {
+            __syncwarp();
+            if ((int)lane < m) {
+                const uint2 q = S.queue[nq - m + lane];
+                const int64_t pb = (int64_t)q.y - shift;
+                const bool mb = mark(pb);
+                unsigned slot = (q.x * 2654435761u) >> (32 - lg);
+                for (int32_t k = S.key[slot]; k != kEmpty; k = S.key[slot]) {
+                    if (k == (int32_t)q.x) {
+                        const unsigned f = c + S.pos[slot];
+                        const int o = place_of(f);
+                        const uint4 r = S.row[o];
+                        const unsigned c2 = hit((marked >> r.w) & 1u, (int64_t)r.y + (f - S.start[o]), mb);
+                        if (c2 & 1u) atomicAdd(&S.cnt[r.w], 1);
+                        if (c2 & 2u) row(pb, 1);
+                    }
+                    slot = (slot + 1) & (slots - 1);
+                }
+            }
+            __syncwarp();
+            nq -= m;
+        };
+        for (unsigned b = b0; b < b1; b += kWarp) {
+            const unsigned c4 = b + lane;
+            unsigned cm = 0;
+            int4 x4 = make_int4(0, 0, 0, 0);
+            if (c4 < b1) {
+                x4 = __ldg(cols4 + c4);
+                auto test = [&](int32_t x) {
+                    const unsigned t = ((unsigned)x * 2654435761u) >> (29 - lg);
+                    return (S.bm[t >> 5] >> (t & 31)) & 1u;
+                };
+                cm = test(x4.x) | test(x4.y) << 1 | test(x4.z) << 2 | test(x4.w) << 3;
+                if (4 * c4 < ulo) cm &= 0xFu << (ulo - 4 * c4);
+                if (4 * c4 + 4 > uhi) cm &= 0xFu >> (4 * c4 + 4 - uhi);
+            }
+#pragma unroll 1
+            for (int q = 0; q < 4; q++) {
+                const int32_t x = q == 0 ? x4.x : q == 1 ? x4.y : q == 2 ? x4.z : x4.w;
+                const bool cand = ((cm >> q) & 1u) && x >= 0;
+                const unsigned m = __ballot_sync(kFull, cand);
+                if (cand) S.queue[nq + __popc(m & lt)] = make_uint2((unsigned)x, 4 * c4 + (unsigned)q);
+                nq += __popc(m);
+                const bool end = q == 3 && b + kWarp >= b1;
+                while (nq >= kWarp || (end && nq > 0)) resolve(nq < kWarp ? nq : kWarp);
+            }
+        }
+    }
+}
 
 // list(i): the edge of entry i, or -1.  mark(e): flag of an edge.  hit(me, pa,
 // mb): a common column, at position pa of N+(v) and an edge of u with flag mb;
 // bit 0 of the result counts it for the entry's edge, bit 1 for the edge of u.
-// row(pb, count) and done(e, count), count > 0: the counts of the edges of u, at
-// the end of a staged piece at the latest, and of the entries.
+// row(pb, count) and done(e, count), count > 0: the counts of the edges of u, once
+// per staged piece (of a long run hit by hit), and of the entries.  Long runs wait
+// for a second turn over the warp's groups.
 template <class List, class Mark, class Hit, class Row, class Done>
 __device__ __forceinline__ void walk_edges(const int32_t* __restrict__ rows, const int32_t* __restrict__ cols,
                                            const RowView& rv, int64_t n, int group, EdgeWalkShared& S, List&& list,
@@ -91,11 +208,14 @@ __device__ __forceinline__ void walk_edges(const int32_t* __restrict__ rows, con
     const unsigned shift = (unsigned)((uintptr_t)cols >> 2) & 3u;
     const int4* __restrict__ cols4 = reinterpret_cast<const int4*>(cols - shift);
     const int64_t nw = (int64_t)gridDim.x * (kOpsBlock / kWarp);
-    for (int64_t g = blockIdx.x * (int64_t)(kOpsBlock / kWarp) + threadIdx.x / kWarp; g * group < n; g += nw) {
+    const int64_t g0 = blockIdx.x * (int64_t)(kOpsBlock / kWarp) + threadIdx.x / kWarp;
+    // a group's entries, one a lane (true: of a row that is to be walked)
+    auto entry = [&](int64_t g, int64_t& e, int32_t& u, int32_t& bv, int32_t& lv, bool& me) {
         const int64_t i = g * group + lane;
-        int64_t e = -1;
-        int32_t u = -1, bv = 0, lv = 0;
-        bool me = false;
+        e = -1;
+        u = -1;
+        bv = lv = 0;
+        me = false;
         if ((int)lane < group && i < n) {
             e = list(i);
             if (e >= 0 && e < rv.n_edges) {
@@ -109,32 +229,59 @@ __device__ __forceinline__ void walk_edges(const int32_t* __restrict__ rows, con
             }
         }
         S.cnt[lane] = 0;
+    };
+    // the lanes of todo with the source of the first of them, and the chunks of
+    // their rows: all of them, or the first where they are too many
+    auto next_run = [&](unsigned todo, int32_t u, int32_t bv, int32_t lv, bool wide, int32_t& ur, int32_t& start,
+                        unsigned& total) {
+        const int first = __ffs(todo) - 1;
+        ur = __shfl_sync(kFull, u, first);
+        const unsigned lo = (unsigned)bv + shift, hi = lo + (unsigned)lv;
+        const int32_t chunks = (int32_t)(((hi + 3) >> 2) - (lo >> 2));
+        unsigned run = wide ? 1u << first : __ballot_sync(kFull, u == ur) & todo;
+        const int32_t len = (run >> lane) & 1u ? chunks : 0;
+        const int32_t incl = warp_incl_scan(len);
+        start = incl - len;
+        total = (unsigned)__shfl_sync(kFull, incl, 31);
+        if (total > kWalkChunks && !wide) {
+            run = 1u << first;
+            start = 0;
+            total = (unsigned)__shfl_sync(kFull, chunks, first);
+        }
+        return run;
+    };
+    auto is_long = [&](int64_t du, unsigned total) {
+        return total > kWalkChunks || (du > kLongRow && du / (4 * kLongRatio) > (int64_t)total);
+    };
+    bool longs = false;
+    for (int64_t g = g0; g * group < n; g += nw) {
+        int64_t e;
+        int32_t u, bv, lv;
+        bool me;
+        entry(g, e, u, bv, lv, me);
         const unsigned marked = __ballot_sync(kFull, me);
         const bool wide = __any_sync(kFull, lv >= (1 << 26));  // 32 of them might overflow a start
         unsigned todo = __ballot_sync(kFull, lv > 0);
         while (todo) {
-            const int first = __ffs(todo) - 1;
-            const int32_t ur = __shfl_sync(kFull, u, first);
-            const unsigned run = wide ? 1u << first : __ballot_sync(kFull, u == ur) & todo;
+            int32_t ur, start;
+            unsigned total;
+            const unsigned run = next_run(todo, u, bv, lv, wide, ur, start, total);
             todo &= ~run;
-            const bool mine = (run >> lane) & 1u;
-            const unsigned lo = (unsigned)bv + shift, hi = lo + (unsigned)lv;
-            const int32_t len = mine ? (int32_t)(((hi + 3) >> 2) - (lo >> 2)) : 0;
-            const int32_t incl = warp_incl_scan(len);
-            const unsigned total = (unsigned)__shfl_sync(kFull, incl, 31);
-            if (mine) {
+            const int64_t bu = rv.begin(ur), eu = rv.end(ur);
+            if (is_long(eu - bu, total)) {
+                longs = true;
+                continue;
+            }
+            if ((run >> lane) & 1u) {
                 const int k = __popc(run & lt);
-                S.start[k] = (unsigned)(incl - len);
-                S.row[k] = make_uint4((unsigned)(incl - len), lo, hi, lane);
+                const unsigned lo = (unsigned)bv + shift;
+                S.start[k] = (unsigned)start;
+                S.row[k] = make_uint4((unsigned)start, lo, lo + (unsigned)lv, lane);
             }
             const int nrun = __popc(run);
-            const int off_shift = wide ? 0 : 5;  // a wide row is alone in its run
-            const int64_t bu = rv.begin(ur), eu = rv.end(ur);
             for (int64_t c = bu; c < eu; c += kWalkKeys) {
                 const int d = (int)(eu - c < kWalkKeys ? eu - c : kWalkKeys);
-                int lg = 33 - __clz(d);  // 2 d rounded up to a power of two, or the next one
-                if (2 * d == 1 << (lg - 1)) lg--;
-                lg = lg < kWalkMinLog2 ? kWalkMinLog2 : lg;
+                const int lg = walk_table_log2(d);
                 const unsigned slots = 1u << lg;
                 for (unsigned k = lane; k < slots / 4; k += kWarp) {
                     reinterpret_cast<int4*>(S.key)[k] = make_int4(kEmpty, kEmpty, kEmpty, kEmpty);
@@ -161,7 +308,7 @@ __device__ __forceinline__ void walk_edges(const int32_t* __restrict__ rows, con
                     if ((int)lane < m) {
                         const uint2 q = S.queue[(head + lane) & (kWalkQueue - 1)];
                         const int32_t x = (int32_t)q.x;
-                        const uint4 r = S.row[wide ? 0u : q.y & 31u];
+                        const uint4 r = S.row[q.y & 31u];
                         unsigned slot = (q.x * 2654435761u) >> (32 - lg);
                         int32_t k = S.key[slot];
                         while (k != x && k != kEmpty) {
@@ -170,17 +317,10 @@ __device__ __forceinline__ void walk_edges(const int32_t* __restrict__ rows, con
                         }
                         if (k == x) {
                             const unsigned kb = S.pos[slot], at = kb & 0x7fffu;
-                            const int64_t pa = (int64_t)r.y + (q.y >> off_shift) - shift;
+                            const int64_t pa = (int64_t)r.y + (q.y >> 5) - shift;
                             const unsigned c2 = hit((marked >> r.w) & 1u, pa, (bool)(kb >> 15));
                             if (c2 & 1u) atomicAdd(&S.cnt[r.w], 1);
-                            if (c2 & 2u) {
-                                const unsigned sh = 16 * (at & 1u);
-                                const unsigned n = ((atomicAdd(&S.hits[at >> 1], 1u << sh) >> sh) & 0xffffu) + 1u;
-                                if (n == kHitsFull) {
-                                    atomicSub(&S.hits[at >> 1], kHitsFull << sh);
-                                    row(c + at, (int32_t)kHitsFull);
-                                }
-                            }
+                            if (c2 & 2u) atomicAdd(&S.hits[at >> 1], 1u << (16 * (at & 1u)));
                         }
                     }
                     __syncwarp();
@@ -211,7 +351,7 @@ __device__ __forceinline__ void walk_edges(const int32_t* __restrict__ rows, con
                         cm = test(x4.x) | test(x4.y) << 1 | test(x4.z) << 2 | test(x4.w) << 3;
                         if (p0 < r.y) cm &= 0xFu << (r.y - p0);
                         if (p0 + 4 > r.z) cm &= 0xFu >> (p0 + 4 - r.z);
-                        ent = ((p0 - r.y) << off_shift) + (unsigned)o;
+                        ent = ((p0 - r.y) << 5) + (unsigned)o;
                     }
                     ob += nb + (Bn == base + kWarp ? 1 : 0);
                     const int32_t xs[4] = {x4.x, x4.y, x4.z, x4.w};
@@ -221,7 +361,7 @@ __device__ __forceinline__ void walk_edges(const int32_t* __restrict__ rows, con
                         const unsigned m = __ballot_sync(kFull, cand);
                         if (cand)
                             S.queue[(head + nq + __popc(m & lt)) & (kWalkQueue - 1)] =
-                                make_uint2((unsigned)xs[q], ent + ((unsigned)q << off_shift));
+                                make_uint2((unsigned)xs[q], ent + ((unsigned)q << 5));
                         nq += __popc(m);
                         if (nq >= kWarp) resolve(kWarp);
                     }
@@ -234,6 +374,28 @@ __device__ __forceinline__ void walk_edges(const int32_t* __restrict__ rows, con
                 }
                 __syncwarp();
             }
+        }
+        const int32_t count = S.cnt[lane];
+        if (count > 0) done(e, count);
+        __syncwarp();
+    }
+    if (!longs) return;
+    for (int64_t g = g0; g * group < n; g += nw) {
+        int64_t e;
+        int32_t u, bv, lv;
+        bool me;
+        entry(g, e, u, bv, lv, me);
+        const unsigned marked = __ballot_sync(kFull, me);
+        const bool wide = __any_sync(kFull, lv >= (1 << 26));
+        unsigned todo = __ballot_sync(kFull, lv > 0);
+        while (todo) {
+            int32_t ur, start;
+            unsigned total;
+            const unsigned run = next_run(todo, u, bv, lv, wide, ur, start, total);
+            todo &= ~run;
+            const int64_t bu = rv.begin(ur), eu = rv.end(ur);
+            if (is_long(eu - bu, total)) walk_long_run(cols, S, run, bv, lv, marked, bu, eu, mark, hit, row);
+            __syncwarp();
         }
         const int32_t count = S.cnt[lane];
         if (count > 0) done(e, count);
