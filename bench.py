@@ -755,8 +755,14 @@ def bench_served_small(dev, srv, num_graphs=4096, rate=20000.0):
 # is its rate x T.  Reported beside the algorithmic bytes, never used for them.
 TRAFFIC_PER_TRIANGLE = {"support": 25.4, "listing": 60.1, "peel": 48.5}
 TRAFFIC_SOURCE = ("ncu capture (dram__bytes_read.sum + dram__bytes_write.sum) of one R-MAT scale-20 "
-                  "decomposition, scaled per triangle; at scale 22, where the supports no longer fit in L2, "
-                  "the peel moves more than that")
+                  "decomposition, scaled per triangle")
+# The same bytes of one decomposition of R-MAT scale 22, edge factor 16, from
+# one-pass captures of its main kernels (in-adjacency and walk 80.4 GB, state 1.5;
+# list offsets 0.7, distribution 68.5 + 69.1; peel 116.2): at this size the
+# supports no longer fit in L2, so the rates of scale 20 fall short.
+TRAFFIC_BY_WORKLOAD = {(22, 16): {"support": 82.0e9, "listing": 138.3e9, "peel": 116.2e9}}
+TRAFFIC_SOURCE_BY_WORKLOAD = ("ncu one-pass captures (dram__bytes_read.sum + dram__bytes_write.sum) of the main "
+                              "kernels of one decomposition of this workload")
 
 
 
@@ -882,8 +888,8 @@ def main_ours(args):
     t_sup, t_list, t_peel, t_post = (phases[k] / n for k in range(4))
     # the decomposition's algorithmic bytes B_dec = 2 B_sup: the support pass,
     # then one re-enumeration of each edge's triangles (listing + peel)
-    mt = {k: v * res.triangles for k, v in TRAFFIC_PER_TRIANGLE.items()}
-    traffic_src = TRAFFIC_SOURCE
+    mt = TRAFFIC_BY_WORKLOAD.get((scale, ef)) or {k: v * res.triangles for k, v in TRAFFIC_PER_TRIANGLE.items()}
+    traffic_src = TRAFFIC_SOURCE_BY_WORKLOAD if (scale, ef) in TRAFFIC_BY_WORKLOAD else TRAFFIC_SOURCE
     if res.listing != 2:
         # the captures behind these figures are of the one-walk listed path
         mt, traffic_src = None, "not captured for this path"

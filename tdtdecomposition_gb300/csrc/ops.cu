@@ -48,14 +48,15 @@ struct RowView {
 // OR-reduction of the row starts inside the step).  A chunk that holds an entry
 // is mapped as a whole, so any alignment of cols will do.  Most entries miss the
 // bitmap; the others go to a queue and are looked up 32 at a time.  Rows of more
-// than kWalkKeys keys are staged in pieces.
+// than kWalkKeys keys are staged in pieces, or, where they are far longer than the
+// run's N+(v) together, streamed (walk_long_run).
 //
 // Bound by issuing the tests.  One edge at a time, its shorter list hashed and
 // the longer one streamed, the update of 0.87 M of 1.86 M edges (R-MAT scale 17,
 // 109 M entries of N+(v)) took 540 us; in groups 416, with the counts of N+(u)
 // kept in shared memory 431, in chunks of four columns 302 (2.4 M edges of a
 // Chung-Lu graph 1,161 -> 564, the saturating support of all of scale 17
-// 1,748 -> 770).  Tables of 128 keys and more blocks per SM: 317.
+// 1,748 -> 770; without a case for wide rows in the loop 281).  Tables of 128 keys and more blocks per SM: 317.
 constexpr int kWalkKeys = 256;                 // keys per pass, load factor <= 1/2
 constexpr int kWalkSlots = 2 * kWalkKeys;
 constexpr int kWalkMinLog2 = 6;
@@ -433,7 +434,7 @@ __global__ void segment_add_kernel(const int32_t* __restrict__ vals, const int32
 // long segment spreads over many warps and a slab of short ones stays in one;
 // one atomic per (slab, segment).  Bound by reading the values; one 64-bit
 // atomic per value on the segments' addresses (14 M values, 512 segments) took
-// 5.6 ms of an 11.7 ms batch, which takes 5.9 ms with this kernel.
+// 5.6 ms of an 11.7 ms batch, which took 5.9 ms with this kernel (4.7 ms now).
 constexpr int kSegMaxUnroll = 4;
 
 __global__ void __launch_bounds__(kOpsBlock) segment_max_kernel(const int32_t* __restrict__ vals,

@@ -482,7 +482,7 @@ __device__ __forceinline__ void pass_min(const PeelArgs& A, int np, int32_t v) {
 // died; until then its dead entries cost a code word each, and until the first
 // rewrite the list is every edge id and is not read at all.  Level changes are
 // bound by these passes on large graphs: rewritten every time 19.1 ms at R-MAT
-// scale 22 (546 levels), 5.7 at 20, 0.99 at 16; now 14.2, 4.7 and 0.83 (a third
+// scale 22 (307 level changes), 5.7 at 20, 0.99 at 16; now 14.2, 4.7 and 0.83 (a third
 // instead of an eighth: 14.7, 4.7, 0.81).
 constexpr int kListSlack = 8;
 
@@ -1405,9 +1405,10 @@ __device__ __forceinline__ void compact_rows(const PeelArgs& A, int r, bool whol
 // kListed: the caller gave a list tail, and whether the lists fit is decided on
 // the device (search otherwise).  Without a tail the search peels have kernels,
 // and their registers, of their own (Chung-Lu, 1 M vertices, without
-// compaction: 121 -> 104 ms).  A fixed level does not compact: most of its work
-// is its first sub-rounds (k = 10 / 100 at R-MAT scale 20 6.7 / 40.0 ms, with
-// compaction 7.0 / 41.7).
+// compaction: 121 -> 104 ms).  A fixed level does not compact: at most levels its
+// work is its first sub-rounds (k = 10 / 100 at R-MAT scale 20 6.7 / 40.0 ms, with
+// compaction 7.0 / 41.7; k = 200 58.2 / 56.3, kmax 58.9 / 60.7; Chung-Lu, 1 M
+// vertices, at kmax 33.9 / 32.1).
 template <int Mode>
 __global__ void __launch_bounds__(kPeelBlock, TDT_PEEL_MINB) peel_kernel(const __grid_constant__ PeelArgs A) {
     __shared__ int32_t s_app_e[kPeelWarps * kAppBuf];  // per-warp append staging

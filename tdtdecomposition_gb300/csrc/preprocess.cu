@@ -22,7 +22,7 @@
 // ran out leaves keys that are none (sort.cuh).
 // Each sort's digit totals are taken by the kernel that makes its keys.  67 M /
 // 65,536 draws: 10.6 ms / 560 us in 108 / 73 launches with five launches a sort
-// pass and an atomic per degree and row count, 7.6 ms / 312 us in 29 / 21.
+// pass and an atomic per degree and row count, 6.3 ms / 246 us in 26 / 18.
 #include "common.cuh"
 #include "sort.cuh"
 

@@ -4,7 +4,10 @@
 // looking back over the tiles before it (tiles are handed out in order, so the
 // tiles waited for are running).  The scan is one launch instead of three; a
 // sort pass is one launch instead of five, and reads its keys once instead of
-// twice, with no digit table of all tiles to scan between.  A pass over 67 M
+// twice, with no digit table of all tiles to scan between.  The methods are
+// published: the scan with look-back by Merrill and Garland (Single-pass Parallel
+// Prefix Scan with Decoupled Look-back, 2016), the sort by Adinets and Merrill
+// (Onesweep: A Faster Least Significant Digit Radix Sort for GPUs, 2022).  A pass over 67 M
 // 64-bit keys: 600 -> 400 us, 350 with the ballots below (bound: 16 bytes a
 // key, 160 us).
 #include "sort.cuh"

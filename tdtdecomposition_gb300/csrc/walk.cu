@@ -45,9 +45,9 @@
 // count walk is followed by a list walk.
 //
 // Measured at R-MAT scale 20 / 22 (support + listing, against a walk from the
-// source with staged entries, compaction and transposition): 21.5 -> 14.3 ms,
-// 106 -> 76 ms; the count alone, with its in-adjacency, at scale 21: 19.3 ->
-// 9.4 ms.  The walk issues 2.6 instructions a cycle per SM (scale 20: 4.1 ms,
+// source with staged entries, compaction and transposition): 21.5 -> 13.7 ms,
+// 106 -> 73.6 ms; the count alone, with its in-adjacency, at scale 21: 19.3 ->
+// 7.7 ms.  The walk issues 2.6 instructions a cycle per SM (scale 20: 4.1 ms,
 // DRAM 29 %); the regrouping moves 13 GB in 4 ms per role.
 #include "common.cuh"
 #include "sort.cuh"
