@@ -298,7 +298,8 @@ __device__ __forceinline__ void walk_long_tails(const WalkArgs& A, const WalkGro
     uint32_t k = Q.longs[lane];
     Q.longs[lane] = kNoEdge;
     while (__any_sync(kFull, k != kNoEdge)) {
-        int32_t eid = 0, n = 0;
+        int32_t eid = 0;
+        uint32_t n = 0;
         int64_t end = 0, e0 = 0;
         const bool mine = k != kNoEdge;
         if (mine) {
@@ -307,17 +308,18 @@ __device__ __forceinline__ void walk_long_tails(const WalkArgs& A, const WalkGro
             k = A.longs[k];
             const int32_t v = __ldg(A.cols + eid);
             e0 = __ldg(A.rp + v);
-            n = (int32_t)(__ldg(A.rp + v + 1) - e0);
+            n = (uint32_t)(__ldg(A.rp + v + 1) - e0);
             end = __ldg(A.rp + u + 1);
             if (list) Q.off[lane] = role_a_slot<M>(A, eid, u, __ldg(A.rp + u), end);
             Q.cnt[lane] = 0u;
         }
         __syncwarp();
-        // pairs (u,v) differ and a tail is longer than its row: at most E in all
-        const int32_t incl = warp_incl_scan(n);
-        const int32_t total = __shfl_sync(kFull, incl, 31), S = incl - n;
-        for (int32_t b = 0; b < total; b += kWarp) {
-            const int32_t at = b + (int32_t)lane;
+        // 32 pairs (u,v) that differ, and rows a quarter of their tails at most: less
+        // than 1.4 E in all, which 32 bits hold
+        const uint32_t incl = warp_incl_scan(n);
+        const uint32_t total = __shfl_sync(kFull, incl, 31), S = incl - n;
+        for (uint32_t b = 0; b < total; b += kWarp) {
+            const uint32_t at = b + lane;
             int own = 0;  // last lane with S <= at
 #pragma unroll
             for (int step = 16; step > 0; step >>= 1)
