@@ -1969,7 +1969,7 @@ struct Layout {
     void* scan_sb;
     void* scan_off;
     void* sort_ws;
-    size_t zero_peel, zero_sort;
+    size_t zero_count, zero_peel, zero_sort;
     size_t total;
 };
 
@@ -1977,8 +1977,9 @@ Layout carve(void* ws, int64_t V, int64_t E) {
     Carver c{reinterpret_cast<char*>(ws)};
     Layout L;
     const size_t e = (size_t)(E > 0 ? E : 1), v = (size_t)(V > 0 ? V : 1);
-    // zeroed at the start of a run, in one go: up to zero_peel for every mode,
-    // up to zero_sort for a decomposition
+    // zeroed at the start of a run, in one go: up to zero_count without a list tail
+    // (three role counts an edge), to zero_peel with one (and the distribution's
+    // counters), to zero_sort for a decomposition
     L.ctl = (PeelCtl*)c.take(4096);
     L.sup_ctl = c.take(256);
     L.scan_cp = c.take(scan_scratch_bytes((int64_t)v));
@@ -1986,6 +1987,7 @@ Layout carve(void* ws, int64_t V, int64_t E) {
     L.scan_off = c.take(scan_scratch_bytes((int64_t)e));
     L.indeg = (int32_t*)c.take(4 * v);
     L.qi[0] = (int4*)c.take(16 * e);
+    L.zero_count = c.off - 4 * e;
     L.zero_peel = c.off;
     L.sort_ws = c.take(radix_scratch(nullptr, (int64_t)e, 4).bytes);
     L.zero_sort = c.off;
@@ -2036,7 +2038,13 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     int rc = device_info(&di);
     if (rc) return rc;
     Layout L = carve(ws, V, E);
-    TDT_CUDA(cudaMemsetAsync(ws, 0, E == 0 ? 4096 : mode == 0 ? L.zero_sort : L.zero_peel, st));
+    // The list tail: final lists grow from its start, the staging slots of the
+    // one walk end at its end.
+    const size_t list_base = (need + 255) & ~(size_t)255;
+    const unsigned long long tail =
+        mode != 2 && ws_bytes > list_base ? (unsigned long long)(ws_bytes - list_base) : 0ull;
+    const size_t zero = mode == 0 ? L.zero_sort : tail > 0 ? L.zero_peel : L.zero_count;
+    TDT_CUDA(cudaMemsetAsync(ws, 0, E == 0 ? 4096 : zero, st));
     if (E == 0) {
         TDT_CUDA(cudaMemsetAsync(stats, 0, sizeof(int64_t) * TDT_STAT_COUNT, st));
         if (mode == 0) {
@@ -2060,11 +2068,6 @@ int run_peel(int mode, const int32_t* rows, const int32_t* cols, const int64_t* 
     int32_t* cA = reinterpret_cast<int32_t*>(L.qi[0]);
     int32_t* cB = cA + E;
     int32_t* cC = cB + E;
-    // The list tail: final lists grow from its start, the staging slots of the
-    // one walk end at its end.
-    const size_t list_base = (need + 255) & ~(size_t)255;
-    const unsigned long long tail =
-        mode != 2 && ws_bytes > list_base ? (unsigned long long)(ws_bytes - list_base) : 0ull;
     int2* lists = reinterpret_cast<int2*>(reinterpret_cast<char*>(ws) + list_base);
     int2* stage_end = lists + tail / 8;
     prof_mark(0, st);
