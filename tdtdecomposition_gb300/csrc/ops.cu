@@ -211,11 +211,11 @@ __device__ __forceinline__ void walk_edges(const int32_t* __restrict__ rows, con
     const int64_t nw = (int64_t)gridDim.x * (kOpsBlock / kWarp);
     const int64_t g0 = blockIdx.x * (int64_t)(kOpsBlock / kWarp) + threadIdx.x / kWarp;
     // a group's entries, one a lane (true: of a row that is to be walked)
-    auto entry = [&](int64_t g, int64_t& e, int32_t& u, int32_t& bv, int32_t& lv, bool& me) {
+    auto entry = [&](int64_t g, int64_t& e, int32_t& u, int32_t& bu, int32_t& eu, int32_t& bv, int32_t& lv, bool& me) {
         const int64_t i = g * group + lane;
         e = -1;
         u = -1;
-        bv = lv = 0;
+        bu = eu = bv = lv = 0;
         me = false;
         if ((int)lane < group && i < n) {
             e = list(i);
@@ -223,6 +223,8 @@ __device__ __forceinline__ void walk_edges(const int32_t* __restrict__ rows, con
                 u = __ldg(rows + e);
                 const int32_t v = __ldg(cols + e);
                 if (rv.valid(u) && rv.valid(v)) {  // a sentinel edge has no triangles
+                    bu = (int32_t)rv.begin(u);
+                    eu = (int32_t)rv.end(u);
                     bv = (int32_t)rv.begin(v);
                     lv = (int32_t)(rv.end(v) - bv);
                     me = mark(e);
@@ -233,10 +235,9 @@ __device__ __forceinline__ void walk_edges(const int32_t* __restrict__ rows, con
     };
     // the lanes of todo with the source of the first of them, and the chunks of
     // their rows: all of them, or the first where they are too many
-    auto next_run = [&](unsigned todo, int32_t u, int32_t bv, int32_t lv, bool wide, int32_t& ur, int32_t& start,
+    auto next_run = [&](unsigned todo, int first, int32_t u, int32_t bv, int32_t lv, bool wide, int32_t& start,
                         unsigned& total) {
-        const int first = __ffs(todo) - 1;
-        ur = __shfl_sync(kFull, u, first);
+        const int32_t ur = __shfl_sync(kFull, u, first);
         const unsigned lo = (unsigned)bv + shift, hi = lo + (unsigned)lv;
         const int32_t chunks = (int32_t)(((hi + 3) >> 2) - (lo >> 2));
         unsigned run = wide ? 1u << first : __ballot_sync(kFull, u == ur) & todo;
@@ -257,18 +258,19 @@ __device__ __forceinline__ void walk_edges(const int32_t* __restrict__ rows, con
     bool longs = false;
     for (int64_t g = g0; g * group < n; g += nw) {
         int64_t e;
-        int32_t u, bv, lv;
+        int32_t u, u0, u1, bv, lv;
         bool me;
-        entry(g, e, u, bv, lv, me);
+        entry(g, e, u, u0, u1, bv, lv, me);
         const unsigned marked = __ballot_sync(kFull, me);
         const bool wide = __any_sync(kFull, lv >= (1 << 26));  // 32 of them might overflow a start
         unsigned todo = __ballot_sync(kFull, lv > 0);
         while (todo) {
-            int32_t ur, start;
+            int32_t start;
             unsigned total;
-            const unsigned run = next_run(todo, u, bv, lv, wide, ur, start, total);
+            const int first = __ffs(todo) - 1;
+            const unsigned run = next_run(todo, first, u, bv, lv, wide, start, total);
             todo &= ~run;
-            const int64_t bu = rv.begin(ur), eu = rv.end(ur);
+            const int64_t bu = __shfl_sync(kFull, u0, first), eu = __shfl_sync(kFull, u1, first);
             if (is_long(eu - bu, total)) {
                 longs = true;
                 continue;
@@ -383,18 +385,19 @@ __device__ __forceinline__ void walk_edges(const int32_t* __restrict__ rows, con
     if (!longs) return;
     for (int64_t g = g0; g * group < n; g += nw) {
         int64_t e;
-        int32_t u, bv, lv;
+        int32_t u, u0, u1, bv, lv;
         bool me;
-        entry(g, e, u, bv, lv, me);
+        entry(g, e, u, u0, u1, bv, lv, me);
         const unsigned marked = __ballot_sync(kFull, me);
         const bool wide = __any_sync(kFull, lv >= (1 << 26));
         unsigned todo = __ballot_sync(kFull, lv > 0);
         while (todo) {
-            int32_t ur, start;
+            int32_t start;
             unsigned total;
-            const unsigned run = next_run(todo, u, bv, lv, wide, ur, start, total);
+            const int first = __ffs(todo) - 1;
+            const unsigned run = next_run(todo, first, u, bv, lv, wide, start, total);
             todo &= ~run;
-            const int64_t bu = rv.begin(ur), eu = rv.end(ur);
+            const int64_t bu = __shfl_sync(kFull, u0, first), eu = __shfl_sync(kFull, u1, first);
             if (is_long(eu - bu, total)) walk_long_run(cols, S, run, bv, lv, marked, bu, eu, mark, hit, row);
             __syncwarp();
         }
