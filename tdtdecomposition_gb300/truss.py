@@ -75,6 +75,14 @@ def stage_bytes(cols, rp, rows=None):
     return 4 * int((d * (d - 1)).sum())
 
 
+def _stage_room(cols, rp, rows=None):
+    """stage_bytes and a little more: graphs of one size whose ties in degree fall
+    another way differ in the last few slots, and a workspace that grows leaves
+    its old memory behind."""
+    n = stage_bytes(cols, rp, rows)
+    return n + n // 64
+
+
 def _list_bytes(ws, cols, rp, lists, base, rows=None, count=False):
     """Bytes for the workspace's list tail, or 0 to let the peel search the
     adjacency instead: the per-edge triangle lists (24 bytes per triangle)
@@ -98,8 +106,7 @@ def _learn(ws, cols, rp, stats, tail):
         ws.triangles[key] = T = stats[STAT_TRIANGLES]
         S = ws.triangles.get(("stage",) + key)
         if stats[STAT_LISTED] == 1 and S is not None and 24 * T + 256 + S <= tail:
-            # this graph has more slots: room for them, and for the next one's
-            ws.triangles[("stage",) + key] = stage_bytes(cols, rp) * 17 // 16
+            ws.triangles[("stage",) + key] = _stage_room(cols, rp)  # this graph has more slots
 
 
 def _list_need(ws, cols, rp, lists, base, rows, count):
@@ -114,7 +121,7 @@ def _list_need(ws, cols, rp, lists, base, rows, count):
     sk = ("stage",) + key
     S = ws.triangles.get(sk)
     if S is None:
-        S = stage_bytes(cols, rp, rows)
+        S = _stage_room(cols, rp, rows)
         ws.triangles[sk] = S
     need = 24 * T + 256
     if S > STAGE_RATIO * (base + need):

@@ -34,7 +34,8 @@ def test_hint_is_of_the_size(monkeypatch):
     monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (1 << 40, 1 << 40))
     ws = T.Workspace("cpu")
     c, rp = _sparse()
-    S = T.stage_bytes(c, rp)
+    S = T._stage_room(c, rp)
+    assert T.stage_bytes(c, rp) <= S <= T.stage_bytes(c, rp) * 65 // 64
     assert T._list_bytes(ws, c, rp, True, 1 << 20) == 24 * 1000 + 256 + S and calls == [1]
     assert T._list_bytes(ws, c.clone(), rp.clone(), "auto", 1 << 20) == 24 * 1000 + 256 + S and calls == [1]
     # a run found more triangles, then one with more slots than were asked for
@@ -45,7 +46,7 @@ def test_hint_is_of_the_size(monkeypatch):
     stats[T.STAT_LISTED] = 1
     c2, rp2 = _clique()
     T._learn(ws, c2, rp2, stats, 24 * 5000 + 256 + S)
-    S2 = T.stage_bytes(c2, rp2) * 17 // 16
+    S2 = T._stage_room(c2, rp2)
     assert T._list_bytes(ws, c2, rp2, True, 1 << 20) == 24 * 5000 + 256 + S2 and calls == [1]
     # what the workspace has is offered; a capture counts
     ws.buf = torch.empty(1, dtype=torch.uint8).expand(1 << 30)

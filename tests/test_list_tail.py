@@ -39,7 +39,7 @@ def _ranked(n, d):
 def test_tail(monkeypatch, graph, tri, base, free, want):
     monkeypatch.setattr(T, "triangle_count_arrays", lambda *a: tri)
     monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (free, free))
-    S = T.stage_bytes(graph.columns, graph.row_ptr)
+    S = T._stage_room(graph.columns, graph.row_ptr)
     tails = {"none": 0, "lists": 24 * tri + 256, "staged": 24 * tri + 256 + S}
     for lists, kind in want.items():
         ws = T.Workspace("cpu")
