@@ -208,11 +208,11 @@ __global__ void pp_ranks(const uint64_t* __restrict__ vkeys, int64_t num_ids, in
     }
 }
 
-// relabel the unique edges
+// relabel the unique edges (last: the largest id)
 __global__ void __launch_bounds__(kPpBlock) pp_relabel(const uint64_t* __restrict__ ukeys,
                                                        const uint32_t* __restrict__ e_out, int B,
                                                        const int32_t* __restrict__ rank,
-                                                       uint64_t* __restrict__ keys2, uint64_t num_ids, int passes,
+                                                       uint64_t* __restrict__ keys2, uint32_t last, int passes,
                                                        uint32_t* hist) {
     __shared__ uint32_t s_hist[kMaxPasses * kRadix];
     DigitHist H{s_hist};
@@ -221,12 +221,8 @@ __global__ void __launch_bounds__(kPpBlock) pp_relabel(const uint64_t* __restric
     const int64_t eo = (int64_t)*e_out;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < eo; i += (int64_t)gridDim.x * blockDim.x) {
         const uint64_t k = ukeys[i];
-        const uint64_t lo = k >> B, hi = k & mask;
-        uint64_t k2 = 0;
-        if (lo < num_ids && hi < num_ids) {
-            const uint64_t a = (uint64_t)rank[lo], b = (uint64_t)rank[hi];
-            k2 = ((a < b ? a : b) << B) | (a < b ? b : a);
-        }
+        const uint64_t a = (uint64_t)rank[min((uint32_t)(k >> B), last)], b = (uint64_t)rank[min((uint32_t)(k & mask), last)];
+        const uint64_t k2 = ((a < b ? a : b) << B) | (a < b ? b : a);
         keys2[i] = k2;
         H.add(k2, passes);
     }
@@ -411,7 +407,7 @@ int run_preprocess(const int32_t* src, const int32_t* dst, int64_t m, int64_t nu
                                                               L.vcount);
     TDT_LAUNCH_CHECK("pp_ranks");
     // 4. relabel + orient, sort by (row, col); the sorted draw keys are no longer needed
-    pp_relabel<<<g_m, tb, 0, st>>>(uk, e_out, B, L.rank, sk, (uint64_t)num_ids, pe, L.s2.hist);
+    pp_relabel<<<g_m, tb, 0, st>>>(uk, e_out, B, L.rank, sk, (uint32_t)(num_ids - 1), pe, L.s2.hist);
     TDT_LAUNCH_CHECK("pp_relabel");
     rc = radix_sort<uint64_t, false>(sk, uk, sk, nullptr, nullptr, m, pe, L.s2, e_out, nullptr, L.status, st);
     if (rc) return rc;

@@ -18,7 +18,8 @@ namespace tdt {
 static long long g_look_back_limit_ns = 0;
 void set_look_back_limit(long long ns) { g_look_back_limit_ns = ns; }
 LookBack look_back(int* status) {
-    return {status, g_look_back_limit_ns > 0 ? (unsigned long long)g_look_back_limit_ns : kLookBackTimeoutNs};
+    if (g_look_back_limit_ns > 0) return {status, (unsigned long long)g_look_back_limit_ns, 0u};
+    return {status, kLookBackTimeoutNs, 63u};
 }
 
 constexpr int kScanBlock = 512;

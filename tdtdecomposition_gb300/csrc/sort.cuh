@@ -29,6 +29,7 @@ constexpr uint64_t kLookBackTimeoutNs = 2ull * 1000ull * 1000ull * 1000ull;
 struct LookBack {
     int* status;
     unsigned long long limit_ns;
+    unsigned clock_mask;         // the clock is read every clock_mask + 1 polls
 };
 LookBack look_back(int* status);  // with the limit in force (tdt_set_lookback_limit_ns)
 
@@ -46,7 +47,7 @@ __device__ __forceinline__ S tile_word_wait(const S* p, const LookBack& L) {
     for (unsigned spins = 1;; spins++) {
         w = *(const volatile S*)p;
         if (w) return w;
-        if ((spins & 7u) == 1u && globaltimer_ns() - t0 > L.limit_ns) {
+        if ((spins & L.clock_mask) == 0 && globaltimer_ns() - t0 > L.limit_ns) {
             atomicMax(L.status, (int)TDT_ERR_TIMEOUT);
             return TileWord<S>::kInclusive;
         }
